@@ -25,6 +25,8 @@
 // output).  The reference's conv2d order belongs to cuDNN, so dense output
 // agrees within rounding, as the reference's own dense/sparse test allows.
 
+#include <cstring>
+
 #include "th_common.cuh"
 #include "th_internal.h"
 
@@ -89,17 +91,24 @@ __device__ __forceinline__ int64_t reflect(int64_t y, int64_t n)
 }
 
 template <int DT>
-__device__ __forceinline__ bool differs(const void* p, int64_t a, int64_t b)
+__device__ __forceinline__ bool differ(typename Elem<DT>::T a, typename Elem<DT>::T b)
 {
-    using T = typename Elem<DT>::T;
     if constexpr (DT == TH_FLOAT16)
-        return __half2float(static_cast<const __half*>(p)[a]) != __half2float(static_cast<const __half*>(p)[b]);
+        return __half2float(a) != __half2float(b);
     else
-        return static_cast<const T*>(p)[a] != static_cast<const T*>(p)[b];
+        return a != b;
 }
 
-// edge_kernel (gaussian_blur_cuda.cu:116-142) folded into tile flags.
-template <int DT>
+// edge_kernel (gaussian_blur_cuda.cu:116-142) folded into tile flags.  A warp
+// owns 32 * V columns of a band of kEdgeRows rows, V elements (16 bytes where
+// the rows are 16-byte aligned, else one) per lane: it issues the band's loads
+// at once and compares from registers, so every row is read once plus one per
+// band, and index arithmetic is left to the few elements that are edges.
+// Bound by the read of the images (one element per thread with 64-bit
+// divisions took 146 us for 32x1024^2 float32, seven times that read).
+constexpr int kEdgeRows = 8;
+
+template <int DT, int V>
 __global__ void __launch_bounds__(256) edge_tiles_kernel(const void* __restrict__ img,
                                                          int64_t B,
                                                          int64_t H,
@@ -109,87 +118,139 @@ __global__ void __launch_bounds__(256) edge_tiles_kernel(const void* __restrict_
                                                          int64_t TW,
                                                          uint8_t* __restrict__ tiles)
 {
-    const int64_t n = B * H * W;
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
+    using T = typename Elem<DT>::T;
+    const T* src = static_cast<const T*>(img);
+    const int64_t chunks = (W + 32 * V - 1) / (32 * V), bands = (H + kEdgeRows - 1) / kEdgeRows;
+    const int64_t units = B * bands * chunks;
+    const int lane = threadIdx.x & 31;
+    const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+    for (int64_t u = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; u < units; u += nwarps)
     {
-        const int64_t x = i % W, y = i / W % H, b = i / (W * H);
-        const bool edge = (x + 1 < W && differs<DT>(img, i, i + 1)) || (y + 1 < H && differs<DT>(img, i, i + W));
-        if (edge)
+        const int64_t chunk = u % chunks, bb = u / chunks;
+        const int64_t band = bb % bands, b = bb / bands;
+        const int64_t x = (chunk * 32 + lane) * V, y0 = band * kEdgeRows;
+        if (x >= W)
+            continue; // with V > 1, W is a multiple of V
+        const T* p = src + (b * H + y0) * W + x;
+        const int rows = static_cast<int>(H - y0 < kEdgeRows + 1 ? H - y0 : kEdgeRows + 1); // with the row below
+        const bool right = x + V < W;
+        T v[kEdgeRows + 1][V], rn[kEdgeRows];
+#pragma unroll
+        for (int i = 0; i <= kEdgeRows; ++i)
         {
-            uint8_t* t = tiles + (b * TH + y / ts) * TW + x / ts;
-            if (*t == 0)
-                *t = 1;
+            // rows past the image repeat its last one: no difference there
+            const T* q = p + static_cast<int64_t>(i < rows ? i : rows - 1) * W;
+            if constexpr (V > 1)
+            {
+                const uint4 w = *reinterpret_cast<const uint4*>(q);
+                memcpy(v[i], &w, sizeof(w));
+            }
+            else
+                v[i][0] = *q;
+            if (i < kEdgeRows)
+                rn[i] = right ? q[V] : v[i][V - 1];
+        }
+#pragma unroll
+        for (int i = 0; i < kEdgeRows; ++i)
+        {
+            uint32_t m = 0;
+#pragma unroll
+            for (int e = 0; e < V; ++e)
+            {
+                // the comparison with itself at the right border is left out (a NaN differs from itself)
+                const bool h = e + 1 < V ? differ<DT>(v[i][e], v[i][e + 1 < V ? e + 1 : e])
+                                         : right && differ<DT>(v[i][e], rn[i]);
+                const bool w = i + 1 < rows && differ<DT>(v[i][e], v[i + 1][e]);
+                m |= (h || w ? 1u : 0u) << e;
+            }
+            if (m == 0 || i >= rows)
+                continue;
+            uint8_t* row = tiles + (b * TH + (y0 + i) / ts) * TW;
+            for (; m; m &= m - 1)
+            {
+                uint8_t* t = row + (x + __ffs(m) - 1) / ts;
+                if (*t == 0)
+                    *t = 1;
+            }
         }
     }
 }
 
-// Weight table (k*k, x offset major) and its sum, in the output type's arithmetic.
+// Weight table (k*k, x offset major) and its sum, in the output type's
+// arithmetic: block 0; the other blocks clear the tile flags (zero_bytes, a
+// multiple of 16).  The weights come from all threads; the sum keeps the
+// reference's order (tap by tap), so one thread adds them, from shared memory
+// for up to kSumTaps taps.  i*i + j*j is symmetric, so the x-major and the
+// y-major table are the same numbers.
+constexpr int kSumTaps = 4096;
+
 template <int OT>
-__global__ void weights_kernel(int k, float sigma, bool normalise, double* __restrict__ w, double* __restrict__ norm)
+__global__ void __launch_bounds__(256) weights_kernel(int k, float sigma, bool normalise, double* __restrict__ w, double* __restrict__ norm,
+                                                      uint4* __restrict__ zero, int64_t zero_bytes)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0)
+    if (blockIdx.x > 0)
+    {
+        const int64_t n = zero_bytes / 16, stride = static_cast<int64_t>(gridDim.x - 1) * blockDim.x;
+        for (int64_t i = static_cast<int64_t>(blockIdx.x - 1) * blockDim.x + threadIdx.x; i < n; i += stride)
+            zero[i] = make_uint4(0u, 0u, 0u, 0u);
         return;
-    const int r = k / 2;
-    const float den = __fmul_rn(__fmul_rn(2.f, sigma), sigma);
-    if (!normalise)
-    {
-        // tile_convolution_kernel (:268-283): kernel_val per tap, normalization += kernel_val
-        double s = 0.0;
-        float sh = 0.f, sf = 0.f;
-        for (int i = -r; i <= r; ++i)
-            for (int j = -r; j <= r; ++j)
-            {
-                const float e = expf(__fdiv_rn(-static_cast<float>(i * i + j * j), den));
-                double v;
-                if constexpr (OT == TH_FLOAT64)
-                {
-                    v = static_cast<double>(e);
-                    s = __dadd_rn(s, v);
-                }
-                else if constexpr (OT == TH_FLOAT32)
-                {
-                    v = static_cast<double>(e);
-                    sf = __fadd_rn(sf, e);
-                }
-                else
-                {
-                    const float eh = round_half(e);
-                    v = static_cast<double>(eh);
-                    sh = round_half(__fadd_rn(sh, eh));
-                }
-                w[(i + r) * k + (j + r)] = v;
-            }
-        *norm = (OT == TH_FLOAT64) ? s : (OT == TH_FLOAT32 ? static_cast<double>(sf) : static_cast<double>(sh));
     }
-    else
+    __shared__ float ev[kSumTaps];
+    __shared__ float total;
+    const int r = k / 2, taps = k * k;
+    const float den = __fmul_rn(__fmul_rn(2.f, sigma), sigma);
+    auto weight = [&](int t) {
+        const int i = t / k - r, j = t % k - r;
+        return expf(__fdiv_rn(-static_cast<float>(i * i + j * j), den));
+    };
+    // tile_convolution_kernel (:268-283) rounds each weight to the output type
+    // and sums in it; create_gaussian_kernel (:20-71) sums the rounded weights
+    // in float32 and divides by that sum.
+    for (int t = threadIdx.x; t < taps; t += blockDim.x)
     {
-        // create_gaussian_kernel (:20-71): kernel[y][x] in the output type,
-        // divided by its float32 sum.  Stored here x offset major like above.
-        float sum = 0.f;
-        for (int y = 0; y < k; ++y)
-            for (int x = 0; x < k; ++x)
-            {
-                const int dy = y - r, dx = x - r;
-                const float e = expf(__fdiv_rn(-static_cast<float>(dy * dy + dx * dx), den));
-                const float ev = (OT == TH_FLOAT16) ? round_half(e) : e;
-                sum = __fadd_rn(sum, ev);
-            }
-        for (int y = 0; y < k; ++y)
-            for (int x = 0; x < k; ++x)
-            {
-                const int dy = y - r, dx = x - r;
-                const float e = expf(__fdiv_rn(-static_cast<float>(dy * dy + dx * dx), den));
-                double v;
-                if constexpr (OT == TH_FLOAT64)
-                    v = __ddiv_rn(static_cast<double>(e), static_cast<double>(sum));
-                else if constexpr (OT == TH_FLOAT32)
-                    v = static_cast<double>(__fdiv_rn(e, sum));
-                else
-                    v = static_cast<double>(round_half(__fdiv_rn(round_half(e), sum)));
-                w[x * k + y] = v;
-            }
-        *norm = 1.0;
+        const float e = weight(t);
+        const float er = OT == TH_FLOAT16 ? round_half(e) : e;
+        if (t < kSumTaps)
+            ev[t] = er;
+        if (!normalise)
+            w[t] = static_cast<double>(er);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        double s = 0.0;
+        float sf = 0.f;
+#pragma unroll 8
+        for (int t = 0; t < taps; ++t)
+        {
+            float e;
+            if (t < kSumTaps)
+                e = ev[t];
+            else
+                e = OT == TH_FLOAT16 ? round_half(weight(t)) : weight(t);
+            if (!normalise && OT == TH_FLOAT64)
+                s = __dadd_rn(s, static_cast<double>(e));
+            else if (!normalise && OT == TH_FLOAT16)
+                sf = round_half(__fadd_rn(sf, e));
+            else
+                sf = __fadd_rn(sf, e);
+        }
+        *norm = normalise ? 1.0 : (OT == TH_FLOAT64 ? s : static_cast<double>(sf));
+        total = sf;
+    }
+    if (!normalise)
+        return;
+    __syncthreads();
+    const float sum = total;
+    for (int t = threadIdx.x; t < taps; t += blockDim.x)
+    {
+        const float e = weight(t);
+        if constexpr (OT == TH_FLOAT64)
+            w[t] = __ddiv_rn(static_cast<double>(e), static_cast<double>(sum));
+        else if constexpr (OT == TH_FLOAT32)
+            w[t] = static_cast<double>(__fdiv_rn(e, sum));
+        else
+            w[t] = static_cast<double>(round_half(__fdiv_rn(round_half(e), sum)));
     }
 }
 
@@ -307,6 +368,360 @@ __global__ void __launch_bounds__(256) blur_kernel(const void* __restrict__ img,
     }
 }
 
+// The device side of dispatch_image_dtype (a block-uniform branch).
+template <class F>
+__device__ __forceinline__ void dispatch_device(int dt, F&& f)
+{
+    switch (dt)
+    {
+    case TH_UINT8:
+        f.template operator()<TH_UINT8>();
+        break;
+    case TH_INT8:
+        f.template operator()<TH_INT8>();
+        break;
+    case TH_INT16:
+        f.template operator()<TH_INT16>();
+        break;
+    case TH_INT32:
+        f.template operator()<TH_INT32>();
+        break;
+    case TH_INT64:
+        f.template operator()<TH_INT64>();
+        break;
+    case TH_FLOAT16:
+        f.template operator()<TH_FLOAT16>();
+        break;
+    case TH_FLOAT32:
+        f.template operator()<TH_FLOAT32>();
+        break;
+    default:
+        f.template operator()<TH_FLOAT64>();
+        break;
+    }
+}
+
+// ---- blocks of 64 x 32 output pixels ---------------------------------------
+//
+// The block stages its pixels and a halo of k/2 in shared memory, converted
+// once to the type the taps are accumulated in (reflected at the image's
+// borders); a thread owns eight pixels of a column and keeps a sliding window
+// of that column in registers, so a shared load serves eight taps.  Per pixel
+// the taps run in the reference's order (x offset outer, y offset inner) with
+// its roundings, so sparse results are the same bits as one pixel per thread.
+// Sparse: a block without an active tile is a copy, whose loads are issued
+// before the tile flags are known.  Bound by the FMA issue (dense) and by the
+// read and write of the images (sparse).  The whole call on GB300: sparse
+// 32x1024^2 float32, k = 9, 1288 -> 195 us; dense 24x501x723 half, k = 13,
+// 3562 -> 179 us (one pixel per thread before, with a global load, two 64-bit
+// reflections and a double weight per tap).
+constexpr int kTileX = 64, kTileY = 32, kTileRows = 8;
+constexpr int kTileSmem = 96 * 1024;
+
+template <int OT, bool SPARSE>
+struct Accumulate
+{
+    using T = float;
+};
+template <bool SPARSE>
+struct Accumulate<TH_FLOAT64, SPARSE>
+{
+    using T = double;
+};
+template <>
+struct Accumulate<TH_FLOAT16, true>
+{
+    using T = __half; // every operation rounds to half
+};
+
+__device__ __forceinline__ float tap(float w, float v, float acc)
+{
+    return __fmaf_rn(w, v, acc);
+}
+__device__ __forceinline__ double tap(double w, double v, double acc)
+{
+    return __fma_rn(w, v, acc);
+}
+// c10::Half multiplies and adds in float and rounds each result to half; the
+// half instructions round the exact result once, which is the same number (a
+// product of halves is exact in float, and float's 24 bits are at least
+// 2 * 11 + 2, so rounding a sum twice changes nothing).
+__device__ __forceinline__ __half tap(__half w, __half v, __half acc)
+{
+    return __hadd_rn(acc, __hmul_rn(w, v));
+}
+
+// as_out with the accumulation's type.
+template <int DT, int OT, typename A>
+__device__ __forceinline__ A tile_value(const void* img, int64_t i)
+{
+    if constexpr (OT == TH_FLOAT64)
+        return load_f64<DT>(img, i);
+    else if constexpr (OT == TH_FLOAT32)
+        return load_f32<DT>(img, i);
+    else if constexpr (sizeof(A) == 2)
+        return __float2half_rn(load_f32<DT>(img, i));
+    else
+        return round_half(load_f32<DT>(img, i));
+}
+
+// Warp w loads the rows w, w + 8, ... of the tile and its halo.
+template <int DT, int OT, typename A>
+__device__ __forceinline__ void load_tile(const void* __restrict__ img, A* tile, const BlurGeom& g, int64_t base, int64_t y0, int64_t x0, int r)
+{
+    const int lane = threadIdx.x & 31;
+    const int sx = kTileX + 2 * r, sy = kTileY + 2 * r;
+    const bool inner = x0 >= r && y0 >= r && x0 + kTileX + r <= g.W && y0 + kTileY + r <= g.H;
+#pragma unroll 2
+    for (int ly = threadIdx.x >> 5; ly < sy; ly += 8)
+    {
+        const int64_t y = y0 - r + ly;
+        const int64_t row = base + (inner ? y : reflect(y, g.H)) * g.W;
+        for (int lx = lane; lx < sx; lx += 32)
+        {
+            int64_t x = x0 - r + lx;
+            if (!inner && (x < 0 || x >= g.W))
+                x = reflect(x, g.W);
+            tile[ly * sx + lx] = tile_value<DT, OT, A>(img, row + x);
+        }
+    }
+}
+
+template <int OT, bool SPARSE>
+__global__ void __launch_bounds__(256, 3) blur_tile_kernel(const void* __restrict__ img,
+                                                        int idt,
+                                                        void* __restrict__ out,
+                                                        BlurGeom g,
+                                                        const uint8_t* __restrict__ tiles,
+                                                        const double* __restrict__ wtab,
+                                                        const double* __restrict__ norm_ptr,
+                                                        int vec)
+{
+    using A = typename Accumulate<OT, SPARSE>::T;
+    using O = typename Elem<OT>::T;
+    extern __shared__ __align__(16) unsigned char blur_smem[];
+    const int tid = threadIdx.x, k = g.k, r = k / 2;
+    const int sx = kTileX + 2 * r, sy = kTileY + 2 * r;
+    A* w = reinterpret_cast<A*>(blur_smem);
+    A* tile = w + k * k;
+    uint8_t* act = reinterpret_cast<uint8_t*>(tile + sx * sy);
+
+    const int64_t bx = (g.W + kTileX - 1) / kTileX, by = (g.H + kTileY - 1) / kTileY;
+    // fewer than 2^31 blocks: bx and by fit 32 bits
+    const uint32_t nbx = static_cast<uint32_t>(bx), nby = static_cast<uint32_t>(by);
+    const uint32_t rest = blockIdx.x / nbx, ib = rest / nby;
+    const int64_t x0 = static_cast<int64_t>(blockIdx.x - rest * nbx) * kTileX, b = ib,
+                  y0 = static_cast<int64_t>(rest - ib * nby) * kTileY;
+    const int64_t base = b * g.H * g.W;
+    const int ts = static_cast<int>(g.ts);
+    int ntx = 0, nty = 0, ox = 0, oy = 0; // the block's tiles, and its first pixel inside the first tile
+    if constexpr (SPARSE)
+    {
+        // vec: same type in and out, rows 16-byte aligned
+        constexpr int kPer = 16 / static_cast<int>(sizeof(O)), kVecs = kTileX / kPer, kIter = kVecs * kTileY / 256;
+        uint4 c[kIter];
+        if (vec)
+        {
+#pragma unroll
+            for (int i = 0; i < kIter; ++i)
+            {
+                const int v = tid + i * 256;
+                const int64_t y = y0 + v / kVecs, x = x0 + (v % kVecs) * kPer;
+                if (y < g.H && x < g.W)
+                    c[i] = __ldg(reinterpret_cast<const uint4*>(static_cast<const O*>(img) + base + y * g.W + x));
+            }
+        }
+        // the tiles of the block's pixels, and those of one tile around them
+        const int64_t xl = x0 + kTileX < g.W ? x0 + kTileX - 1 : g.W - 1, yl = y0 + kTileY < g.H ? y0 + kTileY - 1 : g.H - 1;
+        const int64_t tx0 = x0 / ts, ty0 = y0 / ts;
+        ox = static_cast<int>(x0 - tx0 * ts);
+        oy = static_cast<int>(y0 - ty0 * ts);
+        ntx = static_cast<int>(xl / ts - tx0) + 1;
+        nty = static_cast<int>(yl / ts - ty0) + 1;
+        bool any = false;
+        for (int t = tid; t < (ntx + 2) * (nty + 2); t += 256)
+        {
+            const int64_t yy = ty0 - 1 + t / (ntx + 2), xx = tx0 - 1 + t % (ntx + 2);
+            if (yy >= 0 && yy < g.TH && xx >= 0 && xx < g.TW)
+                any |= tiles[(b * g.TH + yy) * g.TW + xx] != 0;
+        }
+        if (!__syncthreads_or(any))
+        {
+            if (vec)
+            {
+#pragma unroll
+                for (int i = 0; i < kIter; ++i)
+                {
+                    const int v = tid + i * 256;
+                    const int64_t y = y0 + v / kVecs, x = x0 + (v % kVecs) * kPer;
+                    if (y < g.H && x < g.W)
+                        *reinterpret_cast<uint4*>(static_cast<O*>(out) + base + y * g.W + x) = c[i];
+                }
+                return;
+            }
+            const int64_t x = x0 + (tid & 63);
+            auto copy = [&]<int DT>() {
+                double v[kTileRows];
+#pragma unroll
+                for (int j = 0; j < kTileRows; ++j)
+                {
+                    const int64_t y = y0 + (tid >> 6) + 4 * j;
+                    v[j] = x < g.W && y < g.H ? as_out<DT, OT>(img, base + y * g.W + x) : 0.0;
+                }
+#pragma unroll
+                for (int j = 0; j < kTileRows; ++j)
+                {
+                    const int64_t y = y0 + (tid >> 6) + 4 * j;
+                    if (x < g.W && y < g.H)
+                        store_out<OT>(out, base + y * g.W + x, v[j]);
+                }
+            };
+            dispatch_device(idt, copy);
+            return;
+        }
+        for (int t = tid; t < ntx * nty; t += 256)
+        {
+            const int64_t yy = ty0 + t / ntx, xx = tx0 + t % ntx;
+            bool on = false;
+            for (int64_t dy = -1; dy <= 1; ++dy)
+                for (int64_t dx = -1; dx <= 1; ++dx)
+                    if (yy + dy >= 0 && yy + dy < g.TH && xx + dx >= 0 && xx + dx < g.TW)
+                        on |= tiles[(b * g.TH + yy + dy) * g.TW + xx + dx] != 0;
+            act[t] = on ? 1 : 0;
+        }
+    }
+    for (int t = tid; t < k * k; t += 256)
+    {
+        if constexpr (sizeof(A) == 2)
+            w[t] = __float2half_rn(static_cast<float>(wtab[t]));
+        else
+            w[t] = static_cast<A>(wtab[t]);
+    }
+    dispatch_device(idt, [&]<int DT>() { load_tile<DT, OT, A>(img, tile, g, base, y0, x0, r); });
+    __syncthreads();
+
+    const int cx = tid & (kTileX - 1), cy = (tid / kTileX) * kTileRows; // first pixel of the thread's column
+    const int64_t x = x0 + cx;
+    uint32_t on = 0;
+    if constexpr (SPARSE)
+    {
+        if (x < g.W)
+        {
+            const int tx = (ox + cx) / ts;
+#pragma unroll
+            for (int j = 0; j < kTileRows; ++j)
+                if (y0 + cy + j < g.H && act[(oy + cy + j) / ts * ntx + tx])
+                    on |= 1u << j;
+        }
+    }
+    else
+        on = x < g.W ? 0xffu : 0u;
+    A acc[kTileRows];
+#pragma unroll
+    for (int j = 0; j < kTileRows; ++j)
+        acc[j] = A(0.f);
+    if (__any_sync(0xffffffffu, on != 0))
+    {
+        for (int dx = 0; dx < k; ++dx)
+        {
+            const A* col = tile + cy * sx + cx + dx;
+            const A* wd = w + dx * k;
+            A v[2 * kTileRows - 1];
+#pragma unroll
+            for (int j = 0; j < kTileRows - 1; ++j)
+                v[j] = col[j * sx];
+            col += (kTileRows - 1) * sx;
+            auto taps = [&]<int U>() {
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    v[kTileRows - 1 + u] = col[u * sx];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                {
+                    const A wt = wd[u];
+#pragma unroll
+                    for (int j = 0; j < kTileRows; ++j)
+                        acc[j] = tap(wt, v[j + u], acc[j]);
+                }
+#pragma unroll
+                for (int j = 0; j < kTileRows - 1; ++j)
+                    v[j] = v[j + U];
+                col += U * sx;
+                wd += U;
+            };
+            int left = k;
+            for (; left >= 8; left -= 8)
+                taps.template operator()<8>();
+            if (left & 4)
+                taps.template operator()<4>();
+            if (left & 2)
+                taps.template operator()<2>();
+            if (left & 1)
+                taps.template operator()<1>();
+        }
+    }
+    if (x >= g.W)
+        return;
+    const double norm = *norm_ptr;
+#pragma unroll
+    for (int j = 0; j < kTileRows; ++j)
+    {
+        const int64_t y = y0 + cy + j;
+        if (y >= g.H)
+            return;
+        const int64_t i = base + y * g.W + x;
+        if constexpr (sizeof(A) == 2)
+        {
+            const float res = __fdiv_rn(__half2float(acc[j]), static_cast<float>(norm));
+            static_cast<__half*>(out)[i] = (on >> j) & 1u ? __float2half_rn(res) : tile[(cy + j + r) * sx + cx + r];
+        }
+        else
+        {
+            A res = acc[j];
+            if constexpr (SPARSE)
+            {
+                if constexpr (OT == TH_FLOAT64)
+                    res = __ddiv_rn(res, norm);
+                else
+                    res = __fdiv_rn(res, static_cast<float>(norm));
+                if (!((on >> j) & 1u))
+                    res = tile[(cy + j + r) * sx + cx + r];
+            }
+            store_out<OT>(out, i, static_cast<double>(res));
+        }
+    }
+}
+
+// Shared memory of a block, 0 where the kernel is too wide for it (a block per
+// SM would be left, or none): those take blur_kernel.
+template <int OT, bool SPARSE>
+size_t tile_smem(int k, int64_t ts)
+{
+    const int64_t r = k / 2;
+    int64_t bytes = (int64_t{ k } * k + (kTileX + 2 * r) * (kTileY + 2 * r)) *
+                    static_cast<int64_t>(sizeof(typename Accumulate<OT, SPARSE>::T));
+    if (SPARSE)
+        bytes += (kTileX / ts + 2) * (kTileY / ts + 2);
+    return bytes <= kTileSmem ? static_cast<size_t>(bytes) : 0;
+}
+
+template <int OT, bool SPARSE>
+bool launch_tiles(const void* images, int idt, void* out, const BlurGeom& g, const uint8_t* tiles, const double* wtab, const double* norm, cudaStream_t s)
+{
+    const size_t smem = tile_smem<OT, SPARSE>(g.k, g.ts);
+    const int64_t blocks = ((g.W + kTileX - 1) / kTileX) * ((g.H + kTileY - 1) / kTileY) * g.B;
+    if (smem == 0 || blocks >= (int64_t{ 1 } << 31))
+        return false;
+    auto kernel = blur_tile_kernel<OT, SPARSE>;
+    if (smem > 48 * 1024)
+        TH_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem));
+    const int vec = idt == OT && (reinterpret_cast<uintptr_t>(images) | reinterpret_cast<uintptr_t>(out)) % 16 == 0 &&
+                    (g.W * static_cast<int64_t>(sizeof(typename Elem<OT>::T))) % 16 == 0;
+    kernel<<<static_cast<unsigned>(blocks), 256, smem, s>>>(images, idt, out, g, tiles, wtab, norm, vec);
+    TH_LAUNCH_CHECK();
+    return true;
+}
+
 template <int DT, int OT>
 __global__ void __launch_bounds__(256) convert_kernel(const void* __restrict__ img, void* __restrict__ out, int64_t n)
 {
@@ -381,16 +796,35 @@ void launch_gaussian_blur(const void* images,
     const int64_t woff = (tile_bytes + 15) / 16 * 16;
     double* wtab = reinterpret_cast<double*>(scratch + woff);
     double* norm = wtab + static_cast<int64_t>(kernel_size) * kernel_size;
-    dispatch_out(odt, [&]<int OT>() { weights_kernel<OT><<<1, 32, 0, s>>>(kernel_size, sigma, !sparse, wtab, norm); });
+    const int64_t zero_bytes = sparse ? woff : 0;
+    const unsigned zero_blocks = static_cast<unsigned>(grid_for((zero_bytes + 15) / 16, 256 * 4));
+    dispatch_out(odt, [&]<int OT>() {
+        weights_kernel<OT><<<1 + (sparse ? zero_blocks : 0u), 256, 0, s>>>(kernel_size, sigma, !sparse, wtab, norm,
+                                                                            reinterpret_cast<uint4*>(tiles), zero_bytes);
+    });
     TH_LAUNCH_CHECK();
     if (sparse)
     {
-        TH_CUDA(cudaMemsetAsync(tiles, 0, tile_bytes, s));
         dispatch_image_dtype(idt, [&]<int DT>() {
-            edge_tiles_kernel<DT><<<grid, 256, 0, s>>>(images, B, H, W, g.ts, g.TH, g.TW, tiles);
+            constexpr int V = 16 / static_cast<int>(sizeof(typename Elem<DT>::T));
+            const bool vec = reinterpret_cast<uintptr_t>(images) % 16 == 0 && W % V == 0;
+            const int64_t units = B * ((H + kEdgeRows - 1) / kEdgeRows) * ((W + 32 * (vec ? V : 1) - 1) / (32 * (vec ? V : 1)));
+            const int egrid = grid_for(units * 32, 256);
+            if (vec)
+                edge_tiles_kernel<DT, V><<<egrid, 256, 0, s>>>(images, B, H, W, g.ts, g.TH, g.TW, tiles);
+            else
+                edge_tiles_kernel<DT, 1><<<egrid, 256, 0, s>>>(images, B, H, W, g.ts, g.TH, g.TW, tiles);
         });
         TH_LAUNCH_CHECK();
     }
+    bool done = false;
+    dispatch_out(odt, [&]<int OT>() {
+        done = sparse ? launch_tiles<OT, true>(images, idt, out, g, tiles, wtab, norm, s)
+                      : launch_tiles<OT, false>(images, idt, out, g, tiles, wtab, norm, s);
+    });
+    if (done)
+        return;
+    // kernels too wide for a block's shared memory: one pixel per thread
     dispatch_image_dtype(idt, [&]<int DT>() {
         dispatch_out(odt, [&]<int OT>() {
             if (sparse)
