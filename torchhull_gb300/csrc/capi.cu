@@ -377,7 +377,7 @@ namespace
 // Pools and the last result of the public marching cubes.
 struct McSlot
 {
-    DevBuf groups, keys, slots, codes, used, vbase, tiles_soup, tiles_verts, tiles_scan, active, active_soup, ctr;
+    DevBuf bits, rank, edges, cnt, cells, chunk, keys, slots, codes, used, vbase, tiles_soup, tiles_verts, ctr;
     McCounters* host = nullptr; // pinned, mapped copy of the counters
     McCounters* host_d = nullptr; // its device address
     McPlan plan{};
@@ -386,8 +386,8 @@ struct McSlot
 
     std::vector<const DevBuf*> buffers() const
     {
-        return { &groups, &keys, &slots, &codes, &used, &vbase, &tiles_soup, &tiles_verts, &tiles_scan, &active,
-                 &active_soup, &ctr };
+        return { &bits, &rank, &edges, &cnt, &cells, &chunk, &keys, &slots, &codes, &used, &vbase, &tiles_soup,
+                 &tiles_verts, &ctr };
     }
 
     void release()
@@ -1264,21 +1264,56 @@ void run_mc(McSlot& s, const th_mc_args* a, cudaStream_t st)
         if (!a->volume)
             throw ArgError{ TH_ERR_INVALID_ARGUMENT, "volume pointer is NULL" };
         p.volume = a->volume;
-        p.points = D * H * W;
-        p.wide = p.points >= (int64_t{ 1 } << 32);
-        if (!p.wide)
-        {
-            p.div_w = make_fastdiv(static_cast<uint32_t>(W));
-            p.div_h = make_fastdiv(static_cast<uint32_t>(H));
-        }
-        p.ngroups = (p.points + 31) / 32;
+    }
+    // Rows of 32-point words.  A sparse volume takes them when they are at
+    // most kWordsPerEntry per entry (and always below kFewWords): clearing and
+    // counting a word costs about an eighth of what an entry's hash lookups
+    // do, and a word takes 40 bytes of scratch where an entry's table takes 60.
+    constexpr int64_t kWordsPerEntry = 8, kFewWords = int64_t{ 1 } << 18;
+    p.wr = 0;
+    if (W > 0 && H > 0 && D > 0)
+    {
+        const int64_t wr = (W + 31) / 32;
+        const bool fits = H < (int64_t{ 1 } << 32) / wr && D < (int64_t{ 1 } << 32) / (wr * H); // word indices below 2^32
+        p.nwords = fits ? wr * H * D : 0;
+        // fewer than 2^28 entries: packed counts, like the active cells of a dense volume below
+        p.words = fits && (!p.sparse || (p.nnz < (int64_t{ 1 } << 28) &&
+                                         (p.nwords <= kFewWords || p.nwords / kWordsPerEntry <= p.nnz)));
+        if (!p.sparse && !fits)
+            throw ArgError{ TH_ERR_OUT_OF_MEMORY, "marching cubes: the volume has too many rows of 32 points" };
+    }
+    if (p.words)
+    {
+        p.wr = static_cast<uint32_t>((W + 31) / 32);
+        p.div_wr = make_fastdiv(p.wr);
+        p.div_h = make_fastdiv(static_cast<uint32_t>(H));
     }
 
     if (!s.host)
         alloc_mapped(&s.host, &s.host_d);
     s.ctr.ensure(sizeof(McCounters));
     p.ctr = s.ctr.as<McCounters>();
-    if (p.sparse)
+    if (p.words && !(p.sparse && p.nnz == 0))
+    {
+        const size_t n = static_cast<size_t>(p.nwords);
+        s.bits.ensure(sizeof(uint32_t) * n * (p.sparse ? 2 : 1));
+        p.sign = s.bits.as<uint32_t>() + (p.sparse ? n : 0);
+        if (p.sparse)
+        {
+            s.rank.ensure(sizeof(uint32_t) * n);
+            p.present = s.bits.as<uint32_t>();
+            p.rank = s.rank.as<uint32_t>();
+        }
+        s.cnt.ensure(sizeof(uint32_t) * n);
+        s.cells.ensure(sizeof(uint32_t) * n);
+        s.chunk.ensure(sizeof(uint2) * ((n + 31) / 32));
+        s.tiles_soup.ensure(sizeof(unsigned long long) * word_tiles(p.nwords));
+        if (p.unique)
+            s.edges.ensure(sizeof(uint4) * n);
+        p.mesh = WordMesh{ s.cnt.as<uint32_t>(), s.cells.as<uint32_t>(), s.edges.as<uint4>(), s.chunk.as<uint2>(),
+                           s.tiles_soup.as<unsigned long long>() };
+    }
+    else if (p.sparse)
     {
         const int64_t n = p.nnz;
         uint64_t cap = 64;
@@ -1303,22 +1338,6 @@ void run_mc(McSlot& s, const th_mc_args* a, cudaStream_t st)
             p.tiles_verts = s.tiles_verts.as<unsigned long long>();
         }
     }
-    else
-    {
-        s.tiles_soup.ensure(sizeof(unsigned long long) * mc_scan_tiles(p.points));
-        s.codes.ensure(static_cast<size_t>(p.points));
-        s.tiles_scan.ensure(sizeof(unsigned long long) * mc_scan_tiles(mc_scan_tiles(p.points)));
-        p.tiles_soup = s.tiles_soup.as<unsigned long long>();
-        p.tiles_scan = s.tiles_scan.as<unsigned long long>();
-        p.codes = s.codes.as<uint8_t>();
-        if (p.unique)
-        {
-            s.groups.ensure(sizeof(McGroup) * p.ngroups);
-            s.tiles_verts.ensure(sizeof(unsigned long long) * mc_scan_tiles(p.ngroups));
-            p.groups = s.groups.as<McGroup>();
-            p.tiles_verts = s.tiles_verts.as<unsigned long long>();
-        }
-    }
 
     launch_mc_count(p, st);
     small_copy(s.host_d, p.ctr, sizeof(McCounters), st);
@@ -1329,17 +1348,9 @@ void run_mc(McSlot& s, const th_mc_args* a, cudaStream_t st)
     if (c.flags & kMcUnsorted)
         throw ArgError{ TH_ERR_INVALID_ARGUMENT,
                         "sparse volume indices must be coalesced (strictly ascending in (z, y, x))" };
-    if (!p.sparse)
-    {
-        // packed (soup << 32 | active) tile sums: both totals below 2^32
-        if (c.active >= (1ull << 28))
-            throw ArgError{ TH_ERR_INVALID_ARGUMENT, "marching cubes: more than 2^28 active cells" };
-        p.nactive = static_cast<int64_t>(c.active);
-        s.active.ensure(sizeof(int64_t) * std::max<int64_t>(p.nactive, 1));
-        s.active_soup.ensure(sizeof(unsigned long long) * std::max<int64_t>(p.nactive, 1));
-        p.active = s.active.as<int64_t>();
-        p.active_soup = s.active_soup.as<unsigned long long>();
-    }
+    // the counts are summed packed (corners << 32 | vertices): both below 2^32
+    if (!p.sparse && c.active >= (1ull << 28))
+        throw ArgError{ TH_ERR_INVALID_ARGUMENT, "marching cubes: more than 2^28 active cells" };
     s.plan = p;
     s.info.num_faces = static_cast<int64_t>(c.soup / 3);
     s.info.num_verts = static_cast<int64_t>(p.unique ? c.verts : c.soup);

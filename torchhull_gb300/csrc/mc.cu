@@ -9,18 +9,18 @@
 // faces are the soup's inverse indices.  The unique vertices therefore come
 // in edge-id order: by the ravel index of the lower end point, then by axis.
 // Here that order is produced directly: every grid point carries three bits
-// (its +x, +y, +z edge holds a vertex), a scan over the points numbers the
-// set bits, and a face looks up its vertex as the number of set bits before
-// its edge.  The soup order comes from a scan of the per-cell vertex counts,
-// so no sort runs.
+// (its +x, +y, +z edge holds a vertex), prefix sums number the set bits, and a
+// face looks up its vertex as the number of set bits before its edge; no sort
+// runs.  Dense volumes, and sparse ones that are not too empty, do this on
+// words of 32 points (th_words.cuh); a very sparse volume keeps its entries in
+// a hash table.
 //
 // Which edges hold vertices: every cell's triangulation uses exactly the cell
 // edges whose end points lie on different sides of the isolevel (a property
 // of the table, checked by the tests).  In a dense volume with all sizes >= 2
 // every edge belongs to some cell, so the bits follow from the values alone.
 // In a sparse volume an edge counts only when a complete cell (all 8 corners
-// present) holds it, so each active cell marks its edges on the entries of
-// their lower end points.
+// present) holds it.
 //
 // Axes: x runs along the last volume dimension (W), y along H, z along the
 // first (D).  The reference mixes D and W in its index arithmetic; for
@@ -86,43 +86,14 @@ __device__ __forceinline__ void mc_vertex(const McPlan& p, int64_t x, int64_t y,
 // ---------------------------------------------------------------------------
 // dense volumes
 
-template <bool WIDE>
-__device__ __forceinline__ void decode(const McPlan& p, int64_t q, int64_t& x, int64_t& y, int64_t& z)
+// Triangle corners << 32 | vertices of the whole mesh.
+struct WordTotal
 {
-    if (WIDE)
+    McCounters* ctr;
+    __device__ void operator()(unsigned long long t) const
     {
-        const int64_t r = q / p.W;
-        x = q - r * p.W;
-        z = r / p.H;
-        y = r - z * p.H;
-    }
-    else
-    {
-        const uint32_t qq = static_cast<uint32_t>(q);
-        const uint32_t r = fast_div(p.div_w, qq);
-        x = qq - r * p.div_w.d;
-        const uint32_t zz = fast_div(p.div_h, r);
-        z = zz;
-        y = r - zz * p.div_h.d;
-    }
-}
-
-struct GroupCount
-{
-    const McGroup* groups;
-    __device__ unsigned long long operator()(int64_t i) const
-    {
-        const McGroup& e = groups[i];
-        return static_cast<unsigned long long>(__popc(e.x) + __popc(e.y) + __popc(e.z));
-    }
-};
-
-struct GroupEmit
-{
-    McGroup* groups;
-    __device__ void operator()(int64_t i, unsigned long long off, unsigned long long) const
-    {
-        groups[i].base = off;
+        ctr->soup = t >> 32;
+        ctr->verts = t & 0xffffffffull;
     }
 };
 
@@ -135,17 +106,6 @@ struct SoupTotal
     }
 };
 
-// (soup << 32) | active cells of a dense volume
-struct PackedTotal
-{
-    McCounters* ctr;
-    __device__ void operator()(unsigned long long t) const
-    {
-        ctr->soup = t >> 32;
-        ctr->active = t & 0xffffffffull;
-    }
-};
-
 struct VertTotal
 {
     McCounters* ctr;
@@ -155,301 +115,119 @@ struct VertTotal
     }
 };
 
-// Vertex index of the edge from point q along axis: the set edge bits before it.
-__device__ __forceinline__ unsigned long long dense_vertex(const McGroup* groups, int64_t q, int axis)
+// Rows of a volume in words: word k is in row k / wr (y + H * z).
+struct VolumeWords
 {
-    const McGroup e = groups[q >> 5];
-    const int l = static_cast<int>(q & 31);
-    const uint32_t lt = (1u << l) - 1u;
-    unsigned long long r = e.base + __popc(e.x & lt) + __popc(e.y & lt) + __popc(e.z & lt);
-    if (axis >= 1)
-        r += (e.x >> l) & 1u;
-    if (axis == 2)
-        r += (e.y >> l) & 1u;
-    return r;
-}
+    McPlan p;
 
-// Soup of the active cell with base point q and code (generate_faces_dense
-// :242-306): faces into the unique vertex list, or soup vertices with
-// faces = arange.  off: the cell's first soup vertex.
-template <int DT, bool WIDE>
-__device__ __forceinline__ void dense_emit_cell(const McPlan& p, int64_t q, int code, unsigned long long off, int cnt, float* verts, int64_t* faces)
-{
-    int64_t x, y, z;
-    decode<WIDE>(p, q, x, y, z);
-    const int64_t WH = p.W * p.H;
-    for (int j = 0; j < cnt; ++j)
+    __device__ int64_t words() const
     {
-        const uint32_t e = mc_edges[code][j];
-        const int lo = static_cast<int>(e & 7u), axis = static_cast<int>(e >> 3);
-        const int64_t q1 = q + (lo & 1) + ((lo >> 1) & 1) * p.W + ((lo >> 2) & 1) * WH;
-        const int64_t k = static_cast<int64_t>(off) + j;
-        if (p.unique)
-        {
-            faces[k] = static_cast<int64_t>(dense_vertex(p.groups, q1, axis));
-        }
-        else
-        {
-            const int64_t q2 = q1 + (axis == 0 ? 1 : (axis == 1 ? p.W : WH));
-            mc_vertex(p, x + (lo & 1), y + ((lo >> 1) & 1), z + ((lo >> 2) & 1), axis, load_f32<DT>(p.volume, q1),
-                      load_f32<DT>(p.volume, q2), verts + 3 * k);
-            faces[k] = k;
-        }
+        return p.nwords;
     }
-}
-
-// One pass over a dense volume that loads each value once: a block covers
-// 32 x 8 columns (x, y) and marches kMarchZ planes in z, exchanging the
-// below-isolevel bits of each plane (with a one-point halo in +x and +y)
-// through shared memory, double-buffered.  For every point it writes the cell
-// code (0 where no cell starts), ORs its three vertex-edge bits into the
-// group words (unique vertices), and adds (soup vertices << 32 | active cell)
-// to the sum of its 2048-point tile (one atomic per warp and tile).  groups
-// and tiles_soup are zero when it starts.
-constexpr int kMarchX = 32, kMarchY = 8, kMarchZ = 16;
-
-template <int DT>
-__device__ __forceinline__ uint8_t below_at(const McPlan& p, int64_t x, int64_t y, int64_t z)
-{
-    return (x < p.W && y < p.H && z < p.D) ? (below<DT>(p.volume, x + p.W * (y + p.H * z), p.iso) ? 1 : 0) : 0;
-}
-
-template <int DT>
-__global__ void __launch_bounds__(kMarchX * kMarchY) mc_dense_march_kernel(McPlan p)
-{
-    __shared__ uint8_t plane[2][kMarchY + 1][kMarchX + 1];
-    const int tx = threadIdx.x, ty = threadIdx.y, lane = tx;
-    const int64_t x = static_cast<int64_t>(blockIdx.x) * kMarchX + tx;
-    const int64_t y = static_cast<int64_t>(blockIdx.y) * kMarchY + ty;
-    const int64_t z0 = static_cast<int64_t>(blockIdx.z) * kMarchZ;
-    const int64_t z1 = z0 + kMarchZ < p.D ? z0 + kMarchZ : p.D;
-    const bool in = x < p.W && y < p.H;
-
-    // plane z into buffer k: own bit, and the +x / +y halo
-    auto fill = [&](int k, int64_t z) {
-        plane[k][ty][tx] = below_at<DT>(p, x, y, z);
-        if (tx == kMarchX - 1)
-            plane[k][ty][kMarchX] = below_at<DT>(p, x + 1, y, z);
-        if (ty == kMarchY - 1)
-        {
-            plane[k][kMarchY][tx] = below_at<DT>(p, x, y + 1, z);
-            if (tx == kMarchX - 1)
-                plane[k][kMarchY][kMarchX] = below_at<DT>(p, x + 1, y + 1, z);
-        }
-    };
-    fill(0, z0);
-    __syncthreads();
-    int cur = 0;
-    for (int64_t z = z0; z < z1; ++z)
+    __device__ uint32_t sign(uint32_t k) const
     {
-        const int nxt = cur ^ 1;
-        if (z + 1 < p.D)
-            fill(nxt, z + 1);
-        else
-        {
-            plane[nxt][ty][tx] = 0;
-            if (tx == kMarchX - 1)
-                plane[nxt][ty][kMarchX] = 0;
-            if (ty == kMarchY - 1)
-            {
-                plane[nxt][kMarchY][tx] = 0;
-                if (tx == kMarchX - 1)
-                    plane[nxt][kMarchY][kMarchX] = 0;
-            }
-        }
-        __syncthreads();
-        const uint32_t b0 = plane[cur][ty][tx], bx = plane[cur][ty][tx + 1];
-        const uint32_t by = plane[cur][ty + 1][tx], bxy = plane[cur][ty + 1][tx + 1];
-        const uint32_t c0 = plane[nxt][ty][tx], cx = plane[nxt][ty][tx + 1];
-        const uint32_t cy = plane[nxt][ty + 1][tx], cxy = plane[nxt][ty + 1][tx + 1];
-        const int64_t q = x + p.W * (y + p.H * z);
-        // corner i = (i & 1, i >> 1 & 1, i >> 2 & 1)
-        const int code = static_cast<int>(b0 | (bx << 1) | (by << 2) | (bxy << 3) | (c0 << 4) | (cx << 5) | (cy << 6) |
-                                          (cxy << 7));
-        const bool cell = in && x + 1 < p.W && y + 1 < p.H && z + 1 < p.D;
-        const unsigned cnt = cell ? mc_count[code] : 0u;
-        if (in)
-            p.codes[q] = static_cast<uint8_t>(cell ? code : 0);
-        // the warp's 32 points are consecutive in ravel order (or end at the row's end)
-        const int64_t q0 = __shfl_sync(0xffffffffu, q, 0);
-        // per warp: soup vertices (<= 480) << 16 | active cells (<= 32), for
-        // the (at most two) 2048-point tiles the warp's points fall into
-        const unsigned packed = (cnt << 16) | (cnt ? 1u : 0u);
-        const int64_t t0 = q0 >> 11;
-        const bool second = in && (q >> 11) != t0;
-        const unsigned a0 = __reduce_add_sync(0xffffffffu, second ? 0u : packed);
-        const unsigned a1 = __reduce_add_sync(0xffffffffu, second ? packed : 0u);
-        if (lane == 0)
-        {
-            if (a0)
-                atomicAdd(&p.tiles_soup[t0], (static_cast<unsigned long long>(a0 >> 16) << 32) | (a0 & 0xffffu));
-            if (a1)
-                atomicAdd(&p.tiles_soup[t0 + 1], (static_cast<unsigned long long>(a1 >> 16) << 32) | (a1 & 0xffffu));
-        }
-        if (p.unique)
-        {
-            const bool ex = in && x + 1 < p.W && bx != b0;
-            const bool ey = in && y + 1 < p.H && by != b0;
-            const bool ez = in && z + 1 < p.D && c0 != b0;
-            const uint32_t X = __ballot_sync(0xffffffffu, ex), Y = __ballot_sync(0xffffffffu, ey),
-                           Z = __ballot_sync(0xffffffffu, ez);
-            if (lane == 0)
-            {
-                const int64_t g0 = q0 >> 5;
-                const int sh = static_cast<int>(q0 & 31);
-                McGroup& G0 = p.groups[g0];
-                if (X << sh)
-                    atomicOr(&G0.x, X << sh);
-                if (Y << sh)
-                    atomicOr(&G0.y, Y << sh);
-                if (Z << sh)
-                    atomicOr(&G0.z, Z << sh);
-                if (sh)
-                {
-                    McGroup& G1 = p.groups[g0 + 1];
-                    if (X >> (32 - sh))
-                        atomicOr(&G1.x, X >> (32 - sh));
-                    if (Y >> (32 - sh))
-                        atomicOr(&G1.y, Y >> (32 - sh));
-                    if (Z >> (32 - sh))
-                        atomicOr(&G1.z, Z >> (32 - sh));
-                }
-            }
-        }
-        cur = nxt;
-        __syncthreads(); // plane[cur ^ 1] is refilled next
+        return p.sign[k];
     }
-}
-
-// The tile sums of the march into exclusive offsets, in place (a scan reads
-// all counts of a thread before it writes any offset).
-struct TileCount
-{
-    const unsigned long long* tiles;
-    __device__ unsigned long long operator()(int64_t i) const
+    __device__ WordRows rows(uint32_t k) const
     {
-        return tiles[i];
+        WordRows r;
+        const uint32_t row = fast_div(p.div_wr, k), w = k - row * p.wr;
+        r.z = fast_div(p.div_h, row);
+        r.y = row - r.z * p.div_h.d;
+        r.x0 = static_cast<int64_t>(w) * 32;
+        r.next = w + 1 < p.wr;
+        const bool up = r.y + 1 < p.div_h.d, back = static_cast<int64_t>(r.z) + 1 < p.D;
+        const uint32_t plane = p.wr * p.div_h.d;
+        r.idx[0] = k;
+        r.idx[1] = up ? k + p.wr : kNoWord;
+        r.idx[2] = back ? k + plane : kNoWord;
+        r.idx[3] = up && back ? k + p.wr + plane : kNoWord;
+        return r;
     }
 };
 
-struct TileEmit
+template <int DT>
+struct DenseWords : VolumeWords
 {
-    unsigned long long* tiles;
-    __device__ void operator()(int64_t i, unsigned long long off, unsigned long long) const
+    // every edge inside the volume belongs to some cell
+    __device__ EdgeBits edges(uint32_t, const WordRows& r, const uint32_t s[4], const uint32_t sh[4], uint32_t& cells) const
     {
-        tiles[i] = off;
+        const int64_t points = p.W - r.x0; // at least 1
+        const uint32_t in = points >= 32 ? 0xffffffffu : (1u << points) - 1u;
+        const uint32_t start = points > 32 ? 0xffffffffu : (1u << (points - 1)) - 1u; // with a right neighbour
+        cells = r.idx[3] != kNoWord ? start : 0u;
+        return EdgeBits{ (s[0] ^ sh[0]) & start, r.idx[1] != kNoWord ? (s[0] ^ s[1]) & in : 0u,
+                         r.idx[2] != kNoWord ? (s[0] ^ s[2]) & in : 0u };
+    }
+    __device__ int64_t point(uint32_t k, int b, int64_t& x, int64_t& y, int64_t& z) const
+    {
+        const uint32_t row = fast_div(p.div_wr, k), zz = fast_div(p.div_h, row);
+        x = static_cast<int64_t>(k - row * p.wr) * 32 + b;
+        y = row - zz * p.div_h.d;
+        z = zz;
+        return static_cast<int64_t>(row) * p.W + x;
+    }
+    __device__ void vertex(uint32_t k, int b, int axis, float out[3]) const
+    {
+        int64_t x, y, z;
+        const int64_t q = point(k, b, x, y, z);
+        const int64_t q2 = q + (axis == 0 ? 1 : (axis == 1 ? p.W : p.W * p.H));
+        mc_vertex(p, x, y, z, axis, load_f32<DT>(p.volume, q), load_f32<DT>(p.volume, q2), out);
+    }
+    __device__ void values_at(const WordRows& r, int b, unsigned long long* corner) const
+    {
+        const int64_t q = (r.y + static_cast<int64_t>(r.z) * p.H) * p.W + r.x0 + b;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            corner[i] = static_cast<unsigned long long>(q + (i & 1) + (i >> 1 & 1) * p.W + (i >> 2) * (p.W * p.H));
+    }
+    __device__ void soup_vertex(uint32_t k, int b, int lo, int axis, unsigned long long h1, unsigned long long h2, float out[3]) const
+    {
+        int64_t x, y, z;
+        point(k, b, x, y, z);
+        mc_vertex(p, x + (lo & 1), y + (lo >> 1 & 1), z + (lo >> 2 & 1), axis,
+                  load_f32<DT>(p.volume, static_cast<int64_t>(h1)), load_f32<DT>(p.volume, static_cast<int64_t>(h2)), out);
     }
 };
 
-// Pass 2, over the same tiles with kScanItems consecutive points per thread
-// (one 8-byte read of codes, one block scan per tile): every active cell and
-// its first soup vertex into the active list, in cell order.
-__global__ void __launch_bounds__(kScanThreads) mc_dense_compact_kernel(McPlan p)
-{
-    static_assert(kScanItems == 8, "one 8-byte read of codes per thread");
-    const int64_t ntiles = (p.points + kScanTile - 1) / kScanTile;
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-    {
-        // tiles without an active cell (most of a volume) have equal offsets
-        const unsigned long long next =
-                tile + 1 < ntiles ? p.tiles_soup[tile + 1] : ((p.ctr->soup << 32) | p.ctr->active);
-        if ((next & 0xffffffffull) == (p.tiles_soup[tile] & 0xffffffffull))
-            continue;
-        const int64_t base = tile * kScanTile + static_cast<int64_t>(threadIdx.x) * kScanItems;
-        uint32_t lo = 0, hi = 0;
-        if (base + kScanItems <= p.points)
-        {
-            const uint2 w = *reinterpret_cast<const uint2*>(p.codes + base);
-            lo = w.x;
-            hi = w.y;
-        }
-        else
-        {
-            for (int k = 0; k < kScanItems && base + k < p.points; ++k)
-                (k < 4 ? lo : hi) |= static_cast<uint32_t>(p.codes[base + k]) << (8 * (k & 3));
-        }
-        unsigned long long s = 0;
-#pragma unroll
-        for (int k = 0; k < kScanItems; ++k)
-        {
-            const unsigned cnt = mc_count[((k < 4 ? lo : hi) >> (8 * (k & 3))) & 0xffu];
-            s += (static_cast<unsigned long long>(cnt) << 32) | (cnt ? 1ull : 0ull);
-        }
-        unsigned long long tot;
-        unsigned long long off = block_exclusive_scan(s, &tot) + p.tiles_soup[tile];
-        if (s == 0)
-            continue;
-#pragma unroll
-        for (int k = 0; k < kScanItems; ++k)
-        {
-            const unsigned cnt = mc_count[((k < 4 ? lo : hi) >> (8 * (k & 3))) & 0xffu];
-            if (cnt)
-            {
-                const unsigned long long a = off & 0xffffffffull;
-                p.active[a] = base + k;
-                p.active_soup[a] = off >> 32;
-                off += (static_cast<unsigned long long>(cnt) << 32) | 1ull;
-            }
-        }
-    }
-}
+// Sign words of a dense volume: the only pass over its values.  A warp takes
+// kSignWords consecutive words at a time, a point per lane, all loads issued
+// before the first ballot.
+constexpr int kSignWords = 8;
 
-// The soup of every active cell, one thread per cell.
-template <int DT, bool WIDE>
-__global__ void __launch_bounds__(256) mc_dense_faces_kernel(McPlan p, float* __restrict__ verts, int64_t* __restrict__ faces)
-{
-    const int64_t n = static_cast<int64_t>(p.ctr->active);
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
-    {
-        const int64_t q = p.active[i];
-        const int code = p.codes[q];
-        dense_emit_cell<DT, WIDE>(p, q, code, p.active_soup[i], mc_count[code], verts, faces);
-    }
-}
-
-// The unique vertices, in edge-id order.  Each lane of a warp reads one
-// group; the warp then handles its groups with vertex edges one after the
-// other, a lane per point (most groups of a volume have none).
-template <int DT, bool WIDE>
-__global__ void __launch_bounds__(256) mc_dense_verts_kernel(McPlan p, float* __restrict__ verts)
+template <int DT>
+__global__ void __launch_bounds__(256) mc_sign_kernel(McPlan p)
 {
     const int lane = threadIdx.x & 31;
-    const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-    const int64_t WH = p.W * p.H;
-    const uint32_t bit = 1u << lane, lt = bit - 1u;
-    for (int64_t g0 = warp * 32; g0 < p.ngroups; g0 += nwarps * 32)
+    const int64_t groups = (p.nwords + kSignWords - 1) / kSignWords;
+    using T = typename Elem<DT>::T;
+    const T* volume = static_cast<const T*>(p.volume);
+    for (int64_t g = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; g < groups; g += nwarps)
     {
-        const int64_t gl = g0 + lane;
-        const McGroup mine_group = gl < p.ngroups ? p.groups[gl] : McGroup{ 0u, 0u, 0u, 0u, 0ull };
-        uint32_t todo = __ballot_sync(0xffffffffu, (mine_group.x | mine_group.y | mine_group.z) != 0u);
-        while (todo)
-        {
-            const int j = __ffs(todo) - 1;
-            todo &= todo - 1;
-            const uint32_t ex = __shfl_sync(0xffffffffu, mine_group.x, j);
-            const uint32_t ey = __shfl_sync(0xffffffffu, mine_group.y, j);
-            const uint32_t ez = __shfl_sync(0xffffffffu, mine_group.z, j);
-            const unsigned long long base = __shfl_sync(0xffffffffu, mine_group.base, j);
-            const uint32_t mine = ((ex & bit) ? 1u : 0u) | ((ey & bit) ? 2u : 0u) | ((ez & bit) ? 4u : 0u);
-            if (!mine)
-                continue;
-            unsigned long long r = base + __popc(ex & lt) + __popc(ey & lt) + __popc(ez & lt);
-            const int64_t q = (g0 + j) * 32 + lane;
-            int64_t x, y, z;
-            decode<WIDE>(p, q, x, y, z);
-            const float v1 = load_f32<DT>(p.volume, q);
+        T v[kSignWords];
+        uint32_t in = 0;
 #pragma unroll
-            for (int a = 0; a < 3; ++a)
-            {
-                if (!((mine >> a) & 1u))
-                    continue;
-                const int64_t q2 = q + (a == 0 ? 1 : (a == 1 ? p.W : WH));
-                mc_vertex(p, x, y, z, a, v1, load_f32<DT>(p.volume, q2), verts + 3 * r);
-                ++r;
-            }
+        for (int i = 0; i < kSignWords; ++i)
+        {
+            const int64_t kk = g * kSignWords + i;
+            const uint32_t k = static_cast<uint32_t>(kk < p.nwords ? kk : p.nwords - 1);
+            const uint32_t row = fast_div(p.div_wr, k);
+            const int64_t x = static_cast<int64_t>(k - row * p.wr) * 32 + lane;
+            const bool ok = x < p.W;
+            in |= ok ? 1u << i : 0u;
+            v[i] = ok ? volume[static_cast<int64_t>(row) * p.W + x] : T(0);
         }
+        uint32_t mine = 0;
+#pragma unroll
+        for (int i = 0; i < kSignWords; ++i)
+        {
+            const uint32_t word = __ballot_sync(0xffffffffu, ((in >> i) & 1u) && below<DT>(&v[i], 0, p.iso));
+            if (lane == i)
+                mine = word;
+        }
+        if (lane < kSignWords && g * kSignWords + lane < p.nwords)
+            p.sign[g * kSignWords + lane] = mine;
     }
 }
 
@@ -585,6 +363,98 @@ __global__ void __launch_bounds__(256) mc_sparse_classify_kernel(McPlan p)
     }
 }
 
+// Sparse volumes in words: the entries are in row order, so an entry's index
+// is its word's first entry plus the present points before it.
+template <int DT>
+struct SparseWords : VolumeWords
+{
+    __device__ EdgeBits edges(uint32_t k, const WordRows& r, const uint32_t s[4], const uint32_t sh[4], uint32_t& cells) const
+    {
+        cells = 0;
+        if (p.present[k] == 0)
+            return EdgeBits{ 0u, 0u, 0u };
+        const uint32_t plane = p.wr * p.div_h.d;
+        return masked_edges(
+                [&](int dy, int dz) {
+                    const int64_t y = static_cast<int64_t>(r.y) + dy, z = static_cast<int64_t>(r.z) + dz;
+                    return y >= 0 && y < p.H && z >= 0 && z < p.D ? k + dy * p.wr + dz * plane : kNoWord;
+                },
+                [&](uint32_t idx) { return p.present[idx]; }, r.x0 > 0, r.next, s, sh, cells);
+    }
+    __device__ uint32_t entry(uint32_t k, int b) const
+    {
+        return p.rank[k] + static_cast<uint32_t>(__popc(p.present[k] & ((1u << b) - 1u)));
+    }
+    __device__ void vertex(uint32_t k, int b, int axis, float out[3]) const
+    {
+        const WordRows r = rows(k);
+        const uint32_t e1 = entry(k, b);
+        // the edge's other end is an entry: a complete cell holds both
+        const uint32_t e2 = axis == 0 ? e1 + 1 : entry(r.idx[axis], b);
+        mc_vertex(p, r.x0 + b, r.y, r.z, axis, load_f32<DT>(p.values, e1), load_f32<DT>(p.values, e2), out);
+    }
+    __device__ void values_at(const WordRows& r, int b, unsigned long long* corner) const
+    {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            const uint32_t e = entry(r.idx[q], b);
+            corner[2 * q] = e;
+            corner[2 * q + 1] = e + 1;
+        }
+    }
+    __device__ void soup_vertex(uint32_t k, int b, int lo, int axis, unsigned long long h1, unsigned long long h2, float out[3]) const
+    {
+        const WordRows r = rows(k);
+        mc_vertex(p, r.x0 + b + (lo & 1), static_cast<int64_t>(r.y) + (lo >> 1 & 1), static_cast<int64_t>(r.z) + (lo >> 2 & 1),
+                  axis, load_f32<DT>(p.values, static_cast<int64_t>(h1)), load_f32<DT>(p.values, static_cast<int64_t>(h2)), out);
+    }
+};
+
+// The entries' presence and sign bits and each word's first entry; flags
+// entries outside the volume and indices that are not strictly ascending.
+// Entries of one word are neighbours, so a warp ORs each word's bits first.
+template <int DT>
+__global__ void __launch_bounds__(256) mc_sparse_words_kernel(McPlan p)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x - lane; t0 < p.nnz; t0 += stride)
+    {
+        const int64_t t = t0 + lane;
+        const bool valid = t < p.nnz;
+        int64_t x = 0, y = 0, z = 0;
+        const bool in = valid && entry_point(p, t, x, y, z);
+        if (valid && !in)
+            atomicOr(&p.ctr->flags, static_cast<unsigned int>(kMcBadIndex));
+        const uint32_t word = in ? static_cast<uint32_t>((y + p.H * z) * p.wr + (x >> 5)) : kNoWord;
+        // the entry before: the left lane's, or read
+        int64_t px = __shfl_up_sync(0xffffffffu, x, 1), py = __shfl_up_sync(0xffffffffu, y, 1), pz = __shfl_up_sync(0xffffffffu, z, 1);
+        bool pin = __shfl_up_sync(0xffffffffu, in ? 1 : 0, 1) != 0;
+        if (lane == 0)
+            pin = valid && t > 0 && entry_point(p, t - 1, px, py, pz);
+        uint32_t pword = kNoWord;
+        if (in && pin)
+        {
+            pword = static_cast<uint32_t>((py + p.H * pz) * p.wr + (px >> 5));
+            if (px + p.W * (py + p.H * pz) >= x + p.W * (y + p.H * z))
+                atomicOr(&p.ctr->flags, static_cast<unsigned int>(kMcUnsorted));
+        }
+        if (in && pword != word)
+            p.rank[word] = static_cast<uint32_t>(t);
+        const uint32_t bit = in ? 1u << (x & 31) : 0u;
+        const uint32_t low = in && below<DT>(p.values, t, p.iso) ? bit : 0u;
+        const uint32_t peers = __match_any_sync(0xffffffffu, word);
+        const uint32_t bits = __reduce_or_sync(peers, bit), lows = __reduce_or_sync(peers, low);
+        if (in && lane == __ffs(peers) - 1)
+        {
+            atomicOr(p.present + word, bits);
+            if (lows)
+                atomicOr(p.sign + word, lows);
+        }
+    }
+}
+
 struct SparseSoupCount
 {
     const uint8_t* codes;
@@ -681,51 +551,51 @@ struct SparseCellEmit
     }
 };
 
-// Blocks of the two point passes: up to 8 per SM.
-int dense_grid(const McPlan& p)
+template <class Src>
+void words_count(const Src& src, cudaStream_t s)
 {
-    const int64_t tiles = (p.points + kScanTile - 1) / kScanTile;
-    const int64_t cap = 8LL * sm_count();
-    return static_cast<int>(tiles < cap ? tiles : cap);
+    const McPlan& p = src.p;
+    const int grid = words_grid(p.nwords);
+    if (p.unique)
+        words_count_kernel<Src, true><<<grid, kWordThreads, 0, s>>>(src, p.mesh, &p.ctr->scan_soup, &p.ctr->active, WordTotal{ p.ctr });
+    else
+        words_count_kernel<Src, false><<<grid, kWordThreads, 0, s>>>(src, p.mesh, &p.ctr->scan_soup, &p.ctr->active, WordTotal{ p.ctr });
+    TH_LAUNCH_CHECK();
+    words_base_kernel<Src><<<grid, kWordThreads, 0, s>>>(src, p.mesh);
+    TH_LAUNCH_CHECK();
 }
 
-template <int DT, bool WIDE>
+template <class Src>
+void words_emit(const Src& src, float* verts, int64_t* faces, cudaStream_t s)
+{
+    const McPlan& p = src.p;
+    const int grid = grid_for(p.nwords, 32 * kWordExportWarps);
+    if (p.unique)
+        words_export_kernel<Src, true, false><<<grid, 32 * kWordExportWarps, 0, s>>>(src, p.mesh, verts, faces);
+    else
+        words_export_kernel<Src, false, false><<<grid, 32 * kWordExportWarps, 0, s>>>(src, p.mesh, verts, faces);
+    TH_LAUNCH_CHECK();
+}
+
+template <int DT>
 void dense_count(const McPlan& p, cudaStream_t s)
 {
-    const int64_t ntiles = (p.points + kScanTile - 1) / kScanTile;
-    TH_CUDA(cudaMemsetAsync(p.tiles_soup, 0, sizeof(unsigned long long) * ntiles, s));
-    if (p.unique)
-        TH_CUDA(cudaMemsetAsync(p.groups, 0, sizeof(McGroup) * p.ngroups, s));
-    const dim3 grid(static_cast<unsigned>((p.W + kMarchX - 1) / kMarchX),
-                    static_cast<unsigned>((p.H + kMarchY - 1) / kMarchY),
-                    static_cast<unsigned>((p.D + kMarchZ - 1) / kMarchZ));
-    mc_dense_march_kernel<DT><<<grid, dim3(kMarchX, kMarchY), 0, s>>>(p);
+    mc_sign_kernel<DT><<<grid_for(p.nwords * 32 / kSignWords, 256), 256, 0, s>>>(p);
     TH_LAUNCH_CHECK();
-    run_scan(TileCount{ p.tiles_soup }, TileEmit{ p.tiles_soup }, PackedTotal{ p.ctr }, Count{ nullptr, ntiles }, ntiles,
-             p.tiles_scan, &p.ctr->scan_soup, s);
-    if (p.unique)
-        run_scan(GroupCount{ p.groups }, GroupEmit{ p.groups }, VertTotal{ p.ctr }, Count{ nullptr, p.ngroups },
-                 p.ngroups, p.tiles_verts, &p.ctr->scan_verts, s);
-}
-
-template <int DT, bool WIDE>
-void dense_emit(const McPlan& p, float* verts, int64_t* faces, cudaStream_t s)
-{
-    if (p.unique)
-    {
-        mc_dense_verts_kernel<DT, WIDE><<<grid_for(p.ngroups * 32, 256), 256, 0, s>>>(p, verts);
-        TH_LAUNCH_CHECK();
-    }
-    mc_dense_compact_kernel<<<dense_grid(p), kScanThreads, 0, s>>>(p);
-    TH_LAUNCH_CHECK();
-    mc_dense_faces_kernel<DT, WIDE><<<grid_for(p.nactive, 256), 256, 0, s>>>(p, verts, faces);
-    TH_LAUNCH_CHECK();
+    words_count(DenseWords<DT>{ { p } }, s);
 }
 
 template <int DT>
 void sparse_count(const McPlan& p, cudaStream_t s)
 {
     const int grid = grid_for(p.nnz, 256);
+    if (p.words)
+    {
+        mc_sparse_words_kernel<DT><<<grid, 256, 0, s>>>(p);
+        TH_LAUNCH_CHECK();
+        words_count(SparseWords<DT>{ { p } }, s);
+        return;
+    }
     mc_sparse_insert_kernel<<<grid, 256, 0, s>>>(p);
     TH_LAUNCH_CHECK();
     mc_sparse_classify_kernel<DT><<<grid, 256, 0, s>>>(p);
@@ -740,6 +610,11 @@ void sparse_count(const McPlan& p, cudaStream_t s)
 template <int DT>
 void sparse_emit(const McPlan& p, float* verts, int64_t* faces, cudaStream_t s)
 {
+    if (p.words)
+    {
+        words_emit(SparseWords<DT>{ { p } }, verts, faces, s);
+        return;
+    }
     if (p.unique)
     {
         mc_sparse_verts_kernel<DT><<<grid_for(p.nnz, 256), 256, 0, s>>>(p, verts);
@@ -775,20 +650,18 @@ void launch_mc_count(const McPlan& p, cudaStream_t s)
     {
         if (p.nnz == 0)
             return;
-        TH_CUDA(cudaMemsetAsync(p.keys, 0xff, sizeof(unsigned long long) * (p.hmask + 1), s));
-        if (p.unique)
-            TH_CUDA(cudaMemsetAsync(p.used, 0, sizeof(uint32_t) * p.nnz, s));
+        if (p.words)
+            TH_CUDA(cudaMemsetAsync(p.present, 0, 2 * sizeof(uint32_t) * p.nwords, s)); // and the sign words after them
+        else
+        {
+            TH_CUDA(cudaMemsetAsync(p.keys, 0xff, sizeof(unsigned long long) * (p.hmask + 1), s));
+            if (p.unique)
+                TH_CUDA(cudaMemsetAsync(p.used, 0, sizeof(uint32_t) * p.nnz, s));
+        }
         dispatch_value_dtype(p.dtype, [&]<int DT>() { sparse_count<DT>(p, s); });
         return;
     }
-    if (p.points == 0)
-        return;
-    dispatch_value_dtype(p.dtype, [&]<int DT>() {
-        if (p.wide)
-            dense_count<DT, true>(p, s);
-        else
-            dense_count<DT, false>(p, s);
-    });
+    dispatch_value_dtype(p.dtype, [&]<int DT>() { dense_count<DT>(p, s); });
 }
 
 void launch_mc_emit(const McPlan& p, float* verts, int64_t* faces, cudaStream_t s)
@@ -800,14 +673,7 @@ void launch_mc_emit(const McPlan& p, float* verts, int64_t* faces, cudaStream_t 
         dispatch_value_dtype(p.dtype, [&]<int DT>() { sparse_emit<DT>(p, verts, faces, s); });
         return;
     }
-    if (p.points == 0)
-        return;
-    dispatch_value_dtype(p.dtype, [&]<int DT>() {
-        if (p.wide)
-            dense_emit<DT, true>(p, verts, faces, s);
-        else
-            dense_emit<DT, false>(p, verts, faces, s);
-    });
+    dispatch_value_dtype(p.dtype, [&]<int DT>() { words_emit(DenseWords<DT>{ { p } }, verts, faces, s); });
 }
 
 } // namespace th

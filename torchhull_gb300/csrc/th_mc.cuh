@@ -5,6 +5,7 @@
 #include <cstdint>
 
 #include "th_common.cuh"
+#include "th_words.cuh"
 
 namespace th
 {
@@ -26,43 +27,36 @@ struct McCounters
     ScanState scan_verts;
 };
 
-// Edge bits of 32 consecutive grid points of a dense volume: bit l of x / y /
-// z is set when the +x / +y / +z edge of point 32 g + l is a mesh vertex.
-struct McGroup
-{
-    uint32_t x, y, z, pad;
-    unsigned long long base; // vertices of all points before the group
-};
-
 struct McPlan
 {
     int dtype; // TH_FLOAT16, TH_FLOAT32 or TH_FLOAT64
     bool sparse, unique, local;
-    bool wide;             // points >= 2^32: 64-bit index decoding
     int64_t D, H, W;       // volume sizes along z, y, x
-    int64_t points;        // D * H * W
-    FastDiv div_w, div_h;  // by W and by H (points < 2^32)
     float iso;
     float scale[3];        // 2 / (size - 1) along x, y, z
     const void* volume;    // dense: [D, H, W], x fastest
     const int64_t* indices; // sparse: [4, nnz] rows (0, z, y, x)
     const void* values;     // sparse: [nnz]
     int64_t nnz;
-    // pools
-    McGroup* groups;          // dense, unique: ceil(points / 32)
-    int64_t ngroups;
-    unsigned long long* keys; // sparse: open-addressing table of ravel ids
-    int32_t* slots;           // sparse: entry index of each key
+    // Bit words (th_words.cuh): rows of wr words, one bit per grid point; dense
+    // volumes, and sparse ones whose words are few enough for their entries.
+    bool words;
+    int64_t nwords;
+    uint32_t wr;
+    FastDiv div_wr, div_h;    // by wr and by H
+    uint32_t* sign;           // bit: below the isolevel
+    uint32_t* present;        // sparse: bit: the volume has an entry
+    uint32_t* rank;           // sparse: first entry of a word that has any
+    WordMesh mesh;
+    // sparse volumes with few entries for their size
+    unsigned long long* keys; // open-addressing table of ravel ids
+    int32_t* slots;           // entry index of each key
     uint64_t hmask;           // table capacity - 1 (a power of two minus one)
-    uint8_t* codes;           // cell code of each point (dense) or entry (sparse); 0: no cell
-    uint32_t* used;           // sparse, unique: vertex edge bits of each entry
-    unsigned long long* vbase; // sparse, unique: first vertex of each entry
+    uint8_t* codes;           // cell code of each entry; 0: no cell
+    uint32_t* used;           // unique: vertex edge bits of each entry
+    unsigned long long* vbase; // unique: first vertex of each entry
     unsigned long long* tiles_soup;
     unsigned long long* tiles_verts;
-    unsigned long long* tiles_scan; // dense: tile sums of the scan over tiles_soup
-    int64_t* active;                 // dense: active cells (base points), ascending
-    unsigned long long* active_soup; // dense: their first soup vertex
-    int64_t nactive;                 // dense: active cells (known after phase 1)
     McCounters* ctr;
 };
 
