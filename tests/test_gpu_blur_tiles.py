@@ -1,4 +1,4 @@
-"""The blur's blocks of 64 x 32 pixels at their edges: sizes around a block, wide kernels, rows that vector loads cannot take."""
+"""The blur's blocks of 32 x 32 pixels at their edges: sizes around blocks, wide kernels, rows that vector loads cannot take."""
 
 from __future__ import annotations
 
@@ -10,7 +10,7 @@ from oracle import oracle
 
 pytestmark = pytest.mark.gpu
 
-# images (batch, height, width): below, at and above a block's 64 x 32 pixels; smaller than the halo; odd rows
+# images (batch, height, width): below, at and above one or two blocks of 32 x 32 pixels; smaller than the halo; odd rows
 SHAPES = [(2, 31, 63), (1, 32, 64), (3, 33, 65), (1, 70, 130), (1, 5, 7)]
 
 

@@ -25,6 +25,7 @@
 // output).  The reference's conv2d order belongs to cuDNN, so dense output
 // agrees within rounding, as the reference's own dense/sparse test allows.
 
+#include <algorithm>
 #include <cstring>
 
 #include "th_common.cuh"
@@ -83,6 +84,9 @@ __device__ __forceinline__ int64_t reflect(int64_t y, int64_t n)
     if (n == 1)
         return 0;
     const int64_t m = n - 1;
+    // one reflection, the usual case (halos narrower than the image)
+    if (-m < y && y < 2 * m)
+        return y < 0 ? -y : (y > m ? 2 * m - y : y);
     const int64_t flips = y / m + (y < 0 ? 1 : 0);
     int64_t rem = y % m;
     if (rem < 0)
@@ -99,17 +103,33 @@ __device__ __forceinline__ bool differ(typename Elem<DT>::T a, typename Elem<DT>
         return a != b;
 }
 
-// edge_kernel (gaussian_blur_cuda.cu:116-142) folded into tile flags.  A warp
-// owns 32 * V columns of a band of kEdgeRows rows, V elements (16 bytes where
-// the rows are 16-byte aligned, else one) per lane: it issues the band's loads
-// at once and compares from registers, so every row is read once plus one per
+template <class F>
+__device__ __forceinline__ void dispatch_out_device(int odt, F&& f)
+{
+    if (odt == TH_FLOAT16)
+        f.template operator()<TH_FLOAT16>();
+    else if (odt == TH_FLOAT32)
+        f.template operator()<TH_FLOAT32>();
+    else
+        f.template operator()<TH_FLOAT64>();
+}
+
+// edge_kernel (gaussian_blur_cuda.cu:116-142) folded into tile flags, and the
+// copy of every pixel to the output (the pixels that are blurred are written
+// again by the second pass).  A warp owns 32 * V columns of a band of
+// kEdgeRows rows, V elements per lane (16 bytes where input and output have
+// one type and 16-byte aligned rows, else one): it issues the band's loads at
+// once and compares from registers, so every row is read once plus one per
 // band, and index arithmetic is left to the few elements that are edges.
-// Bound by the read of the images (one element per thread with 64-bit
-// divisions took 146 us for 32x1024^2 float32, seven times that read).
+// Bound by the read and the write of the images: 32x1024^2 float32 61 us
+// with the copy (one element per thread with 64-bit divisions took 146 us
+// without it).
 constexpr int kEdgeRows = 8;
 
 template <int DT, int V>
 __global__ void __launch_bounds__(256) edge_tiles_kernel(const void* __restrict__ img,
+                                                         void* __restrict__ out,
+                                                         int odt,
                                                          int64_t B,
                                                          int64_t H,
                                                          int64_t W,
@@ -131,7 +151,8 @@ __global__ void __launch_bounds__(256) edge_tiles_kernel(const void* __restrict_
         const int64_t x = (chunk * 32 + lane) * V, y0 = band * kEdgeRows;
         if (x >= W)
             continue; // with V > 1, W is a multiple of V
-        const T* p = src + (b * H + y0) * W + x;
+        const int64_t at = (b * H + y0) * W + x;
+        const T* p = src + at;
         const int rows = static_cast<int>(H - y0 < kEdgeRows + 1 ? H - y0 : kEdgeRows + 1); // with the row below
         const bool right = x + V < W;
         T v[kEdgeRows + 1][V], rn[kEdgeRows];
@@ -150,6 +171,24 @@ __global__ void __launch_bounds__(256) edge_tiles_kernel(const void* __restrict_
             if (i < kEdgeRows)
                 rn[i] = right ? q[V] : v[i][V - 1];
         }
+        if constexpr (V > 1)
+        {
+#pragma unroll
+            for (int i = 0; i < kEdgeRows; ++i)
+            {
+                uint4 w;
+                memcpy(&w, v[i], sizeof(w));
+                if (i < rows)
+                    *reinterpret_cast<uint4*>(static_cast<T*>(out) + at + i * W) = w;
+            }
+        }
+        else
+            dispatch_out_device(odt, [&]<int OT>() {
+#pragma unroll
+                for (int i = 0; i < kEdgeRows; ++i)
+                    if (i < rows)
+                        store_out<OT>(out, at + i * W, as_out<DT, OT>(&v[i][0], 0));
+            });
 #pragma unroll
         for (int i = 0; i < kEdgeRows; ++i)
         {
@@ -186,7 +225,7 @@ constexpr int kSumTaps = 4096;
 
 template <int OT>
 __global__ void __launch_bounds__(256) weights_kernel(int k, float sigma, bool normalise, double* __restrict__ w, double* __restrict__ norm,
-                                                      uint4* __restrict__ zero, int64_t zero_bytes)
+                                                      uint4* __restrict__ zero, int64_t zero_bytes, uint32_t* __restrict__ ticket)
 {
     if (blockIdx.x > 0)
     {
@@ -197,6 +236,8 @@ __global__ void __launch_bounds__(256) weights_kernel(int k, float sigma, bool n
     }
     __shared__ float ev[kSumTaps];
     __shared__ float total;
+    if (threadIdx.x == 0 && ticket)
+        *ticket = 0;
     const int r = k / 2, taps = k * k;
     const float den = __fmul_rn(__fmul_rn(2.f, sigma), sigma);
     auto weight = [&](int t) {
@@ -401,7 +442,7 @@ __device__ __forceinline__ void dispatch_device(int dt, F&& f)
     }
 }
 
-// ---- blocks of 64 x 32 output pixels ---------------------------------------
+// ---- blocks of 32 x 32 output pixels ---------------------------------------
 //
 // The block stages its pixels and a halo of k/2 in shared memory, converted
 // once to the type the taps are accumulated in (reflected at the image's
@@ -409,13 +450,13 @@ __device__ __forceinline__ void dispatch_device(int dt, F&& f)
 // of that column in registers, so a shared load serves eight taps.  Per pixel
 // the taps run in the reference's order (x offset outer, y offset inner) with
 // its roundings, so sparse results are the same bits as one pixel per thread.
-// Sparse: a block without an active tile is a copy, whose loads are issued
-// before the tile flags are known.  Bound by the FMA issue (dense) and by the
-// read and write of the images (sparse).  The whole call on GB300: sparse
-// 32x1024^2 float32, k = 9, 1288 -> 195 us; dense 24x501x723 half, k = 13,
-// 3562 -> 179 us (one pixel per thread before, with a global load, two 64-bit
-// reflections and a double weight per tap).
-constexpr int kTileX = 64, kTileY = 32, kTileRows = 8;
+// Bound by the FMA and shared-load issue.  The whole call on GB300: sparse
+// 32x1024^2 float32, k = 9, 1288 -> 185 us; dense 24x501x723 half, k = 13,
+// 3562 -> 129 us (one pixel per thread before, with a global load, two 64-bit
+// reflections and a double weight per tap).  Blocks of 64 x 32 pixels took 192
+// and 135 us: more of a block waits at its barriers.
+constexpr int kTileX = 32, kTileY = 32, kTileRows = 8;
+constexpr int kTileThreads = kTileX * kTileY / kTileRows, kTileWarps = kTileThreads / 32;
 constexpr int kTileSmem = 96 * 1024;
 
 template <int OT, bool SPARSE>
@@ -465,137 +506,106 @@ __device__ __forceinline__ A tile_value(const void* img, int64_t i)
         return round_half(load_f32<DT>(img, i));
 }
 
-// Warp w loads the rows w, w + 8, ... of the tile and its halo.
-template <int DT, int OT, typename A>
-__device__ __forceinline__ void load_tile(const void* __restrict__ img, A* tile, const BlurGeom& g, int64_t base, int64_t y0, int64_t x0, int r)
+// The tile and its halo; a thread's loads are issued kLoadAhead at a time.
+constexpr int kLoadAhead = 8;
+
+template <int DT, int OT, typename A, bool INNER>
+__device__ __forceinline__ void load_tile_part(const void* __restrict__ img, A* tile, const BlurGeom& g, int64_t base, int64_t y0, int64_t x0, int r)
 {
-    const int lane = threadIdx.x & 31;
-    const int sx = kTileX + 2 * r, sy = kTileY + 2 * r;
-    const bool inner = x0 >= r && y0 >= r && x0 + kTileX + r <= g.W && y0 + kTileY + r <= g.H;
-#pragma unroll 2
-    for (int ly = threadIdx.x >> 5; ly < sy; ly += 8)
+    const int sx = kTileX + 2 * r, n = sx * (kTileY + 2 * r);
+    const int step_y = kTileThreads / sx, step_x = kTileThreads - step_y * sx;
+    int ly = threadIdx.x / sx, lx = threadIdx.x - ly * sx;
+    const int64_t corner = base + (y0 - r) * g.W + x0 - r;
+    const int W = static_cast<int>(g.W); // INNER: ly * W + lx from the corner, rows of less than 2^31 elements
+    for (int i = threadIdx.x; i < n; i += kTileThreads * kLoadAhead)
     {
-        const int64_t y = y0 - r + ly;
-        const int64_t row = base + (inner ? y : reflect(y, g.H)) * g.W;
-        for (int lx = lane; lx < sx; lx += 32)
+        A v[kLoadAhead];
+#pragma unroll
+        for (int u = 0; u < kLoadAhead; ++u)
         {
-            int64_t x = x0 - r + lx;
-            if (!inner && (x < 0 || x >= g.W))
-                x = reflect(x, g.W);
-            tile[ly * sx + lx] = tile_value<DT, OT, A>(img, row + x);
+            if (i + kTileThreads * u < n)
+            {
+                int64_t at;
+                if constexpr (INNER)
+                    at = corner + static_cast<int64_t>(ly) * W + lx;
+                else
+                    at = base + reflect(y0 - r + ly, g.H) * g.W + reflect(x0 - r + lx, g.W);
+                v[u] = tile_value<DT, OT, A>(img, at);
+            }
+            lx += step_x;
+            ly += step_y;
+            if (lx >= sx)
+            {
+                lx -= sx;
+                ++ly;
+            }
         }
+#pragma unroll
+        for (int u = 0; u < kLoadAhead; ++u)
+            if (i + kTileThreads * u < n)
+                tile[i + kTileThreads * u] = v[u];
     }
 }
 
-template <int OT, bool SPARSE>
-__global__ void __launch_bounds__(256, 3) blur_tile_kernel(const void* __restrict__ img,
-                                                        int idt,
-                                                        void* __restrict__ out,
-                                                        BlurGeom g,
-                                                        const uint8_t* __restrict__ tiles,
-                                                        const double* __restrict__ wtab,
-                                                        const double* __restrict__ norm_ptr,
-                                                        int vec)
+template <int DT, int OT, typename A>
+__device__ __forceinline__ void load_tile(const void* __restrict__ img, A* tile, const BlurGeom& g, int64_t base, int64_t y0, int64_t x0, int r)
 {
-    using A = typename Accumulate<OT, SPARSE>::T;
-    using O = typename Elem<OT>::T;
-    extern __shared__ __align__(16) unsigned char blur_smem[];
-    const int tid = threadIdx.x, k = g.k, r = k / 2;
-    const int sx = kTileX + 2 * r, sy = kTileY + 2 * r;
-    A* w = reinterpret_cast<A*>(blur_smem);
-    A* tile = w + k * k;
-    uint8_t* act = reinterpret_cast<uint8_t*>(tile + sx * sy);
+    if (x0 >= r && y0 >= r && x0 + kTileX + r <= g.W && y0 + kTileY + r <= g.H && g.W < (int64_t{ 1 } << 31))
+        load_tile_part<DT, OT, A, true>(img, tile, g, base, y0, x0, r);
+    else
+        load_tile_part<DT, OT, A, false>(img, tile, g, base, y0, x0, r);
+}
 
-    const int64_t bx = (g.W + kTileX - 1) / kTileX, by = (g.H + kTileY - 1) / kTileY;
-    // fewer than 2^31 blocks: bx and by fit 32 bits
-    const uint32_t nbx = static_cast<uint32_t>(bx), nby = static_cast<uint32_t>(by);
-    const uint32_t rest = blockIdx.x / nbx, ib = rest / nby;
-    const int64_t x0 = static_cast<int64_t>(blockIdx.x - rest * nbx) * kTileX, b = ib,
+// Row stride of the weights in shared memory: rows of 16-byte multiples, read four at a time.
+__host__ __device__ __forceinline__ int weight_stride(int k)
+{
+    return (k + 3) / 4 * 4;
+}
+
+template <typename A>
+struct __align__(4 * sizeof(A)) Four
+{
+    A v[4];
+};
+
+// Convolves block blk of the images (SPARSE: its pixels in active tiles).
+template <int OT, bool SPARSE, typename A>
+__device__ __forceinline__ void blur_block(const void* __restrict__ img,
+                                           int idt,
+                                           void* __restrict__ out,
+                                           const BlurGeom& g,
+                                           const uint8_t* __restrict__ tiles,
+                                           const A* w,
+                                           A* tile,
+                                           uint8_t* act,
+                                           double norm,
+                                           uint32_t blk,
+                                           uint32_t nbx,
+                                           uint32_t nby)
+{
+    const int tid = threadIdx.x, k = g.k, r = k / 2, ws = weight_stride(k);
+    const int sx = kTileX + 2 * r;
+    const uint32_t rest = blk / nbx, ib = rest / nby;
+    const int64_t x0 = static_cast<int64_t>(blk - rest * nbx) * kTileX, b = ib,
                   y0 = static_cast<int64_t>(rest - ib * nby) * kTileY;
     const int64_t base = b * g.H * g.W;
     const int ts = static_cast<int>(g.ts);
-    int ntx = 0, nty = 0, ox = 0, oy = 0; // the block's tiles, and its first pixel inside the first tile
+    int ntx = 0, ox = 0, oy = 0; // the block's tiles along x, and its first pixel inside its first tile
     if constexpr (SPARSE)
     {
-        // vec: same type in and out, rows 16-byte aligned
-        constexpr int kPer = 16 / static_cast<int>(sizeof(O)), kVecs = kTileX / kPer, kIter = kVecs * kTileY / 256;
-        uint4 c[kIter];
-        if (vec)
-        {
-#pragma unroll
-            for (int i = 0; i < kIter; ++i)
-            {
-                const int v = tid + i * 256;
-                const int64_t y = y0 + v / kVecs, x = x0 + (v % kVecs) * kPer;
-                if (y < g.H && x < g.W)
-                    c[i] = __ldg(reinterpret_cast<const uint4*>(static_cast<const O*>(img) + base + y * g.W + x));
-            }
-        }
-        // the tiles of the block's pixels, and those of one tile around them
         const int64_t xl = x0 + kTileX < g.W ? x0 + kTileX - 1 : g.W - 1, yl = y0 + kTileY < g.H ? y0 + kTileY - 1 : g.H - 1;
         const int64_t tx0 = x0 / ts, ty0 = y0 / ts;
         ox = static_cast<int>(x0 - tx0 * ts);
         oy = static_cast<int>(y0 - ty0 * ts);
         ntx = static_cast<int>(xl / ts - tx0) + 1;
-        nty = static_cast<int>(yl / ts - ty0) + 1;
-        bool any = false;
-        for (int t = tid; t < (ntx + 2) * (nty + 2); t += 256)
+        const int nty = static_cast<int>(yl / ts - ty0) + 1;
+        // the flags of the block's tiles and of those around them
+        const int rx = ntx + 2;
+        for (int t = tid; t < rx * (nty + 2); t += kTileThreads)
         {
-            const int64_t yy = ty0 - 1 + t / (ntx + 2), xx = tx0 - 1 + t % (ntx + 2);
-            if (yy >= 0 && yy < g.TH && xx >= 0 && xx < g.TW)
-                any |= tiles[(b * g.TH + yy) * g.TW + xx] != 0;
+            const int64_t yy = ty0 - 1 + t / rx, xx = tx0 - 1 + t % rx;
+            act[t] = yy >= 0 && yy < g.TH && xx >= 0 && xx < g.TW ? tiles[(b * g.TH + yy) * g.TW + xx] : 0;
         }
-        if (!__syncthreads_or(any))
-        {
-            if (vec)
-            {
-#pragma unroll
-                for (int i = 0; i < kIter; ++i)
-                {
-                    const int v = tid + i * 256;
-                    const int64_t y = y0 + v / kVecs, x = x0 + (v % kVecs) * kPer;
-                    if (y < g.H && x < g.W)
-                        *reinterpret_cast<uint4*>(static_cast<O*>(out) + base + y * g.W + x) = c[i];
-                }
-                return;
-            }
-            const int64_t x = x0 + (tid & 63);
-            auto copy = [&]<int DT>() {
-                double v[kTileRows];
-#pragma unroll
-                for (int j = 0; j < kTileRows; ++j)
-                {
-                    const int64_t y = y0 + (tid >> 6) + 4 * j;
-                    v[j] = x < g.W && y < g.H ? as_out<DT, OT>(img, base + y * g.W + x) : 0.0;
-                }
-#pragma unroll
-                for (int j = 0; j < kTileRows; ++j)
-                {
-                    const int64_t y = y0 + (tid >> 6) + 4 * j;
-                    if (x < g.W && y < g.H)
-                        store_out<OT>(out, base + y * g.W + x, v[j]);
-                }
-            };
-            dispatch_device(idt, copy);
-            return;
-        }
-        for (int t = tid; t < ntx * nty; t += 256)
-        {
-            const int64_t yy = ty0 + t / ntx, xx = tx0 + t % ntx;
-            bool on = false;
-            for (int64_t dy = -1; dy <= 1; ++dy)
-                for (int64_t dx = -1; dx <= 1; ++dx)
-                    if (yy + dy >= 0 && yy + dy < g.TH && xx + dx >= 0 && xx + dx < g.TW)
-                        on |= tiles[(b * g.TH + yy + dy) * g.TW + xx + dx] != 0;
-            act[t] = on ? 1 : 0;
-        }
-    }
-    for (int t = tid; t < k * k; t += 256)
-    {
-        if constexpr (sizeof(A) == 2)
-            w[t] = __float2half_rn(static_cast<float>(wtab[t]));
-        else
-            w[t] = static_cast<A>(wtab[t]);
     }
     dispatch_device(idt, [&]<int DT>() { load_tile<DT, OT, A>(img, tile, g, base, y0, x0, r); });
     __syncthreads();
@@ -607,11 +617,22 @@ __global__ void __launch_bounds__(256, 3) blur_tile_kernel(const void* __restric
     {
         if (x < g.W)
         {
-            const int tx = (ox + cx) / ts;
+            const int tx = (ox + cx) / ts, rx = ntx + 2;
+            int last = -1;
+            bool near = false;
 #pragma unroll
             for (int j = 0; j < kTileRows; ++j)
-                if (y0 + cy + j < g.H && act[(oy + cy + j) / ts * ntx + tx])
+            {
+                const int ty = (oy + cy + j) / ts;
+                if (ty != last)
+                {
+                    const uint8_t* a = act + ty * rx + tx; // the tile up and to the left
+                    near = (a[0] | a[1] | a[2] | a[rx] | a[rx + 1] | a[rx + 2] | a[2 * rx] | a[2 * rx + 1] | a[2 * rx + 2]) != 0;
+                    last = ty;
+                }
+                if (y0 + cy + j < g.H && near)
                     on |= 1u << j;
+            }
         }
     }
     else
@@ -624,45 +645,65 @@ __global__ void __launch_bounds__(256, 3) blur_tile_kernel(const void* __restric
     {
         for (int dx = 0; dx < k; ++dx)
         {
+            // a sliding window of the column in two halves that change roles
+            // every eight taps, so no value moves between registers
             const A* col = tile + cy * sx + cx + dx;
-            const A* wd = w + dx * k;
-            A v[2 * kTileRows - 1];
+            const A* wd = w + dx * ws;
+            A lo[kTileRows], hi[kTileRows];
 #pragma unroll
-            for (int j = 0; j < kTileRows - 1; ++j)
-                v[j] = col[j * sx];
-            col += (kTileRows - 1) * sx;
-            auto taps = [&]<int U>() {
+            for (int j = 0; j < kTileRows; ++j)
+                lo[j] = col[j * sx];
+            auto taps = [&]<int U>(const A(&from)[kTileRows], A(&next)[kTileRows]) {
+                col += kTileRows * sx;
 #pragma unroll
-                for (int u = 0; u < U; ++u)
-                    v[kTileRows - 1 + u] = col[u * sx];
+                for (int u = 0; u < (U < kTileRows ? U - 1 : U); ++u)
+                    next[u] = col[u * sx];
 #pragma unroll
-                for (int u = 0; u < U; ++u)
+                for (int u = 0; u < U; u += 4)
                 {
-                    const A wt = wd[u];
+                    const Four<A> wt = *reinterpret_cast<const Four<A>*>(wd + u);
 #pragma unroll
-                    for (int j = 0; j < kTileRows; ++j)
-                        acc[j] = tap(wt, v[j + u], acc[j]);
+                    for (int i = 0; i < 4 && u + i < U; ++i)
+                    {
+#pragma unroll
+                        for (int j = 0; j < kTileRows; ++j)
+                        {
+                            const int at = j + u + i;
+                            acc[j] = tap(wt.v[i], at < kTileRows ? from[at < kTileRows ? at : 0] : next[at < kTileRows ? 0 : at - kTileRows], acc[j]);
+                        }
+                    }
                 }
-#pragma unroll
-                for (int j = 0; j < kTileRows - 1; ++j)
-                    v[j] = v[j + U];
-                col += U * sx;
                 wd += U;
             };
-            int left = k;
-            for (; left >= 8; left -= 8)
-                taps.template operator()<8>();
-            if (left & 4)
-                taps.template operator()<4>();
-            if (left & 2)
-                taps.template operator()<2>();
-            if (left & 1)
-                taps.template operator()<1>();
+            auto rest = [&](const A(&from)[kTileRows], A(&next)[kTileRows]) {
+                // k is odd
+                const int left = k & 7;
+                if (left == 1)
+                    taps.template operator()<1>(from, next);
+                else if (left == 3)
+                    taps.template operator()<3>(from, next);
+                else if (left == 5)
+                    taps.template operator()<5>(from, next);
+                else
+                    taps.template operator()<7>(from, next);
+            };
+            int eights = k >> 3;
+            for (; eights >= 2; eights -= 2)
+            {
+                taps.template operator()<8>(lo, hi);
+                taps.template operator()<8>(hi, lo);
+            }
+            if (eights)
+            {
+                taps.template operator()<8>(lo, hi);
+                rest(hi, lo);
+            }
+            else
+                rest(lo, hi);
         }
     }
     if (x >= g.W)
         return;
-    const double norm = *norm_ptr;
 #pragma unroll
     for (int j = 0; j < kTileRows; ++j)
     {
@@ -672,8 +713,8 @@ __global__ void __launch_bounds__(256, 3) blur_tile_kernel(const void* __restric
         const int64_t i = base + y * g.W + x;
         if constexpr (sizeof(A) == 2)
         {
-            const float res = __fdiv_rn(__half2float(acc[j]), static_cast<float>(norm));
-            static_cast<__half*>(out)[i] = (on >> j) & 1u ? __float2half_rn(res) : tile[(cy + j + r) * sx + cx + r];
+            if ((on >> j) & 1u)
+                static_cast<__half*>(out)[i] = __float2half_rn(__fdiv_rn(__half2float(acc[j]), static_cast<float>(norm)));
         }
         else
         {
@@ -685,9 +726,93 @@ __global__ void __launch_bounds__(256, 3) blur_tile_kernel(const void* __restric
                 else
                     res = __fdiv_rn(res, static_cast<float>(norm));
                 if (!((on >> j) & 1u))
-                    res = tile[(cy + j + r) * sx + cx + r];
+                    continue; // the first pass copied it
             }
             store_out<OT>(out, i, static_cast<double>(res));
+        }
+    }
+}
+
+// Whether block blk has a pixel in an active tile (a warp's lanes look at the
+// flags of its tiles and of one more around them).
+__device__ __forceinline__ bool block_active(const BlurGeom& g, const uint8_t* __restrict__ tiles, uint32_t blk, uint32_t nbx, uint32_t nby)
+{
+    const uint32_t rest = blk / nbx, ib = rest / nby;
+    const int64_t x0 = static_cast<int64_t>(blk - rest * nbx) * kTileX, y0 = static_cast<int64_t>(rest - ib * nby) * kTileY;
+    const int64_t xl = x0 + kTileX < g.W ? x0 + kTileX - 1 : g.W - 1, yl = y0 + kTileY < g.H ? y0 + kTileY - 1 : g.H - 1;
+    const int64_t ts = g.ts;
+    const int64_t tx0 = x0 / ts > 0 ? x0 / ts - 1 : 0, ty0 = y0 / ts > 0 ? y0 / ts - 1 : 0;
+    const int64_t tx1 = xl / ts + 1 < g.TW ? xl / ts + 1 : g.TW - 1, ty1 = yl / ts + 1 < g.TH ? yl / ts + 1 : g.TH - 1;
+    const uint8_t* p = tiles + (ib * g.TH + ty0) * g.TW + tx0;
+    const int nx = static_cast<int>(tx1 - tx0) + 1, n = nx * (static_cast<int>(ty1 - ty0) + 1);
+    bool any = false;
+#pragma unroll 4
+    for (int t = threadIdx.x & 31; t < n; t += 32)
+        any |= p[t / nx * g.TW + t % nx] != 0;
+    return __any_sync(0xffffffffu, any);
+}
+
+// One block of output pixels at a time: dense block blockIdx.x; sparse, a
+// block takes tickets, each for four blocks of pixels that lie far apart (few
+// of them are active at once), looks at their flags with a warp each and
+// convolves the active ones.  (A block per block of pixels, and a fixed share
+// of the image per block, waited for the slowest: 147 and 171 us for
+// 32x1024^2, k = 9, against 132 us.)
+template <int OT, bool SPARSE>
+__global__ void __launch_bounds__(kTileThreads, 6) blur_tile_kernel(const void* __restrict__ img,
+                                                        int idt,
+                                                        void* __restrict__ out,
+                                                        BlurGeom g,
+                                                        const uint8_t* __restrict__ tiles,
+                                                        const double* __restrict__ wtab,
+                                                        const double* __restrict__ norm_ptr,
+                                                        uint32_t nblocks,
+                                                        uint32_t* __restrict__ ticket)
+{
+    using A = typename Accumulate<OT, SPARSE>::T;
+    extern __shared__ __align__(32) unsigned char blur_smem[];
+    __shared__ uint32_t s_ticket, s_active;
+    const int tid = threadIdx.x, k = g.k, r = k / 2;
+    const int sx = kTileX + 2 * r, sy = kTileY + 2 * r, ws = weight_stride(k);
+    A* w = reinterpret_cast<A*>(blur_smem);
+    A* tile = w + k * ws;
+    uint8_t* act = reinterpret_cast<uint8_t*>(tile + sx * sy);
+    const uint32_t nbx = static_cast<uint32_t>((g.W + kTileX - 1) / kTileX), nby = static_cast<uint32_t>((g.H + kTileY - 1) / kTileY);
+    for (int t = tid; t < k * k; t += kTileThreads)
+    {
+        const int at = t / k * ws + t % k;
+        if constexpr (sizeof(A) == 2)
+            w[at] = __float2half_rn(static_cast<float>(wtab[t]));
+        else
+            w[at] = static_cast<A>(wtab[t]);
+    }
+    const double norm = *norm_ptr;
+    if constexpr (!SPARSE)
+        blur_block<OT, SPARSE>(img, idt, out, g, tiles, w, tile, act, norm, blockIdx.x, nbx, nby);
+    else
+    {
+        const uint32_t tickets = (nblocks + kTileWarps - 1) / kTileWarps;
+        for (uint32_t done = 0; done <= tickets; ++done) // ends when the tickets do
+        {
+            __syncthreads();
+            if (tid == 0)
+            {
+                s_ticket = atomicAdd(ticket, 1u);
+                s_active = 0;
+            }
+            __syncthreads();
+            const uint32_t t = s_ticket;
+            if (t >= tickets)
+                break;
+            const uint32_t mine = t + (tid >> 5) * tickets;
+            if (mine < nblocks && block_active(g, tiles, mine, nbx, nby) && (tid & 31) == 0)
+                atomicOr(&s_active, 1u << (tid >> 5));
+            __syncthreads();
+            for (uint32_t left = s_active; left; left &= left - 1)
+            {
+                blur_block<OT, SPARSE>(img, idt, out, g, tiles, w, tile, act, norm, t + (__ffs(left) - 1) * tickets, nbx, nby);
+                __syncthreads();
+            }
         }
     }
 }
@@ -698,15 +823,15 @@ template <int OT, bool SPARSE>
 size_t tile_smem(int k, int64_t ts)
 {
     const int64_t r = k / 2;
-    int64_t bytes = (int64_t{ k } * k + (kTileX + 2 * r) * (kTileY + 2 * r)) *
+    int64_t bytes = (int64_t{ k } * weight_stride(k) + (kTileX + 2 * r) * (kTileY + 2 * r)) *
                     static_cast<int64_t>(sizeof(typename Accumulate<OT, SPARSE>::T));
     if (SPARSE)
-        bytes += (kTileX / ts + 2) * (kTileY / ts + 2);
+        bytes += (kTileX / ts + 4) * (kTileY / ts + 4);
     return bytes <= kTileSmem ? static_cast<size_t>(bytes) : 0;
 }
 
 template <int OT, bool SPARSE>
-bool launch_tiles(const void* images, int idt, void* out, const BlurGeom& g, const uint8_t* tiles, const double* wtab, const double* norm, cudaStream_t s)
+bool launch_tiles(const void* images, int idt, void* out, const BlurGeom& g, const uint8_t* tiles, const double* wtab, const double* norm, uint32_t* ticket, cudaStream_t s)
 {
     const size_t smem = tile_smem<OT, SPARSE>(g.k, g.ts);
     const int64_t blocks = ((g.W + kTileX - 1) / kTileX) * ((g.H + kTileY - 1) / kTileY) * g.B;
@@ -715,9 +840,8 @@ bool launch_tiles(const void* images, int idt, void* out, const BlurGeom& g, con
     auto kernel = blur_tile_kernel<OT, SPARSE>;
     if (smem > 48 * 1024)
         TH_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem));
-    const int vec = idt == OT && (reinterpret_cast<uintptr_t>(images) | reinterpret_cast<uintptr_t>(out)) % 16 == 0 &&
-                    (g.W * static_cast<int64_t>(sizeof(typename Elem<OT>::T))) % 16 == 0;
-    kernel<<<static_cast<unsigned>(blocks), 256, smem, s>>>(images, idt, out, g, tiles, wtab, norm, vec);
+    const unsigned grid = SPARSE ? static_cast<unsigned>(std::min<int64_t>(blocks, 6 * sm_count())) : static_cast<unsigned>(blocks);
+    kernel<<<grid, kTileThreads, smem, s>>>(images, idt, out, g, tiles, wtab, norm, static_cast<uint32_t>(blocks), ticket);
     TH_LAUNCH_CHECK();
     return true;
 }
@@ -754,7 +878,7 @@ int64_t blur_tile_bytes(int64_t B, int64_t H, int64_t W, int kernel_size)
     const int64_t ts = kernel_size / 2;
     if (ts < 1)
         return 0;
-    // tile table plus the weight table (k*k doubles) and its sum
+    // tile table, padding and a ticket (16 bytes), the weight table (k*k doubles) and its sum
     return B * (H / ts + 1) * (W / ts + 1) + 16 + 8 * (static_cast<int64_t>(kernel_size) * kernel_size + 1);
 }
 
@@ -797,30 +921,40 @@ void launch_gaussian_blur(const void* images,
     double* wtab = reinterpret_cast<double*>(scratch + woff);
     double* norm = wtab + static_cast<int64_t>(kernel_size) * kernel_size;
     const int64_t zero_bytes = sparse ? woff : 0;
+    // The second pass's ticket: four bytes of the padding before the weights,
+    // or, where that is shorter, of what it leaves of its 16 bytes at the end
+    // (blur_tile_bytes).
+    uint32_t* ticket = woff - tile_bytes >= 4 ? reinterpret_cast<uint32_t*>(scratch + woff - 4)
+                                              : reinterpret_cast<uint32_t*>(norm + 1);
     const unsigned zero_blocks = static_cast<unsigned>(grid_for((zero_bytes + 15) / 16, 256 * 4));
     dispatch_out(odt, [&]<int OT>() {
         weights_kernel<OT><<<1 + (sparse ? zero_blocks : 0u), 256, 0, s>>>(kernel_size, sigma, !sparse, wtab, norm,
-                                                                            reinterpret_cast<uint4*>(tiles), zero_bytes);
+                                                                            reinterpret_cast<uint4*>(tiles), zero_bytes,
+                                                                            sparse ? ticket : nullptr);
     });
     TH_LAUNCH_CHECK();
     if (sparse)
     {
-        dispatch_image_dtype(idt, [&]<int DT>() {
-            constexpr int V = 16 / static_cast<int>(sizeof(typename Elem<DT>::T));
-            const bool vec = reinterpret_cast<uintptr_t>(images) % 16 == 0 && W % V == 0;
-            const int64_t units = B * ((H + kEdgeRows - 1) / kEdgeRows) * ((W + 32 * (vec ? V : 1) - 1) / (32 * (vec ? V : 1)));
-            const int egrid = grid_for(units * 32, 256);
-            if (vec)
-                edge_tiles_kernel<DT, V><<<egrid, 256, 0, s>>>(images, B, H, W, g.ts, g.TH, g.TW, tiles);
-            else
-                edge_tiles_kernel<DT, 1><<<egrid, 256, 0, s>>>(images, B, H, W, g.ts, g.TH, g.TW, tiles);
-        });
+        auto edges = [&]<int DT, int V>() {
+            const int64_t units = B * ((H + kEdgeRows - 1) / kEdgeRows) * ((W + 32 * V - 1) / (32 * V));
+            const unsigned egrid = static_cast<unsigned>(std::min<int64_t>((units + 7) / 8, 64LL * sm_count()));
+            edge_tiles_kernel<DT, V><<<egrid, 256, 0, s>>>(images, out, odt, B, H, W, g.ts, g.TH, g.TW, tiles);
+        };
+        const bool aligned = (reinterpret_cast<uintptr_t>(images) | reinterpret_cast<uintptr_t>(out)) % 16 == 0;
+        if (aligned && idt == odt && odt == TH_FLOAT16 && W % 8 == 0)
+            edges.template operator()<TH_FLOAT16, 8>();
+        else if (aligned && idt == odt && odt == TH_FLOAT32 && W % 4 == 0)
+            edges.template operator()<TH_FLOAT32, 4>();
+        else if (aligned && idt == odt && odt == TH_FLOAT64 && W % 2 == 0)
+            edges.template operator()<TH_FLOAT64, 2>();
+        else
+            dispatch_image_dtype(idt, [&]<int DT>() { edges.template operator()<DT, 1>(); });
         TH_LAUNCH_CHECK();
     }
     bool done = false;
     dispatch_out(odt, [&]<int OT>() {
-        done = sparse ? launch_tiles<OT, true>(images, idt, out, g, tiles, wtab, norm, s)
-                      : launch_tiles<OT, false>(images, idt, out, g, tiles, wtab, norm, s);
+        done = sparse ? launch_tiles<OT, true>(images, idt, out, g, tiles, wtab, norm, ticket, s)
+                      : launch_tiles<OT, false>(images, idt, out, g, tiles, wtab, norm, nullptr, s);
     });
     if (done)
         return;
