@@ -184,8 +184,9 @@ bool is_image_dtype(int d)
 struct HullSlot
 {
     DevBuf tf, sat, ones, cell_masks, nodes, node_skip, node_out, child_masks, child_skip, child_out, tile_sums, bitmap,
-            word_rank, rowbits, rows, corners, values, codes, emask, soup_off, vbase, counters, flags, sat_scratch;
-    int64_t node_cap = 0, corner_cap = 0, parent_cap = 0;
+            rowbits, rows, row_slot, row_cnt, row_place, present, runs, word_list, rank, sign, word_cnt, word_cells, word_edges, word_chunk,
+            corners, values, counters, flags, sat_scratch;
+    int64_t node_cap = 0, corner_cap = 0, parent_cap = 0, word_cap = 0;
     HullPlan plan{};
     DevCounters* host = nullptr; // pinned, mapped copy of the counters
     DevCounters* host_d = nullptr; // its device address
@@ -194,7 +195,7 @@ struct HullSlot
     ReqConsts* host_rq_d = nullptr; // its device address
     th_hull_info info{};
     bool has_result = false;
-    bool dirty = false; // bitmap rows of the last request still set
+    bool unfinished = false; // the last run was cut short: the bitmaps and the cell masks may hold bits
     cudaEvent_t done = nullptr;
 
     // Captured pipelines, keyed by the plan with the per-request fields cleared.
@@ -218,8 +219,8 @@ struct HullSlot
     std::vector<const DevBuf*> buffers() const
     {
         return { &tf,     &sat,  &ones,  &cell_masks,   &nodes,     &node_skip,   &node_out,  &child_masks, &child_skip, &child_out, &tile_sums,
-                 &bitmap, &word_rank, &rowbits, &rows, &corners,    &values,     &codes,
-                 &emask,  &soup_off, &vbase,   &counters, &flags, &sat_scratch, &rq };
+                 &bitmap, &rowbits, &rows, &row_slot, &row_cnt, &row_place, &present, &runs, &word_list, &rank, &sign, &word_cnt, &word_cells,
+                 &word_edges, &word_chunk, &corners, &values, &counters, &flags, &sat_scratch, &rq };
     }
 
     void release()
@@ -494,6 +495,12 @@ int64_t max_nodes(int level)
     return s;
 }
 
+// Bytes of the counters and the row groups' corner counts (HullPlan::coarse).
+size_t counter_bytes(int64_t R)
+{
+    return sizeof(DevCounters) + sizeof(uint2) * static_cast<size_t>(R * R / 256 + 2);
+}
+
 // Sizes the pools of slot s for request a and fills its plan.
 // batch_slot: the request is part of a batch, whose octree lives in the
 // batch's shared node pool, so the slot keeps no octree pools of its own.
@@ -522,6 +529,11 @@ void prepare(HullSlot& s, const th_hull_args* a, cudaStream_t st, bool field_one
     const int64_t node_cap = std::min<int64_t>(s.node_cap, max_nodes(L));
     const int64_t corner_cap = std::min<int64_t>(s.corner_cap, R * R * R);
     const int64_t parent_cap = std::min<int64_t>(s.parent_cap, node_cap);
+    // words of 32 points of the touched rows: all rows up to 32 M words (level
+    // 9: 4.7 M), more on demand; a batch slot starts at 8 M
+    const int64_t all_words = R * R * 2 * WR;
+    s.word_cap = std::max<int64_t>(s.word_cap, std::min<int64_t>(all_words, int64_t{ 1 } << (batch_slot ? 23 : 25)));
+    const int64_t word_cap = std::min<int64_t>(s.word_cap, all_words);
 
     s.tf.ensure(sizeof(float) * std::max<int64_t>(B, 1) * 16);
     s.sat.ensure(sizeof(float) * std::max<int64_t>(B * H * W, 1));
@@ -543,24 +555,38 @@ void prepare(HullSlot& s, const th_hull_args* a, cudaStream_t st, bool field_one
     s.child_skip.ensure(sizeof(uint32_t) * 8 * parent_cap);
     s.child_out.ensure(sizeof(uint32_t) * 8 * parent_cap);
     s.flags.ensure(sizeof(unsigned int) * 4);
-    const int64_t scan_items = std::max({ node_cap, corner_cap, R * R * WR });
-    s.tile_sums.ensure(sizeof(unsigned long long) * ((scan_items + kScanTile - 1) / kScanTile + 1));
+    s.tile_sums.ensure(sizeof(unsigned long long) *
+                       std::max<int64_t>((node_cap + kScanTile - 1) / kScanTile, word_tiles(word_cap)));
     const int64_t words = R * R * WR;
     const int64_t rwords = (R * R + 31) / 32;
     if (s.bitmap.ensure(sizeof(uint64_t) * words))
         TH_CUDA(cudaMemsetAsync(s.bitmap.p, 0, s.bitmap.bytes, st));
-    s.word_rank.ensure(sizeof(uint32_t) * words);
     if (s.rowbits.ensure(sizeof(uint32_t) * rwords))
         TH_CUDA(cudaMemsetAsync(s.rowbits.p, 0, s.rowbits.bytes, st));
+    if (s.unfinished)
+    {
+        for (const DevBuf* b : { &s.bitmap, &s.rowbits, &s.cell_masks })
+            if (b->p)
+                TH_CUDA(cudaMemsetAsync(b->p, 0, b->bytes, st));
+        s.unfinished = false;
+    }
     s.rows.ensure(sizeof(uint32_t) * R * R);
+    s.row_slot.ensure(sizeof(uint32_t) * R * R);
+    s.row_cnt.ensure(sizeof(uint2) * R * R);
+    s.row_place.ensure(sizeof(RowPlace) * R * R);
+    s.present.ensure(sizeof(uint32_t) * word_cap);
+    s.word_list.ensure(sizeof(uint32_t) * word_cap);
+    s.runs.ensure(sizeof(uint2) * word_cap);
+    s.rank.ensure(sizeof(uint32_t) * word_cap);
+    s.sign.ensure(sizeof(uint32_t) * word_cap);
+    s.word_cnt.ensure(sizeof(uint32_t) * word_cap);
+    s.word_cells.ensure(sizeof(uint32_t) * word_cap);
+    s.word_edges.ensure(sizeof(uint4) * word_cap);
+    s.word_chunk.ensure(sizeof(uint2) * ((word_cap + 31) / 32));
     s.corners.ensure(sizeof(int64_t) * corner_cap);
     s.values.ensure(sizeof(float) * corner_cap);
-    s.codes.ensure(corner_cap);
-    s.emask.ensure((corner_cap + 3) / 4 * 4);
-    s.soup_off.ensure(sizeof(uint32_t) * corner_cap);
-    s.vbase.ensure(sizeof(uint32_t) * corner_cap);
-    if (s.counters.ensure(sizeof(DevCounters)))
-        TH_CUDA(cudaMemsetAsync(s.counters.p, 0, sizeof(DevCounters), st));
+    // the counters and, behind them, the corners of 256 rows each: cleared together
+    s.counters.ensure(counter_bytes(R));
     if (!s.host)
         alloc_mapped(&s.host, &s.host_d);
     if (!s.done)
@@ -609,15 +635,25 @@ void prepare(HullSlot& s, const th_hull_args* a, cudaStream_t st, bool field_one
     p.R = R;
     p.WR = WR;
     p.bitmap = s.bitmap.as<uint64_t>();
-    p.word_rank = s.word_rank.as<uint32_t>();
     p.rowbits = s.rowbits.as<uint32_t>();
     p.rows = s.rows.as<uint32_t>();
+    p.row_slot = s.row_slot.as<uint32_t>();
+    p.row_cnt = s.row_cnt.as<uint2>();
+    p.coarse = reinterpret_cast<uint2*>(s.counters.as<DevCounters>() + 1);
+    p.wr = static_cast<uint32_t>(2 * WR);
+    p.div_wr = make_fastdiv(p.wr);
+    p.div_r = make_fastdiv(static_cast<uint32_t>(R));
+    p.word_cap = word_cap;
+    p.row_place = s.row_place.as<RowPlace>();
+    p.present = s.present.as<uint32_t>();
+    p.runs = s.runs.as<uint2>();
+    p.word_list = s.word_list.as<uint32_t>();
+    p.rank = s.rank.as<uint32_t>();
+    p.sign = s.sign.as<uint32_t>();
+    p.mesh = WordMesh{ s.word_cnt.as<uint32_t>(), s.word_cells.as<uint32_t>(), s.word_edges.as<uint4>(),
+                       s.word_chunk.as<uint2>(), s.tile_sums.as<unsigned long long>() };
     p.corners = s.corners.as<int64_t>();
     p.values = s.values.as<float>();
-    p.codes = s.codes.as<uint8_t>();
-    p.emask = s.emask.as<uint8_t>();
-    p.soup_off = s.soup_off.as<uint32_t>();
-    p.vbase = s.vbase.as<uint32_t>();
     p.corner_cap = corner_cap;
     p.ctr = s.counters.as<DevCounters>();
     // the per-request inputs the carve and field kernels read from the device
@@ -758,12 +794,8 @@ void run_hull_once(th_context* ctx,
                    const CarveVariants& variants,
                    float* carve_ms)
 {
-    if (s.dirty)
-    {
-        TH_CUDA(cudaStreamWaitEvent(st, s.done, 0));
-        launch_cleanup(s.plan, st);
-        s.dirty = false;
-    }
+    if (s.done)
+        TH_CUDA(cudaStreamWaitEvent(st, s.done, 0)); // the last request's exports read the pools
     s.has_result = false;
     const int L = a->level;
     for (int attempt = 0; attempt < 8; ++attempt)
@@ -772,6 +804,7 @@ void run_hull_once(th_context* ctx,
         for (int i = 0; i < kMaxLevel; ++i)
             s.plan.carve_variant[i] = variants[i];
         const HullPlan& p = s.plan;
+        s.unfinished = true;
         if (attempt == 0)
         {
             if (ev)
@@ -789,7 +822,7 @@ void run_hull_once(th_context* ctx,
         else
             enqueue_core(ctx, s, st, ev, carve_ms != nullptr);
         TH_CUDA(cudaStreamSynchronize(st));
-        s.dirty = true;
+        s.unfinished = false;
         const int64_t ovf = s.host->overflow;
         // A level wider than the skip-mask scratch only loses view skipping
         // for its excess parents (results are unchanged): keep the result and
@@ -798,12 +831,12 @@ void run_hull_once(th_context* ctx,
             s.parent_cap *= 4;
         if ((ovf & ~int64_t{ kOverflowParents }) == 0)
             break;
-        launch_cleanup(p, st);
-        s.dirty = false;
         if (ovf & kOverflowNodes)
             s.node_cap *= 4;
         if (ovf & kOverflowCorners)
             s.corner_cap *= 4;
+        if (ovf & kOverflowWords)
+            s.word_cap *= 4;
         if (attempt == 7)
         {
             const DevCounters& c = *s.host;
@@ -914,12 +947,8 @@ void run_batch(th_context* ctx, const th_hull_args* args, int32_t n, cudaStream_
     for (int32_t r = 0; r < n; ++r)
     {
         HullSlot& s = ctx->batch[r];
-        if (s.dirty)
-        {
+        if (s.done)
             TH_CUDA(cudaStreamWaitEvent(st, s.done, 0));
-            launch_cleanup(s.plan, st);
-            s.dirty = false;
-        }
         s.has_result = false;
     }
     for (int attempt = 0; attempt < 8; ++attempt)
@@ -940,7 +969,8 @@ void run_batch(th_context* ctx, const th_hull_args* args, int32_t n, cudaStream_
             const th_hull_args* a = &args[r];
             HullSlot& s = ctx->batch[r];
             prepare(s, a, st, ctx->field_ones, ctx->field_masks, true);
-            launch_zero(s.plan.ctr, sizeof(DevCounters), st);
+            s.unfinished = true;
+            launch_zero(s.plan.ctr, counter_bytes(s.plan.R), st);
             const HullPlan& p = s.plan;
             BatchReq& q = bs.host_reqs[r];
             q = BatchReq{};
@@ -1058,20 +1088,20 @@ void run_batch(th_context* ctx, const th_hull_args* args, int32_t n, cudaStream_
         for (int32_t r = 0; r < n; ++r)
         {
             HullSlot& s = ctx->batch[r];
-            s.dirty = true;
+            s.unfinished = false;
             if (s.host->overflow & kOverflowCorners)
             {
                 s.corner_cap *= 4;
                 retry = true;
             }
+            if (s.host->overflow & kOverflowWords)
+            {
+                s.word_cap *= 4;
+                retry = true;
+            }
         }
         if (!retry)
             break;
-        for (int32_t r = 0; r < n; ++r)
-        {
-            launch_cleanup(ctx->batch[r].plan, st);
-            ctx->batch[r].dirty = false;
-        }
         if (attempt == 7)
             throw ArgError{ TH_ERR_OUT_OF_MEMORY, "batch pools could not be grown enough" };
     }
@@ -1625,7 +1655,7 @@ th_status th_visual_hull_export(th_context* ctx, float* verts, int64_t* faces, v
         {
             if (!verts || !faces)
                 throw ArgError{ TH_ERR_INVALID_ARGUMENT, "verts or faces pointer is NULL" };
-            launch_export(s.plan, verts, faces, st);
+            launch_export(s.plan, s.host->words, verts, faces, st);
         }
         TH_CUDA(cudaEventRecord(s.done, st));
     });
@@ -1835,7 +1865,7 @@ th_status th_visual_hull_batch_export(th_context* ctx, int32_t index, float* ver
         {
             if (!verts || !faces)
                 throw ArgError{ TH_ERR_INVALID_ARGUMENT, "verts or faces pointer is NULL" };
-            launch_export(s.plan, verts, faces, st);
+            launch_export(s.plan, s.host->words, verts, faces, st);
         }
         TH_CUDA(cudaEventRecord(s.done, st));
     });
@@ -1870,7 +1900,7 @@ th_status th_visual_hull_batch_export_all(th_context* ctx, int32_t n, float* con
         {
             HullSlot& s = ctx->batch[i];
             if (s.info.num_faces > 0)
-                launch_export(s.plan, verts[i], faces[i], ns > 1 ? bs.streams[i % ns] : st);
+                launch_export(s.plan, s.host->words, verts[i], faces[i], ns > 1 ? bs.streams[i % ns] : st);
         }
         if (ns > 1)
         {

@@ -424,7 +424,9 @@ int grid_for(int64_t work_items, int threads)
 
 void launch_hull_init(const HullPlan& p, cudaStream_t s)
 {
-    launch_zero(p.ctr, sizeof(DevCounters), s);
+    // the counters and the row groups' corner counts behind them
+    launch_zero(p.ctr, static_cast<size_t>(reinterpret_cast<unsigned char*>(p.coarse) - reinterpret_cast<unsigned char*>(p.ctr)) +
+                               sizeof(uint2) * static_cast<size_t>(p.R * p.R / 256 + 2), s);
     hull_init_kernel<<<1, 32, 0, s>>>(p);
     TH_LAUNCH_CHECK();
 }

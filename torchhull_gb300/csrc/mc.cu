@@ -27,6 +27,7 @@
 // volumes with D == W (all of its tests) that mixing is invisible and the
 // results here are identical.
 
+#include <cstring>
 #include <cuda_fp16.h>
 
 #include "mc_tables.h"
@@ -124,19 +125,29 @@ struct VolumeWords
     {
         return p.nwords;
     }
+    __device__ uint32_t word(uint32_t i) const
+    {
+        return i;
+    }
     __device__ uint32_t sign(uint32_t k) const
     {
-        return p.sign[k];
+        return __ldg(p.sign + k);
+    }
+    // Word k's place: w in its row, y and z.
+    __device__ void place(uint32_t k, uint32_t& w, uint32_t& y, uint32_t& z) const
+    {
+        const uint32_t row = fast_div(p.div_wr, k);
+        w = k - row * p.wr;
+        z = fast_div(p.div_h, row);
+        y = row - z * p.div_h.d;
     }
     __device__ WordRows rows(uint32_t k) const
     {
+        uint32_t w, y, z;
+        place(k, w, y, z);
         WordRows r;
-        const uint32_t row = fast_div(p.div_wr, k), w = k - row * p.wr;
-        r.z = fast_div(p.div_h, row);
-        r.y = row - r.z * p.div_h.d;
-        r.x0 = static_cast<int64_t>(w) * 32;
         r.next = w + 1 < p.wr;
-        const bool up = r.y + 1 < p.div_h.d, back = static_cast<int64_t>(r.z) + 1 < p.D;
+        const bool up = y + 1 < p.div_h.d, back = static_cast<int64_t>(z) + 1 < p.D;
         const uint32_t plane = p.wr * p.div_h.d;
         r.idx[0] = k;
         r.idx[1] = up ? k + p.wr : kNoWord;
@@ -149,10 +160,14 @@ struct VolumeWords
 template <int DT>
 struct DenseWords : VolumeWords
 {
-    // every edge inside the volume belongs to some cell
-    __device__ EdgeBits edges(uint32_t, const WordRows& r, const uint32_t s[4], const uint32_t sh[4], uint32_t& cells) const
+    __device__ bool empty(uint32_t) const
     {
-        const int64_t points = p.W - r.x0; // at least 1
+        return false;
+    }
+    // every edge inside the volume belongs to some cell
+    __device__ EdgeBits edges(uint32_t k, const WordRows& r, const uint32_t s[4], const uint32_t sh[4], uint32_t& cells) const
+    {
+        const int64_t points = p.W - static_cast<int64_t>(k - fast_div(p.div_wr, k) * p.wr) * 32; // at least 1
         const uint32_t in = points >= 32 ? 0xffffffffu : (1u << points) - 1u;
         const uint32_t start = points > 32 ? 0xffffffffu : (1u << (points - 1)) - 1u; // with a right neighbour
         cells = r.idx[3] != kNoWord ? start : 0u;
@@ -161,11 +176,12 @@ struct DenseWords : VolumeWords
     }
     __device__ int64_t point(uint32_t k, int b, int64_t& x, int64_t& y, int64_t& z) const
     {
-        const uint32_t row = fast_div(p.div_wr, k), zz = fast_div(p.div_h, row);
-        x = static_cast<int64_t>(k - row * p.wr) * 32 + b;
-        y = row - zz * p.div_h.d;
+        uint32_t w, yy, zz;
+        place(k, w, yy, zz);
+        x = static_cast<int64_t>(w) * 32 + b;
+        y = yy;
         z = zz;
-        return static_cast<int64_t>(row) * p.W + x;
+        return (y + z * p.H) * p.W + x;
     }
     __device__ void vertex(uint32_t k, int b, int axis, float out[3]) const
     {
@@ -176,7 +192,8 @@ struct DenseWords : VolumeWords
     }
     __device__ void values_at(const WordRows& r, int b, unsigned long long* corner) const
     {
-        const int64_t q = (r.y + static_cast<int64_t>(r.z) * p.H) * p.W + r.x0 + b;
+        int64_t x, y, z;
+        const int64_t q = point(r.idx[0], b, x, y, z);
 #pragma unroll
         for (int i = 0; i < 8; ++i)
             corner[i] = static_cast<unsigned long long>(q + (i & 1) + (i >> 1 & 1) * p.W + (i >> 2) * (p.W * p.H));
@@ -190,44 +207,73 @@ struct DenseWords : VolumeWords
     }
 };
 
-// Sign words of a dense volume: the only pass over its values.  A warp takes
-// kSignWords consecutive words at a time, a point per lane, all loads issued
-// before the first ballot.
-constexpr int kSignWords = 8;
+// Sign words of a dense volume: the only pass over its values.  VEC (rows and
+// volume on 16-byte boundaries): a lane loads 16 bytes, the 32 / V lanes of a
+// word OR their bits by shuffles, a warp makes V words per load and issues
+// kSignLoads of them first.  Else a point per lane and a ballot per word.  The
+// index arithmetic per word bounds the scalar form: 400^3 float32 117 us
+// against 47 us for the vector form (256 MB: 38 us at the copy rate).
+constexpr int kSignLoads = 8;
 
-template <int DT>
+template <int DT, bool VEC>
 __global__ void __launch_bounds__(256) mc_sign_kernel(McPlan p)
 {
-    const int lane = threadIdx.x & 31;
-    const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-    const int64_t groups = (p.nwords + kSignWords - 1) / kSignWords;
     using T = typename Elem<DT>::T;
+    constexpr int V = VEC ? 16 / static_cast<int>(sizeof(T)) : 1; // points per lane = words per load
+    constexpr int kLanes = 32 / V;                                // lanes per word
+    const int lane = threadIdx.x & 31, sub = lane % kLanes;
+    const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+    constexpr int kWords = kSignLoads * V;
+    const int64_t groups = (p.nwords + kWords - 1) / kWords;
     const T* volume = static_cast<const T*>(p.volume);
     for (int64_t g = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; g < groups; g += nwarps)
     {
-        T v[kSignWords];
+        T v[kSignLoads][V];
         uint32_t in = 0;
 #pragma unroll
-        for (int i = 0; i < kSignWords; ++i)
+        for (int i = 0; i < kSignLoads; ++i)
         {
-            const int64_t kk = g * kSignWords + i;
+            const int64_t kk = g * kWords + i * V + lane / kLanes;
             const uint32_t k = static_cast<uint32_t>(kk < p.nwords ? kk : p.nwords - 1);
             const uint32_t row = fast_div(p.div_wr, k);
-            const int64_t x = static_cast<int64_t>(k - row * p.wr) * 32 + lane;
-            const bool ok = x < p.W;
-            in |= ok ? 1u << i : 0u;
-            v[i] = ok ? volume[static_cast<int64_t>(row) * p.W + x] : T(0);
+            const int64_t x = static_cast<int64_t>(k - row * p.wr) * 32 + sub * V;
+            const T* src = volume + static_cast<int64_t>(row) * p.W + x;
+            // VEC: W is a multiple of V, so the V points are in the row or none is
+            if (x < p.W)
+            {
+                in |= 1u << i;
+                if constexpr (VEC)
+                {
+                    const uint4 w = __ldcs(reinterpret_cast<const uint4*>(src));
+                    memcpy(v[i], &w, sizeof(w));
+                }
+                else
+                    v[i][0] = *src;
+            }
         }
-        uint32_t mine = 0;
 #pragma unroll
-        for (int i = 0; i < kSignWords; ++i)
+        for (int i = 0; i < kSignLoads; ++i)
         {
-            const uint32_t word = __ballot_sync(0xffffffffu, ((in >> i) & 1u) && below<DT>(&v[i], 0, p.iso));
-            if (lane == i)
-                mine = word;
+            uint32_t word = 0;
+            if ((in >> i) & 1u)
+            {
+#pragma unroll
+                for (int j = 0; j < V; ++j)
+                    word |= below<DT>(&v[i][j], 0, p.iso) ? 1u << j : 0u;
+            }
+            if constexpr (VEC)
+            {
+                word <<= sub * V;
+#pragma unroll
+                for (int d = kLanes / 2; d > 0; d >>= 1)
+                    word |= __shfl_xor_sync(0xffffffffu, word, d);
+            }
+            else
+                word = __ballot_sync(0xffffffffu, word != 0u);
+            const int64_t k = g * kWords + i * V + lane / kLanes;
+            if (sub == 0 && k < p.nwords)
+                p.sign[k] = word;
         }
-        if (lane < kSignWords && g * kSignWords + lane < p.nwords)
-            p.sign[g * kSignWords + lane] = mine;
     }
 }
 
@@ -368,22 +414,28 @@ __global__ void __launch_bounds__(256) mc_sparse_classify_kernel(McPlan p)
 template <int DT>
 struct SparseWords : VolumeWords
 {
+    __device__ bool empty(uint32_t k) const
+    {
+        return __ldg(p.present + k) == 0;
+    }
     __device__ EdgeBits edges(uint32_t k, const WordRows& r, const uint32_t s[4], const uint32_t sh[4], uint32_t& cells) const
     {
-        cells = 0;
-        if (p.present[k] == 0)
-            return EdgeBits{ 0u, 0u, 0u };
+        uint32_t w, y, z;
+        place(k, w, y, z);
         const uint32_t plane = p.wr * p.div_h.d;
+        const bool low[2] = { y > 0, z > 0 }, high[2] = { y + 1 < p.div_h.d, static_cast<int64_t>(z) + 1 < p.D };
         return masked_edges(
                 [&](int dy, int dz) {
-                    const int64_t y = static_cast<int64_t>(r.y) + dy, z = static_cast<int64_t>(r.z) + dz;
-                    return y >= 0 && y < p.H && z >= 0 && z < p.D ? k + dy * p.wr + dz * plane : kNoWord;
+                    if ((dy < 0 && !low[0]) || (dy > 0 && !high[0]) || (dz < 0 && !low[1]) || (dz > 0 && !high[1]))
+                        return make_uint2(0u, 0u);
+                    const uint32_t* bits = p.present + (k + dy * p.wr + dz * plane);
+                    return word_runs(w > 0 ? __ldg(bits - 1) : 0u, __ldg(bits), r.next ? __ldg(bits + 1) : 0u);
                 },
-                [&](uint32_t idx) { return p.present[idx]; }, r.x0 > 0, r.next, s, sh, cells);
+                s, sh, cells);
     }
     __device__ uint32_t entry(uint32_t k, int b) const
     {
-        return p.rank[k] + static_cast<uint32_t>(__popc(p.present[k] & ((1u << b) - 1u)));
+        return __ldg(p.rank + k) + static_cast<uint32_t>(__popc(__ldg(p.present + k) & ((1u << b) - 1u)));
     }
     __device__ void vertex(uint32_t k, int b, int axis, float out[3]) const
     {
@@ -391,7 +443,9 @@ struct SparseWords : VolumeWords
         const uint32_t e1 = entry(k, b);
         // the edge's other end is an entry: a complete cell holds both
         const uint32_t e2 = axis == 0 ? e1 + 1 : entry(r.idx[axis], b);
-        mc_vertex(p, r.x0 + b, r.y, r.z, axis, load_f32<DT>(p.values, e1), load_f32<DT>(p.values, e2), out);
+        uint32_t w, y, z;
+        place(k, w, y, z);
+        mc_vertex(p, static_cast<int64_t>(w) * 32 + b, y, z, axis, load_f32<DT>(p.values, e1), load_f32<DT>(p.values, e2), out);
     }
     __device__ void values_at(const WordRows& r, int b, unsigned long long* corner) const
     {
@@ -405,9 +459,10 @@ struct SparseWords : VolumeWords
     }
     __device__ void soup_vertex(uint32_t k, int b, int lo, int axis, unsigned long long h1, unsigned long long h2, float out[3]) const
     {
-        const WordRows r = rows(k);
-        mc_vertex(p, r.x0 + b + (lo & 1), static_cast<int64_t>(r.y) + (lo >> 1 & 1), static_cast<int64_t>(r.z) + (lo >> 2 & 1),
-                  axis, load_f32<DT>(p.values, static_cast<int64_t>(h1)), load_f32<DT>(p.values, static_cast<int64_t>(h2)), out);
+        uint32_t w, y, z;
+        place(k, w, y, z);
+        mc_vertex(p, static_cast<int64_t>(w) * 32 + b + (lo & 1), static_cast<int64_t>(y) + (lo >> 1 & 1),
+                  static_cast<int64_t>(z) + (lo >> 2 & 1), axis, load_f32<DT>(p.values, static_cast<int64_t>(h1)), load_f32<DT>(p.values, static_cast<int64_t>(h2)), out);
     }
 };
 
@@ -569,18 +624,26 @@ template <class Src>
 void words_emit(const Src& src, float* verts, int64_t* faces, cudaStream_t s)
 {
     const McPlan& p = src.p;
-    const int grid = grid_for(p.nwords, 32 * kWordExportWarps);
+    const int grid = words_export_grid(p.nwords);
     if (p.unique)
-        words_export_kernel<Src, true, false><<<grid, 32 * kWordExportWarps, 0, s>>>(src, p.mesh, verts, faces);
+    {
+        words_verts_kernel<Src><<<grid, 32 * kWordExportWarps, 0, s>>>(src, p.mesh, verts);
+        TH_LAUNCH_CHECK();
+        words_faces_kernel<Src, true, false><<<grid, 32 * kWordExportWarps, 0, s>>>(src, p.mesh, verts, faces);
+    }
     else
-        words_export_kernel<Src, false, false><<<grid, 32 * kWordExportWarps, 0, s>>>(src, p.mesh, verts, faces);
+        words_faces_kernel<Src, false, false><<<grid, 32 * kWordExportWarps, 0, s>>>(src, p.mesh, verts, faces);
     TH_LAUNCH_CHECK();
 }
 
 template <int DT>
 void dense_count(const McPlan& p, cudaStream_t s)
 {
-    mc_sign_kernel<DT><<<grid_for(p.nwords * 32 / kSignWords, 256), 256, 0, s>>>(p);
+    constexpr int V = 16 / static_cast<int>(sizeof(typename Elem<DT>::T));
+    if (reinterpret_cast<uintptr_t>(p.volume) % 16 == 0 && p.W % V == 0)
+        mc_sign_kernel<DT, true><<<grid_for(p.nwords * 32 / (kSignLoads * V) + 32, 256), 256, 0, s>>>(p);
+    else
+        mc_sign_kernel<DT, false><<<grid_for(p.nwords * 32 / kSignLoads + 32, 256), 256, 0, s>>>(p);
     TH_LAUNCH_CHECK();
     words_count(DenseWords<DT>{ { p } }, s);
 }

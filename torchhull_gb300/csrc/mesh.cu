@@ -3,28 +3,31 @@
 // Corner set.  The reference turns the leaf cells into 8 corner ids each, then
 // radix-sorts and uniques them (visual_hull_cuda.cu:770-825).  Here each leaf
 // sets its corners in a bitmap over the (2^L+1)^3 grid, laid out row by row
-// (x fastest, one row = WR 64-bit words) so that scanning the set bits in
-// memory order yields the ids already ascending and unique.  A second bitmap
-// flags the rows that hold any bit, so only those rows are scanned and later
-// cleared.  The scan also stores, per word, the rank of its first bit, which
-// turns "index of corner v in the sorted list" into one word load, one rank
-// load and a popcount: this replaces the hash map the reference builds for its
-// marching cubes (marching_cubes_cuda.cu:66-70, :133-144).
+// (x fastest, one row = WR 64-bit words) so that the set bits in memory order
+// are the ids already ascending and unique.  A second bitmap flags the rows
+// that hold any bit.  rows_kernel lists those rows and counts their corners,
+// corners_kernel copies their words into a compact array (32 points a word),
+// with the rank of each word's first corner, and writes the sorted list; it
+// clears the bitmaps behind it.  "Index of corner v in the sorted list" is one
+// word load, one rank load and a popcount: this replaces the hash map the
+// reference builds for its marching cubes (marching_cubes_cuda.cu:66-70,
+// :133-144).
 //
-// Hull field.  One thread per corner multiplies the bilinear mask samples of
+// Hull field.  A corner's value is the product of the bilinear mask samples of
 // all views in ascending view order, the order in which the reference's
-// per-view launches (visual_hull_cuda.cu:827-888) multiply them.
+// per-view launches (visual_hull_cuda.cu:827-888) multiply them.  The field
+// also sets the corner's bit in the sign words when its value is below 0.5.
 //
 // Marching cubes.  A corner g is a cell when all 8 cube corners are present
-// (marching_cubes_cuda.cu:180-223).  Its code selects triangles from the
-// table; every edge a triangle uses is marked on the edge's lower corner (3
-// bits per corner, one per axis).  A scan over corners then numbers the marked
-// edges in (corner, axis) order, which is exactly the reference's vertex order
-// after torch::unique_dim over the edge ids (ravel(p1) << 3 | 1 << axis),
-// (:99-112, :674-693), without a sort.  Faces are emitted per cell in
-// ascending corner order and table order, as the reference's soup is.
+// (marching_cubes_cuda.cu:180-223).  Cells, codes and vertex edges come from
+// the presence and sign words by bit operations (th_words.cuh); the vertices
+// are numbered in (corner, axis) order, which is exactly the reference's
+// vertex order after torch::unique_dim over the edge ids (ravel(p1) << 3 |
+// 1 << axis), (:99-112, :674-693), without a sort.  Faces are emitted per cell
+// in ascending corner order and table order, as the reference's soup is.
 
-#include "mc_tables.h"
+#include <algorithm>
+
 #include "th_hull.cuh"
 #include "th_internal.h"
 
@@ -33,50 +36,6 @@ namespace th
 
 namespace
 {
-
-__device__ const uint8_t g_mc_count[256] = TH_MC_TRI_COUNT_INIT;
-__device__ const uint8_t g_mc_edges[256][15] = TH_MC_TRI_EDGES_INIT;
-
-struct TableCache
-{
-    uint8_t count[256];
-    uint8_t edges[256][16];
-};
-
-__device__ __forceinline__ void load_tables(TableCache& t)
-{
-    for (int i = threadIdx.x; i < 256; i += blockDim.x)
-    {
-        t.count[i] = g_mc_count[i];
-#pragma unroll
-        for (int j = 0; j < 15; ++j)
-            t.edges[i][j] = g_mc_edges[i][j];
-    }
-    __syncthreads();
-}
-
-// Rank of grid point (x,y,z) among the set corners, or false if not set.
-__device__ __forceinline__ bool corner_rank(const HullPlan& p, int64_t x, int64_t y, int64_t z, uint32_t& rank)
-{
-    const int64_t row = y + z * p.R;
-    const int64_t w = row * p.WR + (x >> 6);
-    const uint64_t word = p.bitmap[w];
-    const uint64_t bit = 1ull << (x & 63);
-    if (!(word & bit))
-        return false;
-    rank = p.word_rank[w] + static_cast<uint32_t>(__popcll(word & (bit - 1)));
-    return true;
-}
-
-// Rank of a corner known to be set: the bitmap word and its rank word are
-// loaded together (no check of the bit in between).
-__device__ __forceinline__ uint32_t rank_of(const HullPlan& p, int64_t x, int64_t y, int64_t z)
-{
-    const int64_t w = (y + z * p.R) * p.WR + (x >> 6);
-    const uint64_t word = p.bitmap[w];
-    const uint32_t base = p.word_rank[w];
-    return base + static_cast<uint32_t>(__popcll(word & ((1ull << (x & 63)) - 1ull)));
-}
 
 __global__ void __launch_bounds__(256) mark_corners_kernel(HullPlan p)
 {
@@ -110,161 +69,242 @@ __global__ void __launch_bounds__(256) mark_corners_kernel(HullPlan p)
     }
 }
 
-struct RowCount
+// Sum of v over the block, to every thread.
+__device__ __forceinline__ unsigned long long block_sum(unsigned long long v)
 {
-    const uint32_t* rowbits;
-    __device__ unsigned long long operator()(int64_t i) const
-    {
-        return static_cast<unsigned long long>(__popc(rowbits[i]));
-    }
-};
-
-struct RowEmit
-{
-    const uint32_t* rowbits;
-    uint32_t* rows;
-    __device__ void operator()(int64_t i, unsigned long long off, unsigned long long cnt) const
-    {
-        uint32_t w = rowbits[i];
-        while (w)
-        {
-            const int bit = __ffs(w) - 1;
-            rows[off++] = static_cast<uint32_t>(i * 32 + bit);
-            w &= w - 1;
-        }
-    }
-};
-
-struct RowEpilogue
-{
-    DevCounters* ctr;
-    __device__ void operator()(unsigned long long total) const
-    {
-        ctr->rows = static_cast<int64_t>(total);
-    }
-};
-
-// One scan item per bitmap word of the touched rows (item k: word k % WR of
-// row rows[k / WR]), so that a thread emits the corners of a few words, not
-// of several whole rows.
-struct CornerCount
-{
-    HullPlan p;
-    __device__ unsigned long long operator()(int64_t k) const
-    {
-        const uint32_t wr = static_cast<uint32_t>(p.WR), kk = static_cast<uint32_t>(k);
-        const int64_t w = static_cast<int64_t>(p.rows[kk / wr]) * p.WR + (kk % wr);
-        return static_cast<unsigned long long>(__popcll(p.bitmap[w]));
-    }
-};
-
-
-// Position of the set bit of the 64-bit word w with j set bits below it.
-__device__ __forceinline__ int nth_set_bit64(uint64_t w, int j)
-{
-    const uint32_t lo = static_cast<uint32_t>(w);
-    const int c = __popc(lo);
-    return j < c ? nth_set_bit(lo, j) : 32 + nth_set_bit(static_cast<uint32_t>(w >> 32), j - c);
+    unsigned long long total;
+    block_exclusive_scan(v, &total);
+    return total;
 }
 
-// Pass 2 of the corner scan (the counts come from CornerCount's tile sums):
-// a block owns one scan tile of kScanTile words, a warp 8 chunks of 32
-// consecutive words.  Per chunk the warp numbers the words' corners by a
-// warp scan and writes them with all lanes: corner k of the chunk belongs to
-// the word whose offset is the last one <= k, so the stores are coalesced.
-// Also stores each word's rank (word_rank).
-__global__ void __launch_bounds__(kScanThreads) corner_emit_kernel(HullPlan p, const unsigned long long* __restrict__ tile_offsets)
+// Touched rows, their slots and their corner counts.  A block owns
+// kRowBlock words of row flags; the rows before it are counted from the flags
+// themselves (a few thousand words at the usual levels, read 16 bytes at a
+// time), so no pass or wait comes in between.  Headline scene (32 x 1024^2,
+// level 9, 13 M corners) on GB300: 10 us, where two scan passes over the flags
+// took 40 and a pass for the corner counts 14.
+constexpr int kRowBlock = 32;
+
+__global__ void __launch_bounds__(256) rows_kernel(HullPlan p)
 {
-    static_assert(kScanThreads == 256 && kScanItems == 8, "one warp chunk per 32 items");
-    __shared__ unsigned long long warp_totals[kScanThreads / 32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t n = p.ctr->rows * p.WR;
-    const int64_t ntiles = (n + kScanTile - 1) / kScanTile;
-    const uint32_t wr = static_cast<uint32_t>(p.WR), R = static_cast<uint32_t>(p.R);
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
+    __shared__ uint32_t base[kRowBlock];
+    __shared__ unsigned long long s_before;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t nwords = (p.R * p.R + 31) / 32;
+    const int64_t first = static_cast<int64_t>(blockIdx.x) * kRowBlock;
+    unsigned long long before = 0;
+    // first is a multiple of 4 and the buffer is 256-byte aligned
+    for (int64_t i = tid; i < first / 4; i += 256)
     {
-        const int64_t first = tile * kScanTile + static_cast<int64_t>(w) * 256;
-        uint64_t words[8];
-        unsigned long long wsum = 0;
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
+        const uint4 w = reinterpret_cast<const uint4*>(p.rowbits)[i];
+        before += __popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w);
+    }
+    before = block_sum(before);
+    if (warp == 0)
+    {
+        const uint32_t w = first + lane < nwords ? p.rowbits[first + lane] : 0u;
+        const uint32_t incl = warp_inclusive_scan(static_cast<uint32_t>(__popc(w)));
+        base[lane] = incl - __popc(w);
+        if (lane == 31)
+            s_before = before + incl;
+    }
+    __syncthreads();
+    if (tid == 0 && first + kRowBlock >= nwords)
+    {
+        const int64_t rows = static_cast<int64_t>(s_before);
+        p.ctr->rows = rows;
+        if (rows * p.wr > p.word_cap)
+            p.ctr->overflow |= kOverflowWords;
+    }
+    for (int i = warp; i < kRowBlock; i += 8)
+    {
+        const uint32_t w = first + i < nwords ? p.rowbits[first + i] : 0u;
+        if (w == 0)
+            continue;
+        const bool on = (w >> lane) & 1u;
+        const uint32_t slot = static_cast<uint32_t>(before) + base[i] + __popc(w & ((1u << lane) - 1u));
+        uint32_t cnt = 0, used = 0;
+        if (on)
         {
-            const int64_t k = first + c * 32 + lane;
-            words[c] = 0;
-            if (k < n)
+            const int64_t row = (first + i) * 32 + lane;
+            const uint2* bits = reinterpret_cast<const uint2*>(p.bitmap + row * p.WR);
+#pragma unroll 4
+            for (int64_t j = 0; j < p.WR; ++j)
             {
-                const uint32_t kk = static_cast<uint32_t>(k);
-                words[c] = p.bitmap[static_cast<int64_t>(p.rows[kk / wr]) * p.WR + kk % wr];
+                const uint2 b = bits[j];
+                cnt += __popc(b.x) + __popc(b.y);
+                used += (b.x != 0 ? 1u : 0u) + (b.y != 0 ? 1u : 0u);
             }
-            wsum += __popcll(words[c]);
+            p.rows[slot] = static_cast<uint32_t>(row);
+            p.row_slot[row] = slot;
+            p.row_cnt[slot] = make_uint2(cnt, used);
         }
-        // this warp's corners come after those of the tile's earlier warps
-        unsigned long long wtot = wsum;
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1)
-            wtot += __shfl_xor_sync(0xffffffffu, wtot, d);
+        // the slots of a word lie in at most two groups of 256
+        const uint32_t g0 = __shfl_sync(0xffffffffu, slot, __ffs(w) - 1) >> 8;
+        const bool second = (slot >> 8) != g0;
+        const uint32_t c0 = __reduce_add_sync(0xffffffffu, second ? 0u : cnt), c1 = __reduce_add_sync(0xffffffffu, second ? cnt : 0u);
+        const uint32_t u0 = __reduce_add_sync(0xffffffffu, second ? 0u : used), u1 = __reduce_add_sync(0xffffffffu, second ? used : 0u);
         if (lane == 0)
-            warp_totals[w] = wtot;
-        __syncthreads();
-        unsigned long long running = tile_offsets[tile];
-        for (int v = 0; v < w; ++v)
-            running += warp_totals[v];
-        __syncthreads();
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
         {
-            const int64_t k = first + c * 32 + lane;
-            const int cnt = __popcll(words[c]);
-            const int incl = warp_inclusive_scan(cnt);
-            const int excl = incl - cnt;
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
-            uint32_t row = 0, wi = 0;
-            if (k < n)
+            atomicAdd(&p.coarse[g0].x, c0);
+            atomicAdd(&p.coarse[g0].y, u0);
+            if (c1)
             {
-                const uint32_t kk = static_cast<uint32_t>(k);
-                row = p.rows[kk / wr];
-                wi = kk % wr;
-                p.word_rank[static_cast<int64_t>(row) * p.WR + wi] = static_cast<uint32_t>(running + excl);
+                atomicAdd(&p.coarse[g0 + 1].x, c1);
+                atomicAdd(&p.coarse[g0 + 1].y, u1);
             }
-            for (int k0 = 0; k0 < total; k0 += 32)
+        }
+    }
+}
+
+// The sorted corner list and the rows' words.  A block takes a contiguous
+// range of slots, so what comes before it is summed once, 32 rows at a time; a
+// warp takes as many rows as its lanes have 64-bit words for (three at level
+// 9): presence, runs and ranks, the list of words with corners, then per word
+// a lane per point.  The words of the bitmap and the row flags are cleared
+// behind it.  Issue-bound: headline scene 151 -> 119 us (a warp searched the
+// word of every corner before, and the bitmap was cleared by another pass).
+__global__ void __launch_bounds__(256) corners_kernel(HullPlan p)
+{
+    __shared__ uint2 before[33];  // corners and words of the group's rows before a row
+    __shared__ uint32_t row_s[32], yz_s[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t rows = p.ctr->rows;
+    const uint32_t wr = p.wr, R = static_cast<uint32_t>(p.R);
+    const int WR = static_cast<int>(p.WR);
+    const int64_t nflags = (p.R * p.R + 31) / 32;
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + tid; i < nflags; i += static_cast<int64_t>(gridDim.x) * 256)
+        p.rowbits[i] = 0;
+    const int64_t groups = (rows + 31) / 32;
+    const int64_t per = (groups + gridDim.x - 1) / gridDim.x;
+    const int64_t s0 = per * blockIdx.x * 32;
+    const int64_t s1 = s0 + per * 32 < rows ? s0 + per * 32 : rows;
+    if (s0 >= rows)
+        return;
+    // corners below 2^31, words below 2^32: summed packed
+    unsigned long long sum = 0;
+    auto add = [&](uint2 c) { sum += (static_cast<unsigned long long>(c.y) << 32) | c.x; };
+    for (int64_t i = tid; i < s0 / 256; i += 256)
+        add(p.coarse[i]);
+    for (int64_t i = (s0 & ~int64_t{ 255 }) + tid; i < s0; i += 256)
+        add(p.row_cnt[i]);
+    sum = block_sum(sum);
+    uint32_t corners = static_cast<uint32_t>(sum), words = static_cast<uint32_t>(sum >> 32);
+    // rows per warp and step
+    const int G = WR <= 32 ? 32 / WR : 1;
+    const int sub = WR <= 32 ? lane / WR : 0, first = WR <= 32 ? sub * WR : 0;
+    for (int64_t g = s0; g < s1; g += 32)
+    {
+        const int nrows = static_cast<int>(s1 - g < 32 ? s1 - g : 32);
+        __syncthreads();
+        if (warp == 0)
+        {
+            const uint2 c = lane < nrows ? p.row_cnt[g + lane] : make_uint2(0u, 0u);
+            const uint32_t cx = warp_inclusive_scan(c.x), cy = warp_inclusive_scan(c.y);
+            before[lane + 1] = make_uint2(cx, cy);
+            if (lane == 0)
+                before[0] = make_uint2(0u, 0u);
+        }
+        // the rows around each row: 3 * (dy + 1) + dz + 1
+        for (int i = tid; i < nrows * 9; i += 256)
+        {
+            const int r = i / 9, q = i - 9 * r, dy = q / 3 - 1, dz = q - 3 * (q / 3) - 1;
+            const uint32_t row = p.rows[g + r];
+            const uint32_t z = fast_div(p.div_r, row), y = row - z * R;
+            uint32_t near = kNoWord;
+            if (q == 4)
             {
-                const int kk = k0 + lane;
-                const int s = item_slot(excl, kk);
-                const int es = __shfl_sync(0xffffffffu, excl, s);
-                const uint64_t ws = __shfl_sync(0xffffffffu, words[c], s);
-                const uint32_t rs = __shfl_sync(0xffffffffu, row, s);
-                const uint32_t wis = __shfl_sync(0xffffffffu, wi, s);
-                if (kk < total)
+                near = y | (z << 16);
+                row_s[r] = row;
+                yz_s[r] = near;
+            }
+            else if ((dy >= 0 || y > 0) && (dy <= 0 || y + 1 < R) && (dz >= 0 || z > 0) && (dz <= 0 || z + 1 < R))
+            {
+                // the slot of a row that is not touched is stale: out of range, or another row's
+                const uint32_t other = row + dy + dz * R, os = p.row_slot[other];
+                if (os < static_cast<uint32_t>(rows) && p.rows[os] == other)
+                    near = os;
+            }
+            p.row_place[g + r].near[q] = near;
+        }
+        __syncthreads();
+        for (int i0 = warp * G; i0 < nrows; i0 += 8 * G)
+        {
+            const int i = i0 + sub;
+            const bool mine = sub < G && i < nrows;
+            const uint32_t row = mine ? row_s[i] : 0u, yz = mine ? yz_s[i] : 0u;
+            uint32_t at = mine ? corners + before[i].x : 0u, wat = mine ? words + before[i].y : 0u;
+            uint32_t last = 0; // the last 32 points of the words before (WR > 32)
+            for (int w0 = 0; w0 < WR; w0 += 32)
+            {
+                const int w = w0 + lane - first;
+                const bool on = mine && w < WR;
+                uint2* src = reinterpret_cast<uint2*>(p.bitmap + static_cast<int64_t>(row) * WR + w);
+                const uint2 b = on ? *src : make_uint2(0u, 0u);
+                uint32_t after = on && lane == 31 && w + 1 < WR ? src[1].x : 0u;
+                uint32_t prev = __shfl_up_sync(0xffffffffu, b.y, 1);
+                const uint32_t down = __shfl_down_sync(0xffffffffu, b.x, 1);
+                if (w == w0)
+                    prev = last;
+                const uint32_t next = lane == 31 ? after : (w + 1 < WR ? down : 0u);
+                last = __shfl_sync(0xffffffffu, b.y, 31);
+                if (b.x | b.y)
+                    *src = make_uint2(0u, 0u);
+                // ranks inside the row: inclusive scans over the warp less what lies before the row's first lane
+                const uint32_t cnt = __popc(b.x) + __popc(b.y), used = (b.x != 0 ? 1u : 0u) + (b.y != 0 ? 1u : 0u);
+                const uint32_t incl = warp_inclusive_scan((used << 16) | cnt); // 64 * 32 corners at most
+                const uint32_t excl = incl - ((used << 16) | cnt);
+                const uint32_t start = __shfl_sync(0xffffffffu, excl, first & 31);
+                const uint32_t rank = at + ((excl - start) & 0xffffu), wrank = wat + ((excl - start) >> 16);
+                const int64_t k = (g + i) * wr + 2 * w;
+                if (on && k + 1 < p.word_cap)
                 {
-                    const int bit = nth_set_bit64(ws, kk - es);
-                    const int64_t out = static_cast<int64_t>(running) + kk;
-                    if (out < p.corner_cap)
-                    {
-                        p.corners[out] = pack_corner(static_cast<int64_t>(wis) * 64 + bit, rs % R, rs / R);
-                        p.emask[out] = 0;
-                    }
+                    *reinterpret_cast<uint2*>(p.present + k) = b;
+                    *reinterpret_cast<uint2*>(p.rank + k) = make_uint2(rank, rank + __popc(b.x));
+                    *reinterpret_cast<uint2*>(p.sign + k) = make_uint2(0u, 0u);
+                    const uint2 lo = word_runs(prev, b.x, b.y), hi = word_runs(b.x, b.y, next);
+                    *reinterpret_cast<uint4*>(p.runs + k) = make_uint4(lo.x, lo.y, hi.x, hi.y);
+                    if (b.x)
+                        p.word_list[wrank] = static_cast<uint32_t>(k);
+                    if (b.y)
+                        p.word_list[wrank + (b.x != 0 ? 1u : 0u)] = static_cast<uint32_t>(k) + 1;
+                }
+                for (uint32_t todo = __ballot_sync(0xffffffffu, cnt != 0); todo; todo &= todo - 1)
+                {
+                    const int j = __ffs(todo) - 1;
+                    const uint32_t bx = __shfl_sync(0xffffffffu, b.x, j), by = __shfl_sync(0xffffffffu, b.y, j);
+                    const uint32_t r = __shfl_sync(0xffffffffu, rank, j), ryz = __shfl_sync(0xffffffffu, yz, j);
+                    const int x = __shfl_sync(0xffffffffu, w, j) * 64 + lane;
+                    const int64_t id = pack_corner(x, ryz & 0xffffu, ryz >> 16);
+                    const uint32_t lt = (1u << lane) - 1u;
+                    const uint32_t o0 = r + __popc(bx & lt), o1 = r + __popc(bx) + __popc(by & lt);
+                    if (((bx >> lane) & 1u) && o0 < p.corner_cap)
+                        p.corners[o0] = id;
+                    if (((by >> lane) & 1u) && o1 < p.corner_cap)
+                        p.corners[o1] = id + 32;
+                }
+                if (WR > 32)
+                {
+                    const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
+                    at += all & 0xffffu;
+                    wat += all >> 16;
                 }
             }
-            running += static_cast<unsigned long long>(total);
         }
+        corners += before[32].x;
+        words += before[32].y;
+    }
+    if (s1 == rows && tid == 0)
+    {
+        const bool over = static_cast<int64_t>(corners) > p.corner_cap;
+        if (over)
+            p.ctr->overflow |= kOverflowCorners;
+        // an overflowing request is run again: nothing after this looks at its corners
+        const bool none = over || (p.ctr->overflow & kOverflowWords);
+        p.ctr->corners = none ? 0 : corners;
+        p.ctr->words = none ? 0 : words;
     }
 }
-
-struct CornerEpilogue
-{
-    DevCounters* ctr;
-    int64_t cap;
-    __device__ void operator()(unsigned long long total) const
-    {
-        int64_t n = static_cast<int64_t>(total);
-        if (n > cap)
-        {
-            ctr->overflow |= kOverflowCorners;
-            n = cap;
-        }
-        ctr->corners = n;
-    }
-};
 
 template <int DT>
 __device__ __forceinline__ float mask_sample(const HullPlan& p, const void* masks, int64_t b, int64_t y, int64_t x, float pad)
@@ -401,6 +441,34 @@ __global__ void __launch_bounds__(256) ones_kernel(HullPlan p)
     }
 }
 
+// Sets the bits of the corners below the isolevel in the sign words.  A warp's
+// corners are neighbours in the list, so most of them share a few words: one
+// atomic per word and warp.
+__device__ __forceinline__ void mark_sign(const HullPlan& p, bool valid, int64_t gx, int64_t gy, int64_t gz, float value)
+{
+    uint32_t k = kNoWord;
+    if (valid)
+    {
+        const uint32_t row = static_cast<uint32_t>(gy) + static_cast<uint32_t>(gz) * static_cast<uint32_t>(p.R);
+        k = __ldg(p.row_slot + row) * p.wr + static_cast<uint32_t>(gx >> 5);
+    }
+    const bool low = valid && value < 0.5f;
+    if (!__any_sync(0xffffffffu, low))
+        return;
+    const uint32_t peers = __match_any_sync(0xffffffffu, k);
+    const uint32_t bits = __reduce_or_sync(peers, low ? 1u << (gx & 31) : 0u);
+    if (bits && static_cast<int>(threadIdx.x & 31) == __ffs(peers) - 1)
+        atomicOr(p.sign + k, bits);
+}
+
+// Adds the block's evaluated (corner, view) pairs to the request's counter.
+__device__ __forceinline__ void count_items(const HullPlan& p, unsigned long long items)
+{
+    const unsigned long long total = block_sum(items);
+    if (threadIdx.x == 0 && total)
+        atomicAdd(&p.ctr->field_items, total);
+}
+
 // accumulate_hull_counts_{full,partial} (visual_hull_cuda.cu:419-520): the
 // views [b0, b1) multiplied into each corner's running product in ascending
 // view order (b0 == 0 starts it at 1).  Views go in chunks of kFieldViews, one
@@ -428,26 +496,36 @@ __global__ void __launch_bounds__(256) field_kernel(HullPlan p, int64_t b0, int6
     const float Hf = small_i2f(static_cast<int32_t>(p.H)), Wf = small_i2f(static_cast<int32_t>(p.W));
     const float cx = p.rq->corner[0], cy = p.rq->corner[1], cz = p.rq->corner[2], length = p.rq->length;
     const void* masks = p.rq->masks;
+    const int lane = threadIdx.x & 31;
+    const bool final = b1 >= p.B;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < n; t += stride)
+    unsigned long long items = 0;
+    for (int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x - lane; t0 < n; t0 += stride)
     {
-        const int64_t idx = p.corners[t];
-        int64_t gx, gy, gz;
-        unpack_corner(idx, gx, gy, gz);
-        // c + v/r * L fused (visual_hull_cuda.cu:444-448); v/r == v * (1/r) exactly
-        // corner coordinates are at most 2^12
-        const float wx = __fmaf_rn(__fmul_rn(small_i2f(static_cast<int32_t>(gx)), inv_rc), length, cx);
-        const float wy = __fmaf_rn(__fmul_rn(small_i2f(static_cast<int32_t>(gy)), inv_rc), length, cy);
-        const float wz = __fmaf_rn(__fmul_rn(small_i2f(static_cast<int32_t>(gz)), inv_rc), length, cz);
-        float value = b0 == 0 ? 1.f : p.values[t];
-        const unsigned nact = __popc(__activemask());
-        if ((threadIdx.x & 31) == __ffs(__activemask()) - 1)
-            atomicAdd(&p.ctr->field_items, static_cast<unsigned long long>(nact) * nv);
+        const int64_t t = t0 + lane;
+        const bool valid = t < n;
+        int64_t gx = 0, gy = 0, gz = 0;
+        float value = 1.f;
+        if (valid)
+        {
+            unpack_corner(p.corners[t], gx, gy, gz);
+            // c + v/r * L fused (visual_hull_cuda.cu:444-448); v/r == v * (1/r) exactly
+            // corner coordinates are at most 2^12
+            const float wx = __fmaf_rn(__fmul_rn(small_i2f(static_cast<int32_t>(gx)), inv_rc), length, cx);
+            const float wy = __fmaf_rn(__fmul_rn(small_i2f(static_cast<int32_t>(gy)), inv_rc), length, cy);
+            const float wz = __fmaf_rn(__fmul_rn(small_i2f(static_cast<int32_t>(gz)), inv_rc), length, cz);
+            if (b0 > 0)
+                value = p.values[t];
+            items += nv;
 #pragma unroll 4
-        for (int v = 0; v < nv; ++v)
-            value = __fmul_rn(value, view_factor<DT, PARTIAL>(p, masks, b0 + v, rows[v], wx, wy, wz, Hf, Wf));
-        p.values[t] = value;
+            for (int v = 0; v < nv; ++v)
+                value = __fmul_rn(value, view_factor<DT, PARTIAL>(p, masks, b0 + v, rows[v], wx, wy, wz, Hf, Wf));
+            p.values[t] = value;
+        }
+        if (final)
+            mark_sign(p, valid, gx, gy, gz, value);
     }
+    count_items(p, items);
 }
 
 // The cell-mask table (HullPlan::cell_masks): every cell of level L-1
@@ -469,29 +547,23 @@ __global__ void __launch_bounds__(256) cell_masks_kernel(HullPlan p, bool set)
 // cells that are no node hold 0).
 __device__ __forceinline__ uint32_t corner_view_mask(const HullPlan& p, int64_t gx, int64_t gy, int64_t gz)
 {
-    const int li = p.level - 1;
-    const int64_t r = int64_t{ 1 } << li;
-    const int64_t x0 = gx >> 1, y0 = gy >> 1, z0 = gz >> 1;
-    const int64_t x1 = (gx - 1) >> 1, y1 = (gy - 1) >> 1, z1 = (gz - 1) >> 1;
-    const bool two_x = x1 != x0 && gx > 0, two_y = y1 != y0 && gy > 0, two_z = z1 != z0 && gz > 0;
-    // up to eight cells, a fixed unrolled pattern of predicated loads (issued together)
+    // the table has at most 2^27 cells
+    const uint32_t li = p.level - 1, r = 1u << li;
+    const uint32_t x0 = static_cast<uint32_t>(gx) >> 1, y0 = static_cast<uint32_t>(gy) >> 1, z0 = static_cast<uint32_t>(gz) >> 1;
+    const bool x_low = !(gx & 1) && gx > 0, y_low = !(gy & 1) && gy > 0, z_low = !(gz & 1) && gz > 0;
+    const bool x_in = x0 < r, y_in = y0 < r, z_in = z0 < r;
+    const uint32_t* c = p.cell_masks + (x0 + (y0 << li) + (z0 << (2 * li)));
+    // up to eight cells, a fixed pattern of predicated loads (issued together)
     uint32_t m = 0;
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
+    for (int q = 0; q < 4; ++q)
     {
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-        {
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-            {
-                const int64_t cx = i ? x1 : x0, cy = j ? y1 : y0, cz = k ? z1 : z0;
-                const bool use = (i == 0 || two_x) && (j == 0 || two_y) && (k == 0 || two_z) && cx < r && cy < r &&
-                                 cz < r;
-                if (use)
-                    m |= __ldg(p.cell_masks + (cx | (cy << li) | (cz << (2 * li))));
-            }
-        }
+        const bool use = ((q & 1) ? y_low : y_in) && ((q >> 1) ? z_low : z_in);
+        const uint32_t* row = c - ((q & 1) ? int64_t{ 1 } << li : 0) - ((q >> 1) ? int64_t{ 1 } << (2 * li) : 0);
+        if (use && x_in)
+            m |= __ldg(row);
+        if (use && x_low)
+            m |= __ldg(row - 1);
     }
     return m;
 }
@@ -508,7 +580,8 @@ template <int DT, bool PARTIAL>
 __global__ void __launch_bounds__(32 * kMaskedWarps) field_masked_kernel(HullPlan p, int64_t b0, int64_t b1)
 {
     __shared__ float4 rows[32][3];
-    __shared__ float fac_all[kMaskedWarps][32][33];
+    // a warp's items: their corner (lane) << 8 | view, then their factors
+    __shared__ float fac_all[kMaskedWarps][32 * 32];
     const int nv = static_cast<int>(b1 - b0);
     for (int i = threadIdx.x; i < 3 * nv; i += blockDim.x)
     {
@@ -517,7 +590,7 @@ __global__ void __launch_bounds__(32 * kMaskedWarps) field_masked_kernel(HullPla
         rows[v][r] = *reinterpret_cast<const float4*>(p.tf + 16 * (b0 + v) + 4 * row);
     }
     __syncthreads();
-    float(*fac)[33] = fac_all[threadIdx.x >> 5];
+    float* fac = fac_all[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int64_t n = p.ctr->corners;
     const float inv_rc = __fdiv_rn(1.f, static_cast<float>(p.R - 1)); // exact: a power of two
@@ -525,6 +598,8 @@ __global__ void __launch_bounds__(32 * kMaskedWarps) field_masked_kernel(HullPla
     const float cx = p.rq->corner[0], cy = p.rq->corner[1], cz = p.rq->corner[2], length = p.rq->length;
     const void* masks = p.rq->masks;
     const uint32_t vb = nv >= 32 ? 0xffffffffu : ((1u << nv) - 1u);
+    const bool final = b1 >= p.B;
+    unsigned long long items = 0; // lane 0's: of the warp
     const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
     for (int64_t base = warp * 32; base < n; base += nwarps * 32)
@@ -532,10 +607,10 @@ __global__ void __launch_bounds__(32 * kMaskedWarps) field_masked_kernel(HullPla
         const int64_t t = base + lane;
         const bool valid = t < n;
         float wx = 0.f, wy = 0.f, wz = 0.f, value = 1.f;
+        int64_t gx = 0, gy = 0, gz = 0;
         uint32_t skip = 0;
         if (valid)
         {
-            int64_t gx, gy, gz;
             unpack_corner(p.corners[t], gx, gy, gz);
             // c + v/r * L fused (visual_hull_cuda.cu:444-448), as in field_kernel
             wx = __fmaf_rn(__fmul_rn(small_i2f(static_cast<int32_t>(gx)), inv_rc), length, cx);
@@ -549,175 +624,172 @@ __global__ void __launch_bounds__(32 * kMaskedWarps) field_masked_kernel(HullPla
         if (!__any_sync(0xffffffffu, skip != 0))
         {
             const unsigned nvalid = __popc(__ballot_sync(0xffffffffu, valid));
-            if (lane == 0)
-                atomicAdd(&p.ctr->field_items, static_cast<unsigned long long>(nvalid) * nv);
+            items += static_cast<unsigned long long>(nvalid) * nv;
             if (valid)
             {
 #pragma unroll 4
                 for (int v = 0; v < nv; ++v)
                     value = __fmul_rn(value, view_factor<DT, PARTIAL>(p, masks, b0 + v, rows[v], wx, wy, wz, Hf, Wf));
-                p.values[t] = value;
             }
-            continue;
         }
-        const uint32_t active = valid ? (vb & ~skip) : 0u;
-        const int count = __popc(active);
-        const int incl = warp_inclusive_scan(count);
-        const int excl = incl - count;
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        if (lane == 0 && total > 0)
-            atomicAdd(&p.ctr->field_items, static_cast<unsigned long long>(total));
-        for (int k0 = 0; k0 < total; k0 += 32)
+        else
         {
-            const int k = k0 + lane;
-            const int s = item_slot(excl, k);
-            const int es = __shfl_sync(0xffffffffu, excl, s);
-            const uint32_t as = __shfl_sync(0xffffffffu, active, s);
-            const float sx = __shfl_sync(0xffffffffu, wx, s);
-            const float sy = __shfl_sync(0xffffffffu, wy, s);
-            const float sz = __shfl_sync(0xffffffffu, wz, s);
-            if (k < total)
+            const uint32_t active = valid ? (vb & ~skip) : 0u;
+            const int count = __popc(active);
+            const int incl = warp_inclusive_scan(count);
+            const int excl = incl - count;
+            const int total = __shfl_sync(0xffffffffu, incl, 31);
+            items += static_cast<unsigned long long>(total);
+            // each lane lists its corner's items, then the items go to the lanes
+            // in turn (finding an item's corner and view by searching the
+            // lanes' offsets and masks cost half as much as its factor)
+            int at = excl;
+            for (uint32_t m = active; m; m &= m - 1)
+                fac[at++] = __int_as_float((lane << 8) | (__ffs(m) - 1));
+            __syncwarp();
+            for (int k0 = 0; k0 < total; k0 += 32)
             {
-                const int j = k - es;
-                const int v = nth_set_bit(as, j);
-                fac[s][j] = view_factor<DT, PARTIAL>(p, masks, b0 + v, rows[v], sx, sy, sz, Hf, Wf);
+                const int k = k0 + lane;
+                const uint32_t item = k < total ? __float_as_uint(fac[k]) : 0u;
+                const int s = static_cast<int>(item >> 8);
+                const float sx = __shfl_sync(0xffffffffu, wx, s);
+                const float sy = __shfl_sync(0xffffffffu, wy, s);
+                const float sz = __shfl_sync(0xffffffffu, wz, s);
+                if (k < total)
+                {
+                    const int v = static_cast<int>(item & 0xffu);
+                    fac[k] = view_factor<DT, PARTIAL>(p, masks, b0 + v, rows[v], sx, sy, sz, Hf, Wf);
+                }
             }
+            __syncwarp();
+            for (int j = 0; j < count; ++j)
+                value = __fmul_rn(value, fac[excl + j]);
+            __syncwarp();
         }
-        __syncwarp();
-        for (int j = 0; j < count; ++j)
-            value = __fmul_rn(value, fac[lane][j]);
-        __syncwarp();
         if (valid)
             p.values[t] = value;
+        if (final)
+            mark_sign(p, valid, gx, gy, gz, value);
+    }
+    count_items(p, lane == 0 ? items : 0);
+}
+
+// interpolate_vertex (marching_cubes_cuda.cu:72-97) followed by the world
+// transform of to_global_coordinates (visual_hull_cuda.cu:916-939).
+__device__ __forceinline__ void edge_vertex(const HullPlan& p,
+                                            uint32_t x1,
+                                            uint32_t y1,
+                                            uint32_t z1,
+                                            int axis,
+                                            float v1,
+                                            float v2,
+                                            float scale,
+                                            float* out)
+{
+    const float iso = 0.5f, eps = 1e-5f;
+    // 1: snap to p1, 2: snap to p2, 0: interpolate (the reference's check order)
+    int snap = 0;
+    if (fabsf(__fsub_rn(iso, v1)) < eps)
+        snap = 1;
+    else if (fabsf(__fsub_rn(iso, v2)) < eps)
+        snap = 2;
+    else if (fabsf(__fsub_rn(v1, v2)) < eps)
+        snap = 1;
+    const float t = __fdiv_rn(__fsub_rn(iso, v1), __fsub_rn(v2, v1)); // unused after a snap
+    // grid coordinates are below 2^13: exact float conversions by adds (the
+    // 64-bit integer conversions run on GB300's FP64 pipe)
+    const float f1[3] = { small_i2f(static_cast<int32_t>(x1)), small_i2f(static_cast<int32_t>(y1)), small_i2f(static_cast<int32_t>(z1)) };
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+    {
+        const float f2 = a == axis ? __fadd_rn(f1[a], 1.f) : f1[a];
+        const float q = snap == 1 ? f1[a] : (snap == 2 ? f2 : lerp(f1[a], f2, t));
+        out[a] = __fmaf_rn(scale, q, p.corner[a]);
     }
 }
 
-// Ranks of the 8 corners of the cell with base corner t; false if incomplete.
-// Ranks at or beyond n (possible only when the corner pool overflowed and the
-// request is about to be rerun) count as missing, so no access leaves the pools.
-// The points (x, row) and (x + 1, row) are neighbours in the bitmap's order,
-// so when both are set their ranks are consecutive: one rank lookup per row
-// of the cell (three, the base row's rank being t) instead of seven.
-__device__ __forceinline__ bool cell_ranks(const HullPlan& p,
-                                           int64_t t,
-                                           int64_t n,
-                                           int64_t gx,
-                                           int64_t gy,
-                                           int64_t gz,
-                                           uint32_t rk[8])
+// The corner grid's words (th_words.cuh): those of the touched rows.
+struct HullWords
 {
-    const int64_t R = p.R;
-    if (!(gx < R - 1 && gy < R - 1 && gz < R - 1))
-        return false;
-    const int b = static_cast<int>(gx & 63);
-    // the four rows of corners (dy, dz) = (q & 1, q >> 1): their bitmap words
-    // and rank words are loaded together (independent loads), then checked
-    int64_t w[4];
-    uint64_t word[4], nextw[4];
-    uint32_t wrank[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-    {
-        w[q] = ((gy + (q & 1)) + (gz + (q >> 1)) * R) * p.WR + (gx >> 6);
-        word[q] = p.bitmap[w[q]];
-        wrank[q] = q > 0 ? p.word_rank[w[q]] : 0u;
-        // x + 1 < R stays in the row; at bit 63 the +x corner is bit 0 of the next word
-        nextw[q] = b == 63 ? p.bitmap[w[q] + 1] : 0ull;
-    }
-    bool ok = true;
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-    {
-        const bool next = b < 63 ? ((word[q] >> (b + 1)) & 1ull) != 0 : (nextw[q] & 1ull) != 0;
-        ok = ok && next && (q == 0 || ((word[q] >> b) & 1ull) != 0);
-    }
-    if (!ok)
-        return false;
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-    {
-        const uint32_t r = q == 0 ? static_cast<uint32_t>(t)
-                                  : wrank[q] + static_cast<uint32_t>(__popcll(word[q] & ((1ull << b) - 1ull)));
-        if (r + 1 >= n)
-            return false;
-        rk[2 * q] = r;
-        rk[2 * q + 1] = r + 1;
-    }
-    return true;
-}
+    HullPlan p;
+    float scale;
 
-// classify_voxels_sparse (marching_cubes_cuda.cu:180-223) plus edge marking.
-__global__ void __launch_bounds__(256) mc_cells_kernel(HullPlan p)
-{
-    __shared__ TableCache tab;
-    load_tables(tab);
-    const int64_t n = p.ctr->corners;
-    const float iso = 0.5f;
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < n; t += stride)
+    __device__ int64_t words() const
     {
-        const int64_t idx = p.corners[t];
-        int64_t gx, gy, gz;
-        unpack_corner(idx, gx, gy, gz);
-        uint32_t rk[8];
-        uint32_t code = 0;
-        if (cell_ranks(p, t, n, gx, gy, gz, rk))
+        return p.ctr->words;
+    }
+    __device__ uint32_t word(uint32_t i) const
+    {
+        return __ldg(p.word_list + i);
+    }
+    __device__ bool empty(uint32_t) const
+    {
+        return false; // listed words have corners
+    }
+    __device__ uint32_t sign(uint32_t k) const
+    {
+        return __ldg(p.sign + k);
+    }
+    __device__ WordRows rows(uint32_t k) const
+    {
+        const uint32_t slot = fast_div(p.div_wr, k), w = k - slot * p.wr;
+        const uint32_t* near = p.row_place[slot].near;
+        const uint32_t up = __ldg(near + 7), back = __ldg(near + 5), both = __ldg(near + 8);
+        WordRows r;
+        r.next = w + 1 < p.wr;
+        r.idx[0] = k;
+        r.idx[1] = up != kNoWord ? up * p.wr + w : kNoWord;
+        r.idx[2] = back != kNoWord ? back * p.wr + w : kNoWord;
+        r.idx[3] = both != kNoWord ? both * p.wr + w : kNoWord;
+        return r;
+    }
+    __device__ EdgeBits edges(uint32_t k, const WordRows&, const uint32_t s[4], const uint32_t sh[4], uint32_t& cells) const
+    {
+        const uint32_t slot = fast_div(p.div_wr, k), w = k - slot * p.wr;
+        const uint4* place = reinterpret_cast<const uint4*>(p.row_place + slot);
+        const uint4 n0 = __ldg(place), n1 = __ldg(place + 1);
+        const uint32_t near[9] = { n0.x, n0.y, n0.z, n0.w, slot, n1.y, n1.z, n1.w, __ldg(p.row_place[slot].near + 8) };
+        return masked_edges(
+                [&](int dy, int dz) {
+                    const uint32_t n = near[3 * (dy + 1) + dz + 1];
+                    return n != kNoWord ? __ldg(p.runs + (n * p.wr + w)) : make_uint2(0u, 0u);
+                },
+                s, sh, cells);
+    }
+    __device__ uint32_t entry(uint32_t k, int b) const
+    {
+        return __ldg(p.rank + k) + static_cast<uint32_t>(__popc(__ldg(p.present + k) & ((1u << b) - 1u)));
+    }
+    __device__ void vertex(uint32_t k, int b, int axis, float out[3]) const
+    {
+        const uint32_t slot = fast_div(p.div_wr, k), w = k - slot * p.wr;
+        const uint32_t* near = p.row_place[slot].near;
+        const uint32_t yz = __ldg(near + 4);
+        const uint32_t e1 = entry(k, b);
+        // the edge's other end is a corner: a complete cell holds both
+        const uint32_t e2 = axis == 0 ? e1 + 1 : entry(__ldg(near + (axis == 1 ? 7 : 5)) * p.wr + w, b);
+        edge_vertex(p, w * 32 + b, yz & 0xffffu, yz >> 16, axis, __ldg(p.values + e1), __ldg(p.values + e2), scale, out);
+    }
+    __device__ void values_at(const WordRows& r, int b, unsigned long long* corner) const
+    {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
         {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (p.values[rk[i]] < iso)
-                    code |= 1u << i;
-            const int cnt = tab.count[code];
-            uint32_t used = 0; // bit (lo * 3 + axis)
-            for (int j = 0; j < cnt; ++j)
-            {
-                const uint32_t e = tab.edges[code][j];
-                used |= 1u << ((e & 7u) * 3u + (e >> 3));
-            }
-            // the vertex-edge bits of each lower corner, one word read and at
-            // most one atomic per corner (the reads are independent)
-            unsigned int* words[8];
-            uint32_t bits[8], cur[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-            {
-                const uint32_t r1 = rk[i];
-                bits[i] = ((used >> (3 * i)) & 7u) << (8u * (r1 & 3u));
-                words[i] = reinterpret_cast<unsigned int*>(p.emask) + (r1 >> 2);
-                cur[i] = bits[i] ? *words[i] : 0u;
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if ((cur[i] & bits[i]) != bits[i])
-                    atomicOr(words[i], bits[i]);
+            const uint32_t e = entry(r.idx[q], b);
+            corner[2 * q] = e;
+            corner[2 * q + 1] = e + 1;
         }
-        p.codes[t] = static_cast<uint8_t>(code);
     }
-}
-
-struct VertCount
-{
-    const uint8_t* codes;
-    const uint8_t* emask;
-    __device__ unsigned long long operator()(int64_t t) const
+    __device__ void soup_vertex(uint32_t k, int b, int lo, int axis, unsigned long long h1, unsigned long long h2, float out[3]) const
     {
-        return (static_cast<unsigned long long>(g_mc_count[codes[t]]) << 32) |
-               static_cast<unsigned long long>(__popc(emask[t]));
+        const uint32_t slot = fast_div(p.div_wr, k), w = k - slot * p.wr;
+        const uint32_t yz = __ldg(p.row_place[slot].near + 4);
+        edge_vertex(p, w * 32 + b + (lo & 1), (yz & 0xffffu) + (lo >> 1 & 1), (yz >> 16) + (lo >> 2 & 1), axis,
+                    __ldg(p.values + h1), __ldg(p.values + h2), scale, out);
     }
 };
 
-struct VertEmit
-{
-    uint32_t* soup_off;
-    uint32_t* vbase;
-    __device__ void operator()(int64_t t, unsigned long long off, unsigned long long) const
-    {
-        soup_off[t] = static_cast<uint32_t>(off >> 32);
-        vbase[t] = static_cast<uint32_t>(off & 0xffffffffull);
-    }
-};
-
-struct VertEpilogue
+struct MeshTotal
 {
     DevCounters* ctr;
     __device__ void operator()(unsigned long long total) const
@@ -727,326 +799,9 @@ struct VertEpilogue
     }
 };
 
-// interpolate_vertex (marching_cubes_cuda.cu:72-97) followed by the world
-// transform of to_global_coordinates (visual_hull_cuda.cu:916-939).
-__device__ __forceinline__ void edge_vertex(const HullPlan& p,
-                                            int64_t x1,
-                                            int64_t y1,
-                                            int64_t z1,
-                                            int axis,
-                                            float v1,
-                                            float v2,
-                                            float scale,
-                                            float* out)
+HullWords hull_words(const HullPlan& p)
 {
-    const float iso = 0.5f, eps = 1e-5f;
-    const int64_t x2 = x1 + (axis == 0), y2 = y1 + (axis == 1), z2 = z1 + (axis == 2);
-    // 1: snap to p1, 2: snap to p2, 0: interpolate (the reference's check order)
-    int snap = 0;
-    if (fabsf(__fsub_rn(iso, v1)) < eps)
-        snap = 1;
-    else if (fabsf(__fsub_rn(iso, v2)) < eps)
-        snap = 2;
-    else if (fabsf(__fsub_rn(v1, v2)) < eps)
-        snap = 1;
-    // grid coordinates are below 2^13: exact float conversions by adds (the
-    // 64-bit integer conversions run on GB300's FP64 pipe)
-    const float fx1 = small_i2f(static_cast<int32_t>(x1)), fy1 = small_i2f(static_cast<int32_t>(y1)),
-                fz1 = small_i2f(static_cast<int32_t>(z1));
-    const float fx2 = small_i2f(static_cast<int32_t>(x2)), fy2 = small_i2f(static_cast<int32_t>(y2)),
-                fz2 = small_i2f(static_cast<int32_t>(z2));
-    float q[3];
-    if (snap == 1)
-    {
-        q[0] = fx1;
-        q[1] = fy1;
-        q[2] = fz1;
-    }
-    else if (snap == 2)
-    {
-        q[0] = fx2;
-        q[1] = fy2;
-        q[2] = fz2;
-    }
-    else
-    {
-        const float t = __fdiv_rn(__fsub_rn(iso, v1), __fsub_rn(v2, v1));
-        q[0] = lerp(fx1, fx2, t);
-        q[1] = lerp(fy1, fy2, t);
-        q[2] = lerp(fz1, fz2, t);
-    }
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-        out[a] = __fmaf_rn(scale, q[a], p.corner[a]);
-}
-
-// Faces in soup order; with unique vertices they index the edge-numbered
-// vertex list, without they index the soup, which this kernel also writes.
-// Columns 1 and 2 are swapped as flip_faces does (visual_hull_cuda.cu:941-956).
-// A warp takes 32 consecutive corners, whose face entries form one contiguous
-// range of the soup (soup_off is their exclusive prefix sum).  The range's
-// entries are dealt out one per lane (entry k of the range belongs to the
-// cell whose offset is the last one <= k; the cells' corner ranks are parked
-// in shared memory), parked in shared memory at their flipped position, and
-// stored with coalesced writes.  One thread per cell left three quarters of
-// the lanes idle (a quarter of the corners start an active cell, with 1 to 15
-// entries) and scattered each store over ~50 sectors.
-constexpr int kExportWarps = 8;
-
-__global__ void __launch_bounds__(32 * kExportWarps) export_faces_kernel(HullPlan p, float* __restrict__ verts, int64_t* __restrict__ faces)
-{
-    __shared__ TableCache tab;
-    __shared__ int64_t stage_all[kExportWarps][32 * 15];
-    __shared__ uint32_t ranks_all[kExportWarps][32][9];
-    load_tables(tab);
-    int64_t* stage = stage_all[threadIdx.x >> 5];
-    uint32_t(*ranks)[9] = ranks_all[threadIdx.x >> 5];
-    const int lane = threadIdx.x & 31;
-    const int64_t n = p.ctr->corners;
-    const float scale = __fdiv_rn(p.length, static_cast<float>(int64_t{ 1 } << p.level));
-    const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-    for (int64_t wb = warp * 32; wb < n; wb += nwarps * 32)
-    {
-        const int64_t t = wb + lane;
-        const bool valid = t < n;
-        const uint32_t code = valid ? p.codes[t] : 0u;
-        const int cnt = tab.count[code];
-        const unsigned act = __ballot_sync(0xffffffffu, cnt > 0);
-        if (!act)
-            continue;
-        // the warp's range of the soup starts at lane 0's offset (a multiple of 3)
-        const int64_t lo = __shfl_sync(0xffffffffu, valid ? static_cast<int64_t>(p.soup_off[t]) : int64_t{ 0 }, 0);
-        const int64_t id = cnt > 0 ? p.corners[t] : 0;
-        if (cnt > 0)
-        {
-            int64_t gx, gy, gz;
-            unpack_corner(id, gx, gy, gz);
-            uint32_t rk[8];
-            cell_ranks(p, t, n, gx, gy, gz, rk);
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                ranks[lane][i] = rk[i];
-        }
-        const int incl = warp_inclusive_scan(cnt);
-        const int excl = incl - cnt;
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        __syncwarp();
-        for (int k0 = 0; k0 < total; k0 += 32)
-        {
-            const int k = k0 + lane;
-            const int s = item_slot(excl, k);
-            const int es = __shfl_sync(0xffffffffu, excl, s);
-            const uint32_t cs = __shfl_sync(0xffffffffu, code, s);
-            const int64_t ids = __shfl_sync(0xffffffffu, id, s);
-            if (k < total)
-            {
-                const uint32_t e = tab.edges[cs][k - es];
-                const int lo_corner = static_cast<int>(e & 7u), axis = static_cast<int>(e >> 3);
-                const int64_t f = lo + k;
-                const int slot = static_cast<int>(f % 3);
-                const int dst = k - slot + (slot == 0 ? 0 : 3 - slot);
-                const uint32_t r1 = ranks[s][lo_corner];
-                if (p.unique)
-                    stage[dst] = static_cast<int64_t>(p.vbase[r1]) + __popc(p.emask[r1] & ((1u << axis) - 1u));
-                else
-                {
-                    int64_t gx, gy, gz;
-                    unpack_corner(ids, gx, gy, gz);
-                    float v[3];
-                    const int hi_corner = lo_corner | (1 << axis);
-                    edge_vertex(p, gx + (lo_corner & 1), gy + (lo_corner >> 1 & 1), gz + (lo_corner >> 2 & 1), axis,
-                                p.values[r1], p.values[ranks[s][hi_corner]], scale, v);
-                    verts[3 * f + 0] = v[0];
-                    verts[3 * f + 1] = v[1];
-                    verts[3 * f + 2] = v[2];
-                    stage[dst] = f;
-                }
-            }
-        }
-        __syncwarp();
-        for (int i = lane; i < total; i += 32)
-            faces[lo + i] = stage[i];
-        __syncwarp();
-    }
-}
-
-// Unique vertices: vertices and faces in one pass.  A warp takes 128
-// consecutive corners at a time: their data (code, edge bits, id, value) is
-// staged in shared memory with coalesced loads, and their vertices (one per
-// set edge bit, numbered by vbase) and face entries (numbered by soup_off)
-// form two contiguous output ranges, dealt out one entry per lane (the owner
-// of entry k is found by a binary search over the staged prefix sums), so the
-// rank and value gathers run on all lanes although only about a quarter of
-// the corners own any vertex or face.  The +x neighbour of a corner of the
-// mesh has the next rank; other neighbours are looked up in the bitmap.
-// Face columns 1 and 2 are swapped as flip_faces does
-// (visual_hull_cuda.cu:941-956): entry k of a triangle goes to k's mirror.
-constexpr int kExportPer = 4;                   // corners per lane
-constexpr int kExportChunk = 32 * kExportPer;   // corners per warp and iteration
-
-struct ExportStage
-{
-    int64_t id[kExportChunk];
-    float val[kExportChunk];
-    int32_t vpre[kExportChunk]; // exclusive prefix of the vertex counts over the chunk
-    int32_t fpre[kExportChunk]; // exclusive prefix of the face-entry counts
-    uint8_t code[kExportChunk], em[kExportChunk], nv[kExportChunk], nf[kExportChunk];
-};
-
-// Largest c in [0, kExportChunk) with pre[c] <= k (pre non-decreasing, pre[0] = 0).
-__device__ __forceinline__ int stage_owner(const int32_t* pre, int k)
-{
-    int c = 0;
-#pragma unroll
-    for (int step = kExportChunk / 2; step > 0; step >>= 1)
-        if (pre[c + step] <= k)
-            c += step;
-    return c;
-}
-
-__global__ void __launch_bounds__(32 * kExportWarps) export_mesh_kernel(HullPlan p, float* __restrict__ verts, int64_t* __restrict__ faces)
-{
-    __shared__ TableCache tab;
-    __shared__ ExportStage stage_all[kExportWarps];
-    load_tables(tab);
-    __syncthreads();
-    ExportStage& st = stage_all[threadIdx.x >> 5];
-    const int lane = threadIdx.x & 31;
-    const int64_t n = p.ctr->corners;
-    const float scale = __fdiv_rn(p.length, static_cast<float>(int64_t{ 1 } << p.level));
-    const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-    for (int64_t wb = warp * kExportChunk; wb < n; wb += nwarps * kExportChunk)
-    {
-        // stage the chunk (coalesced: corner g * 32 + lane)
-        bool any = false;
-#pragma unroll
-        for (int g = 0; g < kExportPer; ++g)
-        {
-            const int c = g * 32 + lane;
-            const int64_t t = wb + c;
-            const bool valid = t < n;
-            const uint32_t code = valid ? p.codes[t] : 0u;
-            const uint32_t em = valid ? p.emask[t] : 0u;
-            const int nv = __popc(em), nf = tab.count[code];
-            st.code[c] = static_cast<uint8_t>(code);
-            st.em[c] = static_cast<uint8_t>(em);
-            st.nv[c] = static_cast<uint8_t>(nv);
-            st.nf[c] = static_cast<uint8_t>(nf);
-            if (nv > 0 || nf > 0)
-            {
-                st.id[c] = p.corners[t];
-                any = true;
-            }
-            if (nv > 0)
-                st.val[c] = p.values[t];
-        }
-        if (!__any_sync(0xffffffffu, any))
-            continue;
-        __syncwarp();
-        // prefix sums in corner order: lane l owns corners [4l, 4l + 4)
-        int vloc[kExportPer], floc[kExportPer];
-        int vt = 0, ft = 0;
-#pragma unroll
-        for (int g = 0; g < kExportPer; ++g)
-        {
-            const int c = lane * kExportPer + g;
-            vloc[g] = vt;
-            floc[g] = ft;
-            vt += st.nv[c];
-            ft += st.nf[c];
-        }
-        const int vin = warp_inclusive_scan(vt), fin = warp_inclusive_scan(ft);
-        const int vex = vin - vt, fex = fin - ft;
-        const int vtot = __shfl_sync(0xffffffffu, vin, 31), ftot = __shfl_sync(0xffffffffu, fin, 31);
-#pragma unroll
-        for (int g = 0; g < kExportPer; ++g)
-        {
-            st.vpre[lane * kExportPer + g] = vex + vloc[g];
-            st.fpre[lane * kExportPer + g] = fex + floc[g];
-        }
-        __syncwarp();
-
-        // vertices: the chunk's range starts at its first corner's vertex base.
-        // Two entries per lane and iteration, their loads issued together;
-        // every corner looked up here exists, so the rank needs no check.
-        if (vtot > 0)
-        {
-            const int64_t vlo = p.vbase[wb];
-            auto vertex_at = [&](int k, float v[3]) {
-                const int c = stage_owner(st.vpre, k);
-                const int a = nth_set_bit(st.em[c], k - st.vpre[c]);
-                int64_t gx, gy, gz;
-                unpack_corner(st.id[c], gx, gy, gz);
-                // the edge's upper corner (for a = 0 the next rank, wb + c + 1)
-                const uint32_t r2 = rank_of(p, gx + (a == 0), gy + (a == 1), gz + (a == 2));
-                edge_vertex(p, gx, gy, gz, a, st.val[c], p.values[r2], scale, v);
-            };
-            for (int k = lane; k < vtot; k += 64)
-            {
-                const bool two = k + 32 < vtot;
-                float v0[3], v1[3];
-                vertex_at(k, v0);
-                vertex_at(two ? k + 32 : k, v1);
-                int64_t out = vlo + k;
-                verts[3 * out + 0] = v0[0];
-                verts[3 * out + 1] = v0[1];
-                verts[3 * out + 2] = v0[2];
-                if (two)
-                {
-                    out += 32;
-                    verts[3 * out + 0] = v1[0];
-                    verts[3 * out + 1] = v1[1];
-                    verts[3 * out + 2] = v1[2];
-                }
-            }
-        }
-
-        // faces: the chunk's entries are one contiguous range of the soup
-        // (soup_off is their exclusive prefix sum, a multiple of 3)
-        if (ftot > 0)
-        {
-            const int64_t lo = p.soup_off[wb];
-            auto face_at = [&](int k) -> int64_t {
-                const int c = stage_owner(st.fpre, k);
-                const uint32_t e = tab.edges[st.code[c]][k - st.fpre[c]];
-                const int lo_corner = static_cast<int>(e & 7u), axis = static_cast<int>(e >> 3);
-                int64_t gx, gy, gz;
-                unpack_corner(st.id[c], gx, gy, gz);
-                // the edge's lower corner (every corner of a cell with faces exists)
-                const uint32_t r1 = rank_of(p, gx + (lo_corner & 1), gy + (lo_corner >> 1 & 1), gz + (lo_corner >> 2 & 1));
-                return static_cast<int64_t>(p.vbase[r1]) + __popc(p.emask[r1] & ((1u << axis) - 1u));
-            };
-            for (int k = lane; k < ftot; k += 64)
-            {
-                const bool two = k + 32 < ftot;
-                const int64_t f0 = face_at(k);
-                const int64_t f1 = face_at(two ? k + 32 : k);
-                // columns 1 and 2 swapped: entry k of a triangle goes to its mirror
-                const int s0 = k % 3;
-                faces[lo + k - s0 + (s0 == 0 ? 0 : 3 - s0)] = f0;
-                if (two)
-                {
-                    const int k1 = k + 32, s1 = k1 % 3;
-                    faces[lo + k1 - s1 + (s1 == 0 ? 0 : 3 - s1)] = f1;
-                }
-            }
-        }
-        __syncwarp();
-    }
-}
-
-__global__ void __launch_bounds__(256) clear_rows_kernel(HullPlan p)
-{
-    const int64_t n = p.ctr->rows;
-    const int64_t total = n * p.WR;
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride)
-    {
-        const int64_t k = i / p.WR, w = i - k * p.WR;
-        p.bitmap[static_cast<int64_t>(p.rows[k]) * p.WR + w] = 0;
-    }
+    return HullWords{ p, p.length / static_cast<float>(int64_t{ 1 } << p.level) };
 }
 
 } // namespace
@@ -1062,12 +817,9 @@ void launch_corners(const HullPlan& p, cudaStream_t s)
 void launch_rank_corners(const HullPlan& p, cudaStream_t s)
 {
     const int64_t row_words = (p.R * p.R + 31) / 32;
-    run_scan(RowCount{ p.rowbits }, RowEmit{ p.rowbits, p.rows }, RowEpilogue{ p.ctr }, Count{ nullptr, row_words },
-             row_words, p.tile_sums, &p.ctr->scan, s);
-    const int64_t max_words = p.R * p.R * p.WR;
-    run_scan_reduce(CornerCount{ p }, CornerEpilogue{ p.ctr, p.corner_cap }, Count{ &p.ctr->rows, 0, p.WR }, max_words,
-                    p.tile_sums, &p.ctr->scan, s);
-    corner_emit_kernel<<<scan_grid(max_words), kScanThreads, 0, s>>>(p, p.tile_sums);
+    rows_kernel<<<static_cast<unsigned>((row_words + kRowBlock - 1) / kRowBlock), 256, 0, s>>>(p);
+    TH_LAUNCH_CHECK();
+    corners_kernel<<<grid_for(p.R * p.R, 32), 256, 0, s>>>(p);
     TH_LAUNCH_CHECK();
 }
 
@@ -1133,19 +885,29 @@ void launch_field(const HullPlan& p, cudaStream_t s)
 
 void launch_marching_cubes(const HullPlan& p, cudaStream_t s)
 {
-    mc_cells_kernel<<<grid_for(p.corner_cap, 256), 256, 0, s>>>(p);
+    const HullWords src = hull_words(p);
+    const int grid = words_grid(std::min(p.word_cap, p.R * p.R * static_cast<int64_t>(p.wr)));
+    if (p.unique)
+        words_count_kernel<HullWords, true><<<grid, kWordThreads, 0, s>>>(src, p.mesh, &p.ctr->scan, nullptr, MeshTotal{ p.ctr });
+    else
+        words_count_kernel<HullWords, false><<<grid, kWordThreads, 0, s>>>(src, p.mesh, &p.ctr->scan, nullptr, MeshTotal{ p.ctr });
     TH_LAUNCH_CHECK();
-    run_scan(VertCount{ p.codes, p.emask }, VertEmit{ p.soup_off, p.vbase }, VertEpilogue{ p.ctr },
-             Count{ &p.ctr->corners, 0 }, p.corner_cap, p.tile_sums, &p.ctr->scan, s);
+    words_base_kernel<HullWords><<<grid, kWordThreads, 0, s>>>(src, p.mesh);
+    TH_LAUNCH_CHECK();
 }
 
-void launch_export(const HullPlan& p, float* verts, int64_t* faces, cudaStream_t s)
+void launch_export(const HullPlan& p, int64_t words, float* verts, int64_t* faces, cudaStream_t s)
 {
-    const int grid = grid_for(p.corner_cap, 32 * kExportWarps);
+    const HullWords src = hull_words(p);
+    const int grid = words_export_grid(words);
     if (p.unique)
-        export_mesh_kernel<<<grid, 32 * kExportWarps, 0, s>>>(p, verts, faces);
+    {
+        words_verts_kernel<HullWords><<<grid, 32 * kWordExportWarps, 0, s>>>(src, p.mesh, verts);
+        TH_LAUNCH_CHECK();
+        words_faces_kernel<HullWords, true, true><<<grid, 32 * kWordExportWarps, 0, s>>>(src, p.mesh, verts, faces);
+    }
     else
-        export_faces_kernel<<<grid, 32 * kExportWarps, 0, s>>>(p, verts, faces);
+        words_faces_kernel<HullWords, false, true><<<grid, 32 * kWordExportWarps, 0, s>>>(src, p.mesh, verts, faces);
     TH_LAUNCH_CHECK();
 }
 
@@ -1173,13 +935,6 @@ void launch_export_field(const HullPlan& p, int64_t n, int64_t* indices, float* 
         return;
     export_field_kernel<<<grid_for(n, 256), 256, 0, s>>>(p, n, indices, values);
     TH_LAUNCH_CHECK();
-}
-
-void launch_cleanup(const HullPlan& p, cudaStream_t s)
-{
-    clear_rows_kernel<<<grid_for(p.R * p.R * p.WR, 256), 256, 0, s>>>(p);
-    TH_LAUNCH_CHECK();
-    launch_zero(p.rowbits, sizeof(uint32_t) * ((p.R * p.R + 31) / 32), s);
 }
 
 } // namespace th

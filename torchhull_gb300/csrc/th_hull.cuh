@@ -7,6 +7,7 @@
 #include <cstdint>
 
 #include "th_common.cuh"
+#include "th_words.cuh"
 
 namespace th
 {
@@ -17,6 +18,7 @@ enum OverflowBits : int64_t
     kOverflowCorners = 2,
     kOverflowSoup = 4,
     kOverflowParents = 8,
+    kOverflowWords = 16,
 };
 
 struct DevCounters
@@ -25,6 +27,7 @@ struct DevCounters
     int64_t level_off[kMaxLevel + 3];   // start of level i in the node pool
     int64_t rows;                       // bitmap rows holding at least one corner
     int64_t corners;                    // unique leaf corners (the sparse field)
+    int64_t words;                      // words of 32 points with a corner
     int64_t soup;                       // soup vertices, 3 per face
     int64_t verts;                      // unique mesh vertices
     int64_t overflow;                   // OverflowBits
@@ -42,6 +45,14 @@ struct ReqConsts
     float corner[3];
     float length;
     const void* masks;
+};
+
+// A touched row and the slots of its eight neighbours, kNoWord where one is not
+// touched: near[3 * (dy + 1) + dz + 1] without the middle one, which is yz.
+struct RowPlace
+{
+    uint32_t near[9]; // [4]: y | z << 16
+    uint32_t pad[3];
 };
 
 // Per-request constants and buffers, passed to kernels by value.
@@ -102,16 +113,26 @@ struct HullPlan
     // corner grid: R^3 points, one bit each, rows of WR 64-bit words (x fastest)
     int64_t R, WR;
     uint64_t* bitmap;     // [R*R*WR]
-    uint32_t* word_rank;  // [R*R*WR] rank of the word's first bit (valid for touched rows)
     uint32_t* rowbits;    // [ceil(R*R/32)] touched-row flags
-    uint32_t* rows;       // [R*R] touched rows, ascending
-    // sparse field and marching cubes, indexed by corner rank
+    // Touched rows, ascending, and the words of 32 points of those rows only:
+    // word k = slot * wr + w holds the points x = 32 w.. of row rows[slot].
+    uint32_t* rows;       // [R*R]
+    uint32_t* row_slot;   // [R*R] slot of a touched row (others: stale)
+    RowPlace* row_place;  // [R*R] a slot's row and the rows around it
+    uint2* row_cnt;       // [R*R] corners and words with a corner of a slot's row
+    uint2* coarse;        // [R*R / 256 + 2] the same of 256 slots
+    uint32_t wr;          // 2 * WR
+    FastDiv div_wr, div_r; // by wr and by R
+    int64_t word_cap;
+    uint32_t* present;    // [word_cap] corner bits
+    uint2* runs;          // [word_cap] word_runs of the corner bits
+    uint32_t* rank;       // [word_cap] corners before the word
+    uint32_t* sign;       // [word_cap] bits: field value below 0.5
+    uint32_t* word_list;  // [word_cap] the words with a corner, ascending
+    WordMesh mesh;
+    // sparse field, by corner rank
     int64_t* corners;
     float* values;
-    uint8_t* codes;
-    uint8_t* emask; // bit a: the edge from this corner along axis a carries a vertex
-    uint32_t* soup_off;
-    uint32_t* vbase;
     int64_t corner_cap;
     DevCounters* ctr;
     const ReqConsts* rq; // corner, length and masks of the running request (device)
@@ -141,7 +162,8 @@ void launch_carve_level(const HullPlan& p, int level_index, cudaStream_t s);
 void launch_emit_leaves(const HullPlan& p, cudaStream_t s);
 void launch_corners(const HullPlan& p, cudaStream_t s);
 // The part of launch_corners after the bitmap is set: touched rows, sorted
-// unique corners and per-word ranks.
+// unique corners and the rows' words.  Leaves the bitmap and the row flags
+// clear for the next request.
 void launch_rank_corners(const HullPlan& p, cudaStream_t s);
 
 // Sets the 8 corner bits of a leaf cell (x, y, z) at resolution 2^L in a
@@ -209,7 +231,7 @@ __device__ __forceinline__ void mark_children_corners(uint64_t* bitmap, uint32_t
 
 void launch_field(const HullPlan& p, cudaStream_t s);
 void launch_marching_cubes(const HullPlan& p, cudaStream_t s);
-void launch_export(const HullPlan& p, float* verts, int64_t* faces, cudaStream_t s);
-void launch_cleanup(const HullPlan& p, cudaStream_t s);
+// words: the request's DevCounters::words (read back with the counts).
+void launch_export(const HullPlan& p, int64_t words, float* verts, int64_t* faces, cudaStream_t s);
 
 } // namespace th

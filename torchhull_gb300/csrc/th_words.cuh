@@ -11,16 +11,19 @@
 //    cells' bits and the two counts (vertices, triangle corners); tile sums.
 // 2. words_base: the counts' prefix sums: per word the index of its first
 //    vertex, per 32 words the first vertex and triangle corner.
-// 3. words_export: a warp takes 32 words and deals their vertices, then their
-//    active cells and the cells' triangle corners, to its lanes: an edge's
-//    vertex index is its word's base plus the set bits before it.
+// 3. words_verts and words_faces: a warp takes 32 words and deals their
+//    vertices, or their active cells and the cells' triangle corners, to its
+//    lanes: an edge's vertex index is its word's base plus the set bits before it.
 //
 // Vertices come by the lower end point of their edge (in row order), then by
 // axis; triangles by cell, then in table order.  A source (Src) says how words
 // are found:
-//   int64_t words() const             number of words
+//   int64_t words() const             number of items: words in row order, at least
+//                                     those with a present point
+//   uint32_t word(uint32_t i) const   the word of an item
 //   WordRows rows(uint32_t k) const   the words of the cells that start in word k
 //   uint32_t sign(uint32_t k) const   below-isolevel bits of a word
+//   bool empty(uint32_t k) const      none of the word's points is present
 //   EdgeBits edges(k, rows, s, sh, cells) const   vertex edges and complete cells of a word
 //   void vertex(k, bit, axis, out) const          the vertex of an edge
 //   void values_at(rows, bit, corner) const       handles of a cell's eight values (soup)
@@ -28,9 +31,9 @@
 //
 // All three passes are bound by the latency of short dependent load chains on
 // words that stay in L2; the volume itself is read once, by the pass that
-// makes the sign words.  A 400^3 float32 sphere on GB300: 691 -> 269 us a call
+// makes the sign words.  A 400^3 float32 sphere on GB300: 691 -> 203 us a call
 // (447 us of it were one thread per point, exchanging planes through shared
-// memory), its band of 1.5 M entries 395 -> 203 us (eight hash lookups per
+// memory), its band of 1.5 M entries 395 -> 207 us (eight hash lookups per
 // entry before, twice).
 #pragma once
 
@@ -48,10 +51,10 @@ constexpr int kWordThreads = 256;
 
 struct WordMesh
 {
-    uint32_t* cnt;   // per word: vertices | triangle corners << 8
-    uint32_t* cells; // per word: cells the surface passes through
+    uint32_t* cnt;   // per item: vertices | triangle corners << 8
+    uint32_t* cells; // per item: cells the surface passes through
     uint4* edges;    // per word with vertices: x, y and z edge bits, index of the first vertex
-    uint2* chunk;    // per 32 words: first vertex, first triangle corner
+    uint2* chunk;    // per 32 items: first vertex, first triangle corner
     unsigned long long* tiles; // per tile: triangle corners << 32 | vertices, then exclusive offsets
 };
 
@@ -60,9 +63,7 @@ struct WordMesh
 struct WordRows
 {
     uint32_t idx[4];
-    int64_t x0; // first grid point of the word
-    uint32_t y, z;
-    bool next;        // the word has a right neighbour in its row
+    bool next; // the word has a right neighbour in its row
 };
 
 struct EdgeBits
@@ -110,30 +111,19 @@ __device__ __forceinline__ void sign_rows(const Src& src, const WordRows& r, uin
 
 // Vertex edges and complete cells of a word where not every grid point is
 // present: an edge counts when a cell with all its eight corners holds it.
-// Such cells are runs of two present points in four neighbouring rows, so they
-// follow from the presence words of the nine rows around the word's, with the
-// neighbouring bit on either side.  at(dy, dz): the word of the row (y + dy,
-// z + dz), kNoWord where there is none; present(idx): its bits.
-template <class At, class Present>
-__device__ __forceinline__ EdgeBits masked_edges(At&& at, Present&& present, bool prev, bool next, const uint32_t s[4], const uint32_t sh[4], uint32_t& cells)
+// Such cells are runs of two present points in four neighbouring rows.
+// run(dy, dz): for the word in the row (y + dy, z + dz), bits x: the points b
+// and b + 1 are present, bit 0 of y: the points -1 and 0 are; zero where there
+// is no such row.
+template <class Run>
+__device__ __forceinline__ EdgeBits masked_edges(Run&& run, const uint32_t s[4], const uint32_t sh[4], uint32_t& cells)
 {
-    uint32_t run[3][3];   // bit b: the points b and b + 1 are present
-    uint32_t left = 0;    // bit 3 * (dy + 1) + dz + 1: the points -1 and 0 are present
+    uint2 r[3][3];
 #pragma unroll
-    for (int dy = -1; dy <= 1; ++dy)
-    {
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int dz = -1; dz <= 1; ++dz)
-        {
-            const uint32_t idx = at(dy, dz);
-            const bool in = idx != kNoWord;
-            const uint32_t b = in ? present(idx) : 0u;
-            const uint32_t nb = in && next ? present(idx + 1) : 0u;
-            const uint32_t pb = in && prev ? present(idx - 1) : 0u;
-            run[dy + 1][dz + 1] = b & ((b >> 1) | (nb << 31));
-            left |= ((pb >> 31) & b & 1u) << (3 * (dy + 1) + dz + 1);
-        }
-    }
+        for (int j = 0; j < 3; ++j)
+            r[i][j] = run(i - 1, j - 1);
     // complete cells that start in the rows (y - 1 + i, z - 1 + j), and the points they hold in this word
     uint32_t cell[2][2], held[2][2];
 #pragma unroll
@@ -142,14 +132,20 @@ __device__ __forceinline__ EdgeBits masked_edges(At&& at, Present&& present, boo
 #pragma unroll
         for (int j = 0; j < 2; ++j)
         {
-            cell[i][j] = run[i][j] & run[i + 1][j] & run[i][j + 1] & run[i + 1][j + 1];
-            const uint32_t four = 0x1bu << (3 * i + j); // bits 0, 1, 3, 4
-            held[i][j] = cell[i][j] | (cell[i][j] << 1) | ((left & four) == four ? 1u : 0u);
+            cell[i][j] = r[i][j].x & r[i + 1][j].x & r[i][j + 1].x & r[i + 1][j + 1].x;
+            const uint32_t left = r[i][j].y & r[i + 1][j].y & r[i][j + 1].y & r[i + 1][j + 1].y;
+            held[i][j] = cell[i][j] | (cell[i][j] << 1) | left;
         }
     }
     cells = cell[1][1];
     return EdgeBits{ (s[0] ^ sh[0]) & (cell[1][1] | cell[0][1] | cell[1][0] | cell[0][0]),
                      (s[0] ^ s[1]) & (held[1][1] | held[1][0]), (s[0] ^ s[2]) & (held[1][1] | held[0][1]) };
+}
+
+// A word's runs (masked_edges) from its bits and its neighbours' in the row.
+__device__ __forceinline__ uint2 word_runs(uint32_t prev, uint32_t bits, uint32_t next)
+{
+    return make_uint2(bits & ((bits >> 1) | (next << 31)), (prev >> 31) & bits & 1u);
 }
 
 // Exclusive offsets from tile sums by the block that finishes last, like
@@ -210,19 +206,28 @@ __global__ void __launch_bounds__(kWordThreads) words_count_kernel(Src src, Word
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
     {
         unsigned long long sum = 0;
-        for (int i = 0; i < kWordTile / kWordThreads; ++i)
+        for (int t = 0; t < kWordTile / kWordThreads; ++t)
         {
-            const int64_t kk = tile * kWordTile + i * kWordThreads + threadIdx.x;
+            const int64_t kk = tile * kWordTile + t * kWordThreads + threadIdx.x;
             if (kk >= n)
                 break;
-            const uint32_t k = static_cast<uint32_t>(kk);
-            const WordRows r = src.rows(k);
-            uint32_t s[4], sh[4];
-            sign_rows(src, r, s, sh);
+            const uint32_t i = static_cast<uint32_t>(kk), k = src.word(i);
+            uint32_t s[4], sh[4], some = 0, all = 0;
+            WordRows r;
+            if (!src.empty(k))
+            {
+                r = src.rows(k);
+                sign_rows(src, r, s, sh);
+                some = s[0] | s[1] | s[2] | s[3] | sh[0] | sh[1] | sh[2] | sh[3];
+                all = s[0] & s[1] & s[2] & s[3] & sh[0] & sh[1] & sh[2] & sh[3];
+            }
+            if ((some & ~all) == 0)
+            {
+                m.cnt[i] = 0; // all points around the word lie on one side
+                continue;
+            }
             uint32_t cells = 0;
             const EdgeBits e = src.edges(k, r, s, sh, cells);
-            const uint32_t some = s[0] | s[1] | s[2] | s[3] | sh[0] | sh[1] | sh[2] | sh[3];
-            const uint32_t all = s[0] & s[1] & s[2] & s[3] & sh[0] & sh[1] & sh[2] & sh[3];
             cells &= some & ~all;
             uint32_t soup = 0;
             for (uint32_t left = cells; left; left &= left - 1)
@@ -234,9 +239,9 @@ __global__ void __launch_bounds__(kWordThreads) words_count_kernel(Src src, Word
                 if (verts)
                     m.edges[k] = make_uint4(e.x, e.y, e.z, 0u);
             }
-            m.cnt[k] = verts | (soup << 8);
+            m.cnt[i] = verts | (soup << 8);
             if (cells)
-                m.cells[k] = cells;
+                m.cells[i] = cells;
             sum += (static_cast<unsigned long long>(soup) << 32) | verts;
             nactive += __popc(cells);
         }
@@ -298,7 +303,7 @@ __global__ void __launch_bounds__(kWordThreads) words_base_kernel(Src src, WordM
             if (lane == 0)
                 m.chunk[k >> 5] = make_uint2(static_cast<uint32_t>(off), static_cast<uint32_t>(off >> 32));
             if (c[i] & 0xffu)
-                m.edges[k].w = static_cast<uint32_t>(off) + ((incl - mine) & 0xffffu);
+                m.edges[src.word(static_cast<uint32_t>(k))].w = static_cast<uint32_t>(off) + ((incl - mine) & 0xffffu);
             const uint32_t tot = __shfl_sync(0xffffffffu, incl, 31);
             off += (static_cast<unsigned long long>(tot >> 16) << 32) | (tot & 0xffffu);
         }
@@ -317,15 +322,82 @@ __device__ __forceinline__ unsigned long long point_vertices(const uint4& g, int
 
 constexpr int kWordExportWarps = 8;
 
-// Pass 3.  FLIP: the second and third corner of every triangle change places.
-// Without UNIQUE every triangle corner is a vertex of its own.
+// The export passes take a chunk of 32 words per warp; a warp's chunks lie far
+// apart, which spreads the surface over the warps (eight neighbouring chunks
+// per warp took 46 + 80 us for the vertices and faces of a 400^3 sphere,
+// against 26 + 50).  All that says what a chunk holds is loaded at
+// once, whether or not it holds anything.
+
+// Pass 3, the vertices.
+template <class Src>
+__global__ void __launch_bounds__(32 * kWordExportWarps) words_verts_kernel(Src src, WordMesh m, float* __restrict__ verts)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t n = src.words(), nchunks = (n + 31) / 32;
+    const int64_t nwarps = static_cast<int64_t>(gridDim.x) * kWordExportWarps;
+    for (int64_t c = static_cast<int64_t>(blockIdx.x) * kWordExportWarps + (threadIdx.x >> 5); c < nchunks; c += nwarps)
+    {
+        const uint32_t item = static_cast<uint32_t>(c * 32) + lane;
+        const bool in = c * 32 + lane < n;
+        const uint32_t base = __ldg(&m.chunk[c].x);
+        const uint32_t vc = in ? __ldg(m.cnt + item) & 0xffu : 0u;
+        const uint32_t k = in ? src.word(item) : 0u;
+        if (!__any_sync(0xffffffffu, vc != 0))
+            continue;
+        const uint4 g = vc ? __ldg(m.edges + k) : make_uint4(0u, 0u, 0u, 0u);
+        const int incl = warp_inclusive_scan(static_cast<int>(vc));
+        const int excl = incl - static_cast<int>(vc);
+        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        for (int i0 = 0; i0 < total; i0 += 32)
+        {
+            const int i = i0 + lane;
+            const int s = item_slot(excl, i);
+            int j = i - __shfl_sync(0xffffffffu, excl, s);
+            uint32_t ex = __shfl_sync(0xffffffffu, g.x, s), ey = __shfl_sync(0xffffffffu, g.y, s),
+                     ez = __shfl_sync(0xffffffffu, g.z, s);
+            const uint32_t ks = __shfl_sync(0xffffffffu, k, s);
+            if (i < total)
+            {
+                // the point with j vertices before it in the word, then the axis
+                int b = 0;
+#pragma unroll
+                for (int w = 16; w > 0; w >>= 1)
+                {
+                    const uint32_t low = (1u << w) - 1u;
+                    const int before = __popc(ex & low) + __popc(ey & low) + __popc(ez & low);
+                    if (j >= before)
+                    {
+                        j -= before;
+                        b += w;
+                        ex >>= w;
+                        ey >>= w;
+                        ez >>= w;
+                    }
+                }
+                const uint32_t here = (ex & 1u) | ((ey & 1u) << 1) | ((ez & 1u) << 2);
+                const int axis = j == 0 ? __ffs(here) - 1 : (j == 2 || here != 7u ? 31 - __clz(here) : 1);
+                float v[3];
+                src.vertex(ks, b, axis, v);
+                float* out = verts + 3 * (static_cast<int64_t>(base) + i);
+                out[0] = v[0];
+                out[1] = v[1];
+                out[2] = v[2];
+            }
+        }
+    }
+}
+
+// Pass 3, the triangles.  FLIP: the second and third corner of every triangle
+// change places.  Without UNIQUE every triangle corner is a vertex of its own,
+// written here too.
 template <class Src, bool UNIQUE, bool FLIP>
-__global__ void __launch_bounds__(32 * kWordExportWarps) words_export_kernel(Src src, WordMesh m, float* __restrict__ verts, int64_t* __restrict__ faces)
+__global__ void __launch_bounds__(32 * kWordExportWarps) words_faces_kernel(Src src, WordMesh m, float* __restrict__ verts, int64_t* __restrict__ faces)
 {
     __shared__ WordTables tab;
     // per warp and cell of a round: its corners' vertices (point_vertices), or
-    // where their values are (Src::value_at)
+    // where their values are (Src::values_at)
     __shared__ unsigned long long corner_all[kWordExportWarps][32][9];
+    __shared__ uint32_t stage_all[kWordExportWarps][UNIQUE ? 32 * 15 : 1];
     for (int i = threadIdx.x; i < 256; i += blockDim.x)
     {
         tab.count[i] = words_detail::tri_count[i];
@@ -335,73 +407,32 @@ __global__ void __launch_bounds__(32 * kWordExportWarps) words_export_kernel(Src
     }
     __syncthreads();
     unsigned long long(*corner)[9] = corner_all[threadIdx.x >> 5];
+    uint32_t* stage = stage_all[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    const int64_t n = src.words();
-    const int64_t nchunks = (n + 31) / 32;
+    const int64_t n = src.words(), nchunks = (n + 31) / 32;
     const int64_t nwarps = static_cast<int64_t>(gridDim.x) * kWordExportWarps;
     for (int64_t c = static_cast<int64_t>(blockIdx.x) * kWordExportWarps + (threadIdx.x >> 5); c < nchunks; c += nwarps)
     {
-        const uint32_t k0 = static_cast<uint32_t>(c * 32), k = k0 + lane;
-        const uint32_t cn = c * 32 + lane < n ? m.cnt[k] : 0u;
-        if (!__any_sync(0xffffffffu, cn != 0))
+        const uint32_t item = static_cast<uint32_t>(c * 32) + lane;
+        const bool in = c * 32 + lane < n;
+        const uint32_t base = __ldg(&m.chunk[c].y);
+        const uint32_t cn = in ? __ldg(m.cnt + item) : 0u, cl = in ? __ldg(m.cells + item) : 0u;
+        const uint32_t k = in ? src.word(item) : 0u;
+        const uint32_t cells = (cn >> 8) ? cl : 0u;
+        if (!__any_sync(0xffffffffu, cells != 0))
             continue;
-        const uint2 base = m.chunk[c];
-        const uint32_t cells = (cn >> 8) ? m.cells[k] : 0u;
-        if (UNIQUE)
-        {
-            const uint32_t vc = cn & 0xffu;
-            const uint4 g = vc ? m.edges[k] : make_uint4(0u, 0u, 0u, 0u);
-            const int incl = warp_inclusive_scan(static_cast<int>(vc));
-            const int excl = incl - static_cast<int>(vc);
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
-            for (int i0 = 0; i0 < total; i0 += 32)
-            {
-                const int i = i0 + lane;
-                const int s = item_slot(excl, i);
-                int j = i - __shfl_sync(0xffffffffu, excl, s);
-                uint32_t ex = __shfl_sync(0xffffffffu, g.x, s), ey = __shfl_sync(0xffffffffu, g.y, s),
-                         ez = __shfl_sync(0xffffffffu, g.z, s);
-                if (i < total)
-                {
-                    // the point with j vertices before it in the word, then the axis
-                    int b = 0;
-#pragma unroll
-                    for (int w = 16; w > 0; w >>= 1)
-                    {
-                        const uint32_t low = (1u << w) - 1u;
-                        const int before = __popc(ex & low) + __popc(ey & low) + __popc(ez & low);
-                        if (j >= before)
-                        {
-                            j -= before;
-                            b += w;
-                            ex >>= w;
-                            ey >>= w;
-                            ez >>= w;
-                        }
-                    }
-                    const uint32_t here = (ex & 1u) | ((ey & 1u) << 1) | ((ez & 1u) << 2);
-                    const int axis = j == 0 ? __ffs(here) - 1 : (j == 2 || here != 7u ? 31 - __clz(here) : 1);
-                    float v[3];
-                    src.vertex(k0 + s, b, axis, v);
-                    float* out = verts + 3 * (static_cast<int64_t>(base.x) + i);
-                    out[0] = v[0];
-                    out[1] = v[1];
-                    out[2] = v[2];
-                }
-            }
-        }
         const int cc = __popc(cells);
         const int cincl = warp_inclusive_scan(cc);
         const int cexcl = cincl - cc;
         const int ctotal = __shfl_sync(0xffffffffu, cincl, 31);
-        int64_t at = base.y;
+        int64_t at = base;
         for (int i0 = 0; i0 < ctotal; i0 += 32)
         {
             const int i = i0 + lane;
             const int s = item_slot(cexcl, i);
             const int j = i - __shfl_sync(0xffffffffu, cexcl, s);
             const uint32_t cs = __shfl_sync(0xffffffffu, cells, s);
-            const uint32_t ks = k0 + s;
+            const uint32_t ks = __shfl_sync(0xffffffffu, k, s);
             uint32_t code = 0;
             int b = 0;
             if (i < ctotal)
@@ -409,18 +440,24 @@ __global__ void __launch_bounds__(32 * kWordExportWarps) words_export_kernel(Src
                 b = nth_set_bit(cs, j);
                 const WordRows r = src.rows(ks);
                 uint32_t sg[4], sh[4];
+                uint4 g[4];
                 sign_rows(src, r, sg, sh);
+                if constexpr (UNIQUE)
+                {
+                    // a word without vertices holds no edge of this cell: its entry is not read below
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        g[q] = __ldg(m.edges + r.idx[q]);
+                }
                 code = cell_code(sg, sh, b);
                 if constexpr (UNIQUE)
                 {
 #pragma unroll
                     for (int q = 0; q < 4; ++q)
                     {
-                        // a word without vertices holds no edge of this cell: its entry is not read below
-                        const unsigned long long p0 = point_vertices(m.edges[r.idx[q]], b);
-                        corner[lane][2 * q] = p0;
+                        corner[lane][2 * q] = point_vertices(g[q], b);
                         corner[lane][2 * q + 1] =
-                                b < 31 ? point_vertices(m.edges[r.idx[q]], b + 1) : point_vertices(m.edges[r.idx[q] + 1], 0);
+                                b < 31 ? point_vertices(g[q], b + 1) : point_vertices(__ldg(m.edges + r.idx[q] + 1), 0);
                     }
                 }
                 else
@@ -431,35 +468,47 @@ __global__ void __launch_bounds__(32 * kWordExportWarps) words_export_kernel(Src
             const int excl = incl - cnt;
             const int total = __shfl_sync(0xffffffffu, incl, 31);
             __syncwarp();
-            for (int e0 = 0; e0 < total; e0 += 32)
+            if constexpr (UNIQUE)
             {
-                const int e = e0 + lane;
-                const int es = item_slot(excl, e);
-                const int ej = e - __shfl_sync(0xffffffffu, excl, es);
-                const uint32_t ecode = __shfl_sync(0xffffffffu, code, es);
-                const uint32_t ek = __shfl_sync(0xffffffffu, ks, es);
-                const int eb = __shfl_sync(0xffffffffu, b, es);
-                if (e < total)
+                // a lane per cell parks its triangles' vertices, then all lanes write them
+                for (int j = 0; j < cnt; j += 3)
                 {
-                    const uint32_t ed = tab.edges[ecode][ej];
-                    const int lo = static_cast<int>(ed & 7u), axis = static_cast<int>(ed >> 3);
-                    const int slot = e % 3;
-                    const int64_t dst = at + e + (FLIP ? (slot == 0 ? 0 : 3 - 2 * slot) : 0);
-                    if constexpr (UNIQUE)
+#pragma unroll
+                    for (int t = 0; t < 3; ++t)
                     {
-                        const unsigned long long p = corner[es][lo];
-                        faces[dst] = static_cast<int64_t>((p >> 3) & 0xffffffffull) +
-                                     __popc(static_cast<uint32_t>(p) & ((1u << axis) - 1u));
+                        const uint32_t ed = tab.edges[code][j + t];
+                        const unsigned long long p = corner[lane][ed & 7u];
+                        // FLIP: the triangle's second and third corner change places
+                        stage[excl + j + (FLIP && t > 0 ? 3 - t : t)] =
+                                static_cast<uint32_t>(p >> 3) + __popc(static_cast<uint32_t>(p) & ((1u << (ed >> 3)) - 1u));
                     }
-                    else
+                }
+                __syncwarp();
+                for (int e = lane; e < total; e += 32)
+                    faces[at + e] = static_cast<int64_t>(stage[e]);
+            }
+            else
+            {
+                for (int e0 = 0; e0 < total; e0 += 32)
+                {
+                    const int e = e0 + lane;
+                    const int es = item_slot(excl, e);
+                    const int ej = e - __shfl_sync(0xffffffffu, excl, es);
+                    const uint32_t ecode = __shfl_sync(0xffffffffu, code, es);
+                    const uint32_t ek = __shfl_sync(0xffffffffu, ks, es);
+                    const int eb = __shfl_sync(0xffffffffu, b, es);
+                    if (e < total)
                     {
+                        const uint32_t ed = tab.edges[ecode][ej];
+                        const int lo = static_cast<int>(ed & 7u), axis = static_cast<int>(ed >> 3);
+                        const int slot = e % 3;
                         float v[3];
                         src.soup_vertex(ek, eb, lo, axis, corner[es][lo], corner[es][lo | (1 << axis)], v);
                         float* out = verts + 3 * (at + e);
                         out[0] = v[0];
                         out[1] = v[1];
                         out[2] = v[2];
-                        faces[dst] = at + e;
+                        faces[at + e + (FLIP ? (slot == 0 ? 0 : 3 - 2 * slot) : 0)] = at + e;
                     }
                 }
             }
@@ -472,6 +521,13 @@ __global__ void __launch_bounds__(32 * kWordExportWarps) words_export_kernel(Src
 inline int64_t word_tiles(int64_t words)
 {
     return (words + kWordTile - 1) / kWordTile;
+}
+
+// Grid of the vertex and face passes (words: an upper bound).
+inline int words_export_grid(int64_t words)
+{
+    const int64_t blocks = (words + 32 * kWordExportWarps - 1) / (32 * kWordExportWarps), cap = 8LL * sm_count();
+    return static_cast<int>(blocks < 1 ? 1 : (blocks < cap ? blocks : cap));
 }
 
 // Grid of the count and base passes (words: an upper bound).
