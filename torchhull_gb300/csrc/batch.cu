@@ -42,8 +42,11 @@ __global__ void batch_init_kernel(BatchPlan bp)
     for (int i = threadIdx.x; i < bp.nreq; i += blockDim.x)
     {
         bp.nodes[i] = static_cast<int64_t>(i) << kTagShift;
-        bp.node_skip[i] = 0;
-        bp.node_out[i] = 0;
+        for (int w = 0; w < bp.mask_words; ++w)
+        {
+            bp.node_skip[w * bp.node_cap + i] = 0;
+            bp.node_out[w * bp.node_cap + i] = 0;
+        }
     }
     if (threadIdx.x == 0)
         bp.ctr->count[0] = bp.nreq;
@@ -86,12 +89,12 @@ __device__ __forceinline__ int64_t level_entries(const BatchPlan& bp, int li, in
     return n < room ? n : (room > 0 ? room : 0);
 }
 
-template <int VARIANT>
+template <int VARIANT, int MW>
 __global__ void __launch_bounds__(32 * kBatchWarps, 2) batch_carve_kernel(BatchPlan bp)
 {
     cg::grid_group grid = cg::this_grid();
-    __shared__ WarpSlots slots_all[kBatchWarps];
-    WarpSlots& ws = slots_all[threadIdx.x >> 5];
+    __shared__ WarpSlots<MW> slots_all[kBatchWarps];
+    WarpSlots<MW>& ws = slots_all[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     BatchCounters* ctr = bp.ctr;
     const int64_t nwarps = static_cast<int64_t>(gridDim.x) * kBatchWarps;
@@ -121,24 +124,21 @@ __global__ void __launch_bounds__(32 * kBatchWarps, 2) batch_carve_kernel(BatchP
             const BatchReq& q = bp.reqs[static_cast<int>(node >> kTagShift)];
             const bool work = valid && q.level > li && !q.no_carve;
             const bool skips = work && q.skip_ok && (*q.nonbinary == 0);
-            const uint32_t view_bits = q.B >= 32 ? 0xffffffffu : ((1u << q.B) - 1u);
-            const uint32_t skipm = skips ? (bp.node_skip[start + pi] & view_bits) : 0u;
-            // views that see the cell out of the frame for good (partial requests)
-            const uint32_t outm = (work && q.partial) ? (bp.node_out[start + pi] & view_bits) : 0u;
-            const uint32_t skipall = skipm | outm;
-            const int count = work ? (q.B - __popc(skipall)) : 0;
-            const bool last = (li == q.level - 1);
-            ws.empty[lane] = 0;
-            ws.refine[lane] = 0;
-            ws.inside[lane] = (work && q.partial && last && skipm) ? 0xffu : 0u;
+            // skipped views, and those that see the cell out of the frame for good (partial requests)
+            uint32_t skipm[MW], outm[MW], all[MW], skipped = 0;
+            int count = work ? q.B : 0;
 #pragma unroll
-            for (int c = 0; c < 8; ++c)
+            for (int w = 0; w < MW; ++w)
             {
-                ws.cskip[lane][c] = 0;
-                ws.cout[lane][c] = 0;
+                const uint32_t vb = view_bits(q.B, w);
+                skipm[w] = skips ? (bp.node_skip[w * bp.node_cap + start + pi] & vb) : 0u;
+                outm[w] = (work && q.partial) ? (bp.node_out[w * bp.node_cap + start + pi] & vb) : 0u;
+                all[w] = skipm[w] | outm[w];
+                skipped |= skipm[w];
+                count -= work ? __popc(all[w]) : 0;
             }
-            // the children inherit the cell's out-of-frame views
-            ws.cout_all[lane] = outm;
+            const bool last = (li == q.level - 1);
+            ws.clear(lane, (work && q.partial && last && skipped) ? 0xffu : 0u, outm);
             const int incl = warp_inclusive_scan(count);
             const int excl = incl - count;
             const int total = __shfl_sync(0xffffffffu, incl, 31);
@@ -148,43 +148,23 @@ __global__ void __launch_bounds__(32 * kBatchWarps, 2) batch_carve_kernel(BatchP
                 const int k = k0 + lane;
                 const int s = item_slot(excl, k);
                 const int es = __shfl_sync(0xffffffffu, excl, s);
-                const uint32_t ms = __shfl_sync(0xffffffffu, skipall, s);
+                uint32_t alls[MW];
+#pragma unroll
+                for (int w = 0; w < MW; ++w)
+                    alls[w] = __shfl_sync(0xffffffffu, all[w], s);
                 const int64_t is = __shfl_sync(0xffffffffu, node, s);
-                const bool act = k < total;
-                ItemResult res{ 0, 0, 0, 0, 0 };
-                int b = 0;
-                bool produce = false;
-                if (act)
+                if (k < total)
                 {
                     const BatchReq& qq = bp.reqs[static_cast<int>(is >> kTagShift)];
-                    const uint32_t vb = qq.B >= 32 ? 0xffffffffu : ((1u << qq.B) - 1u);
-                    const uint32_t active = vb & ~ms;
-                    const int na = __popc(active);
-                    const int j = k - es;
-                    b = j < na ? select_bit(active, j) : 32 + (j - na);
+                    const int b = item_view<MW>(qq.B, alls, k - es);
                     float wx[3], wy[3], wz[3];
                     lattice_world(qq.corner, qq.length, is & kCellMask, li, inv_rc, wx, wy, wz);
-                    produce = qq.skip_ok && (*qq.nonbinary == 0) && (li + 1 < qq.level);
-                    const bool skip_inside = qq.partial != 0;
-                    const bool want_out = qq.partial && (li + 1 < qq.level) && b < 32;
+                    const bool produce = qq.skip_ok && (*qq.nonbinary == 0) && (li + 1 < qq.level) && b < 32 * MW;
+                    const bool want_out = qq.partial && (li + 1 < qq.level) && b < 32 * MW;
                     const int grow = li + 2 == qq.level ? 1 : 2;
-                    res = batch_item<VARIANT>(qq, b, wx, wy, wz, produce && b < 32, skip_inside, want_out, grow,
-                                              li + 1 == qq.level);
-                    if (res.out == 0xffu)
-                        atomicOr(&ws.cout_all[s], 1u << b);
-                    else
-                        for (uint32_t o = res.out; o; o &= o - 1)
-                            atomicOr(&ws.cout[s][__ffs(o) - 1], 1u << b);
-                    // merge into the slot's words: one shared atomic per non-zero word
-                    if (res.empty)
-                        atomicOr(&ws.empty[s], res.empty);
-                    if (res.refine)
-                        atomicOr(&ws.refine[s], res.refine);
-                    if (res.inside)
-                        atomicOr(&ws.inside[s], res.inside);
-                    if (produce)
-                        for (uint32_t m = res.skip; m; m &= m - 1)
-                            atomicOr(&ws.cskip[s][__ffs(m) - 1], 1u << (b & 31));
+                    merge_item<MW>(ws, s, b,
+                                   batch_item<VARIANT>(qq, b, wx, wy, wz, produce, qq.partial != 0, want_out, grow,
+                                                       li + 1 == qq.level));
                 }
             }
             __syncwarp();
@@ -205,10 +185,15 @@ __global__ void __launch_bounds__(32 * kBatchWarps, 2) batch_carve_kernel(BatchP
                     const bool produce_me = skips && (li + 1 < q.level);
                     const bool produce_out = work && q.partial && (li + 1 < q.level);
 #pragma unroll
-                    for (int c = 0; c < 8; ++c)
+                    for (int w = 0; w < MW; ++w)
                     {
-                        bp.child_skip[pi * 8 + c] = produce_me ? (ws.cskip[lane][c] | skipm) : 0u;
-                        bp.child_out[pi * 8 + c] = produce_out ? (ws.cout[lane][c] | ws.cout_all[lane]) : 0u;
+#pragma unroll
+                        for (int c = 0; c < 8; ++c)
+                        {
+                            const int64_t at = (w * bp.skip_cap + pi) * 8 + c;
+                            bp.child_skip[at] = produce_me ? (ws.cskip[w][lane][c] | skipm[w]) : 0u;
+                            bp.child_out[at] = produce_out ? (ws.cout[w][lane][c] | ws.cout_all[w][lane]) : 0u;
+                        }
                     }
                 }
             }
@@ -271,8 +256,13 @@ __global__ void __launch_bounds__(32 * kBatchWarps, 2) batch_carve_kernel(BatchP
                     if (out < bp.node_cap)
                     {
                         bp.nodes[out] = tag | (gx + (c & 1)) | ((gy + (c >> 1 & 1)) << sh) | ((gz + (c >> 2 & 1)) << (2 * sh));
-                        bp.node_skip[out] = i < bp.skip_cap ? bp.child_skip[i * 8 + c] : 0u;
-                        bp.node_out[out] = i < bp.skip_cap ? bp.child_out[i * 8 + c] : 0u;
+#pragma unroll
+                        for (int w = 0; w < MW; ++w)
+                        {
+                            const int64_t at = (w * bp.skip_cap + i) * 8 + c;
+                            bp.node_skip[w * bp.node_cap + out] = i < bp.skip_cap ? bp.child_skip[at] : 0u;
+                            bp.node_out[w * bp.node_cap + out] = i < bp.skip_cap ? bp.child_out[at] : 0u;
+                        }
                     }
                     else
                         atomicOr(&ctr->overflow, 1ull);
@@ -361,7 +351,9 @@ __global__ void __launch_bounds__(256) batch_cell_masks_kernel(BatchPlan bp, boo
             const int64_t node = bp.nodes[t];
             const BatchReq& q = bp.reqs[static_cast<int>(node >> kTagShift)];
             if (q.cell_masks && li == q.level - 1)
-                q.cell_masks[node & kCellMask] = set ? (bp.node_skip[t] | bp.node_out[t]) : 0u;
+                for (int w = 0; w < q.mask_words; ++w)
+                    q.cell_masks[(static_cast<int64_t>(w) << (3 * li)) + (node & kCellMask)] =
+                            set ? (bp.node_skip[w * bp.node_cap + t] | bp.node_out[w * bp.node_cap + t]) : 0u;
         }
     }
 }
@@ -379,24 +371,12 @@ void launch_batch_carve(const BatchPlan& bp, cudaStream_t s)
 {
     if (bp.max_level <= 0)
         return;
-    void (*kernel)(BatchPlan) = batch_carve_kernel<-1>;
-    switch (bp.variant)
-    {
-    case 0:
-        kernel = batch_carve_kernel<0>;
-        break;
-    case 1:
-        kernel = batch_carve_kernel<1>;
-        break;
-    case 2:
-        kernel = batch_carve_kernel<2>;
-        break;
-    case 3:
-        kernel = batch_carve_kernel<3>;
-        break;
-    default:
-        break;
-    }
+    static constexpr void (*kernels[2][5])(BatchPlan) = {
+        { batch_carve_kernel<-1, 1>, batch_carve_kernel<0, 1>, batch_carve_kernel<1, 1>, batch_carve_kernel<2, 1>, batch_carve_kernel<3, 1> },
+        { batch_carve_kernel<-1, kMaxMaskWords>, batch_carve_kernel<0, kMaxMaskWords>, batch_carve_kernel<1, kMaxMaskWords>,
+          batch_carve_kernel<2, kMaxMaskWords>, batch_carve_kernel<3, kMaxMaskWords> }
+    };
+    void (*kernel)(BatchPlan) = kernels[bp.mask_words > 1 ? 1 : 0][bp.variant >= 0 && bp.variant <= 3 ? bp.variant + 1 : 0];
     int per_sm = 0;
     TH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * kBatchWarps, 0));
     if (per_sm < 1)

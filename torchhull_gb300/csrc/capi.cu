@@ -20,6 +20,7 @@
 #include <sstream>
 
 #include "th_batch.cuh"
+#include "th_classify.cuh"
 #include "th_hull.cuh"
 #include "th_internal.h"
 #include "th_mc.cuh"
@@ -534,6 +535,7 @@ void prepare(HullSlot& s, const th_hull_args* a, cudaStream_t st, bool field_one
     const int64_t all_words = R * R * 2 * WR;
     s.word_cap = std::max<int64_t>(s.word_cap, std::min<int64_t>(all_words, int64_t{ 1 } << (batch_slot ? 23 : 25)));
     const int64_t word_cap = std::min<int64_t>(s.word_cap, all_words);
+    const int mask_words = mask_words_for(B);
 
     s.tf.ensure(sizeof(float) * std::max<int64_t>(B, 1) * 16);
     s.sat.ensure(sizeof(float) * std::max<int64_t>(B * H * W, 1));
@@ -549,11 +551,11 @@ void prepare(HullSlot& s, const th_hull_args* a, cudaStream_t st, bool field_one
     if (field_ones)
         s.ones.ensure(sizeof(uint32_t) * std::max<int64_t>(B * H * WW, 1));
     s.nodes.ensure(sizeof(int64_t) * node_cap);
-    s.node_skip.ensure(sizeof(uint32_t) * node_cap);
-    s.node_out.ensure(sizeof(uint32_t) * node_cap);
+    s.node_skip.ensure(sizeof(uint32_t) * mask_words * node_cap);
+    s.node_out.ensure(sizeof(uint32_t) * mask_words * node_cap);
     s.child_masks.ensure(node_cap);
-    s.child_skip.ensure(sizeof(uint32_t) * 8 * parent_cap);
-    s.child_out.ensure(sizeof(uint32_t) * 8 * parent_cap);
+    s.child_skip.ensure(sizeof(uint32_t) * 8 * mask_words * parent_cap);
+    s.child_out.ensure(sizeof(uint32_t) * 8 * mask_words * parent_cap);
     s.flags.ensure(sizeof(unsigned int) * 4);
     s.tile_sums.ensure(sizeof(unsigned long long) *
                        std::max<int64_t>((node_cap + kScanTile - 1) / kScanTile, word_tiles(word_cap)));
@@ -613,6 +615,7 @@ void prepare(HullSlot& s, const th_hull_args* a, cudaStream_t st, bool field_one
     p.node_cap = node_cap;
     p.child_masks = s.child_masks.as<uint8_t>();
     p.tile_sums = s.tile_sums.as<unsigned long long>();
+    p.mask_words = mask_words;
     p.node_skip = s.node_skip.as<uint32_t>();
     p.child_skip = s.child_skip.as<uint32_t>();
     p.node_out = s.node_out.as<uint32_t>();
@@ -626,7 +629,7 @@ void prepare(HullSlot& s, const th_hull_args* a, cudaStream_t st, bool field_one
     p.own_cell_masks = !batch_slot;
     if (cell_masks)
     {
-        if (s.cell_masks.ensure(sizeof(uint32_t) * (int64_t{ 1 } << (3 * (L - 1)))))
+        if (s.cell_masks.ensure(sizeof(uint32_t) * mask_words * (int64_t{ 1 } << (3 * (L - 1)))))
             TH_CUDA(cudaMemsetAsync(s.cell_masks.p, 0, s.cell_masks.bytes, st));
         p.cell_masks = s.cell_masks.as<uint32_t>();
     }
@@ -955,13 +958,16 @@ void run_batch(th_context* ctx, const th_hull_args* args, int32_t n, cudaStream_
     {
         bs.reqs.ensure(sizeof(BatchReq) * n);
         bs.nodes.ensure(sizeof(int64_t) * bs.node_cap);
-        bs.node_skip.ensure(sizeof(uint32_t) * bs.node_cap);
-        bs.node_out.ensure(sizeof(uint32_t) * bs.node_cap);
+        int mask_words = 1;
+        for (int32_t r = 0; r < n; ++r)
+            mask_words = std::max(mask_words, mask_words_for(args[r].batch));
+        bs.node_skip.ensure(sizeof(uint32_t) * mask_words * bs.node_cap);
+        bs.node_out.ensure(sizeof(uint32_t) * mask_words * bs.node_cap);
         // view-skip masks for up to a quarter of the pool's cells in one level
         const int64_t skip_cap = std::max<int64_t>(bs.node_cap / 4, 1);
         bs.child_masks.ensure(static_cast<size_t>(bs.node_cap));
-        bs.child_skip.ensure(sizeof(uint32_t) * 8 * skip_cap);
-        bs.child_out.ensure(sizeof(uint32_t) * 8 * skip_cap);
+        bs.child_skip.ensure(sizeof(uint32_t) * 8 * mask_words * skip_cap);
+        bs.child_out.ensure(sizeof(uint32_t) * 8 * mask_words * skip_cap);
         bs.block_sums.ensure(sizeof(unsigned long long) * 8 * sm_count());
         bs.ctr.ensure(sizeof(BatchCounters));
         for (int32_t r = 0; r < n; ++r)
@@ -995,6 +1001,7 @@ void run_batch(th_context* ctx, const th_hull_args* args, int32_t n, cudaStream_
             q.R = p.R;
             q.WR = p.WR;
             q.cell_masks = p.cell_masks;
+            q.mask_words = p.mask_words;
         }
         if (attempt == 0)
         {
@@ -1026,6 +1033,7 @@ void run_batch(th_context* ctx, const th_hull_args* args, int32_t n, cudaStream_
         bp.nreq = n;
         bp.max_level = max_level;
         bp.nodes = bs.nodes.as<int64_t>();
+        bp.mask_words = mask_words;
         bp.node_skip = bs.node_skip.as<uint32_t>();
         bp.node_out = bs.node_out.as<uint32_t>();
         bp.node_cap = bs.node_cap;

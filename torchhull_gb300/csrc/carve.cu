@@ -87,8 +87,11 @@ __global__ void hull_init_kernel(HullPlan p)
         c->level_off[0] = 0;
         c->level_off[1] = 1;
         p.nodes[0] = 0;
-        p.node_skip[0] = 0;
-        p.node_out[0] = 0;
+        for (int w = 0; w < p.mask_words; ++w)
+        {
+            p.node_skip[w * p.node_cap] = 0;
+            p.node_out[w * p.node_cap] = 0;
+        }
     }
 }
 
@@ -136,6 +139,15 @@ __device__ __forceinline__ void store_parent(const HullPlan& p, const LevelInfo&
     p.child_masks[pi] = static_cast<uint8_t>(mask);
 }
 
+// Adds the block's evaluated (parent, view) items to the level's counter.
+__device__ __forceinline__ void count_carved(const HullPlan& p, int li, unsigned long long items)
+{
+    unsigned long long total;
+    block_exclusive_scan(items, &total);
+    if (threadIdx.x == 0 && total)
+        atomicAdd(&p.ctr->items[li], total);
+}
+
 // Views over lanes: a group of LANES lanes owns one parent.
 template <int LANES, bool PARTIAL, bool OPENGL>
 __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_views_kernel(HullPlan p, int li)
@@ -146,45 +158,63 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_views_kernel
     const int sub = lane % LANES, grp = lane / LANES;
     const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-    // skip masks can come out of a ballot only when lane == view (<= 32 views)
-    const bool produce = L.produce && LANES == 32 && p.B <= 32;
-    const bool produce_out = L.produce_out && LANES == 32 && p.B <= 32;
+    // skip masks can come out of a ballot only when lane == view (of a word)
+    const bool produce = L.produce && LANES == 32;
+    const bool produce_out = L.produce_out && LANES == 32;
+    unsigned long long items = 0;
     for (int64_t base = warp * G; base < L.n; base += nwarps * G)
     {
         const int64_t pi = base + grp;
         const bool valid = pi < L.n;
-        if (lane == 0)
-            atomicAdd(&p.ctr->items[li],
-                      static_cast<unsigned long long>(p.B * (L.n - base < G ? L.n - base : G)));
-        uint32_t empty = 0, refine = 0, inside = 0, skip = 0, outb = 0;
+        items += static_cast<unsigned long long>(p.B * (L.n - base < G ? L.n - base : G));
+        uint32_t empty = 0, refine = 0, inside = 0;
+        float wx[3], wy[3], wz[3];
         if (valid)
-        {
-            float wx[3], wy[3], wz[3];
             lattice_world(p.rq->corner, p.rq->length, L.parents[pi], li, L.inv_rc, wx, wy, wz);
-            const ViewSource src = make_view_source(p.tf, p.sat, p.H, p.W);
-            for (int64_t b = sub; b < p.B; b += LANES)
+        const ViewSource src = make_view_source(p.tf, p.sat, p.H, p.W);
+        const bool keep = LANES == 32 && pi < p.parent_cap && !L.last; // the children's masks are kept
+        for (int64_t b0 = 0; b0 < p.B; b0 += LANES)
+        {
+            const int64_t b = b0 + sub;
+            uint32_t skip = 0, outb = 0;
+            if (valid && b < p.B)
             {
-                const ItemResult r = classify_item<PARTIAL, OPENGL>(src, b, wx, wy, wz, produce, L.skip_inside,
-                                                                    produce_out, L.skip_grow, L.last);
+                const bool word = b < 32 * kMaxMaskWords;
+                const ItemResult r = classify_item<PARTIAL, OPENGL>(src, b, wx, wy, wz, produce && word, L.skip_inside,
+                                                                    produce_out && word, L.skip_grow, L.last);
                 empty |= r.empty;
                 refine |= r.refine;
                 inside |= r.inside;
-                skip |= r.skip;
-                outb |= r.out;
+                skip = r.skip;
+                outb = r.out;
             }
-        }
-        uint32_t cskip[8], cout[8];
-        if (produce)
-        {
+            const int64_t w = b0 / 32;
+            if (keep && w < p.mask_words)
+            {
+                // one parent per warp: lane c writes the masks of child c
+                uint32_t cskip = 0, cout = 0;
+                if (produce || produce_out)
+                {
 #pragma unroll
-            for (int c = 0; c < 8; ++c)
-                cskip[c] = __ballot_sync(0xffffffffu, (skip >> c) & 1u);
-        }
-        if (produce_out)
-        {
-#pragma unroll
-            for (int c = 0; c < 8; ++c)
-                cout[c] = __ballot_sync(0xffffffffu, (outb >> c) & 1u);
+                    for (int c = 0; c < 8; ++c)
+                    {
+                        const uint32_t sk = __ballot_sync(0xffffffffu, (skip >> c) & 1u), ou = __ballot_sync(0xffffffffu, (outb >> c) & 1u);
+                        if (lane == c)
+                        {
+                            cskip = sk;
+                            cout = ou;
+                        }
+                    }
+                    // the children inherit the parent's skip views (all descendants are object there)
+                    if (produce)
+                        cskip |= L.parent_skip[w * p.node_cap + pi];
+                }
+                if (lane < 8)
+                {
+                    p.child_skip[w * p.parent_cap * 8 + pi * 8 + lane] = cskip;
+                    p.child_out[w * p.parent_cap * 8 + pi * 8 + lane] = cout;
+                }
+            }
         }
 #pragma unroll
         for (int off = LANES / 2; off > 0; off >>= 1)
@@ -196,113 +226,82 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_views_kernel
         if (valid && sub == 0)
         {
             store_parent(p, L, pi, empty, refine, inside, PARTIAL);
-            if (pi < p.parent_cap && !L.last)
+            if (LANES < 32 && pi < p.parent_cap && !L.last)
             {
-                // the children inherit the parent's skip views (all descendants are object there)
-                const uint32_t inherited = produce && L.skips ? L.parent_skip[pi] : 0u;
 #pragma unroll
                 for (int c = 0; c < 8; ++c)
                 {
-                    p.child_skip[pi * 8 + c] = produce ? (cskip[c] | inherited) : 0u;
-                    p.child_out[pi * 8 + c] = produce_out ? cout[c] : 0u;
+                    p.child_skip[pi * 8 + c] = 0u; // at most 16 views: one mask word
+                    p.child_out[pi * 8 + c] = 0u;
                 }
             }
         }
     }
+    count_carved(p, li, lane == 0 ? items : 0);
 }
 
 // (parent, view) items: a warp deals the unskipped views of a chunk of parents
 // out to its lanes.
-template <bool PARTIAL, bool OPENGL>
+template <bool PARTIAL, bool OPENGL, int MW>
 __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_items_kernel(HullPlan p, int li)
 {
-    __shared__ WarpSlots slots_all[kWarps];
-    WarpSlots& ws = slots_all[threadIdx.x >> 5];
+    __shared__ WarpSlots<MW> slots_all[kWarps];
+    WarpSlots<MW>& ws = slots_all[threadIdx.x >> 5];
     const LevelInfo L = level_info(p, li, PARTIAL);
     const int lane = threadIdx.x & 31;
     const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
     const int B = static_cast<int>(p.B);
-    const uint32_t view_bits = B >= 32 ? 0xffffffffu : ((1u << B) - 1u);
     // parents per chunk: enough chunks for every warp, at most one per lane
     const int64_t per = (L.n + nwarps - 1) / nwarps;
     const int ppw = static_cast<int>(per < 1 ? 1 : (per > 32 ? 32 : per));
+    unsigned long long items = 0;
 
     for (int64_t base = warp * ppw; base < L.n; base += nwarps * ppw)
     {
         const int64_t pi = base + lane;
         const bool valid = lane < ppw && pi < L.n;
         const int64_t idx = valid ? L.parents[pi] : 0;
-        const uint32_t skipm = (valid && L.skips) ? (L.parent_skip[pi] & view_bits) : 0u;
-        // views that see the parent out of the frame for good (partial mode)
-        const uint32_t outm = (valid && PARTIAL) ? (L.parent_out[pi] & view_bits) : 0u;
-        const uint32_t skipall = skipm | outm;
-        const int count = valid ? (B - __popc(skipall)) : 0;
-        ws.empty[lane] = 0;
-        ws.refine[lane] = 0;
+        // skipped views, and those that see the parent out of the frame for good (partial mode)
+        uint32_t skipm[MW], outm[MW], all[MW], skipped = 0;
+        int count = valid ? B : 0;
+#pragma unroll
+        for (int w = 0; w < MW; ++w)
+        {
+            const uint32_t vb = view_bits(B, w);
+            skipm[w] = (valid && L.skips) ? (L.parent_skip[w * p.node_cap + pi] & vb) : 0u;
+            outm[w] = (valid && PARTIAL) ? (L.parent_out[w * p.node_cap + pi] & vb) : 0u;
+            all[w] = skipm[w] | outm[w];
+            skipped |= skipm[w];
+            count -= __popc(all[w]);
+        }
         // a skipped view before the last level (partial mode) is one where
         // every child is fully inside the frame
-        ws.inside[lane] = (PARTIAL && L.last && skipm) ? 0xffu : 0u;
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-        {
-            ws.cskip[lane][c] = 0;
-            ws.cout[lane][c] = 0;
-        }
-        // the children inherit the parent's out-of-frame views
-        ws.cout_all[lane] = outm;
+        ws.clear(lane, (PARTIAL && L.last && skipped) ? 0xffu : 0u, outm);
         const int incl = warp_inclusive_scan(count);
         const int excl = incl - count;
         const int total = __shfl_sync(0xffffffffu, incl, 31);
-        if (lane == 0 && total > 0)
-            atomicAdd(&p.ctr->items[li], static_cast<unsigned long long>(total));
+        items += static_cast<unsigned long long>(total);
         __syncwarp();
         for (int k0 = 0; k0 < total; k0 += 32)
         {
             const int k = k0 + lane;
-            // slot s: the last lane whose exclusive offset is <= k
-            int s = 0;
-#pragma unroll
-            for (int step = 16; step > 0; step >>= 1)
-            {
-                const int e = __shfl_sync(0xffffffffu, excl, s + step);
-                if (s + step < 32 && e <= k)
-                    s += step;
-            }
+            const int s = item_slot(excl, k);
             const int es = __shfl_sync(0xffffffffu, excl, s);
-            const uint32_t ms = __shfl_sync(0xffffffffu, skipall, s);
+            uint32_t alls[MW];
+#pragma unroll
+            for (int w = 0; w < MW; ++w)
+                alls[w] = __shfl_sync(0xffffffffu, all[w], s);
             const int64_t is = __shfl_sync(0xffffffffu, idx, s);
-            ItemResult res{ 0, 0, 0, 0, 0 };
-            int b = 0;
-            const bool act = k < total;
-            if (act)
+            if (k < total)
             {
-                const int j = k - es;
-                const uint32_t active = view_bits & ~ms;
-                const int na = __popc(active);
-                b = j < na ? select_bit(active, j) : 32 + (j - na);
+                const int b = item_view<MW>(B, alls, k - es);
                 float wx[3], wy[3], wz[3];
                 lattice_world(p.rq->corner, p.rq->length, is, li, L.inv_rc, wx, wy, wz);
                 const ViewSource src = make_view_source(p.tf, p.sat, p.H, p.W);
-                res = classify_item<PARTIAL, OPENGL>(src, b, wx, wy, wz, L.produce && b < 32, L.skip_inside,
-                                                     L.produce_out && b < 32, L.skip_grow, L.last);
-                if (res.out == 0xffu)
-                    atomicOr(&ws.cout_all[s], 1u << b);
-                else
-                    for (uint32_t o = res.out; o; o &= o - 1)
-                        atomicOr(&ws.cout[s][__ffs(o) - 1], 1u << b);
-                // merge into the slot's words: one shared atomic per non-zero
-                // word (a slot's items sit in neighbouring lanes, so conflicts
-                // are short)
-                if (res.empty)
-                    atomicOr(&ws.empty[s], res.empty);
-                if (res.refine)
-                    atomicOr(&ws.refine[s], res.refine);
-                if (res.inside)
-                    atomicOr(&ws.inside[s], res.inside);
-                if (L.produce)
-                    for (uint32_t m = res.skip; m; m &= m - 1)
-                        atomicOr(&ws.cskip[s][__ffs(m) - 1], 1u << (b & 31));
+                merge_item<MW>(ws, s, b,
+                               classify_item<PARTIAL, OPENGL>(src, b, wx, wy, wz, L.produce && b < 32 * MW, L.skip_inside,
+                                                              L.produce_out && b < 32 * MW, L.skip_grow, L.last));
             }
         }
         __syncwarp();
@@ -312,15 +311,22 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_items_kernel
             if (pi < p.parent_cap && !L.last)
             {
 #pragma unroll
-                for (int c = 0; c < 8; ++c)
+                for (int w = 0; w < MW; ++w)
                 {
-                    p.child_skip[pi * 8 + c] = L.produce ? (ws.cskip[lane][c] | skipm) : 0u;
-                    p.child_out[pi * 8 + c] = L.produce_out ? (ws.cout[lane][c] | ws.cout_all[lane]) : 0u;
+                    uint32_t* cs = p.child_skip + w * p.parent_cap * 8 + pi * 8;
+                    uint32_t* co = p.child_out + w * p.parent_cap * 8 + pi * 8;
+#pragma unroll
+                    for (int c = 0; c < 8; ++c)
+                    {
+                        cs[c] = L.produce ? (ws.cskip[w][lane][c] | skipm[w]) : 0u;
+                        co[c] = L.produce_out ? (ws.cout[w][lane][c] | ws.cout_all[w][lane]) : 0u;
+                    }
                 }
             }
         }
         __syncwarp();
     }
+    count_carved(p, li, lane == 0 ? items : 0);
 }
 
 struct ChildCount
@@ -361,8 +367,12 @@ struct ChildEmit
                 if (out < p.node_cap)
                 {
                     p.nodes[out] = (gx + (k & 1)) | ((gy + (k >> 1 & 1)) << sh) | ((gz + (k >> 2 & 1)) << (2 * sh));
-                    p.node_skip[out] = has_skip ? __ldg(p.child_skip + i * 8 + k) : 0u;
-                    p.node_out[out] = has_skip ? __ldg(p.child_out + i * 8 + k) : 0u;
+                    for (int w = 0; w < p.mask_words; ++w)
+                    {
+                        const int64_t at = w * p.parent_cap * 8 + i * 8 + k;
+                        p.node_skip[w * p.node_cap + out] = has_skip ? __ldg(p.child_skip + at) : 0u;
+                        p.node_out[w * p.node_cap + out] = has_skip ? __ldg(p.child_out + at) : 0u;
+                    }
                 }
                 ++out;
             }
@@ -399,7 +409,11 @@ void launch_classify(const HullPlan& p, int li, int64_t max_parents, cudaStream_
     if (p.carve_variant[li] == 1)
     {
         // about one lane per (parent, view) item when the level is small
-        classify_items_kernel<PARTIAL, OPENGL><<<grid_for(max_parents * p.B, threads), threads, 0, s>>>(p, li);
+        const int grid = grid_for(max_parents * p.B, threads);
+        if (p.mask_words == 1)
+            classify_items_kernel<PARTIAL, OPENGL, 1><<<grid, threads, 0, s>>>(p, li);
+        else
+            classify_items_kernel<PARTIAL, OPENGL, kMaxMaskWords><<<grid, threads, 0, s>>>(p, li);
         return;
     }
     const int grid = grid_for(max_parents * 32, threads);

@@ -538,21 +538,23 @@ __global__ void __launch_bounds__(256) cell_masks_kernel(HullPlan p, bool set)
     const int64_t off = c->level_off[li];
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += stride)
-        p.cell_masks[p.nodes[off + k]] = set ? (p.node_skip[off + k] | p.node_out[off + k]) : 0u;
+        for (int w = 0; w < p.mask_words; ++w)
+            p.cell_masks[(static_cast<int64_t>(w) << (3 * li)) + p.nodes[off + k]] =
+                    set ? (p.node_skip[w * p.node_cap + off + k] | p.node_out[w * p.node_cap + off + k]) : 0u;
 }
 
-// Views of a corner whose field factor is exactly 1: the OR of the cell-mask
+// Views of mask word `word` whose factor at a corner is exactly 1: the OR of the cell-mask
 // entries of the level L-1 cells whose lattice holds the corner (x >> 1, and
 // also (x - 1) >> 1 for an even x > 0, per axis; cells beyond the grid and
 // cells that are no node hold 0).
-__device__ __forceinline__ uint32_t corner_view_mask(const HullPlan& p, int64_t gx, int64_t gy, int64_t gz)
+__device__ __forceinline__ uint32_t corner_view_mask(const HullPlan& p, int word, int64_t gx, int64_t gy, int64_t gz)
 {
-    // the table has at most 2^27 cells
+    // a plane of the table has at most 2^27 cells
     const uint32_t li = p.level - 1, r = 1u << li;
     const uint32_t x0 = static_cast<uint32_t>(gx) >> 1, y0 = static_cast<uint32_t>(gy) >> 1, z0 = static_cast<uint32_t>(gz) >> 1;
     const bool x_low = !(gx & 1) && gx > 0, y_low = !(gy & 1) && gy > 0, z_low = !(gz & 1) && gz > 0;
     const bool x_in = x0 < r, y_in = y0 < r, z_in = z0 < r;
-    const uint32_t* c = p.cell_masks + (x0 + (y0 << li) + (z0 << (2 * li)));
+    const uint32_t* c = p.cell_masks + (static_cast<int64_t>(word) << (3 * li)) + (x0 + (y0 << li) + (z0 << (2 * li)));
     // up to eight cells, a fixed pattern of predicated loads (issued together)
     uint32_t m = 0;
 #pragma unroll
@@ -616,9 +618,9 @@ __global__ void __launch_bounds__(32 * kMaskedWarps) field_masked_kernel(HullPla
             wx = __fmaf_rn(__fmul_rn(small_i2f(static_cast<int32_t>(gx)), inv_rc), length, cx);
             wy = __fmaf_rn(__fmul_rn(small_i2f(static_cast<int32_t>(gy)), inv_rc), length, cy);
             wz = __fmaf_rn(__fmul_rn(small_i2f(static_cast<int32_t>(gz)), inv_rc), length, cz);
-            if (b0 == 0)
-                skip = corner_view_mask(p, gx, gy, gz) & vb;
-            else
+            if (b0 < 32 * p.mask_words)
+                skip = corner_view_mask(p, static_cast<int>(b0 >> 5), gx, gy, gz) & vb;
+            if (b0 > 0)
                 value = p.values[t];
         }
         if (!__any_sync(0xffffffffu, skip != 0))

@@ -26,6 +26,7 @@ struct BatchReq
     uint32_t* rowbits;
     int64_t R, WR;
     uint32_t* cell_masks; // the field's cell-mask table (HullPlan::cell_masks) or nullptr
+    int32_t mask_words;   // its planes
 };
 
 struct BatchCounters
@@ -45,8 +46,9 @@ struct BatchPlan
     int32_t nreq;
     int32_t max_level;
     int64_t* nodes; // level lists back to back (level i starts after levels < i)
-    uint32_t* node_skip;
-    uint32_t* node_out; // out-of-frame views (HullPlan::node_out)
+    int32_t mask_words;  // planes of the masks below (the most any request needs)
+    uint32_t* node_skip; // [mask_words][node_cap]
+    uint32_t* node_out;  // [mask_words][node_cap] out-of-frame views (HullPlan::node_out)
     int64_t node_cap;
     BatchCounters* ctr;
     // (partial << 1) | opengl when every request shares it, -1 otherwise
@@ -54,8 +56,8 @@ struct BatchPlan
     // per cell of the level being carved: refined children, and the
     // children's view-skip masks for the first skip_cap cells
     uint8_t* child_masks;  // [node_cap]
-    uint32_t* child_skip;  // [skip_cap * 8]
-    uint32_t* child_out;   // [skip_cap * 8]
+    uint32_t* child_skip;  // [mask_words][skip_cap * 8]
+    uint32_t* child_out;   // [mask_words][skip_cap * 8]
     int64_t skip_cap;
     unsigned long long* block_sums; // [grid size] children per block
     uint32_t leaf_levels; // bit i: some request ends at level i

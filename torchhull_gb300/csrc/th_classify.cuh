@@ -170,21 +170,65 @@ __device__ __forceinline__ bool box_out(const Box& bb, float Hf, float Wf)
            fabsf(bb.minx) < lim && fabsf(bb.maxx) < lim && fabsf(bb.miny) < lim && fabsf(bb.maxy) < lim;
 }
 
+// View masks hold at most this many words of 32 views (HullPlan::mask_words).
+constexpr int kMaxMaskWords = 2;
+
+inline int mask_words_for(int64_t views)
+{
+    return views > 32 ? kMaxMaskWords : 1;
+}
+
+// The views of mask word w that a request with B views has.
+__device__ __forceinline__ uint32_t view_bits(int B, int w)
+{
+    const int n = B - 32 * w;
+    return n >= 32 ? 0xffffffffu : (n > 0 ? (1u << n) - 1u : 0u);
+}
+
 // Shared-memory accumulators of one warp's chunk of parents (one slot each).
+template <int MW>
 struct WarpSlots
 {
     uint32_t empty[32], refine[32], inside[32];
-    uint32_t cskip[32][8];
+    uint32_t cskip[MW][32][8];
     // out-of-frame view masks of the children: per child, and for all 8
-    uint32_t cout[32][8], cout_all[32];
+    uint32_t cout[MW][32][8], cout_all[MW][32];
+
+    __device__ __forceinline__ void clear(int lane, uint32_t inside_views, const uint32_t (&outm)[MW])
+    {
+        empty[lane] = 0;
+        refine[lane] = 0;
+        inside[lane] = inside_views;
+#pragma unroll
+        for (int w = 0; w < MW; ++w)
+        {
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+            {
+                cskip[w][lane][c] = 0;
+                cout[w][lane][c] = 0;
+            }
+            // the children inherit the parent's out-of-frame views
+            cout_all[w][lane] = outm[w];
+        }
+    }
 };
 
-// Position of the j-th set bit of m (j < popc(m)).
-__device__ __forceinline__ int select_bit(uint32_t m, int j)
+// View of item j of a parent: its j-th view that is not in all (later views
+// than the masks hold come last).
+template <int MW>
+__device__ __forceinline__ int item_view(int B, const uint32_t (&all)[MW], int j)
 {
-    for (int t = 0; t < j; ++t)
-        m &= m - 1;
-    return __ffs(m) - 1;
+#pragma unroll
+    for (int w = 0; w < MW; ++w)
+    {
+        const uint32_t active = view_bits(B, w) & ~all[w];
+        const int n = __popc(active);
+        if (j < n)
+            return 32 * w + nth_set_bit(active, j);
+        j -= n;
+    }
+    return 32 * MW + j;
 }
 
 // World coordinates of the lattice of the cell idx (ravelled at resolution
@@ -373,5 +417,29 @@ __device__ __forceinline__ ItemResult classify_item(const ViewSource& p,
     return out;
 }
 
+// Merges an item's outcome into its slot: one shared atomic per non-zero word
+// (a slot's items sit in neighbouring lanes, so conflicts are short).
+template <int MW>
+__device__ __forceinline__ void merge_item(WarpSlots<MW>& ws, int s, int b, const ItemResult& res)
+{
+    if (b < 32 * MW)
+    {
+        const int w = b >> 5;
+        const uint32_t bit = 1u << (b & 31);
+        if (res.out == 0xffu)
+            atomicOr(&ws.cout_all[w][s], bit);
+        else
+            for (uint32_t o = res.out; o; o &= o - 1)
+                atomicOr(&ws.cout[w][s][__ffs(o) - 1], bit);
+        for (uint32_t m = res.skip; m; m &= m - 1)
+            atomicOr(&ws.cskip[w][s][__ffs(m) - 1], bit);
+    }
+    if (res.empty)
+        atomicOr(&ws.empty[s], res.empty);
+    if (res.refine)
+        atomicOr(&ws.refine[s], res.refine);
+    if (res.inside)
+        atomicOr(&ws.inside[s], res.inside);
+}
 
 } // namespace th

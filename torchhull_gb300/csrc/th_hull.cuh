@@ -73,21 +73,24 @@ struct HullPlan
     int64_t node_cap;
     uint8_t* child_masks; // one byte per parent of the current level
     unsigned long long* tile_sums;
-    // View skipping (binary masks only).  node_skip[k] has bit b (b < 32) set
-    // when view b need not be evaluated for any descendant of node k: the
-    // box of node k or of one of its ancestors, grown by two pixels, lies
-    // inside the image and holds only ones, so every descendant is "object"
-    // there (and, in partial mode, fully inside the frame).  child_skip holds
-    // the same masks for the 8 children of each parent of the current level.
-    uint32_t* node_skip;  // [node_cap]
-    uint32_t* child_skip; // [parent_cap * 8]
+    // View skipping (binary masks only).  node_skip[k] has bit b set when view
+    // b need not be evaluated for any descendant of node k: the box of node k
+    // or of one of its ancestors, grown by two pixels, lies inside the image
+    // and holds only ones, so every descendant is "object" there (and, in
+    // partial mode, fully inside the frame).  child_skip holds the same masks
+    // for the 8 children of each parent of the current level.
+    // All masks have mask_words planes of 32 views each (plane w: views 32 w
+    // to 32 w + 31); later views have no bit and are always evaluated.
+    int mask_words;       // 1 or 2
+    uint32_t* node_skip;  // [mask_words][node_cap]
+    uint32_t* child_skip; // [mask_words][parent_cap * 8]
     // Out-of-frame views (partial mode): node_out[k] has bit b when node k's
     // box in view b lies more than 2 pixels outside the image (box_out); no
     // descendant's item in view b can change anything, so the item kernel
     // skips it and the children inherit the bit.  child_out: the same for
     // the 8 children of each parent of the current level.
-    uint32_t* node_out;   // [node_cap]
-    uint32_t* child_out;  // [parent_cap * 8]
+    uint32_t* node_out;   // [mask_words][node_cap]
+    uint32_t* child_out;  // [mask_words][parent_cap * 8]
     int64_t parent_cap;
     // carve kernel per parent level: 0 = views over lanes, 1 = (parent, view) items
     uint8_t carve_variant[kMaxLevel];
@@ -108,7 +111,7 @@ struct HullPlan
     // weights in [0, 1], or a point out of the frame).  cell_masks is a dense
     // table over the cells of level L-1, scattered before the field and
     // cleared after it (nullptr: no table, every pair is evaluated).
-    uint32_t* cell_masks; // [8^(L-1)]
+    uint32_t* cell_masks; // [mask_words][8^(L-1)]
     bool own_cell_masks;  // launch_field scatters and clears the table (the batched form does it itself)
     // corner grid: R^3 points, one bit each, rows of WR 64-bit words (x fastest)
     int64_t R, WR;
