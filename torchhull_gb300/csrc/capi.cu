@@ -414,7 +414,7 @@ struct th_context
     th::BatchState bstate;
     th::DevBuf blur_scratch;
     th::DevBuf blurred; // masks blurred by th_visual_hull_blurred
-    th::DevBuf sat_aux; // th_integral_image: its 0/1 flag word, then the single pass's scratch
+    th::DevBuf sat_aux; // th_integral_image: its 0/1 flag word, then the bit passes' scratch
     cudaEvent_t sat_aux_done = nullptr; // the last th_integral_image that used sat_aux
     th::McSlot mc;
     bool profiling = false;

@@ -51,20 +51,20 @@ int grid_for(int64_t work_items, int threads);
 // copy-engine memset could.
 void launch_zero(void* p, size_t bytes, cudaStream_t s);
 
-// Scratch of the single-pass integral image (sat.cu): device memory of at
-// least sat_scratch_bytes(B, H, W, dtype) bytes (each launch clears what it needs).
+// Scratch of the integral image of 0/1 masks (sat.cu): 16-byte aligned device
+// memory of at least sat_scratch_bytes(B, H, W, dtype) bytes, contents undefined.
 struct SatScratch
 {
     void* p = nullptr;
 };
 
-// Bytes of scratch the single pass needs, 0 when it does not apply.
+// Bytes of scratch the bit passes need, 0 when they do not apply.
 int64_t sat_scratch_bytes(int64_t B, int64_t H, int64_t W, int dtype);
 
 // Integral image (sat.cu).  masks [B,H,W] of dtype, out [B,H,W] float32.
 // nonbinary (optional, zeroed by the caller) is set non-zero if any mask value
-// is neither 0 nor 1.  With scratch and nonbinary, 0/1 masks take the single
-// pass; otherwise (and after it, gated on the device) the exact two passes.
+// is neither 0 nor 1.  With scratch and nonbinary, 0/1 masks take the bit
+// passes; otherwise (and after them, gated on the device) the exact two passes.
 void launch_integral_image(const void* masks,
                            int dtype,
                            int64_t B,
