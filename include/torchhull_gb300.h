@@ -135,6 +135,10 @@ th_status th_visual_hull_export_candidates(th_context* ctx, int32_t level, int64
  * (2^level+1)^3) and values (visual_hull_cuda.cu:582-894, RavelledSparseTensor). */
 th_status th_visual_hull_export_field(th_context* ctx, int64_t* indices, float* values, void* stream);
 
+/* The same with the indices of a coalesced sparse tensor of size (1, R, R, R):
+ * four rows (0, z, y, x) of num_corners entries each. */
+th_status th_visual_hull_export_field_coo(th_context* ctx, int64_t* indices, float* values, void* stream);
+
 /*
  * gaussian_blur(images, kernel_size, sigma, sparse, dtype) for images
  * [B,H,W,1] contiguous on the device; out is [B,H,W,1] contiguous of

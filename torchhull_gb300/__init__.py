@@ -98,11 +98,6 @@ def sparse_visual_hull_field(
     Indices are (0, z, y, x), values the product of the views' mask samples
     (reference: visual_hull_cuda.cu:522-580, :896-914).
     """
-    idx, values, r = _extension().sparse_visual_hull_field_raw(
+    return _extension().sparse_visual_hull_field(
         masks, transforms, level, cube_corner_bfl, cube_length, masks_partial, transforms_convention
     )
-    z = idx // (r * r)
-    y = idx // r % r
-    x = idx % r
-    indices = torch.stack([torch.zeros_like(idx), z, y, x])
-    return torch.sparse_coo_tensor(indices, values, (1, r, r, r)).coalesce()

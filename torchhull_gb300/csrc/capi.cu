@@ -184,7 +184,7 @@ bool is_image_dtype(int d)
 // Pools and the state of the last request of one context.
 struct HullSlot
 {
-    DevBuf tf, sat, ones, cell_masks, nodes, node_skip, node_out, child_masks, child_skip, child_out, tile_sums, bitmap,
+    DevBuf tf, sat, ones, cell_masks, nodes, node_skip, node_out, child_masks, child_skip, child_out, carve_sums, tile_sums, bitmap,
             rowbits, rows, row_slot, row_cnt, row_place, present, runs, word_list, rank, sign, word_cnt, word_cells, word_edges, word_chunk,
             corners, values, counters, flags, sat_scratch;
     int64_t node_cap = 0, corner_cap = 0, parent_cap = 0, word_cap = 0;
@@ -219,7 +219,7 @@ struct HullSlot
 
     std::vector<const DevBuf*> buffers() const
     {
-        return { &tf,     &sat,  &ones,  &cell_masks,   &nodes,     &node_skip,   &node_out,  &child_masks, &child_skip, &child_out, &tile_sums,
+        return { &tf,     &sat,  &ones,  &cell_masks,   &nodes,     &node_skip,   &node_out,  &child_masks, &child_skip, &child_out, &carve_sums, &tile_sums,
                  &bitmap, &rowbits, &rows, &row_slot, &row_cnt, &row_place, &present, &runs, &word_list, &rank, &sign, &word_cnt, &word_cells,
                  &word_edges, &word_chunk, &corners, &values, &counters, &flags, &sat_scratch, &rq };
     }
@@ -559,6 +559,7 @@ void prepare(HullSlot& s, const th_hull_args* a, cudaStream_t st, bool field_one
     s.flags.ensure(sizeof(unsigned int) * 4);
     s.tile_sums.ensure(sizeof(unsigned long long) *
                        std::max<int64_t>((node_cap + kScanTile - 1) / kScanTile, word_tiles(word_cap)));
+    s.carve_sums.ensure(2 * sizeof(uint32_t) * (node_cap / 1024 + 4));
     const int64_t words = R * R * WR;
     const int64_t rwords = (R * R + 31) / 32;
     if (s.bitmap.ensure(sizeof(uint64_t) * words))
@@ -615,6 +616,8 @@ void prepare(HullSlot& s, const th_hull_args* a, cudaStream_t st, bool field_one
     p.node_cap = node_cap;
     p.child_masks = s.child_masks.as<uint8_t>();
     p.tile_sums = s.tile_sums.as<unsigned long long>();
+    p.carve_sums[0] = s.carve_sums.as<uint32_t>();
+    p.carve_sums[1] = p.carve_sums[0] + node_cap / 1024 + 4;
     p.mask_words = mask_words;
     p.node_skip = s.node_skip.as<uint32_t>();
     p.child_skip = s.child_skip.as<uint32_t>();
@@ -659,12 +662,12 @@ void prepare(HullSlot& s, const th_hull_args* a, cudaStream_t st, bool field_one
     p.values = s.values.as<float>();
     p.corner_cap = corner_cap;
     p.ctr = s.counters.as<DevCounters>();
+    p.host_ctr = s.host_d;
     // the per-request inputs the carve and field kernels read from the device
     s.rq.ensure(sizeof(ReqConsts));
     if (!s.host_rq)
         alloc_mapped(&s.host_rq, &s.host_rq_d);
     *s.host_rq = ReqConsts{ { p.corner[0], p.corner[1], p.corner[2] }, p.length, p.masks };
-    small_copy(s.rq.p, s.host_rq_d, sizeof(ReqConsts), st);
     p.rq = s.rq.as<ReqConsts>();
 }
 
@@ -706,16 +709,18 @@ void enqueue_core(th_context* ctx, HullSlot& s, cudaStream_t st, StageEvents* ev
 {
     const HullPlan& p = s.plan;
     const int L = p.level;
-    launch_hull_init(p, st);
     // With an empty image every child is empty in the first view (the
     // reference samples zeros everywhere), so the octree stops at the root;
     // without views nothing is refined either.  Skip the carve in both cases.
     const bool carve = p.B > 0 && p.H > 0 && p.W > 0;
     if (tune)
         TH_CUDA(cudaEventRecord(ctx->tune_ev[0], st));
+    const int top = carve ? top_levels(p.level) : 0;
+    if (carve)
+        launch_top(p, st);
     for (int li = 0; li < p.level; ++li)
     {
-        if (carve)
+        if (carve && li >= top)
             launch_carve_level(p, li, st);
         if (ev)
             ev->record(2 + li, st);
@@ -733,7 +738,6 @@ void enqueue_core(th_context* ctx, HullSlot& s, cudaStream_t st, StageEvents* ev
     launch_marching_cubes(p, st);
     if (ev)
         ev->record(L + 5, st);
-    small_copy(s.host_d, p.ctr, sizeof(DevCounters), st);
 }
 
 // enqueue_core as a graph: captured once per plan (the per-request corner,
@@ -812,14 +816,15 @@ void run_hull_once(th_context* ctx,
         {
             if (ev)
                 ev->record(0, st);
-            launch_convert_transforms(a->transforms, a->transforms_dtype, a->batch, s.tf.as<float>(), st);
-            launch_zero(s.flags.p, sizeof(unsigned int), st);
+            launch_begin(p, a->transforms, a->transforms_dtype, s.host_rq_d, s.flags.as<unsigned int>(), true, st);
             launch_integral_image(a->masks, a->masks_dtype, a->batch, a->height, a->width, s.sat.as<float>(), st,
                                   s.flags.as<unsigned int>(),
                                   ctx->sat_single_pass ? SatScratch{ s.sat_scratch.p } : SatScratch{});
             if (ev)
                 ev->record(1, st);
         }
+        else
+            launch_begin(p, a->transforms, a->transforms_dtype, s.host_rq_d, s.flags.as<unsigned int>(), false, st);
         if (ctx->graphs && !ev && !carve_ms)
             replay_core(s, st);
         else
@@ -835,7 +840,10 @@ void run_hull_once(th_context* ctx,
         if ((ovf & ~int64_t{ kOverflowParents }) == 0)
             break;
         if (ovf & kOverflowNodes)
+        {
             s.node_cap *= 4;
+            s.unfinished = true; // cells past the pool's end are not cleared from the cell masks
+        }
         if (ovf & kOverflowCorners)
             s.corner_cap *= 4;
         if (ovf & kOverflowWords)
@@ -976,7 +984,8 @@ void run_batch(th_context* ctx, const th_hull_args* args, int32_t n, cudaStream_
             HullSlot& s = ctx->batch[r];
             prepare(s, a, st, ctx->field_ones, ctx->field_masks, true);
             s.unfinished = true;
-            launch_zero(s.plan.ctr, counter_bytes(s.plan.R), st);
+            if (attempt > 0)
+                launch_begin(s.plan, a->transforms, a->transforms_dtype, s.host_rq_d, s.flags.as<unsigned int>(), false, st);
             const HullPlan& p = s.plan;
             BatchReq& q = bs.host_reqs[r];
             q = BatchReq{};
@@ -1015,8 +1024,7 @@ void run_batch(th_context* ctx, const th_hull_args* args, int32_t n, cudaStream_
                 const th_hull_args* a = &args[r];
                 HullSlot& s = ctx->batch[r];
                 cudaStream_t sr = bs.streams[r % nstreams];
-                launch_convert_transforms(a->transforms, a->transforms_dtype, a->batch, s.tf.as<float>(), sr);
-                launch_zero(s.flags.p, sizeof(unsigned int), sr);
+                launch_begin(s.plan, a->transforms, a->transforms_dtype, s.host_rq_d, s.flags.as<unsigned int>(), true, sr);
                 launch_integral_image(a->masks, a->masks_dtype, a->batch, a->height, a->width, s.sat.as<float>(), sr,
                                       s.flags.as<unsigned int>(),
                                       ctx->sat_single_pass ? SatScratch{ s.sat_scratch.p } : SatScratch{});
@@ -1084,8 +1092,6 @@ void run_batch(th_context* ctx, const th_hull_args* args, int32_t n, cudaStream_
         }
         launch_batch_cell_masks(bp, false, st);
         small_copy(bs.host_ctr_d, bp.ctr, sizeof(BatchCounters), st);
-        for (int32_t r = 0; r < n; ++r)
-            small_copy(ctx->batch[r].host_d, ctx->batch[r].plan.ctr, sizeof(DevCounters), st);
         TH_CUDA(cudaStreamSynchronize(st));
         bool retry = false;
         if (bs.host_ctr->overflow)
@@ -1705,6 +1711,24 @@ th_status th_visual_hull_export_field(th_context* ctx, int64_t* indices, float* 
             if (!indices || !values)
                 throw ArgError{ TH_ERR_INVALID_ARGUMENT, "indices or values pointer is NULL" };
             launch_export_field(s.plan, n, indices, values, st);
+        }
+        TH_CUDA(cudaEventRecord(s.done, st));
+    });
+}
+
+th_status th_visual_hull_export_field_coo(th_context* ctx, int64_t* indices, float* values, void* stream)
+{
+    return guarded(ctx, [&] {
+        HullSlot& s = ctx->hull;
+        if (!s.has_result)
+            throw ArgError{ TH_ERR_STATE, "export called without a successful th_visual_hull" };
+        const int64_t n = s.info.num_corners;
+        auto st = static_cast<cudaStream_t>(stream);
+        if (n > 0)
+        {
+            if (!indices || !values)
+                throw ArgError{ TH_ERR_INVALID_ARGUMENT, "indices or values pointer is NULL" };
+            launch_export_field_coo(s.plan, n, indices, values, st);
         }
         TH_CUDA(cudaEventRecord(s.done, st));
     });

@@ -1,4 +1,5 @@
-// Octree carving: one level per launch pair (classify, then compact).
+// Octree carving: the first levels in one launch, then one launch pair per
+// level (classify, then compact), the last level without the second.
 //
 // Reference: classify_children_full / _partial (visual_hull_cuda.cu:168-417)
 // run one thread per child and project each of the child's 8 corners for
@@ -51,12 +52,15 @@
 // unclamped box area; a child whose rounded box leaves the int32 range takes
 // the exact int64 path for that view.
 //
-// The 8 child flags of a parent become one byte; a device-wide scan over the
-// popcounts then writes the refined children (and their skip masks) in the
-// reference's stable order (parent order, then child index), and its last
-// block stores the level size on the device for the next level.
+// The 8 child flags of a parent become one byte; children_kernel writes the
+// refined children (and their masks) in the reference's stable order (parent
+// order, then child index) and stores the level's size on the device for the
+// next one.
 
+#include <algorithm>
 #include <cfloat>
+#include <cooperative_groups.h>
+#include <cstddef>
 
 #include "th_classify.cuh"
 #include "th_hull.cuh"
@@ -78,20 +82,40 @@ constexpr int kWarps = TH_CARVE_WARPS; // warps per block of the classify kernel
 // resident blocks per SM the classify kernels' register budget is cut for
 constexpr int kMinBlocks = TH_CARVE_MIN_BLOCKS;
 
-__global__ void hull_init_kernel(HullPlan p)
+template <int DT>
+__device__ __forceinline__ float transform_value(const void* tf, int64_t i)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0)
+    return load_f32<DT>(tf, i);
+}
+
+__global__ void __launch_bounds__(256) begin_kernel(HullPlan p, const void* tf, int tf_dtype, const ReqConsts* host_rq, ReqConsts* rq, float* out, unsigned int* flags, bool clear_flags)
+{
+    const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t i = t; i < p.B * 16; i += stride)
+        out[i] = tf_dtype == TH_FLOAT32 ? transform_value<TH_FLOAT32>(tf, i)
+                 : tf_dtype == TH_FLOAT64 ? transform_value<TH_FLOAT64>(tf, i) : transform_value<TH_FLOAT16>(tf, i);
+    // the counters: level 0 is the root, level 1 starts behind it
+    constexpr int64_t kWords = sizeof(DevCounters) / 8;
+    constexpr int64_t kCount0 = offsetof(DevCounters, level_count) / 8, kOff1 = offsetof(DevCounters, level_off) / 8 + 1;
+    auto* ctr = reinterpret_cast<unsigned long long*>(p.ctr);
+    for (int64_t i = t; i < kWords; i += stride)
+        ctr[i] = i == kCount0 || i == kOff1 ? 1ull : 0ull;
+    for (int64_t i = t; i < p.R * p.R / 256 + 2; i += stride)
+        p.coarse[i] = make_uint2(0u, 0u);
+    if (t < 4)
+        p.carve_sums[t & 1][t >> 1] = 0;
+    if (t == 0)
     {
-        DevCounters* c = p.ctr;
-        c->level_count[0] = 1;
-        c->level_off[0] = 0;
-        c->level_off[1] = 1;
         p.nodes[0] = 0;
         for (int w = 0; w < p.mask_words; ++w)
         {
             p.node_skip[w * p.node_cap] = 0;
             p.node_out[w * p.node_cap] = 0;
         }
+        *rq = *host_rq;
+        if (clear_flags)
+            *flags = 0;
     }
 }
 
@@ -131,21 +155,66 @@ __device__ __forceinline__ LevelInfo level_info(const HullPlan& p, int li, bool 
     return L;
 }
 
-__device__ __forceinline__ void store_parent(const HullPlan& p, const LevelInfo& L, int64_t pi, uint32_t empty, uint32_t refine, uint32_t inside, bool partial)
+// The refined children of a warp's parents (base: its first parent; valid
+// lanes hold parent pi and cell idx): their mask is kept; before the last
+// level their number goes into the level's sums of 1024 parents, for the
+// compaction; at the last level they are the leaves, whose corners are marked
+// at once (the leaf list itself is written only when its candidates are
+// exported) and counted into leaves.
+__device__ __forceinline__ void finish_parents(const HullPlan& p, const LevelInfo& L, int li, int64_t base, bool valid, int64_t pi, int64_t idx, uint32_t empty, uint32_t refine, uint32_t inside, bool partial, uint32_t& leaves)
 {
-    uint32_t mask = refine & ~empty;
-    if (partial && L.last)
-        mask &= inside;
-    p.child_masks[pi] = static_cast<uint8_t>(mask);
+    uint32_t mask = 0;
+    if (valid)
+    {
+        mask = refine & ~empty;
+        if (partial && L.last)
+            mask &= inside;
+        p.child_masks[pi] = static_cast<uint8_t>(mask);
+    }
+    if (L.last)
+    {
+        if (mask)
+        {
+            const int64_t r = int64_t{ 1 } << li;
+            mark_children_corners(p.bitmap, p.rowbits, p.R, p.WR, 2 * (idx & (r - 1)), 2 * ((idx >> li) & (r - 1)),
+                                  2 * (idx >> (2 * li)), mask);
+            leaves += __popc(mask);
+        }
+        return;
+    }
+    // a warp's parents lie in at most two groups
+    const int64_t g0 = base >> 10;
+    const uint32_t cnt = __popc(mask);
+    const bool second = valid && (pi >> 10) != g0;
+    const uint32_t a = __reduce_add_sync(0xffffffffu, second ? 0u : cnt), b = __reduce_add_sync(0xffffffffu, second ? cnt : 0u);
+    if ((threadIdx.x & 31) == 0)
+    {
+        if (a)
+            atomicAdd(p.carve_sums[li & 1] + g0, a);
+        if (b)
+            atomicAdd(p.carve_sums[li & 1] + g0 + 1, b);
+    }
 }
 
-// Adds the block's evaluated (parent, view) items to the level's counter.
-__device__ __forceinline__ void count_carved(const HullPlan& p, int li, unsigned long long items)
+// Adds the block's evaluated (parent, view) items (lane 0's) and leaves (every
+// lane's) to the request's counters.
+__device__ __forceinline__ void count_carved(const HullPlan& p, int li, uint32_t items, uint32_t leaves)
 {
-    unsigned long long total;
-    block_exclusive_scan(items, &total);
-    if (threadIdx.x == 0 && total)
-        atomicAdd(&p.ctr->items[li], total);
+    __shared__ unsigned long long sums[2];
+    if (threadIdx.x < 2)
+        sums[threadIdx.x] = 0;
+    __syncthreads();
+    leaves = __reduce_add_sync(0xffffffffu, leaves);
+    if ((threadIdx.x & 31) == 0)
+    {
+        if (items)
+            atomicAdd(&sums[0], static_cast<unsigned long long>(items));
+        if (leaves)
+            atomicAdd(&sums[1], static_cast<unsigned long long>(leaves));
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 && sums[threadIdx.x])
+        atomicAdd(threadIdx.x == 0 ? &p.ctr->items[li] : &p.ctr->leaves, sums[threadIdx.x]);
 }
 
 // Views over lanes: a group of LANES lanes owns one parent.
@@ -161,16 +230,17 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_views_kernel
     // skip masks can come out of a ballot only when lane == view (of a word)
     const bool produce = L.produce && LANES == 32;
     const bool produce_out = L.produce_out && LANES == 32;
-    unsigned long long items = 0;
+    uint32_t items = 0, leaves = 0; // a warp's items of one level: below 2^32
     for (int64_t base = warp * G; base < L.n; base += nwarps * G)
     {
         const int64_t pi = base + grp;
         const bool valid = pi < L.n;
-        items += static_cast<unsigned long long>(p.B * (L.n - base < G ? L.n - base : G));
+        items += static_cast<uint32_t>(p.B * (L.n - base < G ? L.n - base : G));
         uint32_t empty = 0, refine = 0, inside = 0;
         float wx[3], wy[3], wz[3];
+        const int64_t idx = valid ? L.parents[pi] : 0;
         if (valid)
-            lattice_world(p.rq->corner, p.rq->length, L.parents[pi], li, L.inv_rc, wx, wy, wz);
+            lattice_world(p.rq->corner, p.rq->length, idx, li, L.inv_rc, wx, wy, wz);
         const ViewSource src = make_view_source(p.tf, p.sat, p.H, p.W);
         const bool keep = LANES == 32 && pi < p.parent_cap && !L.last; // the children's masks are kept
         for (int64_t b0 = 0; b0 < p.B; b0 += LANES)
@@ -223,21 +293,18 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_views_kernel
             refine |= __shfl_xor_sync(0xffffffffu, refine, off);
             inside |= __shfl_xor_sync(0xffffffffu, inside, off);
         }
-        if (valid && sub == 0)
+        finish_parents(p, L, li, base, valid && sub == 0, pi, idx, empty, refine, inside, PARTIAL, leaves);
+        if (LANES < 32 && valid && sub == 0 && pi < p.parent_cap && !L.last)
         {
-            store_parent(p, L, pi, empty, refine, inside, PARTIAL);
-            if (LANES < 32 && pi < p.parent_cap && !L.last)
-            {
 #pragma unroll
-                for (int c = 0; c < 8; ++c)
-                {
-                    p.child_skip[pi * 8 + c] = 0u; // at most 16 views: one mask word
-                    p.child_out[pi * 8 + c] = 0u;
-                }
+            for (int c = 0; c < 8; ++c)
+            {
+                p.child_skip[pi * 8 + c] = 0u; // at most 16 views: one mask word
+                p.child_out[pi * 8 + c] = 0u;
             }
         }
     }
-    count_carved(p, li, lane == 0 ? items : 0);
+    count_carved(p, li, lane == 0 ? items : 0, leaves);
 }
 
 // (parent, view) items: a warp deals the unskipped views of a chunk of parents
@@ -255,7 +322,7 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_items_kernel
     // parents per chunk: enough chunks for every warp, at most one per lane
     const int64_t per = (L.n + nwarps - 1) / nwarps;
     const int ppw = static_cast<int>(per < 1 ? 1 : (per > 32 ? 32 : per));
-    unsigned long long items = 0;
+    uint32_t items = 0, leaves = 0; // a warp's items of one level: below 2^32
 
     for (int64_t base = warp * ppw; base < L.n; base += nwarps * ppw)
     {
@@ -281,7 +348,7 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_items_kernel
         const int incl = warp_inclusive_scan(count);
         const int excl = incl - count;
         const int total = __shfl_sync(0xffffffffu, incl, 31);
-        items += static_cast<unsigned long long>(total);
+        items += static_cast<uint32_t>(total);
         __syncwarp();
         for (int k0 = 0; k0 < total; k0 += 32)
         {
@@ -305,28 +372,25 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_items_kernel
             }
         }
         __syncwarp();
-        if (valid)
+        finish_parents(p, L, li, base, valid, pi, idx, ws.empty[lane], ws.refine[lane], ws.inside[lane], PARTIAL, leaves);
+        if (valid && pi < p.parent_cap && !L.last)
         {
-            store_parent(p, L, pi, ws.empty[lane], ws.refine[lane], ws.inside[lane], PARTIAL);
-            if (pi < p.parent_cap && !L.last)
+#pragma unroll
+            for (int w = 0; w < MW; ++w)
             {
+                uint32_t* cs = p.child_skip + w * p.parent_cap * 8 + pi * 8;
+                uint32_t* co = p.child_out + w * p.parent_cap * 8 + pi * 8;
 #pragma unroll
-                for (int w = 0; w < MW; ++w)
+                for (int c = 0; c < 8; ++c)
                 {
-                    uint32_t* cs = p.child_skip + w * p.parent_cap * 8 + pi * 8;
-                    uint32_t* co = p.child_out + w * p.parent_cap * 8 + pi * 8;
-#pragma unroll
-                    for (int c = 0; c < 8; ++c)
-                    {
-                        cs[c] = L.produce ? (ws.cskip[w][lane][c] | skipm[w]) : 0u;
-                        co[c] = L.produce_out ? (ws.cout[w][lane][c] | ws.cout_all[w][lane]) : 0u;
-                    }
+                    cs[c] = L.produce ? (ws.cskip[w][lane][c] | skipm[w]) : 0u;
+                    co[c] = L.produce_out ? (ws.cout[w][lane][c] | ws.cout_all[w][lane]) : 0u;
                 }
             }
         }
         __syncwarp();
     }
-    count_carved(p, li, lane == 0 ? items : 0);
+    count_carved(p, li, lane == 0 ? items : 0, leaves);
 }
 
 struct ChildCount
@@ -402,6 +466,194 @@ struct ChildEpilogue
     }
 };
 
+// Compaction of a level: the refined children of its cells, in cell order,
+// with their masks, and (the children of level L-2) their entries of the
+// field's cell-mask table.  A block takes a contiguous range of parents; the
+// children before it are the sums of 1024 parents that the classify kernels
+// left, and the masks since.  A parent per thread (a scan pass that gave a
+// thread eight parents in turn took 12 to 28 us at any size, and another launch
+// for the sums 4 to 6, and one for the table 20; this takes 7 us at 4096
+// parents, 52 at the 1.7 M children of the headline scene's level 8).
+__global__ void __launch_bounds__(256) children_kernel(HullPlan p, int li)
+{
+    const DevCounters* c = p.ctr;
+    const int tid = threadIdx.x;
+    const int64_t n = c->level_count[li], start = c->level_off[li], next = c->level_off[li + 1];
+    const uint32_t* sums = p.carve_sums[li & 1];
+    // the next level's sums start at zero
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + tid; i < (8 * n < p.node_cap ? 8 * n : p.node_cap) / 1024 + 2; i += static_cast<int64_t>(gridDim.x) * 256)
+        p.carve_sums[(li + 1) & 1][i] = 0;
+    const int64_t tiles = (n + 255) / 256, per = (tiles + gridDim.x - 1) / gridDim.x;
+    const int64_t t0 = per * blockIdx.x, t1 = t0 + per < tiles ? t0 + per : tiles;
+    if (t0 >= tiles && (blockIdx.x > 0 || n > 0))
+        return;
+    unsigned long long before = 0, total;
+    for (int64_t i = tid; i < t0 / 4; i += 256)
+        before += sums[i];
+    for (int64_t i = t0 / 4 * 1024 + tid; i < t0 * 256; i += 256)
+        before += __popc(p.child_masks[i]);
+    block_exclusive_scan(before, &total);
+    int64_t base = next + static_cast<int64_t>(total);
+    const int sh = li + 1; // children ravel at resolution 2^(li+1)
+    const int64_t low = (int64_t{ 1 } << li) - 1;
+    const bool cells = p.cell_masks && p.own_cell_masks && li + 2 == p.level;
+    for (int64_t tile = t0; tile < t1; ++tile)
+    {
+        const int64_t i = tile * 256 + tid;
+        const uint32_t m = i < n ? p.child_masks[i] : 0u;
+        uint32_t sum;
+        int64_t out = base + block_exclusive_scan(static_cast<uint32_t>(__popc(m)), &sum);
+        base += sum;
+        if (!m)
+            continue;
+        const int64_t idx = __ldg(p.nodes + start + i);
+        const int64_t gx = 2 * (idx & low), gy = 2 * ((idx >> li) & low), gz = 2 * (idx >> (2 * li));
+        const bool masks = i < p.parent_cap;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+        {
+            if (!((m >> k) & 1u))
+                continue;
+            if (out < p.node_cap)
+            {
+                const int64_t child = (gx + (k & 1)) | ((gy + (k >> 1 & 1)) << sh) | ((gz + (k >> 2 & 1)) << (2 * sh));
+                p.nodes[out] = child;
+                for (int w = 0; w < p.mask_words; ++w)
+                {
+                    const int64_t at = w * p.parent_cap * 8 + i * 8 + k;
+                    const uint32_t skip = masks ? __ldg(p.child_skip + at) : 0u, gone = masks ? __ldg(p.child_out + at) : 0u;
+                    p.node_skip[w * p.node_cap + out] = skip;
+                    p.node_out[w * p.node_cap + out] = gone;
+                    if (cells)
+                        p.cell_masks[(static_cast<int64_t>(w) << (3 * sh)) + child] = skip | gone;
+                }
+            }
+            ++out;
+        }
+    }
+    if (t1 == tiles && tid == 0)
+        ChildEpilogue{ p.ctr, li, p.node_cap, p.parent_cap }(static_cast<unsigned long long>(base - next));
+}
+
+// The first levels in one launch: at most 1, 8 and 64 parents, too few for the
+// GPU, so a launch per step would be all latency (the classify, sum and
+// compaction launches of three levels took 47 to 58 us; this takes 15 us
+// for 8 views, 24 for 32).  A cluster of blocks deals (child, view) tasks to
+// its lanes, eight times as many as (parent, view) items; the outcomes are
+// OR-ed into the first block's shared memory, and every block lists the next
+// level's cells for itself.  The first block writes the lists out.
+constexpr int kTopLevels = 3;
+constexpr int kTopCells = 1 + 8 + 64 + 512; // cells of the levels 0 to 3
+constexpr int kTopBlocks = 8, kTopThreads = 512;
+
+struct TopShared
+{
+    uint32_t empty[73], refine[73];                  // per parent of the levels 0 to 2
+    uint32_t cskip[kMaxMaskWords][8 * 73], cout[kMaxMaskWords][8 * 73]; // per child
+    int32_t node[kTopCells];
+    uint32_t skip[kMaxMaskWords][kTopCells], gone[kMaxMaskWords][kTopCells];
+};
+
+template <bool PARTIAL, bool OPENGL>
+__global__ void __cluster_dims__(kTopBlocks, 1, 1) __launch_bounds__(kTopThreads) carve_top_kernel(HullPlan p, int levels)
+{
+    namespace cg = cooperative_groups;
+    __shared__ TopShared sh;
+    cg::cluster_group cluster = cg::this_cluster();
+    TopShared& first = *cluster.map_shared_rank(&sh, 0);
+    const int tid = threadIdx.x, rank = static_cast<int>(cluster.block_rank());
+    const int B = static_cast<int>(p.B);
+    const bool skips = p.skip_ok && *p.nonbinary == 0;
+    const bool items_next = p.carve_variant[levels] == 1; // the masks are for the item kernel
+    const bool produce = skips && items_next, produce_out = PARTIAL && items_next;
+    const ViewSource src = make_view_source(p.tf, p.sat, p.H, p.W);
+    for (int i = tid; i < static_cast<int>(sizeof(TopShared) / 4); i += kTopThreads)
+        reinterpret_cast<uint32_t*>(&sh)[i] = 0;
+    cluster.sync();
+    int n = 1, off = 0;     // cells of the level and their place in the lists
+    int64_t start = 0;      // the same in the node pool
+    for (int li = 0; li < levels && n > 0; ++li)
+    {
+        const float inv_rc = __int_as_float((127 - (li + 1)) << 23);
+        const int grow = li + 2 == p.level ? 1 : 2;
+        const int64_t tasks = static_cast<int64_t>(n) * 8 * B;
+        uint32_t items = 0;
+        for (int64_t t = rank * kTopThreads + tid; t < tasks; t += kTopBlocks * kTopThreads)
+        {
+            const int c = static_cast<int>(t & 7), q = static_cast<int>(t >> 3);
+            const int b = q / n, pi = off + (q - b * n), w = b >> 5;
+            const uint32_t bit = 1u << (b & 31);
+            const bool word = w < p.mask_words;
+            if (word && ((sh.skip[w][pi] | sh.gone[w][pi]) & bit))
+                continue;
+            items += c == 0 ? 1u : 0u;
+            float wx[3], wy[3], wz[3];
+            lattice_world(p.rq->corner, p.rq->length, sh.node[pi], li, inv_rc, wx, wy, wz);
+            const int dx = c & 1, dy = (c >> 1) & 1, dz = c >> 2;
+            const float cx[2] = { dx ? wx[1] : wx[0], dx ? wx[2] : wx[1] };
+            const float cy[2] = { dy ? wy[1] : wy[0], dy ? wy[2] : wy[1] };
+            const float cz[2] = { dz ? wz[1] : wz[0], dz ? wz[2] : wz[1] };
+            const ItemResult r = classify_child<PARTIAL, OPENGL>(src, b, cx, cy, cz, produce && word, produce_out && word, grow);
+            if (r.empty)
+                atomicOr(&first.empty[pi], 1u << c);
+            if (r.refine)
+                atomicOr(&first.refine[pi], 1u << c);
+            if (r.skip)
+                atomicOr(&first.cskip[w][8 * pi + c], bit);
+            if (r.out)
+                atomicOr(&first.cout[w][8 * pi + c], bit);
+        }
+        items = __reduce_add_sync(0xffffffffu, items);
+        if ((tid & 31) == 0 && items)
+            atomicAdd(&p.ctr->items[li], static_cast<unsigned long long>(items));
+        cluster.sync();
+        // every block lists the children; the first one also writes them out
+        uint32_t mask = 0, total;
+        if (tid < n)
+            mask = first.refine[off + tid] & ~first.empty[off + tid];
+        uint32_t at = block_exclusive_scan(static_cast<uint32_t>(__popc(mask)), &total);
+        const int noff = off + n;
+        const int64_t nstart = start + n;
+        const bool cells = rank == 0 && p.cell_masks && p.own_cell_masks && li + 2 == p.level;
+        const int s = li + 1;
+        for (; mask; mask &= mask - 1)
+        {
+            const int c = __ffs(mask) - 1, pi = off + tid;
+            const int idx = sh.node[pi], low = (1 << li) - 1;
+            const int child = (2 * (idx & low) + (c & 1)) | ((2 * ((idx >> li) & low) + (c >> 1 & 1)) << s) |
+                              ((2 * (idx >> (2 * li)) + (c >> 2)) << (2 * s));
+            sh.node[noff + at] = child;
+            if (rank == 0)
+                p.nodes[nstart + at] = child;
+            for (int w = 0; w < p.mask_words; ++w)
+            {
+                const uint32_t skip = produce ? (first.cskip[w][8 * pi + c] | sh.skip[w][pi]) : 0u;
+                const uint32_t gone = produce_out ? (first.cout[w][8 * pi + c] | sh.gone[w][pi]) : 0u;
+                sh.skip[w][noff + at] = skip;
+                sh.gone[w][noff + at] = gone;
+                if (rank == 0)
+                {
+                    p.node_skip[w * p.node_cap + nstart + at] = skip;
+                    p.node_out[w * p.node_cap + nstart + at] = gone;
+                }
+                if (cells)
+                    p.cell_masks[(static_cast<int64_t>(w) << (3 * s)) + child] = skip | gone;
+            }
+            ++at;
+        }
+        if (rank == 0 && tid == 0)
+        {
+            p.ctr->level_count[li + 1] = total;
+            p.ctr->level_off[li + 2] = nstart + total;
+        }
+        off = noff;
+        start = nstart;
+        n = static_cast<int>(total);
+        __syncthreads();
+    }
+    cluster.sync(); // the first block's shared memory is read until here
+}
+
 template <bool PARTIAL, bool OPENGL>
 void launch_classify(const HullPlan& p, int li, int64_t max_parents, cudaStream_t s)
 {
@@ -436,12 +688,39 @@ int grid_for(int64_t work_items, int threads)
     return static_cast<int>(blocks < 1 ? 1 : (blocks < cap ? blocks : cap));
 }
 
-void launch_hull_init(const HullPlan& p, cudaStream_t s)
+void launch_begin(const HullPlan& p, const void* tf, int tf_dtype, const ReqConsts* host_rq, unsigned int* flags, bool clear_flags, cudaStream_t s)
 {
-    // the counters and the row groups' corner counts behind them
-    launch_zero(p.ctr, static_cast<size_t>(reinterpret_cast<unsigned char*>(p.coarse) - reinterpret_cast<unsigned char*>(p.ctr)) +
-                               sizeof(uint2) * static_cast<size_t>(p.R * p.R / 256 + 2), s);
-    hull_init_kernel<<<1, 32, 0, s>>>(p);
+    const int64_t items = std::max<int64_t>(p.B * 16, p.R * p.R / 256 + 2);
+    begin_kernel<<<grid_for(items, 256), 256, 0, s>>>(p, tf, tf_dtype, host_rq, const_cast<ReqConsts*>(p.rq), const_cast<float*>(p.tf),
+                                                      flags, clear_flags);
+    TH_LAUNCH_CHECK();
+}
+
+// The last level marks corners, which the top kernel does not.
+int top_levels(int level)
+{
+    return level - 1 < kTopLevels ? (level > 1 ? level - 1 : 0) : kTopLevels;
+}
+
+void launch_top(const HullPlan& p, cudaStream_t s)
+{
+    const int levels = top_levels(p.level);
+    if (levels == 0)
+        return;
+    if (p.partial)
+    {
+        if (p.opengl)
+            carve_top_kernel<true, true><<<kTopBlocks, kTopThreads, 0, s>>>(p, levels);
+        else
+            carve_top_kernel<true, false><<<kTopBlocks, kTopThreads, 0, s>>>(p, levels);
+    }
+    else
+    {
+        if (p.opengl)
+            carve_top_kernel<false, true><<<kTopBlocks, kTopThreads, 0, s>>>(p, levels);
+        else
+            carve_top_kernel<false, false><<<kTopBlocks, kTopThreads, 0, s>>>(p, levels);
+    }
     TH_LAUNCH_CHECK();
 }
 
@@ -465,18 +744,13 @@ void launch_carve_level(const HullPlan& p, int li, cudaStream_t s)
             launch_classify<false, false>(p, li, max_parents, s);
     }
     TH_LAUNCH_CHECK();
+    // The leaves are not written out: the last level marked their corners and
+    // counted them (rows_kernel closes the count), and the leaf list is emitted
+    // only when the candidates of the last level are exported.
     if (li + 1 == p.level)
-    {
-        // The leaves are not written out: their corners are marked from the
-        // parents' child masks (launch_corners), and the leaf list is emitted
-        // only when the candidates of the last level are exported.  The count
-        // (and the pool check) is still taken here.
-        run_scan_reduce(ChildCount{ p.child_masks }, ChildEpilogue{ p.ctr, li, p.node_cap, p.parent_cap },
-                        Count{ &p.ctr->level_count[li], 0 }, max_parents, p.tile_sums, &p.ctr->scan, s);
         return;
-    }
-    run_scan(ChildCount{ p.child_masks }, ChildEmit{ p, li }, ChildEpilogue{ p.ctr, li, p.node_cap, p.parent_cap },
-             Count{ &p.ctr->level_count[li], 0 }, max_parents, p.tile_sums, &p.ctr->scan, s);
+    children_kernel<<<grid_for(max_parents, 256), 256, 0, s>>>(p, li);
+    TH_LAUNCH_CHECK();
 }
 
 void launch_emit_leaves(const HullPlan& p, cudaStream_t s)

@@ -96,6 +96,7 @@ struct WordTotal
         ctr->soup = t >> 32;
         ctr->verts = t & 0xffffffffull;
     }
+    __device__ void block() const {}
 };
 
 struct SoupTotal
@@ -129,6 +130,7 @@ struct VolumeWords
     {
         return i;
     }
+    __device__ void tail() const {}
     __device__ uint32_t sign(uint32_t k) const
     {
         return __ldg(p.sign + k);
@@ -625,15 +627,7 @@ void words_emit(const Src& src, float* verts, int64_t* faces, cudaStream_t s)
 {
     const McPlan& p = src.p;
     const int grid = words_export_grid(p.nwords);
-    if (p.unique)
-    {
-        words_verts_kernel<Src><<<grid, 32 * kWordExportWarps, 0, s>>>(src, p.mesh, verts);
-        TH_LAUNCH_CHECK();
-        words_faces_kernel<Src, true, false><<<grid, 32 * kWordExportWarps, 0, s>>>(src, p.mesh, verts, faces);
-    }
-    else
-        words_faces_kernel<Src, false, false><<<grid, 32 * kWordExportWarps, 0, s>>>(src, p.mesh, verts, faces);
-    TH_LAUNCH_CHECK();
+    launch_words_export<Src, false>(src, p.mesh, p.unique, grid, verts, faces, s);
 }
 
 template <int DT>

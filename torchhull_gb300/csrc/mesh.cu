@@ -37,36 +37,11 @@ namespace th
 namespace
 {
 
-__global__ void __launch_bounds__(256) mark_corners_kernel(HullPlan p)
+// Level 0: the root is the only leaf (deeper leaves are marked by the carve).
+__global__ void mark_root_kernel(HullPlan p)
 {
-    const DevCounters* c = p.ctr;
-    const int L = p.level;
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (L == 0)
-    {
-        // the root is the only leaf
-        if (t0 == 0 && c->level_count[0] > 0)
-            mark_cell_corners(p.bitmap, p.rowbits, p.R, p.WR, 0, 0, 0);
-        return;
-    }
-    // the leaves are the refined children of the level L-1 cells (their
-    // child masks), which the carve does not write out
-    if (c->level_count[L] == 0)
-        return;
-    const int li = L - 1;
-    const int64_t n = c->level_count[li];
-    const int64_t* parents = p.nodes + c->level_off[li];
-    const int64_t r = int64_t{ 1 } << li;
-    for (int64_t t = t0; t < n; t += stride)
-    {
-        uint32_t m = p.child_masks[t];
-        if (!m)
-            continue;
-        const int64_t idx = parents[t];
-        mark_children_corners(p.bitmap, p.rowbits, p.R, p.WR, 2 * (idx & (r - 1)), 2 * ((idx >> li) & (r - 1)),
-                              2 * (idx >> (2 * li)), m);
-    }
+    if (threadIdx.x == 0)
+        mark_cell_corners(p.bitmap, p.rowbits, p.R, p.WR, 0, 0, 0);
 }
 
 // Sum of v over the block, to every thread.
@@ -111,10 +86,27 @@ __global__ void __launch_bounds__(256) rows_kernel(HullPlan p)
     __syncthreads();
     if (tid == 0 && first + kRowBlock >= nwords)
     {
+        DevCounters* c = p.ctr;
         const int64_t rows = static_cast<int64_t>(s_before);
-        p.ctr->rows = rows;
+        c->rows = rows;
         if (rows * p.wr > p.word_cap)
-            p.ctr->overflow |= kOverflowWords;
+            c->overflow |= kOverflowWords;
+        const int L = p.level;
+        if (L > 0 && p.own_cell_masks)
+        {
+            // the last level's count, with the checks of the levels before it
+            const int64_t start = c->level_off[L];
+            int64_t n = static_cast<int64_t>(c->leaves);
+            if (c->level_count[L - 1] > p.parent_cap)
+                c->overflow |= kOverflowParents;
+            if (start + n > p.node_cap)
+            {
+                c->overflow |= kOverflowNodes;
+                n = 0;
+            }
+            c->level_count[L] = n;
+            c->level_off[L + 1] = start + n;
+        }
     }
     for (int i = warp; i < kRowBlock; i += 8)
     {
@@ -528,21 +520,6 @@ __global__ void __launch_bounds__(256) field_kernel(HullPlan p, int64_t b0, int6
     count_items(p, items);
 }
 
-// The cell-mask table (HullPlan::cell_masks): every cell of level L-1
-// writes its skip and out-of-frame views (set) or 0 (clear).
-__global__ void __launch_bounds__(256) cell_masks_kernel(HullPlan p, bool set)
-{
-    const DevCounters* c = p.ctr;
-    const int li = p.level - 1;
-    const int64_t n = c->level_count[li];
-    const int64_t off = c->level_off[li];
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += stride)
-        for (int w = 0; w < p.mask_words; ++w)
-            p.cell_masks[(static_cast<int64_t>(w) << (3 * li)) + p.nodes[off + k]] =
-                    set ? (p.node_skip[w * p.node_cap + off + k] | p.node_out[w * p.node_cap + off + k]) : 0u;
-}
-
 // Views of mask word `word` whose factor at a corner is exactly 1: the OR of the cell-mask
 // entries of the level L-1 cells whose lattice holds the corner (x >> 1, and
 // also (x - 1) >> 1 for an even x > 0, per axis; cells beyond the grid and
@@ -724,6 +701,17 @@ struct HullWords
     {
         return __ldg(p.word_list + i);
     }
+    // After the field: its cell-mask table is left clear for the next request.
+    __device__ void tail() const
+    {
+        if (!p.cell_masks || !p.own_cell_masks)
+            return;
+        const int li = p.level - 1;
+        const int64_t n = p.ctr->level_count[li], off = p.ctr->level_off[li], stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+        for (int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += stride)
+            for (int w = 0; w < p.mask_words; ++w)
+                p.cell_masks[(static_cast<int64_t>(w) << (3 * li)) + p.nodes[off + k]] = 0;
+    }
     __device__ bool empty(uint32_t) const
     {
         return false; // listed words have corners
@@ -791,13 +779,22 @@ struct HullWords
     }
 };
 
+// The last counters of a request; the block that writes them then copies all
+// of them to the host.
 struct MeshTotal
 {
     DevCounters* ctr;
+    DevCounters* host;
     __device__ void operator()(unsigned long long total) const
     {
         ctr->soup = static_cast<int64_t>(total >> 32);
         ctr->verts = static_cast<int64_t>(total & 0xffffffffull);
+    }
+    __device__ void block() const
+    {
+        __syncthreads();
+        for (int i = threadIdx.x; i < static_cast<int>(sizeof(DevCounters) / 8); i += blockDim.x)
+            reinterpret_cast<volatile unsigned long long*>(host)[i] = reinterpret_cast<const volatile unsigned long long*>(ctr)[i];
     }
 };
 
@@ -810,9 +807,11 @@ HullWords hull_words(const HullPlan& p)
 
 void launch_corners(const HullPlan& p, cudaStream_t s)
 {
-    const int64_t max_leaves = p.node_cap;
-    mark_corners_kernel<<<grid_for(max_leaves, 256), 256, 0, s>>>(p);
-    TH_LAUNCH_CHECK();
+    if (p.level == 0)
+    {
+        mark_root_kernel<<<1, 32, 0, s>>>(p);
+        TH_LAUNCH_CHECK();
+    }
     launch_rank_corners(p, s);
 }
 
@@ -839,13 +838,6 @@ void launch_field(const HullPlan& p, cudaStream_t s)
     }
     if (p.cell_masks)
     {
-        const int64_t cells = p.level >= 1 ? (int64_t{ 1 } << (3 * (p.level - 1))) : 1;
-        const int mgrid = grid_for(cells < p.node_cap ? cells : p.node_cap, 256);
-        if (p.own_cell_masks)
-        {
-            cell_masks_kernel<<<mgrid, 256, 0, s>>>(p, true);
-            TH_LAUNCH_CHECK();
-        }
         const int grid = grid_for(p.corner_cap, 32 * kMaskedWarps);
         // at least one launch, so that B == 0 still writes the empty product 1
         for (int64_t b0 = 0; b0 == 0 || b0 < p.B; b0 += 32)
@@ -859,11 +851,6 @@ void launch_field(const HullPlan& p, cudaStream_t s)
             });
             if (!ok)
                 throw CudaError{ cudaErrorInvalidValue, "hull field: unsupported mask dtype" };
-            TH_LAUNCH_CHECK();
-        }
-        if (p.own_cell_masks)
-        {
-            cell_masks_kernel<<<mgrid, 256, 0, s>>>(p, false);
             TH_LAUNCH_CHECK();
         }
         return;
@@ -890,9 +877,9 @@ void launch_marching_cubes(const HullPlan& p, cudaStream_t s)
     const HullWords src = hull_words(p);
     const int grid = words_grid(std::min(p.word_cap, p.R * p.R * static_cast<int64_t>(p.wr)));
     if (p.unique)
-        words_count_kernel<HullWords, true><<<grid, kWordThreads, 0, s>>>(src, p.mesh, &p.ctr->scan, nullptr, MeshTotal{ p.ctr });
+        words_count_kernel<HullWords, true><<<grid, kWordThreads, 0, s>>>(src, p.mesh, &p.ctr->scan, nullptr, MeshTotal{ p.ctr, p.host_ctr });
     else
-        words_count_kernel<HullWords, false><<<grid, kWordThreads, 0, s>>>(src, p.mesh, &p.ctr->scan, nullptr, MeshTotal{ p.ctr });
+        words_count_kernel<HullWords, false><<<grid, kWordThreads, 0, s>>>(src, p.mesh, &p.ctr->scan, nullptr, MeshTotal{ p.ctr, p.host_ctr });
     TH_LAUNCH_CHECK();
     words_base_kernel<HullWords><<<grid, kWordThreads, 0, s>>>(src, p.mesh);
     TH_LAUNCH_CHECK();
@@ -902,20 +889,13 @@ void launch_export(const HullPlan& p, int64_t words, float* verts, int64_t* face
 {
     const HullWords src = hull_words(p);
     const int grid = words_export_grid(words);
-    if (p.unique)
-    {
-        words_verts_kernel<HullWords><<<grid, 32 * kWordExportWarps, 0, s>>>(src, p.mesh, verts);
-        TH_LAUNCH_CHECK();
-        words_faces_kernel<HullWords, true, true><<<grid, 32 * kWordExportWarps, 0, s>>>(src, p.mesh, verts, faces);
-    }
-    else
-        words_faces_kernel<HullWords, false, true><<<grid, 32 * kWordExportWarps, 0, s>>>(src, p.mesh, verts, faces);
-    TH_LAUNCH_CHECK();
+    launch_words_export<HullWords, true>(src, p.mesh, p.unique, grid, verts, faces, s);
 }
 
 namespace
 {
 
+template <bool COO>
 __global__ void __launch_bounds__(256) export_field_kernel(HullPlan p, int64_t n, int64_t* __restrict__ indices, float* __restrict__ values)
 {
     const int64_t R = p.R;
@@ -924,7 +904,15 @@ __global__ void __launch_bounds__(256) export_field_kernel(HullPlan p, int64_t n
     {
         int64_t x, y, z;
         unpack_corner(p.corners[t], x, y, z);
-        indices[t] = x + y * R + z * R * R;
+        if constexpr (COO)
+        {
+            indices[t] = 0;
+            indices[n + t] = z;
+            indices[2 * n + t] = y;
+            indices[3 * n + t] = x;
+        }
+        else
+            indices[t] = x + y * R + z * R * R;
         values[t] = p.values[t];
     }
 }
@@ -935,7 +923,15 @@ void launch_export_field(const HullPlan& p, int64_t n, int64_t* indices, float* 
 {
     if (n <= 0)
         return;
-    export_field_kernel<<<grid_for(n, 256), 256, 0, s>>>(p, n, indices, values);
+    export_field_kernel<false><<<grid_for(n, 256), 256, 0, s>>>(p, n, indices, values);
+    TH_LAUNCH_CHECK();
+}
+
+void launch_export_field_coo(const HullPlan& p, int64_t n, int64_t* indices, float* values, cudaStream_t s)
+{
+    if (n <= 0)
+        return;
+    export_field_kernel<true><<<grid_for(n, 256), 256, 0, s>>>(p, n, indices, values);
     TH_LAUNCH_CHECK();
 }
 

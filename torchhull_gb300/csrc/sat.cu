@@ -366,14 +366,6 @@ bool bits_apply(int64_t B, int64_t H, int64_t W, int dtype)
            B * ((H + kBandRows - 1) / kBandRows) < (int64_t{ 1 } << 31);
 }
 
-template <int DT>
-__global__ void convert_transforms_kernel(const void* __restrict__ tf, int64_t n, float* __restrict__ out)
-{
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n)
-        out[i] = load_f32<DT>(tf, i);
-}
-
 } // namespace
 
 int64_t sat_scratch_bytes(int64_t B, int64_t H, int64_t W, int dtype)
@@ -441,29 +433,6 @@ void launch_integral_image(const void* masks,
     const int64_t rows = B * H;
     const unsigned grid_rows = static_cast<unsigned>((rows + 32 * kRowWarps - 1) / (32 * kRowWarps));
     sat_rows_kernel<<<grid_rows, 32 * kRowWarps, 0, s>>>(out, rows, W, gate);
-    TH_LAUNCH_CHECK();
-}
-
-void launch_convert_transforms(const void* tf, int dtype, int64_t B, float* out, cudaStream_t s)
-{
-    const int64_t n = B * 16;
-    if (n == 0)
-        return;
-    const unsigned grid = static_cast<unsigned>((n + 255) / 256);
-    switch (dtype)
-    {
-    case TH_FLOAT16:
-        convert_transforms_kernel<TH_FLOAT16><<<grid, 256, 0, s>>>(tf, n, out);
-        break;
-    case TH_FLOAT32:
-        convert_transforms_kernel<TH_FLOAT32><<<grid, 256, 0, s>>>(tf, n, out);
-        break;
-    case TH_FLOAT64:
-        convert_transforms_kernel<TH_FLOAT64><<<grid, 256, 0, s>>>(tf, n, out);
-        break;
-    default:
-        throw CudaError{ cudaErrorInvalidValue, "transforms: unsupported dtype" };
-    }
     TH_LAUNCH_CHECK();
 }
 

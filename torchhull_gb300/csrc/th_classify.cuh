@@ -417,6 +417,65 @@ __device__ __forceinline__ ItemResult classify_item(const ViewSource& p,
     return out;
 }
 
+// One child of a parent in view b (the top levels, where a lane per child is
+// wanted for latency): classify_item's outcome for child c alone, from the same
+// operations on its eight corners.  The fields of the result are 0 or 1.
+template <bool PARTIAL, bool OPENGL>
+__device__ __forceinline__ ItemResult classify_child(const ViewSource& p,
+                                                     int64_t b,
+                                                     const float wx[2],
+                                                     const float wy[2],
+                                                     const float wz[2],
+                                                     bool want_skip,
+                                                     bool want_out,
+                                                     int grow)
+{
+    const int32_t H = static_cast<int32_t>(p.H), W = static_cast<int32_t>(p.W);
+    const float* m = p.tf + 16 * b;
+    const float4 rx = *reinterpret_cast<const float4*>(m);
+    const float4 ry = *reinterpret_cast<const float4*>(m + 4);
+    const float4 rd = *reinterpret_cast<const float4*>(m + (OPENGL ? 12 : 8));
+    float px[8], py[8];
+    bool front = true, nan = false;
+#pragma unroll
+    for (int z = 0; z < 2; ++z)
+    {
+        const float tzx = __fmaf_rn(rx.z, wz[z], rx.w), tzy = __fmaf_rn(ry.z, wz[z], ry.w), tzd = __fmaf_rn(rd.z, wz[z], rd.w);
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+        {
+            const float tyx = __fmaf_rn(rx.y, wy[y], tzx), tyy = __fmaf_rn(ry.y, wy[y], tzy), tyd = __fmaf_rn(rd.y, wy[y], tzd);
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+            {
+                const int k = x + 2 * y + 4 * z;
+                const float cx = __fmaf_rn(rx.x, wx[x], tyx), cy = __fmaf_rn(ry.x, wx[x], tyy), cd = __fmaf_rn(rd.x, wx[x], tyd);
+                const float nx = __fdiv_rn(cx, cd), ny = __fdiv_rn(cy, cd);
+                if (OPENGL)
+                {
+                    px[k] = __fsub_rn(__fmul_rn(__fmul_rn(__fadd_rn(nx, 1.f), p.Wf), 0.5f), 0.5f);
+                    py[k] = __fsub_rn(__fmul_rn(__fmul_rn(__fadd_rn(ny, 1.f), p.Hf), 0.5f), 0.5f);
+                }
+                else
+                {
+                    px[k] = __fsub_rn(nx, 0.5f);
+                    py[k] = __fsub_rn(ny, 0.5f);
+                }
+                front = front && cd > 0.f;
+                nan = nan || !(px[k] == px[k] && py[k] == py[k]);
+            }
+        }
+    }
+    Box bb{ px[0], py[0], px[0], py[0] };
+#pragma unroll
+    for (int k = 1; k < 8; ++k)
+        bb = merge(bb, Box{ px[k], py[k], px[k], py[k] });
+    const bool in2 = !nan && bb.minx >= 1.5f && bb.maxx < __fsub_rn(p.Wf, 2.5f) && bb.miny >= 1.5f && bb.maxy < __fsub_rn(p.Hf, 2.5f);
+    const ViewResult r = classify_view<PARTIAL>(p.sat + b * p.H * p.W, H, W, p.Hf, p.Wf, bb, want_skip && front && (!PARTIAL || in2), grow);
+    return ItemResult{ r.cls == kEmpty ? 1u : 0u, r.cls == kRefine ? 1u : 0u, 0u, r.skip ? 1u : 0u,
+                       PARTIAL && want_out && front && box_out(bb, p.Hf, p.Wf) ? 1u : 0u };
+}
+
 // Merges an item's outcome into its slot: one shared atomic per non-zero word
 // (a slot's items sit in neighbouring lanes, so conflicts are short).
 template <int MW>

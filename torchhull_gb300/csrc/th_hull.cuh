@@ -32,6 +32,7 @@ struct DevCounters
     int64_t verts;                      // unique mesh vertices
     int64_t overflow;                   // OverflowBits
     int64_t row_words;                  // words of the row-occupancy bitmap
+    unsigned long long leaves;          // refined children of the last level
     unsigned long long items[kMaxLevel];  // (parent, view) items the carve evaluated per parent level
     unsigned long long field_items;       // (corner, view) pairs the field evaluated
     ScanState scan;
@@ -72,6 +73,7 @@ struct HullPlan
     int64_t* nodes;
     int64_t node_cap;
     uint8_t* child_masks; // one byte per parent of the current level
+    uint32_t* carve_sums[2]; // children of 1024 parents each, of even and of odd levels
     unsigned long long* tile_sums;
     // View skipping (binary masks only).  node_skip[k] has bit b set when view
     // b need not be evaluated for any descendant of node k: the box of node k
@@ -112,7 +114,7 @@ struct HullPlan
     // table over the cells of level L-1, scattered before the field and
     // cleared after it (nullptr: no table, every pair is evaluated).
     uint32_t* cell_masks; // [mask_words][8^(L-1)]
-    bool own_cell_masks;  // launch_field scatters and clears the table (the batched form does it itself)
+    bool own_cell_masks;  // the carve fills and the mesh stages clear the table (the batched form does it itself)
     // corner grid: R^3 points, one bit each, rows of WR 64-bit words (x fastest)
     int64_t R, WR;
     uint64_t* bitmap;     // [R*R*WR]
@@ -138,6 +140,7 @@ struct HullPlan
     float* values;
     int64_t corner_cap;
     DevCounters* ctr;
+    DevCounters* host_ctr; // mapped host memory the finished counters are written to
     const ReqConsts* rq; // corner, length and masks of the running request (device)
 };
 
@@ -156,9 +159,17 @@ __device__ __forceinline__ void unpack_corner(int64_t v, int64_t& x, int64_t& y,
     z = v >> 42;
 }
 
-void launch_hull_init(const HullPlan& p, cudaStream_t s);
+// Everything a request starts from, in one launch: its transforms as float32,
+// its ReqConsts (host_rq: device address of mapped host memory), cleared
+// counters, the root cell and (clear_flags) the 0/1 flag of its masks.
+void launch_begin(const HullPlan& p, const void* tf, int tf_dtype, const ReqConsts* host_rq, unsigned int* flags, bool clear_flags, cudaStream_t s);
+// Levels launch_top carves in one launch (the first levels of the octree).
+int top_levels(int level);
+void launch_top(const HullPlan& p, cudaStream_t s);
 // Sparse field export: ravelled ids (x + y*R + z*R*R) and values.
 void launch_export_field(const HullPlan& p, int64_t n, int64_t* indices, float* values, cudaStream_t s);
+// The same with the indices of a sparse tensor: four rows of n (0, z, y, x).
+void launch_export_field_coo(const HullPlan& p, int64_t n, int64_t* indices, float* values, cudaStream_t s);
 void launch_carve_level(const HullPlan& p, int level_index, cudaStream_t s);
 // The leaf list (level L) from the last level's child masks; the carve itself
 // only counts the leaves.
@@ -193,42 +204,48 @@ __device__ __forceinline__ void mark_cell_corners(uint64_t* bitmap, uint32_t* ro
 // Sets the corner bits of the refined children (child mask m) of a cell whose
 // lattice starts at (x, y, z) at resolution 2^L: per lattice row (y + dy,
 // z + dz) one OR of the x bits its children cover, instead of four words per
-// child (neighbouring children share 27 of their 64 corners).
+// child (neighbouring children share 27 of their 64 corners).  Most bits are
+// set already by a neighbour: the nine words are read first, together, and
+// only what is missing is written (a row whose bits are all set has its flag
+// from whoever set them).
 __device__ __forceinline__ void mark_children_corners(uint64_t* bitmap, uint32_t* rowbits, int64_t R, int64_t WR,
                                                       int64_t x, int64_t y, int64_t z, uint32_t m)
 {
+    const uint32_t wx = static_cast<uint32_t>(x >> 6);
+    const int b = static_cast<int>(x & 63);
+    uint32_t xb[9]; // lattice x bits 0..2 of the rows
+    uint64_t have[9];
+    uint64_t* const first = bitmap + (y + z * R) * WR + wx;
 #pragma unroll
-    for (int dz = 0; dz < 3; ++dz)
+    for (int q = 0; q < 9; ++q)
     {
+        const int dy = q % 3, dz = q / 3;
+        xb[q] = 0;
 #pragma unroll
-        for (int dy = 0; dy < 3; ++dy)
+        for (int c = 0; c < 8; ++c)
         {
-            uint32_t xb = 0; // lattice x bits 0..2 of this row
-#pragma unroll
-            for (int c = 0; c < 8; ++c)
-            {
-                const int cx = c & 1, cy = (c >> 1) & 1, cz = c >> 2;
-                if (((m >> c) & 1u) && (dy == cy || dy == cy + 1) && (dz == cz || dz == cz + 1))
-                    xb |= 3u << cx;
-            }
-            if (!xb)
-                continue;
-            const int64_t row = (y + dy) + (z + dz) * R;
-            const int64_t w = row * WR + (x >> 6);
-            const int b = static_cast<int>(x & 63);
-            const uint64_t lo = static_cast<uint64_t>(xb) << b;
-            if (lo && (bitmap[w] & lo) != lo)
-                atomicOr(reinterpret_cast<unsigned long long*>(bitmap + w), static_cast<unsigned long long>(lo));
-            if (b > 61)
-            {
-                const uint64_t hi = static_cast<uint64_t>(xb) >> (64 - b);
-                if (hi && (bitmap[w + 1] & hi) != hi)
-                    atomicOr(reinterpret_cast<unsigned long long*>(bitmap + w + 1), static_cast<unsigned long long>(hi));
-            }
-            const uint32_t rb = 1u << (row & 31);
-            if (!(rowbits[row >> 5] & rb))
-                atomicOr(rowbits + (row >> 5), rb);
+            const int cx = c & 1, cy = (c >> 1) & 1, cz = c >> 2;
+            if ((dy == cy || dy == cy + 1) && (dz == cz || dz == cz + 1) && ((m >> c) & 1u))
+                xb[q] |= 3u << cx;
         }
+        have[q] = xb[q] ? __ldcg(first + (dy + dz * R) * WR) : 0ull;
+    }
+#pragma unroll
+    for (int q = 0; q < 9; ++q)
+    {
+        const uint64_t lo = static_cast<uint64_t>(xb[q]) << b;
+        const bool spill = b > 61 && (xb[q] >> (64 - b)) != 0; // into the next word
+        if ((have[q] & lo) == lo && !spill)
+            continue;
+        const int64_t row = (y + q % 3) + (z + q / 3) * R;
+        uint64_t* w = first + (q % 3 + q / 3 * R) * WR;
+        if (lo)
+            atomicOr(reinterpret_cast<unsigned long long*>(w), static_cast<unsigned long long>(lo));
+        if (spill)
+            atomicOr(reinterpret_cast<unsigned long long*>(w + 1), static_cast<unsigned long long>(xb[q] >> (64 - b)));
+        const uint32_t rb = 1u << (row & 31);
+        if (!(__ldcg(rowbits + (row >> 5)) & rb))
+            atomicOr(rowbits + (row >> 5), rb);
     }
 }
 

@@ -75,9 +75,6 @@ void launch_integral_image(const void* masks,
                            unsigned int* nonbinary = nullptr,
                            SatScratch scratch = {});
 
-// Transform conversion to float32 row-major [B,16] (sat.cu).
-void launch_convert_transforms(const void* tf, int dtype, int64_t B, float* out, cudaStream_t s);
-
 // Gaussian blur (blur.cu).  edge_tiles: scratch of tiles_bytes(B,H,W,k) bytes.
 int64_t blur_tile_bytes(int64_t B, int64_t H, int64_t W, int kernel_size);
 void launch_gaussian_blur(const void* images,

@@ -11,7 +11,7 @@
 //    cells' bits and the two counts (vertices, triangle corners); tile sums.
 // 2. words_base: the counts' prefix sums: per word the index of its first
 //    vertex, per 32 words the first vertex and triangle corner.
-// 3. words_verts and words_faces: a warp takes 32 words and deals their
+// 3. words_export: a warp takes 32 words and deals their
 //    vertices, or their active cells and the cells' triangle corners, to its
 //    lanes: an edge's vertex index is its word's base plus the set bits before it.
 //
@@ -21,6 +21,7 @@
 //   int64_t words() const             number of items: words in row order, at least
 //                                     those with a present point
 //   uint32_t word(uint32_t i) const   the word of an item
+//   void tail() const                 more work for the threads of the base pass
 //   WordRows rows(uint32_t k) const   the words of the cells that start in word k
 //   uint32_t sign(uint32_t k) const   below-isolevel bits of a word
 //   bool empty(uint32_t k) const      none of the word's points is present
@@ -189,10 +190,12 @@ __device__ __forceinline__ void finish_word_tiles(int64_t ntiles, unsigned long 
         state->blocks_done = 0;
         epi(carry);
     }
+    epi.block();
 }
 
 // Pass 1.  A thread per word; most words see one side only and leave after the
-// loads.  epi(total) gets the triangle corners << 32 | vertices.
+// loads.  epi(total) gets the triangle corners << 32 | vertices on one
+// thread, then epi.block() runs on the same block.
 template <class Src, bool UNIQUE, class EpiF>
 __global__ void __launch_bounds__(kWordThreads) words_count_kernel(Src src, WordMesh m, ScanState* state, unsigned long long* active, EpiF epi)
 {
@@ -308,6 +311,7 @@ __global__ void __launch_bounds__(kWordThreads) words_base_kernel(Src src, WordM
             off += (static_cast<unsigned long long>(tot >> 16) << 32) | (tot & 0xffffu);
         }
     }
+    src.tail();
 }
 
 // Index of the first vertex of the point at bit b of a word, and the point's
@@ -328,14 +332,14 @@ constexpr int kWordExportWarps = 8;
 // against 26 + 50).  All that says what a chunk holds is loaded at
 // once, whether or not it holds anything.
 
-// Pass 3, the vertices.
+// Pass 3, the vertices, by block `block` of `blocks`.
 template <class Src>
-__global__ void __launch_bounds__(32 * kWordExportWarps) words_verts_kernel(Src src, WordMesh m, float* __restrict__ verts)
+__device__ __forceinline__ void export_verts(const Src& src, const WordMesh& m, float* __restrict__ verts, uint32_t block, uint32_t blocks)
 {
     const int lane = threadIdx.x & 31;
     const int64_t n = src.words(), nchunks = (n + 31) / 32;
-    const int64_t nwarps = static_cast<int64_t>(gridDim.x) * kWordExportWarps;
-    for (int64_t c = static_cast<int64_t>(blockIdx.x) * kWordExportWarps + (threadIdx.x >> 5); c < nchunks; c += nwarps)
+    const int64_t nwarps = static_cast<int64_t>(blocks) * kWordExportWarps;
+    for (int64_t c = static_cast<int64_t>(block) * kWordExportWarps + (threadIdx.x >> 5); c < nchunks; c += nwarps)
     {
         const uint32_t item = static_cast<uint32_t>(c * 32) + lane;
         const bool in = c * 32 + lane < n;
@@ -387,12 +391,19 @@ __global__ void __launch_bounds__(32 * kWordExportWarps) words_verts_kernel(Src 
     }
 }
 
-// Pass 3, the triangles.  FLIP: the second and third corner of every triangle
-// change places.  Without UNIQUE every triangle corner is a vertex of its own,
-// written here too.
+// Pass 3.  UNIQUE: the even blocks write vertices, the odd ones triangles (one
+// launch, so that a small mesh does not wait for two).  FLIP: the second and
+// third corner of every triangle change places.  Without UNIQUE every triangle
+// corner is a vertex of its own, written with the triangles.
 template <class Src, bool UNIQUE, bool FLIP>
-__global__ void __launch_bounds__(32 * kWordExportWarps) words_faces_kernel(Src src, WordMesh m, float* __restrict__ verts, int64_t* __restrict__ faces)
+__global__ void __launch_bounds__(32 * kWordExportWarps) words_export_kernel(Src src, WordMesh m, float* __restrict__ verts, int64_t* __restrict__ faces)
 {
+    if (UNIQUE && blockIdx.x % 2 == 0)
+    {
+        export_verts(src, m, verts, blockIdx.x / 2, gridDim.x / 2);
+        return;
+    }
+    const uint32_t block = UNIQUE ? blockIdx.x / 2 : blockIdx.x, blocks = UNIQUE ? gridDim.x / 2 : gridDim.x;
     __shared__ WordTables tab;
     // per warp and cell of a round: its corners' vertices (point_vertices), or
     // where their values are (Src::values_at)
@@ -410,8 +421,8 @@ __global__ void __launch_bounds__(32 * kWordExportWarps) words_faces_kernel(Src 
     uint32_t* stage = stage_all[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int64_t n = src.words(), nchunks = (n + 31) / 32;
-    const int64_t nwarps = static_cast<int64_t>(gridDim.x) * kWordExportWarps;
-    for (int64_t c = static_cast<int64_t>(blockIdx.x) * kWordExportWarps + (threadIdx.x >> 5); c < nchunks; c += nwarps)
+    const int64_t nwarps = static_cast<int64_t>(blocks) * kWordExportWarps;
+    for (int64_t c = static_cast<int64_t>(block) * kWordExportWarps + (threadIdx.x >> 5); c < nchunks; c += nwarps)
     {
         const uint32_t item = static_cast<uint32_t>(c * 32) + lane;
         const bool in = c * 32 + lane < n;
@@ -528,6 +539,18 @@ inline int words_export_grid(int64_t words)
 {
     const int64_t blocks = (words + 32 * kWordExportWarps - 1) / (32 * kWordExportWarps), cap = 8LL * sm_count();
     return static_cast<int>(blocks < 1 ? 1 : (blocks < cap ? blocks : cap));
+}
+
+// Pass 3 on stream s; grid: words_export_grid.
+template <class Src, bool FLIP>
+inline void launch_words_export(const Src& src, const WordMesh& m, bool unique, int grid, float* verts, int64_t* faces, cudaStream_t s)
+{
+    if (unique)
+        words_export_kernel<Src, true, FLIP><<<2 * grid, 32 * kWordExportWarps, 0, s>>>(src, m, verts, faces);
+    else
+        words_export_kernel<Src, false, FLIP><<<grid, 32 * kWordExportWarps, 0, s>>>(src, m, verts, faces);
+    check_launch("mesh export");
+    note_launches(1);
 }
 
 // Grid of the count and base passes (words: an upper bound).

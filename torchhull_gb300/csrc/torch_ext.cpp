@@ -183,6 +183,7 @@ HullOutputs run_visual_hull(const at::Tensor& masks_in,
                             bool unique_verts,
                             bool want_candidates,
                             bool want_field,
+                            bool field_coo = false,
                             int blur_kernel_size = 0,
                             float blur_sigma = 0.f)
 {
@@ -218,10 +219,11 @@ HullOutputs run_visual_hull(const at::Tensor& masks_in,
     }
     if (want_field)
     {
-        out.field_indices = at::empty({ info.num_corners }, at::TensorOptions().dtype(at::kLong).device(dev));
+        const auto index = at::TensorOptions().dtype(at::kLong).device(dev);
+        out.field_indices = field_coo ? at::empty({ 4, info.num_corners }, index) : at::empty({ info.num_corners }, index);
         out.field_values = at::empty({ info.num_corners }, at::TensorOptions().dtype(at::kFloat).device(dev));
-        check(th_visual_hull_export_field(dc.ctx, out.field_indices.data_ptr<int64_t>(),
-                                          out.field_values.data_ptr<float>(), stream),
+        check((field_coo ? th_visual_hull_export_field_coo : th_visual_hull_export_field)(
+                      dc.ctx, out.field_indices.data_ptr<int64_t>(), out.field_values.data_ptr<float>(), stream),
               dc.ctx);
     }
     return out;
@@ -257,7 +259,7 @@ std::tuple<at::Tensor, at::Tensor> visual_hull_blurred(const at::Tensor& masks,
 {
     TORCH_CHECK(kernel_size != 0, "Check failed: kernel_size > 0 (0 vs. 0)");
     auto o = run_visual_hull(masks, transforms, level, cube_corner_bfl, cube_length, masks_partial,
-                             transforms_convention, unique_verts, false, false, kernel_size, sigma);
+                             transforms_convention, unique_verts, false, false, false, kernel_size, sigma);
     return { o.verts, o.faces };
 }
 
@@ -289,6 +291,24 @@ std::tuple<at::Tensor, at::Tensor, int64_t> sparse_visual_hull_field_raw(const a
     auto o = run_visual_hull(masks, transforms, level, cube_corner_bfl, cube_length, masks_partial,
                              transforms_convention, true, false, true);
     return { o.field_indices, o.field_values, (int64_t{ 1 } << level) + 1 };
+}
+
+// The sparse field as torchhull's coalesced COO tensor of size (1, R, R, R)
+// (visual_hull_cuda.cu:522-580): its indices (0, z, y, x) leave the library in
+// ascending order, so nothing is sorted or checked here.
+at::Tensor sparse_visual_hull_field(const at::Tensor& masks,
+                                    const at::Tensor& transforms,
+                                    int level,
+                                    const std::array<float, 3>& cube_corner_bfl,
+                                    float cube_length,
+                                    bool masks_partial,
+                                    const std::string& transforms_convention)
+{
+    auto o = run_visual_hull(masks, transforms, level, cube_corner_bfl, cube_length, masks_partial,
+                             transforms_convention, true, false, true, true);
+    const int64_t r = (int64_t{ 1 } << level) + 1;
+    return at::_sparse_coo_tensor_unsafe(o.field_indices, o.field_values, { 1, r, r, r }, o.field_values.options().layout(at::kSparse),
+                                         true);
 }
 
 at::Tensor gaussian_blur(const at::Tensor& images_in,
@@ -697,6 +717,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m)
     m.def("visual_hull_with_candidate_voxels", &visual_hull_with_candidate_voxels, "masks"_a, "transforms"_a, "level"_a,
           "cube_corner_bfl"_a, "cube_length"_a, "masks_partial"_a, "transforms_convention"_a, "unique_verts"_a = true,
           "visual_hull plus the ravelled candidate cells of every octree level.");
+    m.def("sparse_visual_hull_field", &sparse_visual_hull_field, "masks"_a, "transforms"_a, "level"_a,
+          "cube_corner_bfl"_a, "cube_length"_a, "masks_partial"_a, "transforms_convention"_a);
     m.def("sparse_visual_hull_field_raw", &sparse_visual_hull_field_raw, "masks"_a, "transforms"_a, "level"_a,
           "cube_corner_bfl"_a, "cube_length"_a, "masks_partial"_a, "transforms_convention"_a,
           "Sparse hull field as (ravelled indices, values, grid size).");
