@@ -53,7 +53,7 @@ __global__ void batch_init_kernel(BatchPlan bp)
 }
 
 // VARIANT: (partial << 1) | opengl shared by every request of the batch, or
-// -1 to branch per request.
+// -1 to take each request's own.
 template <int VARIANT>
 __device__ __forceinline__ ItemResult batch_item(const BatchReq& q,
                                                  int64_t b,
@@ -67,18 +67,8 @@ __device__ __forceinline__ ItemResult batch_item(const BatchReq& q,
                                                  bool want_inside)
 {
     const ViewSource src = make_view_source(q.tf, q.sat, q.H, q.W);
-    if constexpr (VARIANT >= 0)
-        return classify_item<(VARIANT >> 1) != 0, (VARIANT & 1) != 0>(src, b, wx, wy, wz, want_skip, skip_inside,
-                                                                      want_out, grow, want_inside);
-    if (q.partial)
-        return q.opengl ? classify_item<true, true>(src, b, wx, wy, wz, want_skip, skip_inside, want_out, grow,
-                                                    want_inside)
-                        : classify_item<true, false>(src, b, wx, wy, wz, want_skip, skip_inside, want_out, grow,
-                                                     want_inside);
-    return q.opengl ? classify_item<false, true>(src, b, wx, wy, wz, want_skip, skip_inside, want_out, grow,
-                                                 want_inside)
-                    : classify_item<false, false>(src, b, wx, wy, wz, want_skip, skip_inside, want_out, grow,
-                                                  want_inside);
+    return classify_item(VARIANT >= 0 ? (VARIANT >> 1) != 0 : q.partial != 0, VARIANT >= 0 ? (VARIANT & 1) != 0 : q.opengl != 0,
+                         src, b, wx, wy, wz, want_skip, skip_inside, want_out, grow, want_inside);
 }
 
 // Entries of level li that were written (a pool overflow drops the rest).

@@ -612,6 +612,8 @@ void prepare(HullSlot& s, const th_hull_args* a, cudaStream_t st, bool field_one
     p.corner[2] = a->cube_corner_bfl[2];
     p.length = a->cube_length;
     p.level = L;
+    p.mark_apart = L >= kMarkApartLevel;
+    p.sms = sm_count();
     p.nodes = s.nodes.as<int64_t>();
     p.node_cap = node_cap;
     p.child_masks = s.child_masks.as<uint8_t>();

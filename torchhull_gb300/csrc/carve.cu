@@ -81,6 +81,7 @@ constexpr int kWarps = TH_CARVE_WARPS; // warps per block of the classify kernel
 #endif
 // resident blocks per SM the classify kernels' register budget is cut for
 constexpr int kMinBlocks = TH_CARVE_MIN_BLOCKS;
+constexpr int kGridPerSm = 16; // blocks of the item kernel's grid per SM
 
 template <int DT>
 __device__ __forceinline__ float transform_value(const void* tf, int64_t i)
@@ -158,9 +159,9 @@ __device__ __forceinline__ LevelInfo level_info(const HullPlan& p, int li, bool 
 // The refined children of a warp's parents (base: its first parent; valid
 // lanes hold parent pi and cell idx): their mask is kept; before the last
 // level their number goes into the level's sums of 1024 parents, for the
-// compaction; at the last level they are the leaves, whose corners are marked
-// at once (the leaf list itself is written only when its candidates are
-// exported) and counted into leaves.
+// compaction; at the last level they are the leaves, which are counted into
+// leaves and, unless that is left to another launch, marked at once (the leaf
+// list itself is written only when its candidates are exported).
 __device__ __forceinline__ void finish_parents(const HullPlan& p, const LevelInfo& L, int li, int64_t base, bool valid, int64_t pi, int64_t idx, uint32_t empty, uint32_t refine, uint32_t inside, bool partial, uint32_t& leaves)
 {
     uint32_t mask = 0;
@@ -173,12 +174,12 @@ __device__ __forceinline__ void finish_parents(const HullPlan& p, const LevelInf
     }
     if (L.last)
     {
-        if (mask)
+        leaves += __popc(mask);
+        if (mask && !p.mark_apart)
         {
             const int64_t r = int64_t{ 1 } << li;
             mark_children_corners(p.bitmap, p.rowbits, p.R, p.WR, 2 * (idx & (r - 1)), 2 * ((idx >> li) & (r - 1)),
                                   2 * (idx >> (2 * li)), mask);
-            leaves += __popc(mask);
         }
         return;
     }
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_views_kernel
             if (valid && b < p.B)
             {
                 const bool word = b < 32 * kMaxMaskWords;
-                const ItemResult r = classify_item<PARTIAL, OPENGL>(src, b, wx, wy, wz, produce && word, L.skip_inside,
+                const ItemResult r = classify_item(PARTIAL, OPENGL, src, b, wx, wy, wz, produce && word, L.skip_inside,
                                                                     produce_out && word, L.skip_grow, L.last);
                 empty |= r.empty;
                 refine |= r.refine;
@@ -319,8 +320,18 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_items_kernel
     const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
     const int B = static_cast<int>(p.B);
-    // parents per chunk: enough chunks for every warp, at most one per lane
-    const int64_t per = (L.n + nwarps - 1) / nwarps;
+    // Parents per chunk: a chunk for each of 16 blocks per SM where that
+    // leaves at least eight parents (their items must fill 32 lanes), else for
+    // half as many, at most one parent per lane.  Two blocks fit an SM; the
+    // others start as those end, which evens out what parents cost, and the
+    // warps of a block take neighbouring chunks, whose integral-image reads
+    // meet in L1.  (Headline scene, levels 7 and 8: 433 and 656 us with 8
+    // blocks per SM, 376 and 625 so, 512 and 673 with resident blocks only;
+    // chunks handed out by a counter scattered the reads: 64x2048^2, level 8,
+    // 599 us against 360.)
+    const int64_t share = static_cast<int64_t>(kGridPerSm) * kWarps * p.sms;
+    const int64_t fine = (L.n + share - 1) / share, coarse = (2 * L.n + share - 1) / share;
+    const int64_t per = fine >= 8 ? fine : (coarse < 8 ? coarse : 8);
     const int ppw = static_cast<int>(per < 1 ? 1 : (per > 32 ? 32 : per));
     uint32_t items = 0, leaves = 0; // a warp's items of one level: below 2^32
 
@@ -367,7 +378,7 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_items_kernel
                 lattice_world(p.rq->corner, p.rq->length, is, li, L.inv_rc, wx, wy, wz);
                 const ViewSource src = make_view_source(p.tf, p.sat, p.H, p.W);
                 merge_item<MW>(ws, s, b,
-                               classify_item<PARTIAL, OPENGL>(src, b, wx, wy, wz, L.produce && b < 32 * MW, L.skip_inside,
+                               classify_item(PARTIAL, OPENGL, src, b, wx, wy, wz, L.produce && b < 32 * MW, L.skip_inside,
                                                               L.produce_out && b < 32 * MW, L.skip_grow, L.last));
             }
         }
@@ -593,7 +604,7 @@ __global__ void __cluster_dims__(kTopBlocks, 1, 1) __launch_bounds__(kTopThreads
             const float cx[2] = { dx ? wx[1] : wx[0], dx ? wx[2] : wx[1] };
             const float cy[2] = { dy ? wy[1] : wy[0], dy ? wy[2] : wy[1] };
             const float cz[2] = { dz ? wz[1] : wz[0], dz ? wz[2] : wz[1] };
-            const ItemResult r = classify_child<PARTIAL, OPENGL>(src, b, cx, cy, cz, produce && word, produce_out && word, grow);
+            const ItemResult r = classify_child(PARTIAL, OPENGL, src, b, cx, cy, cz, produce && word, produce_out && word, grow);
             if (r.empty)
                 atomicOr(&first.empty[pi], 1u << c);
             if (r.refine)
@@ -661,7 +672,7 @@ void launch_classify(const HullPlan& p, int li, int64_t max_parents, cudaStream_
     if (p.carve_variant[li] == 1)
     {
         // about one lane per (parent, view) item when the level is small
-        const int grid = grid_for(max_parents * p.B, threads);
+        const int grid = static_cast<int>(std::min<int64_t>((max_parents * p.B + threads - 1) / threads, static_cast<int64_t>(kGridPerSm) * p.sms));
         if (p.mask_words == 1)
             classify_items_kernel<PARTIAL, OPENGL, 1><<<grid, threads, 0, s>>>(p, li);
         else
@@ -744,8 +755,8 @@ void launch_carve_level(const HullPlan& p, int li, cudaStream_t s)
             launch_classify<false, false>(p, li, max_parents, s);
     }
     TH_LAUNCH_CHECK();
-    // The leaves are not written out: the last level marked their corners and
-    // counted them (rows_kernel closes the count), and the leaf list is emitted
+    // The leaves are not written out: the last level counted them (rows_kernel
+    // closes the count), their corners are marked from the child masks, and the leaf list is emitted
     // only when the candidates of the last level are exported.
     if (li + 1 == p.level)
         return;

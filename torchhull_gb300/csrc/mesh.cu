@@ -44,6 +44,81 @@ __global__ void mark_root_kernel(HullPlan p)
         mark_cell_corners(p.bitmap, p.rowbits, p.R, p.WR, 0, 0, 0);
 }
 
+// The corners of the leaves, the refined children of the level L-1 cells, from
+// their child masks (HullPlan::mark_apart).  256 consecutive cells are close
+// together and share most of their corners' words, so a block collects the
+// words' bits in a table in shared memory and writes each word once: atomics
+// of neighbouring cells on one word of the bitmap queued behind each other
+// (headline scene: 147 to 171 us, this 103).
+__global__ void __launch_bounds__(256) mark_corners_kernel(HullPlan p)
+{
+    __shared__ MarkTable table;
+    const int tid = threadIdx.x, li = p.level - 1;
+    const int64_t n = p.ctr->level_count[li];
+    const int64_t* parents = p.nodes + p.ctr->level_off[li];
+    const uint32_t R = static_cast<uint32_t>(p.R), wr = p.wr, low = (1u << li) - 1u;
+    uint32_t* bitmap = reinterpret_cast<uint32_t*>(p.bitmap);
+    for (int64_t t0 = static_cast<int64_t>(blockIdx.x) * 256; t0 < n; t0 += static_cast<int64_t>(gridDim.x) * 256)
+    {
+        const int64_t t = t0 + tid;
+        const uint32_t m = t < n ? p.child_masks[t] : 0u;
+        const int64_t idx = t < n ? parents[t] : 0;
+        for (int i = tid; i < kMarkSlots; i += 256)
+        {
+            table.key[i] = kNoWord;
+            table.bits[i] = 0;
+        }
+        __syncthreads();
+        if (m)
+        {
+            const uint32_t x = 2 * (static_cast<uint32_t>(idx) & low), y = 2 * (static_cast<uint32_t>(idx >> li) & low),
+                           z = 2 * static_cast<uint32_t>(idx >> (2 * li));
+            const uint32_t first = (y + z * R) * wr + (x >> 5);
+            const int b = static_cast<int>(x & 31); // even: bit 30 is the last, one bit into the next word
+#pragma unroll
+            for (int q = 0; q < 9; ++q)
+            {
+                uint32_t xb = 0; // lattice x bits 0..2 of the row (y + q % 3, z + q / 3)
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                {
+                    const int cx = c & 1, cy = (c >> 1) & 1, cz = c >> 2, dy = q % 3, dz = q / 3;
+                    if ((dy == cy || dy == cy + 1) && (dz == cz || dz == cz + 1) && ((m >> c) & 1u))
+                        xb |= 3u << cx;
+                }
+                if (!xb)
+                    continue;
+                const uint32_t w = first + (q % 3 + q / 3 * R) * wr;
+                const uint32_t lo = xb << b, hi = b > 29 ? xb >> (32 - b) : 0u;
+                if (lo && !mark_word(table, w, lo))
+                {
+                    atomicOr(bitmap + w, lo);
+                    const uint32_t row = w / wr;
+                    atomicOr(p.rowbits + (row >> 5), 1u << (row & 31));
+                }
+                if (hi && !mark_word(table, w + 1, hi))
+                {
+                    atomicOr(bitmap + w + 1, hi);
+                    const uint32_t row = w / wr;
+                    atomicOr(p.rowbits + (row >> 5), 1u << (row & 31));
+                }
+            }
+        }
+        __syncthreads();
+        for (int i = tid; i < kMarkSlots; i += 256)
+        {
+            const uint32_t w = table.key[i];
+            if (w == kNoWord)
+                continue;
+            atomicOr(bitmap + w, table.bits[i]);
+            const uint32_t row = fast_div(p.div_wr, w), rb = 1u << (row & 31);
+            if (!(__ldcg(p.rowbits + (row >> 5)) & rb))
+                atomicOr(p.rowbits + (row >> 5), rb);
+        }
+        __syncthreads();
+    }
+}
+
 // Sum of v over the block, to every thread.
 __device__ __forceinline__ unsigned long long block_sum(unsigned long long v)
 {
@@ -150,16 +225,18 @@ __global__ void __launch_bounds__(256) rows_kernel(HullPlan p)
 }
 
 // The sorted corner list and the rows' words.  A block takes a contiguous
-// range of slots, so what comes before it is summed once, 32 rows at a time; a
+// range of slots, so what comes before it is summed once, 256 rows at a time; a
 // warp takes as many rows as its lanes have 64-bit words for (three at level
 // 9): presence, runs and ranks, the list of words with corners, then per word
 // a lane per point.  The words of the bitmap and the row flags are cleared
-// behind it.  Issue-bound: headline scene 151 -> 119 us (a warp searched the
+// behind it.  Issue-bound: headline scene 151 -> 97 us (a warp searched the
 // word of every corner before, and the bitmap was cleared by another pass).
+constexpr int kRowGroup = 256; // rows whose places a block works out together
+
 __global__ void __launch_bounds__(256) corners_kernel(HullPlan p)
 {
-    __shared__ uint2 before[33];  // corners and words of the group's rows before a row
-    __shared__ uint32_t row_s[32], yz_s[32];
+    __shared__ uint2 before[kRowGroup]; // corners and words before each of the group's rows
+    __shared__ uint32_t row_s[kRowGroup], yz_s[kRowGroup];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t rows = p.ctr->rows;
     const uint32_t wr = p.wr, R = static_cast<uint32_t>(p.R);
@@ -185,18 +262,18 @@ __global__ void __launch_bounds__(256) corners_kernel(HullPlan p)
     // rows per warp and step
     const int G = WR <= 32 ? 32 / WR : 1;
     const int sub = WR <= 32 ? lane / WR : 0, first = WR <= 32 ? sub * WR : 0;
-    for (int64_t g = s0; g < s1; g += 32)
+    for (int64_t g = s0; g < s1; g += kRowGroup)
     {
-        const int nrows = static_cast<int>(s1 - g < 32 ? s1 - g : 32);
+        const int nrows = static_cast<int>(s1 - g < kRowGroup ? s1 - g : kRowGroup);
         __syncthreads();
-        if (warp == 0)
+        unsigned long long mine_sum = 0, group_sum;
+        if (tid < nrows)
         {
-            const uint2 c = lane < nrows ? p.row_cnt[g + lane] : make_uint2(0u, 0u);
-            const uint32_t cx = warp_inclusive_scan(c.x), cy = warp_inclusive_scan(c.y);
-            before[lane + 1] = make_uint2(cx, cy);
-            if (lane == 0)
-                before[0] = make_uint2(0u, 0u);
+            const uint2 c = p.row_cnt[g + tid];
+            mine_sum = (static_cast<unsigned long long>(c.y) << 32) | c.x;
         }
+        const unsigned long long ahead = block_exclusive_scan(mine_sum, &group_sum);
+        before[tid] = make_uint2(static_cast<uint32_t>(ahead), static_cast<uint32_t>(ahead >> 32));
         // the rows around each row: 3 * (dy + 1) + dz + 1
         for (int i = tid; i < nrows * 9; i += 256)
         {
@@ -283,8 +360,8 @@ __global__ void __launch_bounds__(256) corners_kernel(HullPlan p)
                 }
             }
         }
-        corners += before[32].x;
-        words += before[32].y;
+        corners += static_cast<uint32_t>(group_sum);
+        words += static_cast<uint32_t>(group_sum >> 32);
     }
     if (s1 == rows && tid == 0)
     {
@@ -810,6 +887,11 @@ void launch_corners(const HullPlan& p, cudaStream_t s)
     if (p.level == 0)
     {
         mark_root_kernel<<<1, 32, 0, s>>>(p);
+        TH_LAUNCH_CHECK();
+    }
+    else if (p.mark_apart)
+    {
+        mark_corners_kernel<<<grid_for(p.node_cap, 256), 256, 0, s>>>(p);
         TH_LAUNCH_CHECK();
     }
     launch_rank_corners(p, s);

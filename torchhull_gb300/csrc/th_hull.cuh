@@ -21,6 +21,13 @@ enum OverflowBits : int64_t
     kOverflowWords = 16,
 };
 
+// From this level on the corners of the leaves are marked by a launch of their
+// own: at level 7 (13 x 437x611) marking them in the last classify kernel took
+// 85 us for both against 91, but that kernel keeps 16 warps on an SM, too few for the
+// waits on the bitmap when there are many leaves (level 9 headline scene: 906
+// us against 625 + 103).
+constexpr int kMarkApartLevel = 8;
+
 struct DevCounters
 {
     int64_t level_count[kMaxLevel + 2]; // cells of level i (level 0: the root)
@@ -69,6 +76,8 @@ struct HullPlan
     float corner[3];
     float length;
     int level;
+    int sms;         // SMs of the device
+    bool mark_apart; // the last level's corners are marked by a launch of their own
     // octree node pool: all levels back to back
     int64_t* nodes;
     int64_t node_cap;
@@ -247,6 +256,33 @@ __device__ __forceinline__ void mark_children_corners(uint64_t* bitmap, uint32_t
         if (!(__ldcg(rowbits + (row >> 5)) & rb))
             atomicOr(rowbits + (row >> 5), rb);
     }
+}
+
+// mark_children_corners into a block's table of bitmap words (kMarkSlots
+// entries, keys kNoWord when free): false when the table is full.
+constexpr int kMarkSlots = 2048;
+
+struct MarkTable
+{
+    uint32_t key[kMarkSlots]; // word of 32 points of the bitmap
+    uint32_t bits[kMarkSlots];
+};
+
+__device__ __forceinline__ bool mark_word(MarkTable& t, uint32_t word, uint32_t bits)
+{
+    uint32_t slot = (word * 2654435761u) >> 21; // Knuth's multiplicative hash, 11 bits
+    for (int k = 0; k < 64; ++k)
+    {
+        const uint32_t had = atomicCAS(&t.key[slot], kNoWord, word);
+        if (had == kNoWord || had == word)
+        {
+            if ((*static_cast<volatile uint32_t*>(&t.bits[slot]) & bits) != bits)
+                atomicOr(&t.bits[slot], bits);
+            return true;
+        }
+        slot = (slot + 1) % kMarkSlots;
+    }
+    return false;
 }
 
 void launch_field(const HullPlan& p, cudaStream_t s);
