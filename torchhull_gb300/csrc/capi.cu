@@ -14,12 +14,12 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <numeric>
 #include <string>
 #include <vector>
 
 #include <sstream>
 
-#include "th_batch.cuh"
 #include "th_classify.cuh"
 #include "th_hull.cuh"
 #include "th_internal.h"
@@ -181,13 +181,34 @@ bool is_image_dtype(int d)
     return d >= TH_UINT8 && d <= TH_FLOAT64;
 }
 
+// What a request needs while it runs and not afterwards: the octree, the corner
+// bitmap and the field's cell-mask table (both clear between requests), sums.
+// The requests of a batch that follow each other on a stream share one.
+struct WorkPool
+{
+    DevBuf nodes, node_skip, node_out, child_masks, child_skip, child_out, carve_sums, tile_sums, cell_masks, bitmap, rowbits;
+    int64_t node_cap = 0, parent_cap = 0;
+    bool unfinished = false; // a run was cut short: the bitmaps and the cell masks may hold bits
+
+    std::vector<const DevBuf*> buffers() const
+    {
+        return { &nodes, &node_skip, &node_out, &child_masks, &child_skip, &child_out, &carve_sums, &tile_sums, &cell_masks,
+                 &bitmap, &rowbits };
+    }
+    void release()
+    {
+        for (const DevBuf* b : buffers())
+            const_cast<DevBuf*>(b)->release();
+    }
+};
+
 // Pools and the state of the last request of one context.
 struct HullSlot
 {
-    DevBuf tf, sat, ones, cell_masks, nodes, node_skip, node_out, child_masks, child_skip, child_out, carve_sums, tile_sums, bitmap,
-            rowbits, rows, row_slot, row_cnt, row_place, present, runs, word_list, rank, sign, word_cnt, word_cells, word_edges, word_chunk,
-            corners, values, counters, flags, sat_scratch;
-    int64_t node_cap = 0, corner_cap = 0, parent_cap = 0, word_cap = 0;
+    WorkPool work; // plain requests; a batch's slots use its streams' pools
+    DevBuf tf, sat, ones, rows, row_slot, row_cnt, row_place, present, runs, word_list, rank, sign, word_cnt, word_cells, word_edges,
+            word_chunk, corners, values, counters, flags, sat_scratch;
+    int64_t corner_cap = 0, word_cap = 0;
     HullPlan plan{};
     DevCounters* host = nullptr; // pinned, mapped copy of the counters
     DevCounters* host_d = nullptr; // its device address
@@ -196,7 +217,6 @@ struct HullSlot
     ReqConsts* host_rq_d = nullptr; // its device address
     th_hull_info info{};
     bool has_result = false;
-    bool unfinished = false; // the last run was cut short: the bitmaps and the cell masks may hold bits
     cudaEvent_t done = nullptr;
 
     // Captured pipelines, keyed by the plan with the per-request fields cleared.
@@ -219,9 +239,12 @@ struct HullSlot
 
     std::vector<const DevBuf*> buffers() const
     {
-        return { &tf,     &sat,  &ones,  &cell_masks,   &nodes,     &node_skip,   &node_out,  &child_masks, &child_skip, &child_out, &carve_sums, &tile_sums,
-                 &bitmap, &rowbits, &rows, &row_slot, &row_cnt, &row_place, &present, &runs, &word_list, &rank, &sign, &word_cnt, &word_cells,
-                 &word_edges, &word_chunk, &corners, &values, &counters, &flags, &sat_scratch, &rq };
+        std::vector<const DevBuf*> all = { &tf, &sat, &ones, &rows, &row_slot, &row_cnt, &row_place, &present, &runs, &word_list,
+                                           &rank, &sign, &word_cnt, &word_cells, &word_edges, &word_chunk, &corners, &values,
+                                           &counters, &flags, &sat_scratch, &rq };
+        for (const DevBuf* b : work.buffers())
+            all.push_back(b);
+        return all;
     }
 
     void release()
@@ -329,39 +352,26 @@ namespace th
 namespace
 {
 
-// Shared state of the batched form: the tagged node pool of the persistent
-// carve, the request table, and the streams the per-request stages run on.
+// Shared state of the batched form: the streams its requests run on, with a
+// work pool each.
 struct BatchState
 {
-    DevBuf reqs, nodes, node_skip, node_out, ctr, child_masks, child_skip, child_out, block_sums;
-    BatchReq* host_reqs = nullptr; // pinned, mapped
-    BatchReq* host_reqs_d = nullptr; // its device address
-    int32_t host_reqs_cap = 0;
-    BatchCounters* host_ctr = nullptr; // pinned, mapped
-    BatchCounters* host_ctr_d = nullptr; // its device address
-    int64_t node_cap = 0;
+    std::vector<WorkPool> pools;
     std::vector<cudaStream_t> streams;
     std::vector<cudaEvent_t> joins;
     cudaEvent_t fork = nullptr;
 
     void release()
     {
-        for (DevBuf* b : { &reqs, &nodes, &node_skip, &node_out, &ctr, &child_masks, &child_skip, &child_out, &block_sums })
-            b->release();
-        if (host_reqs)
-            cudaFreeHost(host_reqs);
-        if (host_ctr)
-            cudaFreeHost(host_ctr);
-        host_reqs = nullptr;
-        host_ctr = nullptr;
-        host_reqs_d = nullptr;
-        host_ctr_d = nullptr;
+        for (auto& w : pools)
+            w.release();
         for (auto s : streams)
             cudaStreamDestroy(s);
         for (auto e : joins)
             cudaEventDestroy(e);
         if (fork)
             cudaEventDestroy(fork);
+        pools.clear();
         streams.clear();
         joins.clear();
         fork = nullptr;
@@ -449,6 +459,9 @@ int64_t pool_bytes(const th_context* ctx)
         total += static_cast<int64_t>(d->bytes);
     for (const auto& s : ctx->batch)
         total += sum(s);
+    for (const auto& w : ctx->bstate.pools)
+        for (const DevBuf* d : w.buffers())
+            total += static_cast<int64_t>(d->bytes);
     return total;
 }
 
@@ -503,9 +516,8 @@ size_t counter_bytes(int64_t R)
 }
 
 // Sizes the pools of slot s for request a and fills its plan.
-// batch_slot: the request is part of a batch, whose octree lives in the
-// batch's shared node pool, so the slot keeps no octree pools of its own.
-void prepare(HullSlot& s, const th_hull_args* a, cudaStream_t st, bool field_ones, bool field_masks, bool batch_slot = false)
+// Work happens in pool w.  batch_slot: one of many, which starts smaller.
+void prepare(HullSlot& s, WorkPool& w, const th_hull_args* a, cudaStream_t st, bool field_ones, bool field_masks, bool batch_slot = false)
 {
     const int L = a->level;
     const int64_t B = a->batch, H = a->height, W = a->width;
@@ -515,21 +527,13 @@ void prepare(HullSlot& s, const th_hull_args* a, cudaStream_t st, bool field_one
     // to 16 M nodes and corners (about 0.5 GB; a level-9 hull of 32 megapixel
     // views fits without a rerun), whatever smaller requests the context
     // served before; beyond that the pools grow x4 per rerun.  Batch slots
-    // keep no octree of their own and start at 4 M corners.
-    if (batch_slot)
-    {
-        s.node_cap = std::max<int64_t>(s.node_cap, 1);
-        s.parent_cap = std::max<int64_t>(s.parent_cap, 1);
-    }
-    else
-    {
-        s.node_cap = std::max<int64_t>(s.node_cap, std::min<int64_t>(max_nodes(L), int64_t{ 1 } << 24));
-        s.parent_cap = std::max<int64_t>(s.parent_cap, std::min<int64_t>(max_nodes(L), int64_t{ 1 } << 22));
-    }
+    // start at 4 M corners.
+    w.node_cap = std::max<int64_t>(w.node_cap, std::min<int64_t>(max_nodes(L), int64_t{ 1 } << 24));
+    w.parent_cap = std::max<int64_t>(w.parent_cap, std::min<int64_t>(max_nodes(L), int64_t{ 1 } << 22));
     s.corner_cap = std::max<int64_t>(s.corner_cap, std::min<int64_t>(R * R * R, int64_t{ 1 } << (batch_slot ? 22 : 24)));
-    const int64_t node_cap = std::min<int64_t>(s.node_cap, max_nodes(L));
+    const int64_t node_cap = std::min<int64_t>(w.node_cap, max_nodes(L));
     const int64_t corner_cap = std::min<int64_t>(s.corner_cap, R * R * R);
-    const int64_t parent_cap = std::min<int64_t>(s.parent_cap, node_cap);
+    const int64_t parent_cap = std::min<int64_t>(w.parent_cap, node_cap);
     // words of 32 points of the touched rows: all rows up to 32 M words (level
     // 9: 4.7 M), more on demand; a batch slot starts at 8 M
     const int64_t all_words = R * R * 2 * WR;
@@ -550,28 +554,28 @@ void prepare(HullSlot& s, const th_hull_args* a, cudaStream_t st, bool field_one
     field_ones = field_ones && !cell_masks;
     if (field_ones)
         s.ones.ensure(sizeof(uint32_t) * std::max<int64_t>(B * H * WW, 1));
-    s.nodes.ensure(sizeof(int64_t) * node_cap);
-    s.node_skip.ensure(sizeof(uint32_t) * mask_words * node_cap);
-    s.node_out.ensure(sizeof(uint32_t) * mask_words * node_cap);
-    s.child_masks.ensure(node_cap);
-    s.child_skip.ensure(sizeof(uint32_t) * 8 * mask_words * parent_cap);
-    s.child_out.ensure(sizeof(uint32_t) * 8 * mask_words * parent_cap);
+    w.nodes.ensure(sizeof(int64_t) * node_cap);
+    w.node_skip.ensure(sizeof(uint32_t) * mask_words * node_cap);
+    w.node_out.ensure(sizeof(uint32_t) * mask_words * node_cap);
+    w.child_masks.ensure(node_cap);
+    w.child_skip.ensure(sizeof(uint32_t) * 8 * mask_words * parent_cap);
+    w.child_out.ensure(sizeof(uint32_t) * 8 * mask_words * parent_cap);
     s.flags.ensure(sizeof(unsigned int) * 4);
-    s.tile_sums.ensure(sizeof(unsigned long long) *
+    w.tile_sums.ensure(sizeof(unsigned long long) *
                        std::max<int64_t>((node_cap + kScanTile - 1) / kScanTile, word_tiles(word_cap)));
-    s.carve_sums.ensure(2 * sizeof(uint32_t) * (node_cap / 1024 + 4));
+    w.carve_sums.ensure(2 * sizeof(uint32_t) * (node_cap / 1024 + 4));
     const int64_t words = R * R * WR;
     const int64_t rwords = (R * R + 31) / 32;
-    if (s.bitmap.ensure(sizeof(uint64_t) * words))
-        TH_CUDA(cudaMemsetAsync(s.bitmap.p, 0, s.bitmap.bytes, st));
-    if (s.rowbits.ensure(sizeof(uint32_t) * rwords))
-        TH_CUDA(cudaMemsetAsync(s.rowbits.p, 0, s.rowbits.bytes, st));
-    if (s.unfinished)
+    if (w.bitmap.ensure(sizeof(uint64_t) * words))
+        TH_CUDA(cudaMemsetAsync(w.bitmap.p, 0, w.bitmap.bytes, st));
+    if (w.rowbits.ensure(sizeof(uint32_t) * rwords))
+        TH_CUDA(cudaMemsetAsync(w.rowbits.p, 0, w.rowbits.bytes, st));
+    if (w.unfinished)
     {
-        for (const DevBuf* b : { &s.bitmap, &s.rowbits, &s.cell_masks })
+        for (const DevBuf* b : { &w.bitmap, &w.rowbits, &w.cell_masks })
             if (b->p)
                 TH_CUDA(cudaMemsetAsync(b->p, 0, b->bytes, st));
-        s.unfinished = false;
+        w.unfinished = false;
     }
     s.rows.ensure(sizeof(uint32_t) * R * R);
     s.row_slot.ensure(sizeof(uint32_t) * R * R);
@@ -614,36 +618,35 @@ void prepare(HullSlot& s, const th_hull_args* a, cudaStream_t st, bool field_one
     p.level = L;
     p.mark_apart = L >= kMarkApartLevel;
     p.sms = sm_count();
-    p.nodes = s.nodes.as<int64_t>();
+    p.nodes = w.nodes.as<int64_t>();
     p.node_cap = node_cap;
-    p.child_masks = s.child_masks.as<uint8_t>();
-    p.tile_sums = s.tile_sums.as<unsigned long long>();
-    p.carve_sums[0] = s.carve_sums.as<uint32_t>();
+    p.child_masks = w.child_masks.as<uint8_t>();
+    p.tile_sums = w.tile_sums.as<unsigned long long>();
+    p.carve_sums[0] = w.carve_sums.as<uint32_t>();
     p.carve_sums[1] = p.carve_sums[0] + node_cap / 1024 + 4;
     p.mask_words = mask_words;
-    p.node_skip = s.node_skip.as<uint32_t>();
-    p.child_skip = s.child_skip.as<uint32_t>();
-    p.node_out = s.node_out.as<uint32_t>();
-    p.child_out = s.child_out.as<uint32_t>();
+    p.node_skip = w.node_skip.as<uint32_t>();
+    p.child_skip = w.child_skip.as<uint32_t>();
+    p.node_out = w.node_out.as<uint32_t>();
+    p.child_out = w.child_out.as<uint32_t>();
     p.parent_cap = parent_cap;
     p.nonbinary = s.flags.as<unsigned int>();
     // exact integer box sums need every SAT sum of two entries below 2^24
     p.skip_ok = B > 0 && H > 0 && W > 0 && H * W <= (int64_t{ 1 } << 23);
     p.field_ones = field_ones && B > 0 && H > 0 && W > 0;
     p.cell_masks = nullptr;
-    p.own_cell_masks = !batch_slot;
     if (cell_masks)
     {
-        if (s.cell_masks.ensure(sizeof(uint32_t) * mask_words * (int64_t{ 1 } << (3 * (L - 1)))))
-            TH_CUDA(cudaMemsetAsync(s.cell_masks.p, 0, s.cell_masks.bytes, st));
-        p.cell_masks = s.cell_masks.as<uint32_t>();
+        if (w.cell_masks.ensure(sizeof(uint32_t) * mask_words * (int64_t{ 1 } << (3 * (L - 1)))))
+            TH_CUDA(cudaMemsetAsync(w.cell_masks.p, 0, w.cell_masks.bytes, st));
+        p.cell_masks = w.cell_masks.as<uint32_t>();
     }
     p.ones = field_ones ? s.ones.as<uint32_t>() : nullptr;
     p.WW = WW;
     p.R = R;
     p.WR = WR;
-    p.bitmap = s.bitmap.as<uint64_t>();
-    p.rowbits = s.rowbits.as<uint32_t>();
+    p.bitmap = w.bitmap.as<uint64_t>();
+    p.rowbits = w.rowbits.as<uint32_t>();
     p.rows = s.rows.as<uint32_t>();
     p.row_slot = s.row_slot.as<uint32_t>();
     p.row_cnt = s.row_cnt.as<uint2>();
@@ -659,7 +662,7 @@ void prepare(HullSlot& s, const th_hull_args* a, cudaStream_t st, bool field_one
     p.rank = s.rank.as<uint32_t>();
     p.sign = s.sign.as<uint32_t>();
     p.mesh = WordMesh{ s.word_cnt.as<uint32_t>(), s.word_cells.as<uint32_t>(), s.word_edges.as<uint4>(),
-                       s.word_chunk.as<uint2>(), s.tile_sums.as<unsigned long long>() };
+                       s.word_chunk.as<uint2>(), w.tile_sums.as<unsigned long long>() };
     p.corners = s.corners.as<int64_t>();
     p.values = s.values.as<float>();
     p.corner_cap = corner_cap;
@@ -809,11 +812,11 @@ void run_hull_once(th_context* ctx,
     const int L = a->level;
     for (int attempt = 0; attempt < 8; ++attempt)
     {
-        prepare(s, a, st, ctx->field_ones, ctx->field_masks);
+        prepare(s, s.work, a, st, ctx->field_ones, ctx->field_masks);
         for (int i = 0; i < kMaxLevel; ++i)
             s.plan.carve_variant[i] = variants[i];
         const HullPlan& p = s.plan;
-        s.unfinished = true;
+        s.work.unfinished = true;
         if (attempt == 0)
         {
             if (ev)
@@ -832,19 +835,19 @@ void run_hull_once(th_context* ctx,
         else
             enqueue_core(ctx, s, st, ev, carve_ms != nullptr);
         TH_CUDA(cudaStreamSynchronize(st));
-        s.unfinished = false;
+        s.work.unfinished = false;
         const int64_t ovf = s.host->overflow;
         // A level wider than the skip-mask scratch only loses view skipping
         // for its excess parents (results are unchanged): keep the result and
         // grow the scratch for the next request.
         if (ovf & kOverflowParents)
-            s.parent_cap *= 4;
+            s.work.parent_cap *= 4;
         if ((ovf & ~int64_t{ kOverflowParents }) == 0)
             break;
         if (ovf & kOverflowNodes)
         {
-            s.node_cap *= 4;
-            s.unfinished = true; // cells past the pool's end are not cleared from the cell masks
+            s.work.node_cap *= 4;
+            s.work.unfinished = true; // cells past the pool's end are not cleared from the cell masks
         }
         if (ovf & kOverflowCorners)
             s.corner_cap *= 4;
@@ -913,9 +916,11 @@ void run_hull(th_context* ctx, HullSlot& s, const th_hull_args* a, cudaStream_t 
     ctx->carve_tuned[key] = (t_items < t_views) ? items_from_level4() : views_everywhere();
 }
 
-// Batched form: every request's SAT, then one persistent carve over all
-// octrees, one launch marking all leaves' corners, then the per-request
-// stages spread over a few streams; one device->host read at the end.
+// Batched form: the requests' pipelines side by side on up to eight streams,
+// the ones with most work first, with a single wait at the end.  (One
+// persistent cooperative kernel over all octrees, before, took 3.8 ms for the
+// carve of 16 mixed requests alone, whose neighbouring cells it scattered over
+// the SMs: 7393 -> 5611 us with the faster stages around it, 4495 so.)
 void run_batch(th_context* ctx, const th_hull_args* args, int32_t n, cudaStream_t st, th_hull_info* infos)
 {
     for (int32_t r = 0; r < n; ++r)
@@ -935,186 +940,89 @@ void run_batch(th_context* ctx, const th_hull_args* args, int32_t n, cudaStream_
         bs.streams.push_back(s);
         bs.joins.push_back(e);
     }
+    if (static_cast<int>(bs.pools.size()) < nstreams)
+        bs.pools.resize(nstreams);
     if (!bs.fork)
         TH_CUDA(cudaEventCreateWithFlags(&bs.fork, cudaEventDisableTiming));
-    if (bs.host_reqs_cap < n)
-    {
-        if (bs.host_reqs)
-            TH_CUDA(cudaFreeHost(bs.host_reqs));
-        alloc_mapped(&bs.host_reqs, &bs.host_reqs_d, n);
-        bs.host_reqs_cap = n;
-    }
-    if (!bs.host_ctr)
-        alloc_mapped(&bs.host_ctr, &bs.host_ctr_d);
-    int max_level = 0;
-    int64_t want_nodes = 0;
-    for (int32_t r = 0; r < n; ++r)
-    {
-        max_level = std::max(max_level, args[r].level);
-        want_nodes += std::min<int64_t>(max_nodes(args[r].level), int64_t{ 1 } << 24);
-    }
-    if (bs.node_cap == 0)
-        bs.node_cap = std::min<int64_t>(want_nodes, int64_t{ 1 } << 26);
-    bs.node_cap = std::max<int64_t>(bs.node_cap, n);
-
     for (int32_t r = 0; r < n; ++r)
     {
         HullSlot& s = ctx->batch[r];
         if (s.done)
-            TH_CUDA(cudaStreamWaitEvent(st, s.done, 0));
+            TH_CUDA(cudaStreamWaitEvent(st, s.done, 0)); // the last batch's exports read the pools
         s.has_result = false;
     }
+    std::vector<int32_t> order(n);
+    std::iota(order.begin(), order.end(), 0);
+    auto work = [&](int32_t r) { return static_cast<double>(args[r].batch) * static_cast<double>(int64_t{ 1 } << (2 * args[r].level)); };
+    std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) { return work(x) > work(y); });
     for (int attempt = 0; attempt < 8; ++attempt)
     {
-        bs.reqs.ensure(sizeof(BatchReq) * n);
-        bs.nodes.ensure(sizeof(int64_t) * bs.node_cap);
-        int mask_words = 1;
-        for (int32_t r = 0; r < n; ++r)
-            mask_words = std::max(mask_words, mask_words_for(args[r].batch));
-        bs.node_skip.ensure(sizeof(uint32_t) * mask_words * bs.node_cap);
-        bs.node_out.ensure(sizeof(uint32_t) * mask_words * bs.node_cap);
-        // view-skip masks for up to a quarter of the pool's cells in one level
-        const int64_t skip_cap = std::max<int64_t>(bs.node_cap / 4, 1);
-        bs.child_masks.ensure(static_cast<size_t>(bs.node_cap));
-        bs.child_skip.ensure(sizeof(uint32_t) * 8 * mask_words * skip_cap);
-        bs.child_out.ensure(sizeof(uint32_t) * 8 * mask_words * skip_cap);
-        bs.block_sums.ensure(sizeof(unsigned long long) * 8 * sm_count());
-        bs.ctr.ensure(sizeof(BatchCounters));
-        for (int32_t r = 0; r < n; ++r)
-        {
-            const th_hull_args* a = &args[r];
-            HullSlot& s = ctx->batch[r];
-            prepare(s, a, st, ctx->field_ones, ctx->field_masks, true);
-            s.unfinished = true;
-            if (attempt > 0)
-                launch_begin(s.plan, a->transforms, a->transforms_dtype, s.host_rq_d, s.flags.as<unsigned int>(), false, st);
-            const HullPlan& p = s.plan;
-            BatchReq& q = bs.host_reqs[r];
-            q = BatchReq{};
-            q.tf = p.tf;
-            q.sat = p.sat;
-            q.H = p.H;
-            q.W = p.W;
-            q.B = static_cast<int32_t>(p.B);
-            q.level = p.level;
-            q.partial = p.partial ? 1 : 0;
-            q.opengl = p.opengl ? 1 : 0;
-            q.skip_ok = p.skip_ok ? 1 : 0;
-            // empty images or no views: the octree stops at the root (see run_hull_once)
-            q.no_carve = (p.B > 0 && p.H > 0 && p.W > 0) ? 0 : 1;
-            q.nonbinary = p.nonbinary;
-            q.corner[0] = p.corner[0];
-            q.corner[1] = p.corner[1];
-            q.corner[2] = p.corner[2];
-            q.length = p.length;
-            q.bitmap = p.bitmap;
-            q.rowbits = p.rowbits;
-            q.R = p.R;
-            q.WR = p.WR;
-            q.cell_masks = p.cell_masks;
-            q.mask_words = p.mask_words;
-        }
-        if (attempt == 0)
-        {
-            // the requests' integral images side by side on the streams (each
-            // walks its columns and rows sequentially and leaves the GPU idle)
-            TH_CUDA(cudaEventRecord(bs.fork, st));
-            for (int i = 0; i < nstreams; ++i)
-                TH_CUDA(cudaStreamWaitEvent(bs.streams[i], bs.fork, 0));
-            for (int32_t r = 0; r < n; ++r)
-            {
-                const th_hull_args* a = &args[r];
-                HullSlot& s = ctx->batch[r];
-                cudaStream_t sr = bs.streams[r % nstreams];
-                launch_begin(s.plan, a->transforms, a->transforms_dtype, s.host_rq_d, s.flags.as<unsigned int>(), true, sr);
-                launch_integral_image(a->masks, a->masks_dtype, a->batch, a->height, a->width, s.sat.as<float>(), sr,
-                                      s.flags.as<unsigned int>(),
-                                      ctx->sat_single_pass ? SatScratch{ s.sat_scratch.p } : SatScratch{});
-            }
-            for (int i = 0; i < nstreams; ++i)
-            {
-                TH_CUDA(cudaEventRecord(bs.joins[i], bs.streams[i]));
-                TH_CUDA(cudaStreamWaitEvent(st, bs.joins[i], 0));
-            }
-        }
-        small_copy(bs.reqs.p, bs.host_reqs_d, sizeof(BatchReq) * n, st);
-        BatchPlan bp{};
-        bp.reqs = bs.reqs.as<BatchReq>();
-        bp.nreq = n;
-        bp.max_level = max_level;
-        bp.nodes = bs.nodes.as<int64_t>();
-        bp.mask_words = mask_words;
-        bp.node_skip = bs.node_skip.as<uint32_t>();
-        bp.node_out = bs.node_out.as<uint32_t>();
-        bp.node_cap = bs.node_cap;
-        bp.ctr = bs.ctr.as<BatchCounters>();
-        bp.child_masks = bs.child_masks.as<uint8_t>();
-        bp.child_skip = bs.child_skip.as<uint32_t>();
-        bp.child_out = bs.child_out.as<uint32_t>();
-        bp.skip_cap = skip_cap;
-        bp.block_sums = bs.block_sums.as<unsigned long long>();
-        bp.leaf_levels = 0;
-        bp.mask_levels = 0;
-        for (int32_t r = 0; r < n; ++r)
-        {
-            const BatchReq& q = bs.host_reqs[r];
-            bp.leaf_levels |= 1u << q.level;
-            if (q.cell_masks && q.level >= 1)
-                bp.mask_levels |= 1u << (q.level - 1);
-        }
-        bp.variant = -1;
-        for (int32_t r = 0; r < n; ++r)
-        {
-            const BatchReq& q = bs.host_reqs[r];
-            const int32_t v = (q.partial << 1) | q.opengl;
-            bp.variant = (r == 0 || bp.variant == v) ? v : -2;
-        }
-        if (bp.variant < 0)
-            bp.variant = -1;
-        launch_batch_init(bp, st);
-        launch_batch_carve(bp, st);
-        launch_batch_mark(bp, st);
-        launch_batch_cell_masks(bp, true, st);
-        // per-request stages, spread over the streams
         TH_CUDA(cudaEventRecord(bs.fork, st));
         for (int i = 0; i < nstreams; ++i)
             TH_CUDA(cudaStreamWaitEvent(bs.streams[i], bs.fork, 0));
-        for (int32_t r = 0; r < n; ++r)
+        // until the wait below, no pool is known to be clear
+        auto unfinished = [&](bool u) {
+            for (int i = 0; i < nstreams; ++i)
+                bs.pools[i].unfinished = u;
+        };
+        try
         {
-            const HullPlan& p = ctx->batch[r].plan;
-            cudaStream_t sr = bs.streams[r % nstreams];
-            launch_rank_corners(p, sr);
-            launch_field(p, sr);
-            launch_marching_cubes(p, sr);
+            for (int32_t k = 0; k < n; ++k)
+            {
+                const int32_t r = order[k];
+                const th_hull_args* a = &args[r];
+                HullSlot& s = ctx->batch[r];
+                WorkPool& w = bs.pools[k % nstreams];
+                const cudaStream_t sr = bs.streams[k % nstreams];
+                prepare(s, w, a, sr, ctx->field_ones, ctx->field_masks, true);
+                const auto tuned = ctx->carve_tuned.find(tune_key(a));
+                const CarveVariants variants = ctx->carve_mode == 1 ? views_everywhere()
+                                               : ctx->carve_mode == 2 || tuned == ctx->carve_tuned.end() ? items_from_level4()
+                                                                                                         : tuned->second;
+                for (int i = 0; i < kMaxLevel; ++i)
+                    s.plan.carve_variant[i] = variants[i];
+                launch_begin(s.plan, a->transforms, a->transforms_dtype, s.host_rq_d, s.flags.as<unsigned int>(), attempt == 0, sr);
+                if (attempt == 0)
+                    launch_integral_image(a->masks, a->masks_dtype, a->batch, a->height, a->width, s.sat.as<float>(), sr,
+                                          s.flags.as<unsigned int>(),
+                                          ctx->sat_single_pass ? SatScratch{ s.sat_scratch.p } : SatScratch{});
+                enqueue_core(ctx, s, sr, nullptr, false);
+            }
         }
+        catch (...)
+        {
+            unfinished(true);
+            throw;
+        }
+        unfinished(true);
         for (int i = 0; i < nstreams; ++i)
         {
             TH_CUDA(cudaEventRecord(bs.joins[i], bs.streams[i]));
             TH_CUDA(cudaStreamWaitEvent(st, bs.joins[i], 0));
         }
-        launch_batch_cell_masks(bp, false, st);
-        small_copy(bs.host_ctr_d, bp.ctr, sizeof(BatchCounters), st);
         TH_CUDA(cudaStreamSynchronize(st));
+        unfinished(false);
         bool retry = false;
-        if (bs.host_ctr->overflow)
+        for (int32_t k = 0; k < n; ++k)
         {
-            bs.node_cap *= 4;
-            retry = true;
-        }
-        for (int32_t r = 0; r < n; ++r)
-        {
-            HullSlot& s = ctx->batch[r];
-            s.unfinished = false;
-            if (s.host->overflow & kOverflowCorners)
+            HullSlot& s = ctx->batch[order[k]];
+            WorkPool& w = bs.pools[k % nstreams];
+            const int64_t ovf = s.host->overflow;
+            // as for a plain request: only view skipping was lost
+            if (ovf & kOverflowParents)
+                w.parent_cap = std::max(w.parent_cap, 4 * s.plan.parent_cap);
+            if (ovf & kOverflowNodes)
             {
+                w.node_cap = std::max(w.node_cap, 4 * s.plan.node_cap);
+                // cells past the pool's end are not cleared from the cell
+                // masks, which later requests of the stream read: all run again
+                w.unfinished = true;
+            }
+            if (ovf & kOverflowCorners)
                 s.corner_cap *= 4;
-                retry = true;
-            }
-            if (s.host->overflow & kOverflowWords)
-            {
+            if (ovf & kOverflowWords)
                 s.word_cap *= 4;
-                retry = true;
-            }
+            retry = retry || (ovf & ~int64_t{ kOverflowParents }) != 0;
         }
         if (!retry)
             break;

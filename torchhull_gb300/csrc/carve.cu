@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(256) children_kernel(HullPlan p, int li)
     int64_t base = next + static_cast<int64_t>(total);
     const int sh = li + 1; // children ravel at resolution 2^(li+1)
     const int64_t low = (int64_t{ 1 } << li) - 1;
-    const bool cells = p.cell_masks && p.own_cell_masks && li + 2 == p.level;
+    const bool cells = p.cell_masks && li + 2 == p.level;
     for (int64_t tile = t0; tile < t1; ++tile)
     {
         const int64_t i = tile * 256 + tid;
@@ -625,7 +625,7 @@ __global__ void __cluster_dims__(kTopBlocks, 1, 1) __launch_bounds__(kTopThreads
         uint32_t at = block_exclusive_scan(static_cast<uint32_t>(__popc(mask)), &total);
         const int noff = off + n;
         const int64_t nstart = start + n;
-        const bool cells = rank == 0 && p.cell_masks && p.own_cell_masks && li + 2 == p.level;
+        const bool cells = rank == 0 && p.cell_masks && li + 2 == p.level;
         const int s = li + 1;
         for (; mask; mask &= mask - 1)
         {

@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(256) rows_kernel(HullPlan p)
         if (rows * p.wr > p.word_cap)
             c->overflow |= kOverflowWords;
         const int L = p.level;
-        if (L > 0 && p.own_cell_masks)
+        if (L > 0)
         {
             // the last level's count, with the checks of the levels before it
             const int64_t start = c->level_off[L];
@@ -781,7 +781,7 @@ struct HullWords
     // After the field: its cell-mask table is left clear for the next request.
     __device__ void tail() const
     {
-        if (!p.cell_masks || !p.own_cell_masks)
+        if (!p.cell_masks)
             return;
         const int li = p.level - 1;
         const int64_t n = p.ctr->level_count[li], off = p.ctr->level_off[li], stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
