@@ -424,6 +424,7 @@ struct th_context
     th::BatchState bstate;
     th::DevBuf blur_scratch;
     th::DevBuf blurred; // masks blurred by th_visual_hull_blurred
+    cudaEvent_t blur_done = nullptr; // the last blur that used blur_scratch
     th::DevBuf sat_aux; // th_integral_image: its 0/1 flag word, then the bit passes' scratch
     cudaEvent_t sat_aux_done = nullptr; // the last th_integral_image that used sat_aux
     th::McSlot mc;
@@ -991,6 +992,9 @@ void run_batch(th_context* ctx, const th_hull_args* args, int32_t n, cudaStream_
         }
         catch (...)
         {
+            // what is queued reads the callers' masks and the slots' buffers
+            for (int i = 0; i < nstreams; ++i)
+                cudaStreamSynchronize(bs.streams[i]);
             unfinished(true);
             throw;
         }
@@ -1048,11 +1052,10 @@ void run_batch(th_context* ctx, const th_hull_args* args, int32_t n, cudaStream_
 }
 
 // With routing on, a request whose octree alone fills the GPU (level >= 8
-// and at least 16 M mask pixels) runs through the per-request pipeline (graph
-// replay, autotuned carve kernels) and the others share the persistent carve.
-// Off by default: on a batch of four such requests routing gained 2 %, on a
-// mixed batch it lost 16 % (the routed requests no longer overlap the
-// others).  Results are identical either way.
+// and at least 16 M mask pixels) runs by itself, as th_visual_hull does, and
+// the others side by side.  Off by default: a batch's requests run through the
+// same pipeline on its streams, where the small ones fill the large ones' gaps.
+// Results are identical either way.
 bool fills_gpu(const th_hull_args& a)
 {
     return a.level >= 8 && a.batch * a.height * a.width >= (int64_t{ 1 } << 24);
@@ -1151,6 +1154,31 @@ void check_blur_args(int32_t images_dtype, int32_t kernel_size, float sigma, int
     if (!is_image_dtype(images_dtype))
         throw ArgError{ TH_ERR_UNSUPPORTED_DTYPE,
                         std::string("\"edge_kernel\" not implemented for '") + dtype_name(images_dtype) + "'" };
+}
+
+// Blurs on different streams share blur_scratch: each waits for the one before.
+// A blur recorded into a caller's graph takes no part: its order against others
+// is the graph's (an event from outside a capture cannot be waited on in it).
+bool in_capture(cudaStream_t st)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    TH_CUDA(cudaStreamIsCapturing(st, &status));
+    return status != cudaStreamCaptureStatusNone;
+}
+
+void wait_for_blur(th_context* ctx, cudaStream_t st)
+{
+    if (ctx->blur_done && !in_capture(st))
+        TH_CUDA(cudaStreamWaitEvent(st, ctx->blur_done, 0));
+}
+
+void record_blur(th_context* ctx, cudaStream_t st)
+{
+    if (in_capture(st))
+        return;
+    if (!ctx->blur_done)
+        TH_CUDA(cudaEventCreateWithFlags(&ctx->blur_done, cudaEventDisableTiming));
+    TH_CUDA(cudaEventRecord(ctx->blur_done, st));
 }
 
 // Element size of a float dtype code.
@@ -1350,6 +1378,8 @@ void th_context_destroy(th_context* ctx)
     ctx->sat_aux.release();
     if (ctx->sat_aux_done)
         cudaEventDestroy(ctx->sat_aux_done);
+    if (ctx->blur_done)
+        cudaEventDestroy(ctx->blur_done);
     ctx->mc.release();
     ctx->bstate.release();
     ctx->events.destroy();
@@ -1556,10 +1586,12 @@ th_status th_visual_hull_blurred(th_context* ctx,
         {
             ctx->blurred.ensure(float_size(args->masks_dtype) * static_cast<size_t>(n));
             const int64_t bytes = blur_tile_bytes(args->batch, args->height, args->width, kernel_size);
+            wait_for_blur(ctx, st);
             if (bytes > 0)
                 ctx->blur_scratch.ensure(static_cast<size_t>(bytes));
             launch_gaussian_blur(args->masks, args->masks_dtype, args->batch, args->height, args->width, kernel_size,
                                  sigma, true, ctx->blurred.p, args->masks_dtype, ctx->blur_scratch.as<uint8_t>(), st);
+            record_blur(ctx, st);
             a.masks = ctx->blurred.p;
         }
         run_hull(ctx, ctx->hull, &a, st, ctx->profiling ? &ctx->events : nullptr);
@@ -1667,10 +1699,13 @@ th_status th_gaussian_blur(th_context* ctx,
         if (!images || !out)
             throw ArgError{ TH_ERR_INVALID_ARGUMENT, "images or out pointer is NULL" };
         const int64_t bytes = blur_tile_bytes(batch, height, width, kernel_size);
+        const cudaStream_t st = static_cast<cudaStream_t>(stream);
+        wait_for_blur(ctx, st);
         if (bytes > 0)
             ctx->blur_scratch.ensure(static_cast<size_t>(bytes));
         launch_gaussian_blur(images, images_dtype, batch, height, width, kernel_size, sigma, sparse != 0, out, out_dtype,
-                             ctx->blur_scratch.as<uint8_t>(), static_cast<cudaStream_t>(stream));
+                             ctx->blur_scratch.as<uint8_t>(), st);
+        record_blur(ctx, st);
     });
 }
 
