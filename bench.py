@@ -12,8 +12,8 @@ OpenGL-rendered dataset.  Each request's masks are 128 MiB, so the inputs
 exceed L2 between timed iterations.
 
 GB300 arm: inputs resident in HBM.  `value` is hulls/s of the batched form
-(all Q requests of a step in one th_visual_hull_batch call: one persistent
-carve launch over the Q octrees).  Beside it: the plain drop-in
+(all Q requests of a step in one th_visual_hull_batch call, side by side on
+the batch's streams).  Beside it: the plain drop-in
 (torchhull_gb300.visual_hull, one request per call) as hulls/s and p50/p99
 per hull (as a caller runs it: the pipeline replayed as a CUDA graph), stage
 times from a separate profiled pass, whose CUDA events between the stages
@@ -81,12 +81,12 @@ METRIC = "hulls/s, level 9, 32x1024^2 views, partial masks (batched form; plain 
 WORKLOAD = ("partial-view visual hull: 32 views of 1024x1024 float32 masks, level 9, masks_partial=True, "
             "unique_verts=True, OpenGL, 8 ellipsoids + 20 capsules")
 MEASURED_PEAKS = ROOT / "MEASURED_PEAKS.json"
-# DRAM bytes (read + write) per launch of a stage's dominant kernel, from one ncu capture of the
-# same workload's first request (not measured by this run): dram__bytes_read.sum +
-# dram__bytes_write.sum of the level-8 classify_items_kernel launch.
-NCU_TRAFFIC = {"carve_level_8": 60.8e6}
-NCU_TRAFFIC_SOURCE = ("ncu --set full capture of classify_items_kernel, level 8, first request of this workload "
-                      "(dram__bytes_read.sum + dram__bytes_write.sum); a separate capture, not this run")
+# DRAM bytes (read + write) per launch of a stage's dominant kernel, from one ncu capture of a
+# request of the same workload (not measured by this run): dram__bytes.sum.per_second times
+# the duration of the level-8 classify_items_kernel launch.
+NCU_TRAFFIC = {"carve_level_8": 56.1e6}
+NCU_TRAFFIC_SOURCE = ("ncu capture of classify_items_kernel, level 8, a request of this workload "
+                      "(dram__bytes.sum.per_second times its duration); a separate capture, not this run")
 
 
 def peaks() -> tuple[float, str]:
@@ -266,12 +266,12 @@ def timed_plain(th, reqs, steps: int, dev, world: int, local: int, profile: bool
 def host_copy(th, method: str):
     """The copy the end-to-end legs move their bytes with, on the current stream: "sm" is
     torchhull_gb300's copy kernel (th_copy: a few blocks of SMs over the pinned buffers' device
-    mappings), "dma" is cudaMemcpyAsync (a copy engine).  With copy-engine copies overlapping the
-    hulls, about one loop of three on GB300 lost ~70-80 ms: a few consecutive copies ran at a
-    tenth of their rate (raw cudaMemcpyAsync as well as torch's copies, either direction).  Plain hulls: the copy kernel showed no
-    stall in 40 loops and ran ~5% below the stall-free copy-engine loops.  Batched hulls: its few
-    blocks find little room beside the persistent carve kernel (~232 against ~342 hulls/s for
-    stall-free copy-engine loops), so that leg keeps the copy engines."""
+    mappings), "dma" is cudaMemcpyAsync (a copy engine).  The copy
+    engines are the default of both legs: plain hulls 422 hulls/s against 281 with the copy kernel,
+    batched ones 480 against 250, because the hulls' kernels leave its few blocks little room.  One
+    copy-engine loop in eight (one in three while a hull took 3.1 ms) loses 70-80 ms: a few
+    consecutive copies run at a tenth of their rate (raw cudaMemcpyAsync as well as torch's copies,
+    either direction; 239 hulls/s then).  The copy kernel showed no such stall."""
     if method == "sm":
         return th._C.copy_on_sms
 
@@ -559,7 +559,7 @@ def run_gb300(args) -> dict | None:
         "data": "synthetic: seeded ray-ellipsoid/capsule masks (stand-in for the reference's rendered dataset)",
         "config": {"workload": WORKLOAD, "requests_per_step": Q, "level": LEVEL, "views": VIEWS, "side": SIDE,
                    "l2": "inputs larger than L2 (128 MiB of masks + 128 MiB SAT per request)",
-                   "path": "batched form (th_visual_hull_batch: one persistent carve launch per step)",
+                   "path": "batched form (th_visual_hull_batch: one call per step)",
                    "field_ones": args.field_ones, "field_masks": args.field_masks,
                    "mesh_verts": nv, "mesh_faces": nf, "leaves": levels[-1], "corners": corners},
         "plain": {"value": plain_value, "unit": "hulls/s", "p50_ms": percentile(per_hull, 50),
@@ -1025,11 +1025,11 @@ def main() -> None:
     ap.add_argument("--no-reference-cuda", action="store_true")
     ap.add_argument("--no-hetero", action="store_true")
     ap.add_argument("--no-serve", action="store_true")
-    ap.add_argument("--e2e-copy", choices=["dma", "sm"], default="sm",
+    ap.add_argument("--e2e-copy", choices=["dma", "sm"], default="dma",
                     help="plain end-to-end leg: host <-> device copies by the copy kernel or by copy engines")
     ap.add_argument("--e2e-batched-copy", choices=["dma", "sm"], default="dma",
                     help="batched end-to-end leg: copy engines (the copy kernel's few blocks starve beside "
-                         "the batch's persistent carve kernel)")
+                         "the batch's kernels)")
     ap.add_argument("--batch-route", choices=["on", "off"], default="off",
                     help="batched form: requests that fill the GPU alone through the per-request pipeline")
     ap.add_argument("--field-ones", choices=["on", "off"], default="on",

@@ -314,9 +314,9 @@ typedef enum th_option
      * one by one.  Profiled and autotuning runs always launch directly. */
     TH_OPTION_GRAPHS = 2,
     /* 1: th_visual_hull_batch runs requests that fill the GPU alone (level >= 8
-     * and at least 16 M mask pixels) through the per-request pipeline and the
-     * others through the shared persistent carve; 0 (default): every request
-     * through the shared carve.  Results are identical. */
+     * and at least 16 M mask pixels) one after the other, as th_visual_hull
+     * does, and the others side by side; 0 (default): all side by side.
+     * Results are identical. */
     TH_OPTION_BATCH_ROUTE = 3,
     /* 1 (default): where the field has no cell masks (below), it first
      * builds a bitmap of the 2x2 pixel footprints whose four mask values are
@@ -329,9 +329,9 @@ typedef enum th_option
      * factors are exactly 1, and it skips them; 0: every pair is evaluated.
      * Results are identical. */
     TH_OPTION_FIELD_MASKS = 5,
-    /* 1 (default): integral images of 0/1 masks (H*W <= 2^24, W <= 4096) are
-     * built in one banded pass (exact integer sums, any order); 0: always the
-     * two sequential passes in torch's addition order.  Results are identical. */
+    /* 1 (default): integral images of 0/1 masks (H*W <= 2^24) are built from
+     * bit words, each mask read once (exact integer sums, any order); 0: always
+     * the two sequential passes in torch's addition order.  Results are identical. */
     TH_OPTION_SAT_SINGLE_PASS = 6
 } th_option;
 th_status th_context_set_option(th_context* ctx, int32_t option, int64_t value);

@@ -689,7 +689,8 @@ public:
     }
 
     // A batch of requests (the tuples of visual_hull_batch) on this context:
-    // one persistent carve launch over all of them, on the current stream.
+    // their pipelines side by side on the context's streams, ordered after and
+    // before the current stream's work.
     std::vector<std::tuple<at::Tensor, at::Tensor>> visual_hull_batch(const pybind11::list& requests)
     {
         return run_batch_on(requests, ctx_, &lock_, device_);

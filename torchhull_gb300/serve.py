@@ -15,8 +15,8 @@ is free and the device memory it needs fits in the admission budget together
 with the requests already running; otherwise it waits, and later requests
 that do fit may go first (no head-of-line blocking).  With ``max_batch > 1`` a
 free slot takes all the pending requests that fit (up to that many) and runs
-them as one batch: one persistent carve launch over all their octrees, their
-integral images and mesh stages side by side on the slot's context.  Every
+them as one batch, their pipelines side by side on streams of the slot's
+context.  Every
 request's result is identical to running it alone: the kernels are
 deterministic and slots share no state.
 
@@ -45,26 +45,30 @@ def _max_nodes(level: int) -> int:
 def estimate_bytes(req: HullRequest) -> int:
     """Device bytes a request holds while it runs: its inputs plus the pools it needs.
 
-    Mirrors the pool sizing of the C library (csrc/capi.cu: prepare): SAT,
-    node and corner pools (capped at 16 M entries, the initial capacity), the
-    field's all-ones footprint bitmap and cell-mask table, and the corner
-    bitmap with its rank words.
+    Mirrors the pool sizing of the C library (csrc/capi.cu: prepare): the
+    integral images and their bit words, node and corner pools (capped at 16 M
+    entries, the initial capacity), the view masks (a second word beyond 32
+    views), the field's all-ones footprint bitmap and cell-mask table, the
+    corner bitmap, and the touched rows with their words (capped at 32 M).
     """
     B, H, W = req.masks.shape[:3]
     inputs = req.masks.numel() * req.masks.element_size() + req.transforms.numel() * req.transforms.element_size()
     L = req.level
     R = (1 << L) + 1
     WR = (R + 63) // 64
+    mask_words = 2 if B > 32 else 1
     nodes = min(_max_nodes(L), 1 << 24)
     corners = min(R**3, 1 << 24)
     parents = min(_max_nodes(L), 1 << 22)
-    sat = 4 * B * H * W
+    words = min(R * R * 2 * WR, 1 << 25)
+    sat = 4 * B * H * W + 8 * B * ((H + 31) // 32) * (W + 3)
     ones = 4 * B * H * ((W + 31) // 32)
-    cell_masks = 4 * 8 ** (L - 1) if 1 <= L <= 10 else 0
-    node_pool = nodes * (8 + 4 + 4 + 1) + parents * 64
-    corner_pool = corners * (8 + 4 + 1 + 1 + 4 + 4)
-    bitmap = R * R * WR * (8 + 4) + R * R * 4 + (R * R + 31) // 32 * 4
-    return int(inputs + sat + ones + cell_masks + node_pool + corner_pool + bitmap)
+    cell_masks = 4 * mask_words * 8 ** (L - 1) if 1 <= L <= 10 else 0
+    node_pool = nodes * (8 + 1 + 8 * mask_words) + parents * 64 * mask_words
+    corner_pool = corners * (8 + 4)
+    word_pool = words * (4 * 4 + 8 + 4 + 4 + 16) + words // 4
+    bitmap = R * R * WR * 8 + R * R * (4 + 4 + 8 + 48) + (R * R + 31) // 32 * 4
+    return int(inputs + sat + ones + cell_masks + node_pool + corner_pool + word_pool + bitmap)
 
 
 @dataclasses.dataclass(eq=False)  # jobs compare by identity (their requests hold tensors)
@@ -90,9 +94,8 @@ class HullServer:
         so the block scheduler prefers their kernels; "none": all requests alike.
 
         max_batch > 1: a slot that becomes free takes up to max_batch of the pending requests that
-        fit the budget together and runs them as one batch (th_visual_hull_batch: one persistent
-        carve launch over all of their octrees, their integral images and mesh stages side by
-        side); requests above large_bytes still run alone.  Results are the same either way."""
+        fit the budget together and runs them as one batch (th_visual_hull_batch: their pipelines
+        side by side on streams, one wait for all); requests above large_bytes still run alone.  Results are the same either way."""
         if priority not in ("exclusive_large", "large_first", "small_first", "none"):
             raise ValueError(f"unknown priority policy {priority!r}")
         if max_batch < 1:
