@@ -22,8 +22,8 @@
 //    coherent and best while every view must be evaluated;
 //  * (parent, view) items: a warp takes a chunk of parents, lists the views
 //    each parent still needs (below) and deals the items out to its lanes;
-//    results are OR-reduced over runs of lanes of the same parent, then
-//    merged in shared memory.  Best when many views are skipped.
+//    results are merged in the parent's slot by shared atomics.  Best when
+//    many views are skipped.
 // The host picks one per level (autotuned by measuring both).
 //
 // View skipping (binary masks).  When a child's pixel box grown by two pixels
@@ -309,16 +309,25 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_views_kernel
 }
 
 // (parent, view) items: a warp deals the unskipped views of a chunk of parents
-// out to its lanes.
-template <bool PARTIAL, bool OPENGL, int MW>
+// out to its lanes, or, with POOL, a block those of its warps' chunks to all
+// its threads.  The pool evens out the chunks and fills the lanes, but its
+// warps wait for the slowest three times a chunk.  At the last level, whose
+// items hand no masks on, that is less than it gives (32x1024^2, level 8: 625
+// -> 536 us; 64x2048^2, level 9: 455 -> 382; 13x437x611, level 6: 85 -> 79);
+// above it is more (level 7 of the first 378 -> 470, level 8 of the second
+// 367 -> 454).
+template <bool PARTIAL, bool OPENGL, int MW, bool POOL>
 __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_items_kernel(HullPlan p, int li)
 {
     __shared__ WarpSlots<MW> slots_all[kWarps];
-    WarpSlots<MW>& ws = slots_all[threadIdx.x >> 5];
+    constexpr int kPool = POOL ? 32 * kWarps : 1;
+    __shared__ int64_t parent_id[kPool];
+    __shared__ uint32_t parent_done[MW][kPool]; // views that are no items
+    __shared__ int first_item[kPool], warp_items[kWarps];
+    const int wi = threadIdx.x >> 5;
+    WarpSlots<MW>& ws = slots_all[wi];
     const LevelInfo L = level_info(p, li, PARTIAL);
     const int lane = threadIdx.x & 31;
-    const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
     const int B = static_cast<int>(p.B);
     // Parents per chunk: a chunk for each of 16 blocks per SM where that
     // leaves at least eight parents (their items must fill 32 lanes), else for
@@ -335,8 +344,9 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_items_kernel
     const int ppw = static_cast<int>(per < 1 ? 1 : (per > 32 ? 32 : per));
     uint32_t items = 0, leaves = 0; // a warp's items of one level: below 2^32
 
-    for (int64_t base = warp * ppw; base < L.n; base += nwarps * ppw)
+    for (int64_t first = static_cast<int64_t>(blockIdx.x) * kWarps * ppw; first < L.n; first += static_cast<int64_t>(gridDim.x) * kWarps * ppw)
     {
+        const int64_t base = first + wi * ppw;
         const int64_t pi = base + lane;
         const bool valid = lane < ppw && pi < L.n;
         const int64_t idx = valid ? L.parents[pi] : 0;
@@ -357,32 +367,75 @@ __global__ void __launch_bounds__(32 * kWarps, kMinBlocks) classify_items_kernel
         // every child is fully inside the frame
         ws.clear(lane, (PARTIAL && L.last && skipped) ? 0xffu : 0u, outm);
         const int incl = warp_inclusive_scan(count);
-        const int excl = incl - count;
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        items += static_cast<uint32_t>(total);
-        __syncwarp();
-        for (int k0 = 0; k0 < total; k0 += 32)
+        const int sum = __shfl_sync(0xffffffffu, incl, 31);
+        items += static_cast<uint32_t>(sum);
+        if constexpr (POOL)
         {
-            const int k = k0 + lane;
-            const int s = item_slot(excl, k);
-            const int es = __shfl_sync(0xffffffffu, excl, s);
-            uint32_t alls[MW];
+            if (lane == 31)
+                warp_items[wi] = sum;
+            parent_id[threadIdx.x] = idx;
 #pragma unroll
             for (int w = 0; w < MW; ++w)
-                alls[w] = __shfl_sync(0xffffffffu, all[w], s);
-            const int64_t is = __shfl_sync(0xffffffffu, idx, s);
-            if (k < total)
+                parent_done[w][threadIdx.x] = all[w];
+            __syncthreads();
+            int before = 0, total = 0;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w)
             {
-                const int b = item_view<MW>(B, alls, k - es);
-                float wx[3], wy[3], wz[3];
-                lattice_world(p.rq->corner, p.rq->length, is, li, L.inv_rc, wx, wy, wz);
-                const ViewSource src = make_view_source(p.tf, p.sat, p.H, p.W);
-                merge_item<MW>(ws, s, b,
-                               classify_item(PARTIAL, OPENGL, src, b, wx, wy, wz, L.produce && b < 32 * MW, L.skip_inside,
-                                                              L.produce_out && b < 32 * MW, L.skip_grow, L.last));
+                const int n = warp_items[w];
+                before += w < wi ? n : 0;
+                total += n;
             }
+            first_item[threadIdx.x] = before + incl - count;
+            __syncthreads();
+            for (int k = threadIdx.x; k < total; k += 32 * kWarps)
+            {
+                // the last parent whose first item is not past k
+                int s = 0;
+#pragma unroll
+                for (int step = 16 * kWarps; step > 0; step >>= 1)
+                    s += first_item[s + step] <= k ? step : 0;
+                uint32_t alls[MW];
+#pragma unroll
+                for (int w = 0; w < MW; ++w)
+                    alls[w] = parent_done[w][s];
+                const int b = item_view<MW>(B, alls, k - first_item[s]);
+                float wx[3], wy[3], wz[3];
+                lattice_world(p.rq->corner, p.rq->length, parent_id[s], li, L.inv_rc, wx, wy, wz);
+                const ViewSource src = make_view_source(p.tf, p.sat, p.H, p.W);
+                merge_item<MW>(slots_all[s >> 5], s & 31, b,
+                               classify_item(PARTIAL, OPENGL, src, b, wx, wy, wz, L.produce && b < 32 * MW, L.skip_inside,
+                                             L.produce_out && b < 32 * MW, L.skip_grow, L.last));
+            }
+            __syncthreads();
         }
-        __syncwarp();
+        else
+        {
+            const int excl = incl - count;
+            __syncwarp();
+            for (int k0 = 0; k0 < sum; k0 += 32)
+            {
+                const int k = k0 + lane;
+                const int s = item_slot(excl, k);
+                const int es = __shfl_sync(0xffffffffu, excl, s);
+                uint32_t alls[MW];
+#pragma unroll
+                for (int w = 0; w < MW; ++w)
+                    alls[w] = __shfl_sync(0xffffffffu, all[w], s);
+                const int64_t is = __shfl_sync(0xffffffffu, idx, s);
+                if (k < sum)
+                {
+                    const int b = item_view<MW>(B, alls, k - es);
+                    float wx[3], wy[3], wz[3];
+                    lattice_world(p.rq->corner, p.rq->length, is, li, L.inv_rc, wx, wy, wz);
+                    const ViewSource src = make_view_source(p.tf, p.sat, p.H, p.W);
+                    merge_item<MW>(ws, s, b,
+                                   classify_item(PARTIAL, OPENGL, src, b, wx, wy, wz, L.produce && b < 32 * MW, L.skip_inside,
+                                                                  L.produce_out && b < 32 * MW, L.skip_grow, L.last));
+                }
+            }
+            __syncwarp();
+        }
         finish_parents(p, L, li, base, valid, pi, idx, ws.empty[lane], ws.refine[lane], ws.inside[lane], PARTIAL, leaves);
         if (valid && pi < p.parent_cap && !L.last)
         {
@@ -673,10 +726,12 @@ void launch_classify(const HullPlan& p, int li, int64_t max_parents, cudaStream_
     {
         // about one lane per (parent, view) item when the level is small
         const int grid = static_cast<int>(std::min<int64_t>((max_parents * p.B + threads - 1) / threads, static_cast<int64_t>(kGridPerSm) * p.sms));
+        const bool pool = li + 1 == p.level;
         if (p.mask_words == 1)
-            classify_items_kernel<PARTIAL, OPENGL, 1><<<grid, threads, 0, s>>>(p, li);
+            (pool ? classify_items_kernel<PARTIAL, OPENGL, 1, true> : classify_items_kernel<PARTIAL, OPENGL, 1, false>)<<<grid, threads, 0, s>>>(p, li);
         else
-            classify_items_kernel<PARTIAL, OPENGL, kMaxMaskWords><<<grid, threads, 0, s>>>(p, li);
+            (pool ? classify_items_kernel<PARTIAL, OPENGL, kMaxMaskWords, true>
+                  : classify_items_kernel<PARTIAL, OPENGL, kMaxMaskWords, false>)<<<grid, threads, 0, s>>>(p, li);
         return;
     }
     const int grid = grid_for(max_parents * 32, threads);
