@@ -395,6 +395,7 @@ struct McSlot
     McPlan plan{};
     th_mc_info info{};
     bool has_result = false;
+    cudaEvent_t done = nullptr; // the last export that read the buffers
 
     std::vector<const DevBuf*> buffers() const
     {
@@ -409,6 +410,9 @@ struct McSlot
         if (host)
             cudaFreeHost(host);
         host = nullptr;
+        if (done)
+            cudaEventDestroy(done);
+        done = nullptr;
     }
 };
 
@@ -1156,9 +1160,6 @@ void check_blur_args(int32_t images_dtype, int32_t kernel_size, float sigma, int
                         std::string("\"edge_kernel\" not implemented for '") + dtype_name(images_dtype) + "'" };
 }
 
-// Blurs on different streams share blur_scratch: each waits for the one before.
-// A blur recorded into a caller's graph takes no part: its order against others
-// is the graph's (an event from outside a capture cannot be waited on in it).
 bool in_capture(cudaStream_t st)
 {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
@@ -1166,6 +1167,9 @@ bool in_capture(cudaStream_t st)
     return status != cudaStreamCaptureStatusNone;
 }
 
+// Blurs on different streams share blur_scratch: each waits for the one before.
+// A blur recorded into a caller's graph takes no part: its order against others
+// is the graph's (an event from outside a capture cannot be waited on in it).
 void wait_for_blur(th_context* ctx, cudaStream_t st)
 {
     if (ctx->blur_done && !in_capture(st))
@@ -1271,6 +1275,11 @@ void run_mc(McSlot& s, const th_mc_args* a, cudaStream_t st)
         p.div_h = make_fastdiv(static_cast<uint32_t>(H));
     }
 
+    // the last mesh may still be read from the buffers on another stream
+    if (s.done)
+        TH_CUDA(cudaStreamWaitEvent(st, s.done, 0));
+    else
+        TH_CUDA(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
     if (!s.host)
         alloc_mapped(&s.host, &s.host_d);
     s.ctr.ensure(sizeof(McCounters));
@@ -1321,9 +1330,18 @@ void run_mc(McSlot& s, const th_mc_args* a, cudaStream_t st)
         }
     }
 
-    launch_mc_count(p, st);
-    small_copy(s.host_d, p.ctr, sizeof(McCounters), st);
-    TH_CUDA(cudaStreamSynchronize(st));
+    try
+    {
+        launch_mc_count(p, st);
+        small_copy(s.host_d, p.ctr, sizeof(McCounters), st);
+        TH_CUDA(cudaStreamSynchronize(st));
+    }
+    catch (...)
+    {
+        // what is queued writes the buffers, which the next call may use on another stream
+        cudaStreamSynchronize(st);
+        throw;
+    }
     const McCounters& c = *s.host;
     if (c.flags & kMcBadIndex)
         throw ArgError{ TH_ERR_INVALID_ARGUMENT, "sparse volume indices lie outside the volume" };
@@ -1770,7 +1788,12 @@ th_status th_marching_cubes_export(th_context* ctx, float* verts, int64_t* faces
         {
             if (!verts || !faces)
                 throw ArgError{ TH_ERR_INVALID_ARGUMENT, "verts or faces pointer is NULL" };
-            launch_mc_emit(s.plan, verts, faces, static_cast<cudaStream_t>(stream));
+            const cudaStream_t st = static_cast<cudaStream_t>(stream);
+            launch_mc_emit(s.plan, verts, faces, st);
+            // an export recorded into a caller's graph is not ordered here: its
+            // event could not be waited on outside the graph
+            if (!in_capture(st))
+                TH_CUDA(cudaEventRecord(s.done, st));
         }
     });
 }
