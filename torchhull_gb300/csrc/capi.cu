@@ -13,6 +13,7 @@
 #include <atomic>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <numeric>
 #include <string>
@@ -419,6 +420,128 @@ struct McSlot
 } // namespace
 } // namespace th
 
+namespace th
+{
+namespace
+{
+
+bool in_capture(cudaStream_t st)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    TH_CUDA(cudaStreamIsCapturing(st, &status));
+    return status != cudaStreamCaptureStatusNone;
+}
+
+// Scratch of the calls that a caller records into a graph.  The graph's
+// kernels keep the addresses they were recorded with, for as long as the graph
+// or anything instantiated from it lives, and run in no order with the calls
+// outside it.  So each recorded call has a block of its own, which the graph
+// holds through a CUDA user object; when that is gone, the block is for the
+// next recording.  Blocks have power-of-two sizes and are freed with the
+// context: there are as many as were held at one time.
+class GraphScratch
+{
+public:
+    // A block of at least `bytes`, held by the graph that st is capturing.
+    void* take(cudaStream_t st, size_t bytes)
+    {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        cudaGraph_t graph = nullptr;
+        TH_CUDA(cudaStreamGetCaptureInfo(st, &status, nullptr, &graph));
+        if (status != cudaStreamCaptureStatusActive)
+            throw CudaError{ cudaErrorStreamCaptureInvalidated, "scratch of a recorded call" };
+        size_t size = 256;
+        while (size < bytes)
+            size *= 2;
+        void* p = nullptr;
+        {
+            std::lock_guard<std::mutex> g(blocks_->lock);
+            for (Block& b : blocks_->all)
+            {
+                if (!b.held && b.size == size)
+                {
+                    b.held = true;
+                    p = b.p;
+                    break;
+                }
+            }
+        }
+        if (!p)
+        {
+            // an allocation is no part of the graph: allowed in the relaxed mode
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            TH_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+            const cudaError_t e = cudaMalloc(&p, size);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            TH_CUDA(e);
+            std::lock_guard<std::mutex> g(blocks_->lock);
+            blocks_->all.push_back(Block{ p, size, true });
+        }
+        Lease* lease = new Lease{ blocks_, p };
+        cudaUserObject_t held = nullptr;
+        const cudaError_t e = cudaUserObjectCreate(&held, lease, &GraphScratch::end, 1, cudaUserObjectNoDestructorSync);
+        if (e != cudaSuccess)
+        {
+            end(lease);
+            throw CudaError{ e, "cudaUserObjectCreate" };
+        }
+        const cudaError_t r = cudaGraphRetainUserObject(graph, held, 1, cudaGraphUserObjectMove);
+        if (r != cudaSuccess)
+        {
+            cudaUserObjectRelease(held, 1);
+            throw CudaError{ r, "cudaGraphRetainUserObject" };
+        }
+        return p;
+    }
+    int64_t bytes() const
+    {
+        std::lock_guard<std::mutex> g(blocks_->lock);
+        int64_t total = 0;
+        for (const Block& b : blocks_->all)
+            total += static_cast<int64_t>(b.size);
+        return total;
+    }
+    // Frees all blocks: graphs recorded with the context are not replayed after it.
+    void release()
+    {
+        std::lock_guard<std::mutex> g(blocks_->lock);
+        for (Block& b : blocks_->all)
+            cudaFree(b.p);
+        blocks_->all.clear();
+    }
+
+private:
+    struct Block
+    {
+        void* p;
+        size_t size;
+        bool held;
+    };
+    struct Blocks
+    {
+        std::mutex lock;
+        std::vector<Block> all;
+    };
+    struct Lease
+    {
+        std::shared_ptr<Blocks> blocks; // a graph may outlive the context
+        void* p;
+    };
+    static void CUDART_CB end(void* data)
+    {
+        std::unique_ptr<Lease> lease(static_cast<Lease*>(data));
+        std::lock_guard<std::mutex> g(lease->blocks->lock);
+        for (Block& b : lease->blocks->all)
+            if (b.p == lease->p)
+                b.held = false;
+    }
+
+    std::shared_ptr<Blocks> blocks_ = std::make_shared<Blocks>();
+};
+
+} // namespace
+} // namespace th
+
 struct th_context
 {
     int device = 0;
@@ -431,6 +554,7 @@ struct th_context
     cudaEvent_t blur_done = nullptr; // the last blur that used blur_scratch
     th::DevBuf sat_aux; // th_integral_image: its 0/1 flag word, then the bit passes' scratch
     cudaEvent_t sat_aux_done = nullptr; // the last th_integral_image that used sat_aux
+    th::GraphScratch graph_scratch; // the same for blurs and integral images recorded into a caller's graph
     th::McSlot mc;
     bool profiling = false;
     th::StageEvents events;
@@ -459,7 +583,8 @@ int64_t pool_bytes(const th_context* ctx)
         return b;
     };
     int64_t total = sum(ctx->hull) + static_cast<int64_t>(ctx->blur_scratch.bytes) +
-                    static_cast<int64_t>(ctx->blurred.bytes) + static_cast<int64_t>(ctx->sat_aux.bytes);
+                    static_cast<int64_t>(ctx->blurred.bytes) + static_cast<int64_t>(ctx->sat_aux.bytes) +
+                    ctx->graph_scratch.bytes();
     for (const DevBuf* d : ctx->mc.buffers())
         total += static_cast<int64_t>(d->bytes);
     for (const auto& s : ctx->batch)
@@ -1160,29 +1285,23 @@ void check_blur_args(int32_t images_dtype, int32_t kernel_size, float sigma, int
                         std::string("\"edge_kernel\" not implemented for '") + dtype_name(images_dtype) + "'" };
 }
 
-bool in_capture(cudaStream_t st)
+// Runs launch(scratch) on st with scratch of at least `bytes`.  Calls on
+// different streams share the context's buffer: each waits for the one before.
+// A call that is recorded into a caller's graph takes a block of its own.
+template <class F>
+void with_scratch(th_context* ctx, DevBuf& buf, cudaEvent_t& done, size_t bytes, cudaStream_t st, F&& launch)
 {
-    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    TH_CUDA(cudaStreamIsCapturing(st, &status));
-    return status != cudaStreamCaptureStatusNone;
-}
-
-// Blurs on different streams share blur_scratch: each waits for the one before.
-// A blur recorded into a caller's graph takes no part: its order against others
-// is the graph's (an event from outside a capture cannot be waited on in it).
-void wait_for_blur(th_context* ctx, cudaStream_t st)
-{
-    if (ctx->blur_done && !in_capture(st))
-        TH_CUDA(cudaStreamWaitEvent(st, ctx->blur_done, 0));
-}
-
-void record_blur(th_context* ctx, cudaStream_t st)
-{
+    if (bytes == 0)
+        return launch(nullptr);
     if (in_capture(st))
-        return;
-    if (!ctx->blur_done)
-        TH_CUDA(cudaEventCreateWithFlags(&ctx->blur_done, cudaEventDisableTiming));
-    TH_CUDA(cudaEventRecord(ctx->blur_done, st));
+        return launch(ctx->graph_scratch.take(st, bytes));
+    if (done)
+        TH_CUDA(cudaStreamWaitEvent(st, done, 0));
+    else
+        TH_CUDA(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+    buf.ensure(bytes);
+    launch(buf.p);
+    TH_CUDA(cudaEventRecord(done, st));
 }
 
 // Element size of a float dtype code.
@@ -1394,6 +1513,7 @@ void th_context_destroy(th_context* ctx)
     ctx->blur_scratch.release();
     ctx->blurred.release();
     ctx->sat_aux.release();
+    ctx->graph_scratch.release();
     if (ctx->sat_aux_done)
         cudaEventDestroy(ctx->sat_aux_done);
     if (ctx->blur_done)
@@ -1604,12 +1724,10 @@ th_status th_visual_hull_blurred(th_context* ctx,
         {
             ctx->blurred.ensure(float_size(args->masks_dtype) * static_cast<size_t>(n));
             const int64_t bytes = blur_tile_bytes(args->batch, args->height, args->width, kernel_size);
-            wait_for_blur(ctx, st);
-            if (bytes > 0)
-                ctx->blur_scratch.ensure(static_cast<size_t>(bytes));
-            launch_gaussian_blur(args->masks, args->masks_dtype, args->batch, args->height, args->width, kernel_size,
-                                 sigma, true, ctx->blurred.p, args->masks_dtype, ctx->blur_scratch.as<uint8_t>(), st);
-            record_blur(ctx, st);
+            with_scratch(ctx, ctx->blur_scratch, ctx->blur_done, static_cast<size_t>(bytes), st, [&](void* scratch) {
+                launch_gaussian_blur(args->masks, args->masks_dtype, args->batch, args->height, args->width, kernel_size,
+                                     sigma, true, ctx->blurred.p, args->masks_dtype, static_cast<uint8_t*>(scratch), st);
+            });
             a.masks = ctx->blurred.p;
         }
         run_hull(ctx, ctx->hull, &a, st, ctx->profiling ? &ctx->events : nullptr);
@@ -1718,12 +1836,10 @@ th_status th_gaussian_blur(th_context* ctx,
             throw ArgError{ TH_ERR_INVALID_ARGUMENT, "images or out pointer is NULL" };
         const int64_t bytes = blur_tile_bytes(batch, height, width, kernel_size);
         const cudaStream_t st = static_cast<cudaStream_t>(stream);
-        wait_for_blur(ctx, st);
-        if (bytes > 0)
-            ctx->blur_scratch.ensure(static_cast<size_t>(bytes));
-        launch_gaussian_blur(images, images_dtype, batch, height, width, kernel_size, sigma, sparse != 0, out, out_dtype,
-                             ctx->blur_scratch.as<uint8_t>(), st);
-        record_blur(ctx, st);
+        with_scratch(ctx, ctx->blur_scratch, ctx->blur_done, static_cast<size_t>(bytes), st, [&](void* scratch) {
+            launch_gaussian_blur(images, images_dtype, batch, height, width, kernel_size, sigma, sparse != 0, out, out_dtype,
+                                 static_cast<uint8_t*>(scratch), st);
+        });
     });
 }
 
@@ -1748,24 +1864,17 @@ th_status th_integral_image(th_context* ctx,
             throw ArgError{ TH_ERR_INVALID_ARGUMENT, "masks or out pointer is NULL" };
         const cudaStream_t st = static_cast<cudaStream_t>(stream);
         const int64_t sb = ctx->sat_single_pass ? sat_scratch_bytes(batch, height, width, masks_dtype) : 0;
-        unsigned int* flag = nullptr;
-        SatScratch sc{};
-        if (sb > 0)
-        {
-            constexpr int64_t kFlagBytes = 256;
-            // calls on different streams share sat_aux: each waits for the previous one
-            if (!ctx->sat_aux_done)
-                TH_CUDA(cudaEventCreateWithFlags(&ctx->sat_aux_done, cudaEventDisableTiming));
-            else
-                TH_CUDA(cudaStreamWaitEvent(st, ctx->sat_aux_done, 0));
-            ctx->sat_aux.ensure(static_cast<size_t>(kFlagBytes + sb));
-            flag = ctx->sat_aux.as<unsigned int>();
-            launch_zero(flag, sizeof(unsigned int), st);
-            sc = SatScratch{ static_cast<unsigned char*>(ctx->sat_aux.p) + kFlagBytes };
-        }
-        launch_integral_image(masks, masks_dtype, batch, height, width, out, st, flag, sc);
-        if (sb > 0)
-            TH_CUDA(cudaEventRecord(ctx->sat_aux_done, st));
+        constexpr int64_t kFlagBytes = 256;
+        with_scratch(ctx, ctx->sat_aux, ctx->sat_aux_done, sb > 0 ? static_cast<size_t>(kFlagBytes + sb) : 0, st, [&](void* scratch) {
+            unsigned int* flag = static_cast<unsigned int*>(scratch);
+            SatScratch sc{};
+            if (flag)
+            {
+                launch_zero(flag, sizeof(unsigned int), st);
+                sc = SatScratch{ static_cast<unsigned char*>(scratch) + kFlagBytes };
+            }
+            launch_integral_image(masks, masks_dtype, batch, height, width, out, st, flag, sc);
+        });
     });
 }
 
