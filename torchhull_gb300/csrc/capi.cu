@@ -926,6 +926,13 @@ void replay_core(HullSlot& s, cudaStream_t st)
     note_launches(static_cast<int>(g->kernels));
 }
 
+// What no larger pool helps against.  The request's pool is left unfinished then.
+void refuse_overflow(int64_t overflow)
+{
+    if (overflow & kOverflowIndices)
+        throw ArgError{ TH_ERR_INVALID_ARGUMENT, "visual hull: 2^32 or more corners of leaf cells" };
+}
+
 // One complete run of a request with the given carve kernels.  carve_ms
 // (optional) receives the time of the carve stage, for the autotuner.
 void run_hull_once(th_context* ctx,
@@ -965,8 +972,9 @@ void run_hull_once(th_context* ctx,
         else
             enqueue_core(ctx, s, st, ev, carve_ms != nullptr);
         TH_CUDA(cudaStreamSynchronize(st));
-        s.work.unfinished = false;
         const int64_t ovf = s.host->overflow;
+        refuse_overflow(ovf);
+        s.work.unfinished = false;
         // A level wider than the skip-mask scratch only loses view skipping
         // for its excess parents (results are unchanged): keep the result and
         // grow the scratch for the next request.
@@ -1135,6 +1143,12 @@ void run_batch(th_context* ctx, const th_hull_args* args, int32_t n, cudaStream_
         }
         TH_CUDA(cudaStreamSynchronize(st));
         unfinished(false);
+        for (int32_t r = 0; r < n; ++r)
+        {
+            if (ctx->batch[r].host->overflow & kOverflowIndices)
+                unfinished(true);
+            refuse_overflow(ctx->batch[r].host->overflow);
+        }
         bool retry = false;
         for (int32_t k = 0; k < n; ++k)
         {

@@ -138,7 +138,7 @@ constexpr int kRowBlock = 32;
 __global__ void __launch_bounds__(256) rows_kernel(HullPlan p)
 {
     __shared__ uint32_t base[kRowBlock];
-    __shared__ unsigned long long s_before;
+    __shared__ unsigned long long s_before, s_corners;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t nwords = (p.R * p.R + 31) / 32;
     const int64_t first = static_cast<int64_t>(blockIdx.x) * kRowBlock;
@@ -156,7 +156,10 @@ __global__ void __launch_bounds__(256) rows_kernel(HullPlan p)
         const uint32_t incl = warp_inclusive_scan(static_cast<uint32_t>(__popc(w)));
         base[lane] = incl - __popc(w);
         if (lane == 31)
+        {
             s_before = before + incl;
+            s_corners = 0;
+        }
     }
     __syncthreads();
     if (tid == 0 && first + kRowBlock >= nwords)
@@ -183,6 +186,7 @@ __global__ void __launch_bounds__(256) rows_kernel(HullPlan p)
             c->level_off[L + 1] = start + n;
         }
     }
+    unsigned long long corners = 0; // lane 0's: of the warp
     for (int i = warp; i < kRowBlock; i += 8)
     {
         const uint32_t w = first + i < nwords ? p.rowbits[first + i] : 0u;
@@ -220,8 +224,14 @@ __global__ void __launch_bounds__(256) rows_kernel(HullPlan p)
                 atomicAdd(&p.coarse[g0 + 1].x, c1);
                 atomicAdd(&p.coarse[g0 + 1].y, u1);
             }
+            corners += c0 + c1;
         }
     }
+    if (corners)
+        atomicAdd(&s_corners, corners);
+    __syncthreads();
+    if (tid == 0 && s_corners)
+        atomicAdd(&p.ctr->row_corners, s_corners);
 }
 
 // The sorted corner list and the rows' words.  A block takes a contiguous
@@ -250,7 +260,13 @@ __global__ void __launch_bounds__(256) corners_kernel(HullPlan p)
     const int64_t s1 = s0 + per * 32 < rows ? s0 + per * 32 : rows;
     if (s0 >= rows)
         return;
-    // corners below 2^31, words below 2^32: summed packed
+    if (p.ctr->row_corners >> 32)
+    {
+        if (s0 == 0 && tid == 0)
+            p.ctr->overflow |= kOverflowIndices; // corners and words stay 0: nothing after this has any to look at
+        return;
+    }
+    // corners and words below 2^32: summed packed
     unsigned long long sum = 0;
     auto add = [&](uint2 c) { sum += (static_cast<unsigned long long>(c.y) << 32) | c.x; };
     for (int64_t i = tid; i < s0 / 256; i += 256)

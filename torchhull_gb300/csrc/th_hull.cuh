@@ -16,7 +16,7 @@ enum OverflowBits : int64_t
 {
     kOverflowNodes = 1,
     kOverflowCorners = 2,
-    kOverflowSoup = 4,
+    kOverflowIndices = 4, // more corners than 32-bit indices number: refused
     kOverflowParents = 8,
     kOverflowWords = 16,
 };
@@ -40,6 +40,7 @@ struct DevCounters
     int64_t overflow;                   // OverflowBits
     int64_t row_words;                  // words of the row-occupancy bitmap
     unsigned long long leaves;          // refined children of the last level
+    unsigned long long row_corners;     // corners of the touched rows (corners: once they are known to fit)
     unsigned long long items[kMaxLevel];  // (parent, view) items the carve evaluated per parent level
     unsigned long long field_items;       // (corner, view) pairs the field evaluated
     ScanState scan;
