@@ -58,3 +58,41 @@ extern "C" int64_t counters_bytes(int level)
     const int64_t R = (int64_t{ 1 } << level) + 1;
     return sizeof(DevCounters) + sizeof(uint2) * (R * R / 256 + 2);
 }
+
+namespace th
+{
+namespace
+{
+
+// n words around which every cell has four triangles (the corners of a cell
+// lie on alternating sides) but the last of a word, and no vertices.
+struct Checkers
+{
+    int64_t n;
+    __device__ int64_t words() const { return n; }
+    __device__ uint32_t word(uint32_t i) const { return i; }
+    __device__ bool empty(uint32_t) const { return false; }
+    __device__ uint32_t sign(uint32_t i) const { return (i & 3u) == 0 || (i & 3u) == 3 ? 0x55555555u : 0xaaaaaaaau; }
+    __device__ WordRows rows(uint32_t k) const { return WordRows{ { 4 * k, 4 * k + 1, 4 * k + 2, 4 * k + 3 }, false }; }
+    __device__ EdgeBits edges(uint32_t, const WordRows&, const uint32_t*, const uint32_t*, uint32_t& cells) const
+    {
+        cells = 0x7fffffffu;
+        return EdgeBits{ 0u, 0u, 0u };
+    }
+};
+
+} // namespace
+} // namespace th
+
+// Triangle corners of such words; result: overflow bits, corners.
+extern "C" int triangles_probe(int64_t words, uint32_t* cnt, uint32_t* cells, unsigned long long* tiles, void* counters, int64_t* result)
+{
+    DevCounters* ctr = static_cast<DevCounters*>(counters);
+    const WordMesh mesh{ cnt, cells, nullptr, nullptr, tiles };
+    words_count_kernel<Checkers, true><<<words_grid(words), kWordThreads>>>(Checkers{ words }, mesh, &ctr->scan, nullptr, MeshTotal{ ctr, ctr + 1 });
+    DevCounters c;
+    const cudaError_t e = cudaMemcpy(&c, ctr + 1, sizeof(c), cudaMemcpyDeviceToHost);
+    result[0] = c.overflow;
+    result[1] = c.soup;
+    return e;
+}

@@ -73,3 +73,19 @@ def test_corners_that_fit(probe, cuda):
     x = torch.arange(4097, device=cuda)
     want = torch.cat([x, x + (1 << 21), x[:100] + (2 << 21)])
     assert torch.equal(corners[: len(want)], want)
+
+
+@pytest.mark.parametrize("words", [1000, (1 << 32) // 372, (1 << 32) // 372 + 1, 12_000_000])
+def test_triangle_corners_beyond_32_bits(probe, cuda, words):
+    """31 cells of 12 triangle corners in each word."""
+    ints = lambda n: torch.zeros(n, dtype=torch.int32, device=cuda)  # noqa: E731
+    cnt, cells, tiles = ints(words), ints(words), ints(2 * (words // 1024 + 1))
+    counters = torch.zeros(2 * probe.counters_bytes(1), dtype=torch.uint8, device=cuda)
+    result = (ctypes.c_longlong * 2)()
+    torch.cuda.synchronize()
+    at = [ctypes.c_void_p(t.data_ptr()) for t in (cnt, cells, tiles, counters)]
+    rc = probe.triangles_probe(ctypes.c_longlong(words), *at, result)
+    assert rc == 0
+    assert bool(result[0] & INDICES) == (words * 372 >= 1 << 32)
+    if not result[0]:
+        assert result[1] == words * 372

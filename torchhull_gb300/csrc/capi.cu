@@ -930,7 +930,7 @@ void replay_core(HullSlot& s, cudaStream_t st)
 void refuse_overflow(int64_t overflow)
 {
     if (overflow & kOverflowIndices)
-        throw ArgError{ TH_ERR_INVALID_ARGUMENT, "visual hull: 2^32 or more corners of leaf cells" };
+        throw ArgError{ TH_ERR_INVALID_ARGUMENT, "visual hull: 2^32 or more corners of leaf cells or of triangles" };
 }
 
 // One complete run of a request with the given carve kernels.  carve_ms

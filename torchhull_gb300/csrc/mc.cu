@@ -87,11 +87,12 @@ __device__ __forceinline__ void mc_vertex(const McPlan& p, int64_t x, int64_t y,
 // ---------------------------------------------------------------------------
 // dense volumes
 
-// Triangle corners << 32 | vertices of the whole mesh.
+// Triangle corners << 32 | vertices of the whole mesh (more than 2^28 active
+// cells, 15 corners each, are refused: no total that is used has wrapped).
 struct WordTotal
 {
     McCounters* ctr;
-    __device__ void operator()(unsigned long long t) const
+    __device__ void operator()(unsigned long long t, bool) const
     {
         ctr->soup = t >> 32;
         ctr->verts = t & 0xffffffffull;

@@ -878,8 +878,10 @@ struct MeshTotal
 {
     DevCounters* ctr;
     DevCounters* host;
-    __device__ void operator()(unsigned long long total) const
+    __device__ void operator()(unsigned long long total, bool wrapped) const
     {
+        if (wrapped)
+            ctr->overflow |= kOverflowIndices;
         ctr->soup = static_cast<int64_t>(total >> 32);
         ctr->verts = static_cast<int64_t>(total & 0xffffffffull);
     }

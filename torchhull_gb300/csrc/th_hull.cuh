@@ -16,7 +16,7 @@ enum OverflowBits : int64_t
 {
     kOverflowNodes = 1,
     kOverflowCorners = 2,
-    kOverflowIndices = 4, // more corners than 32-bit indices number: refused
+    kOverflowIndices = 4, // more corners, or triangle corners, than 32 bits number: refused
     kOverflowParents = 8,
     kOverflowWords = 16,
 };

@@ -150,7 +150,10 @@ __device__ __forceinline__ uint2 word_runs(uint32_t prev, uint32_t bits, uint32_
 }
 
 // Exclusive offsets from tile sums by the block that finishes last, like
-// finish_tile_sums, eight sums per thread and round.
+// finish_tile_sums, eight sums per thread and round.  A round's triangle
+// corners are below 2^32 (2048 tiles of 1024 words, 480 corners a word), and
+// every vertex is some triangle's corner, so the packed total wraps exactly
+// when there are 2^32 triangle corners or more; epi is told.
 template <class EpiF>
 __device__ __forceinline__ void finish_word_tiles(int64_t ntiles, unsigned long long* tiles, ScanState* state, EpiF epi)
 {
@@ -163,6 +166,7 @@ __device__ __forceinline__ void finish_word_tiles(int64_t ntiles, unsigned long 
         return;
     __threadfence();
     unsigned long long carry = 0;
+    bool wrapped = false;
     for (int64_t base = 0; base < ntiles; base += 8 * kWordThreads)
     {
         const int64_t t0 = base + 8 * static_cast<int64_t>(threadIdx.x);
@@ -182,19 +186,20 @@ __device__ __forceinline__ void finish_word_tiles(int64_t ntiles, unsigned long 
                 tiles[t0 + i] = off;
             off += v[i];
         }
+        wrapped |= carry + tot < carry;
         carry += tot;
     }
     if (threadIdx.x == 0)
     {
         state->total = carry;
         state->blocks_done = 0;
-        epi(carry);
+        epi(carry, wrapped);
     }
     epi.block();
 }
 
 // Pass 1.  A thread per word; most words see one side only and leave after the
-// loads.  epi(total) gets the triangle corners << 32 | vertices on one
+// loads.  epi(total, wrapped) gets the triangle corners << 32 | vertices on one
 // thread, then epi.block() runs on the same block.
 template <class Src, bool UNIQUE, class EpiF>
 __global__ void __launch_bounds__(kWordThreads) words_count_kernel(Src src, WordMesh m, ScanState* state, unsigned long long* active, EpiF epi)
@@ -263,7 +268,7 @@ __global__ void __launch_bounds__(kWordThreads) words_count_kernel(Src src, Word
     finish_word_tiles(ntiles, m.tiles, state, epi);
 }
 
-// Pass 2: a warp numbers 8 chunks of 32 consecutive words of a tile.
+// Pass 2: a warp numbers 4 chunks of 32 consecutive words of a tile.
 template <class Src>
 __global__ void __launch_bounds__(kWordThreads) words_base_kernel(Src src, WordMesh m)
 {
