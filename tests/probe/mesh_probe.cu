@@ -70,6 +70,7 @@ struct Checkers
 {
     int64_t n;
     __device__ int64_t words() const { return n; }
+    __device__ int64_t counted() const { return 0; }
     __device__ uint32_t word(uint32_t i) const { return i; }
     __device__ bool empty(uint32_t) const { return false; }
     __device__ uint32_t sign(uint32_t i) const { return (i & 3u) == 0 || (i & 3u) == 3 ? 0x55555555u : 0xaaaaaaaau; }
@@ -88,7 +89,7 @@ struct Checkers
 extern "C" int triangles_probe(int64_t words, uint32_t* cnt, uint32_t* cells, unsigned long long* tiles, void* counters, int64_t* result)
 {
     DevCounters* ctr = static_cast<DevCounters*>(counters);
-    const WordMesh mesh{ cnt, cells, nullptr, nullptr, tiles };
+    const WordMesh mesh{ cnt, cells, nullptr, nullptr, tiles, nullptr };
     words_count_kernel<Checkers, true><<<words_grid(words), kWordThreads>>>(Checkers{ words }, mesh, &ctr->scan, nullptr, MeshTotal{ ctr, ctr + 1 });
     DevCounters c;
     const cudaError_t e = cudaMemcpy(&c, ctr + 1, sizeof(c), cudaMemcpyDeviceToHost);

@@ -390,7 +390,7 @@ namespace
 // Pools and the last result of the public marching cubes.
 struct McSlot
 {
-    DevBuf bits, rank, edges, cnt, cells, chunk, keys, slots, codes, used, vbase, tiles_soup, tiles_verts, ctr;
+    DevBuf bits, rank, edges, cnt, cells, chunk, start, keys, slots, codes, used, vbase, tiles_soup, tiles_verts, ctr;
     McCounters* host = nullptr; // pinned, mapped copy of the counters
     McCounters* host_d = nullptr; // its device address
     McPlan plan{};
@@ -400,7 +400,7 @@ struct McSlot
 
     std::vector<const DevBuf*> buffers() const
     {
-        return { &bits, &rank, &edges, &cnt, &cells, &chunk, &keys, &slots, &codes, &used, &vbase, &tiles_soup,
+        return { &bits, &rank, &edges, &cnt, &cells, &chunk, &start, &keys, &slots, &codes, &used, &vbase, &tiles_soup,
                  &tiles_verts, &ctr };
     }
 
@@ -792,7 +792,7 @@ void prepare(HullSlot& s, WorkPool& w, const th_hull_args* a, cudaStream_t st, b
     p.rank = s.rank.as<uint32_t>();
     p.sign = s.sign.as<uint32_t>();
     p.mesh = WordMesh{ s.word_cnt.as<uint32_t>(), s.word_cells.as<uint32_t>(), s.word_edges.as<uint4>(),
-                       s.word_chunk.as<uint2>(), w.tile_sums.as<unsigned long long>() };
+                       s.word_chunk.as<uint2>(), w.tile_sums.as<unsigned long long>(), nullptr };
     p.corners = s.corners.as<int64_t>();
     p.values = s.values.as<float>();
     p.corner_cap = corner_cap;
@@ -1393,8 +1393,26 @@ void run_mc(McSlot& s, const th_mc_args* a, cudaStream_t st)
     if (W > 0 && H > 0 && D > 0)
     {
         const int64_t wr = (W + 31) / 32;
-        const bool fits = H < (int64_t{ 1 } << 32) / wr && D < (int64_t{ 1 } << 32) / (wr * H); // word indices below 2^32
+        bool fits = H < (int64_t{ 1 } << 32) / wr && D < (int64_t{ 1 } << 32) / (wr * H); // word indices below 2^32
         p.nwords = fits ? wr * H * D : 0;
+        p.slab = D;
+        if (!p.sparse && H < (int64_t{ 1 } << 32) / wr)
+        {
+            // A word takes 28 bytes of scratch, however few points its row has:
+            // slabs keep it below 1.75 bytes a point (what rows of 16 points and
+            // more need), or 3.8 GB where that is less.  A slab's words are
+            // counted twice, now and for the export (12000 x 12000 x 3 float32,
+            // two slabs: 16.4 ms; 11100 x 12000 x 3 at once: 8.2).
+            const int64_t plane = wr * H;
+            const int64_t most = std::min<int64_t>(std::max<int64_t>(int64_t{ 1 } << 27, D * H * W / 16), (int64_t{ 1 } << 32) - 1);
+            if (!fits || p.nwords > most)
+            {
+                p.slab = std::max<int64_t>(most / plane - 2, 1);
+                p.nwords = std::min<int64_t>(p.slab + 2, D) * plane; // of the largest slab
+                fits = p.nwords < (int64_t{ 1 } << 32);
+            }
+        }
+        p.own = p.nwords;
         // fewer than 2^28 entries: packed counts, like the active cells of a dense volume below
         p.words = fits && (!p.sparse || (p.nnz < (int64_t{ 1 } << 28) &&
                                          (p.nwords <= kFewWords || p.nwords / kWordsPerEntry <= p.nnz)));
@@ -1435,7 +1453,12 @@ void run_mc(McSlot& s, const th_mc_args* a, cudaStream_t st)
         if (p.unique)
             s.edges.ensure(sizeof(uint4) * n);
         p.mesh = WordMesh{ s.cnt.as<uint32_t>(), s.cells.as<uint32_t>(), s.edges.as<uint4>(), s.chunk.as<uint2>(),
-                           s.tiles_soup.as<unsigned long long>() };
+                           s.tiles_soup.as<unsigned long long>(), nullptr };
+        if (p.slab < D)
+        {
+            s.start.ensure(sizeof(unsigned long long));
+            p.mesh.start = s.start.as<unsigned long long>();
+        }
     }
     else if (p.sparse)
     {

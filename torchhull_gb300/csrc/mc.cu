@@ -127,6 +127,10 @@ struct VolumeWords
     {
         return p.nwords;
     }
+    __device__ int64_t counted() const
+    {
+        return p.own;
+    }
     __device__ uint32_t word(uint32_t i) const
     {
         return i;
@@ -191,7 +195,7 @@ struct DenseWords : VolumeWords
         int64_t x, y, z;
         const int64_t q = point(k, b, x, y, z);
         const int64_t q2 = q + (axis == 0 ? 1 : (axis == 1 ? p.W : p.W * p.H));
-        mc_vertex(p, x, y, z, axis, load_f32<DT>(p.volume, q), load_f32<DT>(p.volume, q2), out);
+        mc_vertex(p, x, y, z + p.z0, axis, load_f32<DT>(p.volume, q), load_f32<DT>(p.volume, q2), out);
     }
     __device__ void values_at(const WordRows& r, int b, unsigned long long* corner) const
     {
@@ -205,7 +209,7 @@ struct DenseWords : VolumeWords
     {
         int64_t x, y, z;
         point(k, b, x, y, z);
-        mc_vertex(p, x + (lo & 1), y + (lo >> 1 & 1), z + (lo >> 2 & 1), axis,
+        mc_vertex(p, x + (lo & 1), y + (lo >> 1 & 1), z + p.z0 + (lo >> 2 & 1), axis,
                   load_f32<DT>(p.volume, static_cast<int64_t>(h1)), load_f32<DT>(p.volume, static_cast<int64_t>(h2)), out);
     }
 };
@@ -610,7 +614,7 @@ struct SparseCellEmit
 };
 
 template <class Src>
-void words_count(const Src& src, cudaStream_t s)
+void words_count(const Src& src, bool number, cudaStream_t s)
 {
     const McPlan& p = src.p;
     const int grid = words_grid(p.nwords);
@@ -619,6 +623,8 @@ void words_count(const Src& src, cudaStream_t s)
     else
         words_count_kernel<Src, false><<<grid, kWordThreads, 0, s>>>(src, p.mesh, &p.ctr->scan_soup, &p.ctr->active, WordTotal{ p.ctr });
     TH_LAUNCH_CHECK();
+    if (!number)
+        return;
     words_base_kernel<Src><<<grid, kWordThreads, 0, s>>>(src, p.mesh);
     TH_LAUNCH_CHECK();
 }
@@ -632,7 +638,7 @@ void words_emit(const Src& src, float* verts, int64_t* faces, cudaStream_t s)
 }
 
 template <int DT>
-void dense_count(const McPlan& p, cudaStream_t s)
+void dense_signs(const McPlan& p, cudaStream_t s)
 {
     constexpr int V = 16 / static_cast<int>(sizeof(typename Elem<DT>::T));
     if (reinterpret_cast<uintptr_t>(p.volume) % 16 == 0 && p.W % V == 0)
@@ -640,7 +646,53 @@ void dense_count(const McPlan& p, cudaStream_t s)
     else
         mc_sign_kernel<DT, false><<<grid_for(p.nwords * 32 / kSignLoads + 32, 256), 256, 0, s>>>(p);
     TH_LAUNCH_CHECK();
-    words_count(DenseWords<DT>{ { p } }, s);
+}
+
+template <int DT>
+void dense_count(const McPlan& p, cudaStream_t s)
+{
+    dense_signs<DT>(p, s);
+    words_count(DenseWords<DT>{ { p } }, true, s);
+}
+
+// The numbering that the next slab goes on from: what comes before word p.own,
+// or the total when there is no halo.
+__global__ void __launch_bounds__(32) mc_slab_end_kernel(McPlan p)
+{
+    unsigned long long at = p.ctr->scan_soup.total;
+    if (p.own < p.nwords)
+    {
+        const int64_t first = p.own & ~int64_t{ 31 };
+        const uint32_t c = first + threadIdx.x < p.own ? p.mesh.cnt[first + threadIdx.x] : 0u;
+        const uint2 base = p.mesh.chunk[first >> 5];
+        at = (static_cast<unsigned long long>(base.y + __reduce_add_sync(0xffffffffu, c >> 8)) << 32) |
+             (base.x + __reduce_add_sync(0xffffffffu, c & 0xffu));
+    }
+    if (threadIdx.x == 0)
+    {
+        *p.mesh.start = at;
+        WordTotal{ p.ctr }(at, false);
+    }
+}
+
+// Slab by slab: the counts, or (emit) the numbering again and the mesh.
+template <int DT>
+void dense_slabs(const McPlan& p, bool emit, float* verts, int64_t* faces, cudaStream_t s)
+{
+    TH_CUDA(cudaMemsetAsync(p.mesh.start, 0, sizeof(unsigned long long), s));
+    for (int64_t z0 = 0; z0 < p.D; z0 += p.slab)
+    {
+        McPlan q = dense_slab(p, z0);
+        dense_signs<DT>(q, s);
+        if (!emit)
+            q.nwords = q.own; // the halo is only looked at
+        words_count(DenseWords<DT>{ { q } }, emit, s);
+        mc_slab_end_kernel<<<1, 32, 0, s>>>(q);
+        TH_LAUNCH_CHECK();
+        q.nwords = q.own;
+        if (emit)
+            words_emit(DenseWords<DT>{ { q } }, verts, faces, s);
+    }
 }
 
 template <int DT>
@@ -651,7 +703,7 @@ void sparse_count(const McPlan& p, cudaStream_t s)
     {
         mc_sparse_words_kernel<DT><<<grid, 256, 0, s>>>(p);
         TH_LAUNCH_CHECK();
-        words_count(SparseWords<DT>{ { p } }, s);
+        words_count(SparseWords<DT>{ { p } }, true, s);
         return;
     }
     mc_sparse_insert_kernel<<<grid, 256, 0, s>>>(p);
@@ -701,6 +753,18 @@ void dispatch_value_dtype(int dt, F&& f)
 
 } // namespace
 
+McPlan dense_slab(const McPlan& p, int64_t z0)
+{
+    McPlan q = p;
+    q.z0 = z0;
+    const int64_t planes = p.D - z0 < p.slab ? p.D - z0 : p.slab, size = p.dtype == TH_FLOAT64 ? 8 : (p.dtype == TH_FLOAT32 ? 4 : 2);
+    q.volume = static_cast<const unsigned char*>(p.volume) + z0 * p.H * p.W * size;
+    q.D = p.D - z0 < planes + 2 ? p.D - z0 : planes + 2;
+    q.nwords = q.D * p.H * p.wr;
+    q.own = planes * p.H * p.wr;
+    return q;
+}
+
 void launch_mc_count(const McPlan& p, cudaStream_t s)
 {
     TH_CUDA(cudaMemsetAsync(p.ctr, 0, sizeof(McCounters), s));
@@ -719,7 +783,12 @@ void launch_mc_count(const McPlan& p, cudaStream_t s)
         dispatch_value_dtype(p.dtype, [&]<int DT>() { sparse_count<DT>(p, s); });
         return;
     }
-    dispatch_value_dtype(p.dtype, [&]<int DT>() { dense_count<DT>(p, s); });
+    dispatch_value_dtype(p.dtype, [&]<int DT>() {
+        if (p.slab < p.D)
+            dense_slabs<DT>(p, false, nullptr, nullptr, s);
+        else
+            dense_count<DT>(p, s);
+    });
 }
 
 void launch_mc_emit(const McPlan& p, float* verts, int64_t* faces, cudaStream_t s)
@@ -731,7 +800,12 @@ void launch_mc_emit(const McPlan& p, float* verts, int64_t* faces, cudaStream_t 
         dispatch_value_dtype(p.dtype, [&]<int DT>() { sparse_emit<DT>(p, verts, faces, s); });
         return;
     }
-    dispatch_value_dtype(p.dtype, [&]<int DT>() { words_emit(DenseWords<DT>{ { p } }, verts, faces, s); });
+    dispatch_value_dtype(p.dtype, [&]<int DT>() {
+        if (p.slab < p.D)
+            dense_slabs<DT>(p, true, verts, faces, s);
+        else
+            words_emit(DenseWords<DT>{ { p } }, verts, faces, s);
+    });
 }
 
 } // namespace th

@@ -790,6 +790,10 @@ struct HullWords
     {
         return p.ctr->words;
     }
+    __device__ int64_t counted() const
+    {
+        return 0; // not asked for
+    }
     __device__ uint32_t word(uint32_t i) const
     {
         return __ldg(p.word_list + i);

@@ -42,6 +42,11 @@ struct McPlan
     // volumes, and sparse ones whose words are few enough for their entries.
     bool words;
     int64_t nwords;
+    // A dense volume that would need too much scratch goes slab by slab of
+    // `slab` planes, through the same kernels: a plan of a slab (dense_slab) has the
+    // volume and D of its planes, z0 its first plane, and `own` words that are
+    // no halo.  The slab's numbering goes on from mesh.start.
+    int64_t slab, z0, own;
     uint32_t wr;
     FastDiv div_wr, div_h;    // by wr and by H
     uint32_t* sign;           // bit: below the isolevel
@@ -66,6 +71,10 @@ inline int64_t mc_scan_tiles(int64_t n)
     return (n + kScanTile - 1) / kScanTile;
 }
 
+// Slab `z0` of the dense volume of plan p: its own planes, and behind them the
+// one whose vertices its last cells use, with the one that gives those their
+// z edges.
+McPlan dense_slab(const McPlan& p, int64_t z0);
 // Phase 1: the soup and vertex counts (ctr) and the vertex numbering.
 void launch_mc_count(const McPlan& p, cudaStream_t s);
 // Phase 2: vertices [verts, 3] and faces [soup / 3, 3] into caller buffers.

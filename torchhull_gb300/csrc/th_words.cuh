@@ -20,6 +20,7 @@
 // are found:
 //   int64_t words() const             number of items: words in row order, at least
 //                                     those with a present point
+//   int64_t counted() const           items whose active cells are counted
 //   uint32_t word(uint32_t i) const   the word of an item
 //   void tail() const                 more work for the threads of the base pass
 //   WordRows rows(uint32_t k) const   the words of the cells that start in word k
@@ -57,6 +58,7 @@ struct WordMesh
     uint4* edges;    // per word with vertices: x, y and z edge bits, index of the first vertex
     uint2* chunk;    // per 32 items: first vertex, first triangle corner
     unsigned long long* tiles; // per tile: triangle corners << 32 | vertices, then exclusive offsets
+    unsigned long long* start; // triangle corners << 32 | vertices before the first word; nullptr: none
 };
 
 // The four rows of cell corners (row q: y + (q & 1), z + (q >> 1)) of the
@@ -155,7 +157,7 @@ __device__ __forceinline__ uint2 word_runs(uint32_t prev, uint32_t bits, uint32_
 // every vertex is some triangle's corner, so the packed total wraps exactly
 // when there are 2^32 triangle corners or more; epi is told.
 template <class EpiF>
-__device__ __forceinline__ void finish_word_tiles(int64_t ntiles, unsigned long long* tiles, ScanState* state, EpiF epi)
+__device__ __forceinline__ void finish_word_tiles(int64_t ntiles, unsigned long long* tiles, const unsigned long long* start, ScanState* state, EpiF epi)
 {
     __threadfence();
     __shared__ bool is_last;
@@ -165,7 +167,7 @@ __device__ __forceinline__ void finish_word_tiles(int64_t ntiles, unsigned long 
     if (!is_last)
         return;
     __threadfence();
-    unsigned long long carry = 0;
+    unsigned long long carry = start ? *start : 0ull;
     bool wrapped = false;
     for (int64_t base = 0; base < ntiles; base += 8 * kWordThreads)
     {
@@ -208,7 +210,7 @@ __global__ void __launch_bounds__(kWordThreads) words_count_kernel(Src src, Word
     for (int i = threadIdx.x; i < 256; i += kWordThreads)
         count[i] = words_detail::tri_count[i];
     __syncthreads();
-    const int64_t n = src.words();
+    const int64_t n = src.words(), counted = src.counted();
     const int64_t ntiles = (n + kWordTile - 1) / kWordTile;
     unsigned long long nactive = 0;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
@@ -251,7 +253,7 @@ __global__ void __launch_bounds__(kWordThreads) words_count_kernel(Src src, Word
             if (cells)
                 m.cells[i] = cells;
             sum += (static_cast<unsigned long long>(soup) << 32) | verts;
-            nactive += __popc(cells);
+            nactive += kk < counted ? __popc(cells) : 0;
         }
         unsigned long long tot;
         block_exclusive_scan(sum, &tot);
@@ -265,7 +267,7 @@ __global__ void __launch_bounds__(kWordThreads) words_count_kernel(Src src, Word
         if (threadIdx.x == 0 && tot)
             atomicAdd(active, tot);
     }
-    finish_word_tiles(ntiles, m.tiles, state, epi);
+    finish_word_tiles(ntiles, m.tiles, m.start, state, epi);
 }
 
 // Pass 2: a warp numbers 4 chunks of 32 consecutive words of a tile.
