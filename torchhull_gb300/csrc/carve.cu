@@ -605,17 +605,16 @@ __global__ void __launch_bounds__(256) children_kernel(HullPlan p, int li)
 // for 8 views, 24 for 32).  A cluster of blocks deals (child, view) tasks to
 // its lanes, eight times as many as (parent, view) items; the outcomes are
 // OR-ed into the first block's shared memory, and every block lists the next
-// level's cells for itself.  The first block writes the lists out.
+// level's cells for itself.  The first block writes the lists out.  No view is
+// ruled out here: the masks begin with the children of the level kTopLevels.
 constexpr int kTopLevels = 3;
 constexpr int kTopCells = 1 + 8 + 64 + 512; // cells of the levels 0 to 3
 constexpr int kTopBlocks = 8, kTopThreads = 512;
 
 struct TopShared
 {
-    uint32_t empty[73], refine[73];                  // per parent of the levels 0 to 2
-    uint32_t cskip[kMaxMaskWords][8 * 73], cout[kMaxMaskWords][8 * 73]; // per child
+    uint32_t empty[73], refine[73]; // per parent of the levels 0 to 2
     int32_t node[kTopCells];
-    uint32_t skip[kMaxMaskWords][kTopCells], gone[kMaxMaskWords][kTopCells];
 };
 
 template <bool PARTIAL, bool OPENGL>
@@ -627,9 +626,6 @@ __global__ void __cluster_dims__(kTopBlocks, 1, 1) __launch_bounds__(kTopThreads
     TopShared& first = *cluster.map_shared_rank(&sh, 0);
     const int tid = threadIdx.x, rank = static_cast<int>(cluster.block_rank());
     const int B = static_cast<int>(p.B);
-    const bool skips = p.skip_ok && *p.nonbinary == 0;
-    const bool items_next = p.carve_variant[levels] == 1; // the masks are for the item kernel
-    const bool produce = skips && items_next, produce_out = PARTIAL && items_next;
     const ViewSource src = make_view_source(p.tf, p.sat, p.H, p.W);
     for (int i = tid; i < static_cast<int>(sizeof(TopShared) / 4); i += kTopThreads)
         reinterpret_cast<uint32_t*>(&sh)[i] = 0;
@@ -639,17 +635,12 @@ __global__ void __cluster_dims__(kTopBlocks, 1, 1) __launch_bounds__(kTopThreads
     for (int li = 0; li < levels && n > 0; ++li)
     {
         const float inv_rc = __int_as_float((127 - (li + 1)) << 23);
-        const int grow = li + 2 == p.level ? 1 : 2;
         const int64_t tasks = static_cast<int64_t>(n) * 8 * B;
         uint32_t items = 0;
         for (int64_t t = rank * kTopThreads + tid; t < tasks; t += kTopBlocks * kTopThreads)
         {
             const int c = static_cast<int>(t & 7), q = static_cast<int>(t >> 3);
-            const int b = q / n, pi = off + (q - b * n), w = b >> 5;
-            const uint32_t bit = 1u << (b & 31);
-            const bool word = w < p.mask_words;
-            if (word && ((sh.skip[w][pi] | sh.gone[w][pi]) & bit))
-                continue;
+            const int b = q / n, pi = off + (q - b * n);
             items += c == 0 ? 1u : 0u;
             float wx[3], wy[3], wz[3];
             lattice_world(p.rq->corner, p.rq->length, sh.node[pi], li, inv_rc, wx, wy, wz);
@@ -657,15 +648,11 @@ __global__ void __cluster_dims__(kTopBlocks, 1, 1) __launch_bounds__(kTopThreads
             const float cx[2] = { dx ? wx[1] : wx[0], dx ? wx[2] : wx[1] };
             const float cy[2] = { dy ? wy[1] : wy[0], dy ? wy[2] : wy[1] };
             const float cz[2] = { dz ? wz[1] : wz[0], dz ? wz[2] : wz[1] };
-            const ItemResult r = classify_child(PARTIAL, OPENGL, src, b, cx, cy, cz, produce && word, produce_out && word, grow);
-            if (r.empty)
+            const uint32_t cls = classify_child(PARTIAL, OPENGL, src, b, cx, cy, cz);
+            if (cls == kEmpty)
                 atomicOr(&first.empty[pi], 1u << c);
-            if (r.refine)
+            else if (cls == kRefine)
                 atomicOr(&first.refine[pi], 1u << c);
-            if (r.skip)
-                atomicOr(&first.cskip[w][8 * pi + c], bit);
-            if (r.out)
-                atomicOr(&first.cout[w][8 * pi + c], bit);
         }
         items = __reduce_add_sync(0xffffffffu, items);
         if ((tid & 31) == 0 && items)
@@ -678,7 +665,6 @@ __global__ void __cluster_dims__(kTopBlocks, 1, 1) __launch_bounds__(kTopThreads
         uint32_t at = block_exclusive_scan(static_cast<uint32_t>(__popc(mask)), &total);
         const int noff = off + n;
         const int64_t nstart = start + n;
-        const bool cells = rank == 0 && p.cell_masks && li + 2 == p.level;
         const int s = li + 1;
         for (; mask; mask &= mask - 1)
         {
@@ -688,20 +674,13 @@ __global__ void __cluster_dims__(kTopBlocks, 1, 1) __launch_bounds__(kTopThreads
                               ((2 * (idx >> (2 * li)) + (c >> 2)) << (2 * s));
             sh.node[noff + at] = child;
             if (rank == 0)
-                p.nodes[nstart + at] = child;
-            for (int w = 0; w < p.mask_words; ++w)
             {
-                const uint32_t skip = produce ? (first.cskip[w][8 * pi + c] | sh.skip[w][pi]) : 0u;
-                const uint32_t gone = produce_out ? (first.cout[w][8 * pi + c] | sh.gone[w][pi]) : 0u;
-                sh.skip[w][noff + at] = skip;
-                sh.gone[w][noff + at] = gone;
-                if (rank == 0)
+                p.nodes[nstart + at] = child;
+                for (int w = 0; w < p.mask_words; ++w)
                 {
-                    p.node_skip[w * p.node_cap + nstart + at] = skip;
-                    p.node_out[w * p.node_cap + nstart + at] = gone;
+                    p.node_skip[w * p.node_cap + nstart + at] = 0;
+                    p.node_out[w * p.node_cap + nstart + at] = 0;
                 }
-                if (cells)
-                    p.cell_masks[(static_cast<int64_t>(w) << (3 * s)) + child] = skip | gone;
             }
             ++at;
         }

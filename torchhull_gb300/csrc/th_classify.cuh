@@ -1,6 +1,6 @@
-// Per-(parent, view) carve routine shared by the plain and the batched
-// carve kernels: the 3x3x3 lattice of a parent projected into one view and
-// the classification of its eight children (see carve.cu for the design).
+// Per-(parent, view) routine of the carve kernels: the 3x3x3 lattice of a
+// parent projected into one view and the classification of its eight children
+// (see carve.cu for the design).
 #pragma once
 
 #include <cfloat>
@@ -544,27 +544,22 @@ __device__ __forceinline__ ItemResult classify_item(bool PARTIAL,
     return out;
 }
 
-// One child of a parent in view b (the top levels, where a lane per child is
-// wanted for latency): classify_item's outcome for child c alone, from the same
-// operations on its eight corners.  The fields of the result are 0 or 1.
-__device__ __forceinline__ ItemResult classify_child(bool PARTIAL,
-                                                     bool OPENGL,
-                                                     const ViewSource& p,
-                                                     int64_t b,
-                                                     const float wx[2],
-                                                     const float wy[2],
-                                                     const float wz[2],
-                                                     bool want_skip,
-                                                     bool want_out,
-                                                     int grow)
+// ViewClass of one child of a parent in view b (the top levels, where a lane per
+// child is wanted for latency): classify_item's outcome for that child alone, from
+// the same operations on its eight corners.
+__device__ __forceinline__ uint32_t classify_child(bool PARTIAL,
+                                                   bool OPENGL,
+                                                   const ViewSource& p,
+                                                   int64_t b,
+                                                   const float wx[2],
+                                                   const float wy[2],
+                                                   const float wz[2])
 {
-    const int32_t H = static_cast<int32_t>(p.H), W = static_cast<int32_t>(p.W);
     const float* m = p.tf + 16 * b;
     const float4 rx = *reinterpret_cast<const float4*>(m);
     const float4 ry = *reinterpret_cast<const float4*>(m + 4);
     const float4 rd = *reinterpret_cast<const float4*>(m + (OPENGL ? 12 : 8));
     float px[8], py[8];
-    bool front = true, nan = false;
 #pragma unroll
     for (int z = 0; z < 2; ++z)
     {
@@ -580,18 +575,8 @@ __device__ __forceinline__ ItemResult classify_child(bool PARTIAL,
                 const float cx = __fmaf_rn(rx.x, wx[x], tyx), cy = __fmaf_rn(ry.x, wx[x], tyy), cd = __fmaf_rn(rd.x, wx[x], tyd);
                 float nx, ny;
                 divide_pair(cx, cy, cd, nx, ny);
-                if (OPENGL)
-                {
-                    px[k] = __fsub_rn(__fmul_rn(__fmul_rn(__fadd_rn(nx, 1.f), p.Wf), 0.5f), 0.5f);
-                    py[k] = __fsub_rn(__fmul_rn(__fmul_rn(__fadd_rn(ny, 1.f), p.Hf), 0.5f), 0.5f);
-                }
-                else
-                {
-                    px[k] = __fsub_rn(nx, 0.5f);
-                    py[k] = __fsub_rn(ny, 0.5f);
-                }
-                front = front && cd > 0.f;
-                nan = nan || !(px[k] == px[k] && py[k] == py[k]);
+                px[k] = pixel_of(OPENGL, nx, p.Wf);
+                py[k] = pixel_of(OPENGL, ny, p.Hf);
             }
         }
     }
@@ -599,10 +584,7 @@ __device__ __forceinline__ ItemResult classify_child(bool PARTIAL,
 #pragma unroll
     for (int k = 1; k < 8; ++k)
         bb = merge(bb, Box{ px[k], py[k], px[k], py[k] });
-    const bool in2 = !nan && bb.minx >= 1.5f && bb.maxx < __fsub_rn(p.Wf, 2.5f) && bb.miny >= 1.5f && bb.maxy < __fsub_rn(p.Hf, 2.5f);
-    const ViewResult r = classify_view(PARTIAL, p.sat + b * p.H * p.W, H, W, p.Hf, p.Wf, bb, want_skip && front && (!PARTIAL || in2), grow);
-    return ItemResult{ r.cls == kEmpty ? 1u : 0u, r.cls == kRefine ? 1u : 0u, 0u, r.skip ? 1u : 0u,
-                       PARTIAL && want_out && front && box_out(bb, p.Hf, p.Wf) ? 1u : 0u };
+    return classify_view(PARTIAL, p.sat + b * p.H * p.W, static_cast<int32_t>(p.H), static_cast<int32_t>(p.W), p.Hf, p.Wf, bb, false).cls;
 }
 
 // Merges an item's outcome into its slot: one shared atomic per non-zero word
