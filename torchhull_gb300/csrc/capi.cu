@@ -691,11 +691,12 @@ void prepare(HullSlot& s, WorkPool& w, const th_hull_args* a, cudaStream_t st, b
     w.child_skip.ensure(sizeof(uint32_t) * 8 * mask_words * parent_cap);
     w.child_out.ensure(sizeof(uint32_t) * 8 * mask_words * parent_cap);
     s.flags.ensure(sizeof(unsigned int) * 4);
+    const int64_t rwords = (R * R + 31) / 32;
+    const int64_t row_blocks = (rwords + kRowBlock - 1) / kRowBlock;
     w.tile_sums.ensure(sizeof(unsigned long long) *
-                       std::max<int64_t>((node_cap + kScanTile - 1) / kScanTile, word_tiles(word_cap)));
+                       std::max<int64_t>({ (node_cap + kScanTile - 1) / kScanTile, word_tiles(word_cap), row_blocks }));
     w.carve_sums.ensure(2 * sizeof(uint32_t) * (node_cap / 1024 + 4));
     const int64_t words = R * R * WR;
-    const int64_t rwords = (R * R + 31) / 32;
     if (w.bitmap.ensure(sizeof(uint64_t) * words))
         TH_CUDA(cudaMemsetAsync(w.bitmap.p, 0, w.bitmap.bytes, st));
     if (w.rowbits.ensure(sizeof(uint32_t) * rwords))
@@ -777,6 +778,7 @@ void prepare(HullSlot& s, WorkPool& w, const th_hull_args* a, cudaStream_t st, b
     p.WR = WR;
     p.bitmap = w.bitmap.as<uint64_t>();
     p.rowbits = w.rowbits.as<uint32_t>();
+    p.block_rows = row_blocks >= kCountRowBlocks ? w.tile_sums.as<uint32_t>() : nullptr; // free until the mesh passes
     p.rows = s.rows.as<uint32_t>();
     p.row_slot = s.row_slot.as<uint32_t>();
     p.row_cnt = s.row_cnt.as<uint2>();

@@ -132,8 +132,19 @@ __device__ __forceinline__ unsigned long long block_sum(unsigned long long v)
 // themselves (a few thousand words at the usual levels, read 16 bytes at a
 // time), so no pass or wait comes in between.  Headline scene (32 x 1024^2,
 // level 9, 13 M corners) on GB300: 10 us, where two scan passes over the flags
-// took 40 and a pass for the corner counts 14.
-constexpr int kRowBlock = 32;
+// took 40 and a pass for the corner counts 14.  The flags read so grow 16-fold
+// per level, so from kCountRowBlocks blocks on (levels 11 and 12)
+// row_counts_kernel counts the blocks' flags first (HullPlan::block_rows).  All
+// passes over the corners of a thin rod: level 11 102 -> 55 us, level 12 936 ->
+// 99; level 10, with 1027 blocks, takes 39 us either way.
+__global__ void __launch_bounds__(256) row_counts_kernel(HullPlan p)
+{
+    const int64_t nwords = (p.R * p.R + 31) / 32;
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; // a warp per block of rows_kernel
+    const uint32_t n = __reduce_add_sync(0xffffffffu, i < nwords ? __popc(p.rowbits[i]) : 0u);
+    if ((threadIdx.x & 31) == 0 && i < nwords)
+        p.block_rows[i / kRowBlock] = n;
+}
 
 __global__ void __launch_bounds__(256) rows_kernel(HullPlan p)
 {
@@ -143,11 +154,19 @@ __global__ void __launch_bounds__(256) rows_kernel(HullPlan p)
     const int64_t nwords = (p.R * p.R + 31) / 32;
     const int64_t first = static_cast<int64_t>(blockIdx.x) * kRowBlock;
     unsigned long long before = 0;
-    // first is a multiple of 4 and the buffer is 256-byte aligned
-    for (int64_t i = tid; i < first / 4; i += 256)
+    if (p.block_rows)
     {
-        const uint4 w = reinterpret_cast<const uint4*>(p.rowbits)[i];
-        before += __popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w);
+        for (uint32_t i = tid; i < blockIdx.x; i += 256)
+            before += p.block_rows[i];
+    }
+    else
+    {
+        // first is a multiple of 4 and the buffer is 256-byte aligned
+        for (int64_t i = tid; i < first / 4; i += 256)
+        {
+            const uint4 w = reinterpret_cast<const uint4*>(p.rowbits)[i];
+            before += __popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w);
+        }
     }
     before = block_sum(before);
     if (warp == 0)
@@ -922,6 +941,11 @@ void launch_corners(const HullPlan& p, cudaStream_t s)
 void launch_rank_corners(const HullPlan& p, cudaStream_t s)
 {
     const int64_t row_words = (p.R * p.R + 31) / 32;
+    if (p.block_rows)
+    {
+        row_counts_kernel<<<static_cast<unsigned>((row_words + 255) / 256), 256, 0, s>>>(p);
+        TH_LAUNCH_CHECK();
+    }
     rows_kernel<<<static_cast<unsigned>((row_words + kRowBlock - 1) / kRowBlock), 256, 0, s>>>(p);
     TH_LAUNCH_CHECK();
     corners_kernel<<<grid_for(p.R * p.R, 32), 256, 0, s>>>(p);

@@ -28,6 +28,9 @@ enum OverflowBits : int64_t
 // us against 625 + 103).
 constexpr int kMarkApartLevel = 8;
 
+constexpr int kRowBlock = 32;           // words of row flags a block of rows_kernel owns
+constexpr int64_t kCountRowBlocks = 2048; // blocks from which their flags are counted first
+
 struct DevCounters
 {
     int64_t level_count[kMaxLevel + 2]; // cells of level i (level 0: the root)
@@ -130,6 +133,7 @@ struct HullPlan
     uint32_t* rowbits;    // [ceil(R*R/32)] touched-row flags
     // Touched rows, ascending, and the words of 32 points of those rows only:
     // word k = slot * wr + w holds the points x = 32 w.. of row rows[slot].
+    uint32_t* block_rows; // touched rows of each block of rows_kernel, counted first (nullptr: by the blocks themselves)
     uint32_t* rows;       // [R*R]
     uint32_t* row_slot;   // [R*R] slot of a touched row (others: stale)
     RowPlace* row_place;  // [R*R] a slot's row and the rows around it
