@@ -137,13 +137,19 @@ struct DevBuf
     void* p = nullptr;
     size_t bytes = 0;
 
-    // Returns true when fresh memory was allocated (contents undefined).
-    bool ensure(size_t need)
+    // Returns true when fresh memory was allocated (contents undefined).  What
+    // uses the memory it replaces must be queued on st, or on a stream that st
+    // waits for: a batch's requests share the pool of their stream, and one that
+    // needs more is prepared while those before it still run.
+    bool ensure(size_t need, cudaStream_t st)
     {
         if (need <= bytes && p)
             return false;
         if (p)
+        {
+            TH_CUDA(cudaStreamSynchronize(st));
             TH_CUDA(cudaFree(p));
+        }
         p = nullptr;
         bytes = 0;
         size_t sz = std::max<size_t>(need, 256);
@@ -671,11 +677,11 @@ void prepare(HullSlot& s, WorkPool& w, const th_hull_args* a, cudaStream_t st, b
     const int64_t word_cap = std::min<int64_t>(s.word_cap, all_words);
     const int mask_words = mask_words_for(B);
 
-    s.tf.ensure(sizeof(float) * std::max<int64_t>(B, 1) * 16);
-    s.sat.ensure(sizeof(float) * std::max<int64_t>(B * H * W, 1));
+    s.tf.ensure(sizeof(float) * std::max<int64_t>(B, 1) * 16, st);
+    s.sat.ensure(sizeof(float) * std::max<int64_t>(B * H * W, 1), st);
     const int64_t sat_scratch = sat_scratch_bytes(B, H, W, a->masks_dtype);
     if (sat_scratch > 0)
-        s.sat_scratch.ensure(static_cast<size_t>(sat_scratch));
+        s.sat_scratch.ensure(static_cast<size_t>(sat_scratch), st);
     const int64_t WW = (W + 31) / 32;
     // the field's cell-mask table of level L-1 (up to 2^27 cells, 512 MB:
     // level 10) skips most pairs; the all-ones bitmap only pays without it
@@ -683,23 +689,23 @@ void prepare(HullSlot& s, WorkPool& w, const th_hull_args* a, cudaStream_t st, b
                             (a->masks_partial != 0 || (B > 0 && H > 0 && W > 0 && H * W <= (int64_t{ 1 } << 23)));
     field_ones = field_ones && !cell_masks;
     if (field_ones)
-        s.ones.ensure(sizeof(uint32_t) * std::max<int64_t>(B * H * WW, 1));
-    w.nodes.ensure(sizeof(int64_t) * node_cap);
-    w.node_skip.ensure(sizeof(uint32_t) * mask_words * node_cap);
-    w.node_out.ensure(sizeof(uint32_t) * mask_words * node_cap);
-    w.child_masks.ensure(node_cap);
-    w.child_skip.ensure(sizeof(uint32_t) * 8 * mask_words * parent_cap);
-    w.child_out.ensure(sizeof(uint32_t) * 8 * mask_words * parent_cap);
-    s.flags.ensure(sizeof(unsigned int) * 4);
+        s.ones.ensure(sizeof(uint32_t) * std::max<int64_t>(B * H * WW, 1), st);
+    w.nodes.ensure(sizeof(int64_t) * node_cap, st);
+    w.node_skip.ensure(sizeof(uint32_t) * mask_words * node_cap, st);
+    w.node_out.ensure(sizeof(uint32_t) * mask_words * node_cap, st);
+    w.child_masks.ensure(node_cap, st);
+    w.child_skip.ensure(sizeof(uint32_t) * 8 * mask_words * parent_cap, st);
+    w.child_out.ensure(sizeof(uint32_t) * 8 * mask_words * parent_cap, st);
+    s.flags.ensure(sizeof(unsigned int) * 4, st);
     const int64_t rwords = (R * R + 31) / 32;
     const int64_t row_blocks = (rwords + kRowBlock - 1) / kRowBlock;
     w.tile_sums.ensure(sizeof(unsigned long long) *
-                       std::max<int64_t>({ (node_cap + kScanTile - 1) / kScanTile, word_tiles(word_cap), row_blocks }));
-    w.carve_sums.ensure(2 * sizeof(uint32_t) * (node_cap / 1024 + 4));
+                       std::max<int64_t>({ (node_cap + kScanTile - 1) / kScanTile, word_tiles(word_cap), row_blocks }), st);
+    w.carve_sums.ensure(2 * sizeof(uint32_t) * (node_cap / 1024 + 4), st);
     const int64_t words = R * R * WR;
-    if (w.bitmap.ensure(sizeof(uint64_t) * words))
+    if (w.bitmap.ensure(sizeof(uint64_t) * words, st))
         TH_CUDA(cudaMemsetAsync(w.bitmap.p, 0, w.bitmap.bytes, st));
-    if (w.rowbits.ensure(sizeof(uint32_t) * rwords))
+    if (w.rowbits.ensure(sizeof(uint32_t) * rwords, st))
         TH_CUDA(cudaMemsetAsync(w.rowbits.p, 0, w.rowbits.bytes, st));
     if (w.unfinished)
     {
@@ -708,23 +714,23 @@ void prepare(HullSlot& s, WorkPool& w, const th_hull_args* a, cudaStream_t st, b
                 TH_CUDA(cudaMemsetAsync(b->p, 0, b->bytes, st));
         w.unfinished = false;
     }
-    s.rows.ensure(sizeof(uint32_t) * R * R);
-    s.row_slot.ensure(sizeof(uint32_t) * R * R);
-    s.row_cnt.ensure(sizeof(uint2) * R * R);
-    s.row_place.ensure(sizeof(RowPlace) * R * R);
-    s.present.ensure(sizeof(uint32_t) * word_cap);
-    s.word_list.ensure(sizeof(uint32_t) * word_cap);
-    s.runs.ensure(sizeof(uint2) * word_cap);
-    s.rank.ensure(sizeof(uint32_t) * word_cap);
-    s.sign.ensure(sizeof(uint32_t) * word_cap);
-    s.word_cnt.ensure(sizeof(uint32_t) * word_cap);
-    s.word_cells.ensure(sizeof(uint32_t) * word_cap);
-    s.word_edges.ensure(sizeof(uint4) * word_cap);
-    s.word_chunk.ensure(sizeof(uint2) * ((word_cap + 31) / 32));
-    s.corners.ensure(sizeof(int64_t) * corner_cap);
-    s.values.ensure(sizeof(float) * corner_cap);
+    s.rows.ensure(sizeof(uint32_t) * R * R, st);
+    s.row_slot.ensure(sizeof(uint32_t) * R * R, st);
+    s.row_cnt.ensure(sizeof(uint2) * R * R, st);
+    s.row_place.ensure(sizeof(RowPlace) * R * R, st);
+    s.present.ensure(sizeof(uint32_t) * word_cap, st);
+    s.word_list.ensure(sizeof(uint32_t) * word_cap, st);
+    s.runs.ensure(sizeof(uint2) * word_cap, st);
+    s.rank.ensure(sizeof(uint32_t) * word_cap, st);
+    s.sign.ensure(sizeof(uint32_t) * word_cap, st);
+    s.word_cnt.ensure(sizeof(uint32_t) * word_cap, st);
+    s.word_cells.ensure(sizeof(uint32_t) * word_cap, st);
+    s.word_edges.ensure(sizeof(uint4) * word_cap, st);
+    s.word_chunk.ensure(sizeof(uint2) * ((word_cap + 31) / 32), st);
+    s.corners.ensure(sizeof(int64_t) * corner_cap, st);
+    s.values.ensure(sizeof(float) * corner_cap, st);
     // the counters and, behind them, the corners of 256 rows each: cleared together
-    s.counters.ensure(counter_bytes(R));
+    s.counters.ensure(counter_bytes(R), st);
     if (!s.host)
         alloc_mapped(&s.host, &s.host_d);
     if (!s.done)
@@ -768,7 +774,7 @@ void prepare(HullSlot& s, WorkPool& w, const th_hull_args* a, cudaStream_t st, b
     p.cell_masks = nullptr;
     if (cell_masks)
     {
-        if (w.cell_masks.ensure(sizeof(uint32_t) * mask_words * (int64_t{ 1 } << (3 * (L - 1)))))
+        if (w.cell_masks.ensure(sizeof(uint32_t) * mask_words * (int64_t{ 1 } << (3 * (L - 1))), st))
             TH_CUDA(cudaMemsetAsync(w.cell_masks.p, 0, w.cell_masks.bytes, st));
         p.cell_masks = w.cell_masks.as<uint32_t>();
     }
@@ -801,7 +807,7 @@ void prepare(HullSlot& s, WorkPool& w, const th_hull_args* a, cudaStream_t st, b
     p.ctr = s.counters.as<DevCounters>();
     p.host_ctr = s.host_d;
     // the per-request inputs the carve and field kernels read from the device
-    s.rq.ensure(sizeof(ReqConsts));
+    s.rq.ensure(sizeof(ReqConsts), st);
     if (!s.host_rq)
         alloc_mapped(&s.host_rq, &s.host_rq_d);
     *s.host_rq = ReqConsts{ { p.corner[0], p.corner[1], p.corner[2] }, p.length, p.masks };
@@ -1315,7 +1321,7 @@ void with_scratch(th_context* ctx, DevBuf& buf, cudaEvent_t& done, size_t bytes,
         TH_CUDA(cudaStreamWaitEvent(st, done, 0));
     else
         TH_CUDA(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
-    buf.ensure(bytes);
+    buf.ensure(bytes, st);
     launch(buf.p);
     TH_CUDA(cudaEventRecord(done, st));
 }
@@ -1435,30 +1441,30 @@ void run_mc(McSlot& s, const th_mc_args* a, cudaStream_t st)
         TH_CUDA(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
     if (!s.host)
         alloc_mapped(&s.host, &s.host_d);
-    s.ctr.ensure(sizeof(McCounters));
+    s.ctr.ensure(sizeof(McCounters), st);
     p.ctr = s.ctr.as<McCounters>();
     if (p.words && !(p.sparse && p.nnz == 0))
     {
         const size_t n = static_cast<size_t>(p.nwords);
-        s.bits.ensure(sizeof(uint32_t) * n * (p.sparse ? 2 : 1));
+        s.bits.ensure(sizeof(uint32_t) * n * (p.sparse ? 2 : 1), st);
         p.sign = s.bits.as<uint32_t>() + (p.sparse ? n : 0);
         if (p.sparse)
         {
-            s.rank.ensure(sizeof(uint32_t) * n);
+            s.rank.ensure(sizeof(uint32_t) * n, st);
             p.present = s.bits.as<uint32_t>();
             p.rank = s.rank.as<uint32_t>();
         }
-        s.cnt.ensure(sizeof(uint32_t) * n);
-        s.cells.ensure(sizeof(uint32_t) * n);
-        s.chunk.ensure(sizeof(uint2) * ((n + 31) / 32));
-        s.tiles_soup.ensure(sizeof(unsigned long long) * word_tiles(p.nwords));
+        s.cnt.ensure(sizeof(uint32_t) * n, st);
+        s.cells.ensure(sizeof(uint32_t) * n, st);
+        s.chunk.ensure(sizeof(uint2) * ((n + 31) / 32), st);
+        s.tiles_soup.ensure(sizeof(unsigned long long) * word_tiles(p.nwords), st);
         if (p.unique)
-            s.edges.ensure(sizeof(uint4) * n);
+            s.edges.ensure(sizeof(uint4) * n, st);
         p.mesh = WordMesh{ s.cnt.as<uint32_t>(), s.cells.as<uint32_t>(), s.edges.as<uint4>(), s.chunk.as<uint2>(),
                            s.tiles_soup.as<unsigned long long>(), nullptr };
         if (p.slab < D)
         {
-            s.start.ensure(sizeof(unsigned long long));
+            s.start.ensure(sizeof(unsigned long long), st);
             p.mesh.start = s.start.as<unsigned long long>();
         }
     }
@@ -1468,10 +1474,10 @@ void run_mc(McSlot& s, const th_mc_args* a, cudaStream_t st)
         uint64_t cap = 64;
         while (cap < 2 * static_cast<uint64_t>(n))
             cap <<= 1;
-        s.keys.ensure(sizeof(unsigned long long) * cap);
-        s.slots.ensure(sizeof(int32_t) * cap);
-        s.codes.ensure(static_cast<size_t>(n));
-        s.tiles_soup.ensure(sizeof(unsigned long long) * mc_scan_tiles(n));
+        s.keys.ensure(sizeof(unsigned long long) * cap, st);
+        s.slots.ensure(sizeof(int32_t) * cap, st);
+        s.codes.ensure(static_cast<size_t>(n), st);
+        s.tiles_soup.ensure(sizeof(unsigned long long) * mc_scan_tiles(n), st);
         p.keys = s.keys.as<unsigned long long>();
         p.slots = s.slots.as<int32_t>();
         p.hmask = cap - 1;
@@ -1479,9 +1485,9 @@ void run_mc(McSlot& s, const th_mc_args* a, cudaStream_t st)
         p.tiles_soup = s.tiles_soup.as<unsigned long long>();
         if (p.unique)
         {
-            s.used.ensure(sizeof(uint32_t) * n);
-            s.vbase.ensure(sizeof(unsigned long long) * n);
-            s.tiles_verts.ensure(sizeof(unsigned long long) * mc_scan_tiles(n));
+            s.used.ensure(sizeof(uint32_t) * n, st);
+            s.vbase.ensure(sizeof(unsigned long long) * n, st);
+            s.tiles_verts.ensure(sizeof(unsigned long long) * mc_scan_tiles(n), st);
             p.used = s.used.as<uint32_t>();
             p.vbase = s.vbase.as<unsigned long long>();
             p.tiles_verts = s.tiles_verts.as<unsigned long long>();
@@ -1761,7 +1767,7 @@ th_status th_visual_hull_blurred(th_context* ctx,
         const int64_t n = args->batch * args->height * args->width;
         if (n > 0)
         {
-            ctx->blurred.ensure(float_size(args->masks_dtype) * static_cast<size_t>(n));
+            ctx->blurred.ensure(float_size(args->masks_dtype) * static_cast<size_t>(n), st);
             const int64_t bytes = blur_tile_bytes(args->batch, args->height, args->width, kernel_size);
             with_scratch(ctx, ctx->blur_scratch, ctx->blur_done, static_cast<size_t>(bytes), st, [&](void* scratch) {
                 launch_gaussian_blur(args->masks, args->masks_dtype, args->batch, args->height, args->width, kernel_size,
