@@ -438,6 +438,30 @@ bool in_capture(cudaStream_t st)
     return status != cudaStreamCaptureStatusNone;
 }
 
+// Runs launch(), the kernels of an export on st, and records `done` behind them
+// for the next request.  Exports of one result may be on several streams: each
+// waits for the one before, as some use scratch (the leaf list, the words of a
+// volume in slabs), and so the last event stands for them all.  An export
+// recorded into a caller's graph is not ordered here: its event could not be
+// waited on outside the graph.
+template <class F>
+void export_on(cudaEvent_t done, cudaStream_t st, F&& launch)
+{
+    if (in_capture(st))
+        return launch();
+    TH_CUDA(cudaStreamWaitEvent(st, done, 0));
+    try
+    {
+        launch();
+    }
+    catch (...)
+    {
+        cudaEventRecord(done, st); // what is queued
+        throw;
+    }
+    TH_CUDA(cudaEventRecord(done, st));
+}
+
 // Scratch of the calls that a caller records into a graph.  The graph's
 // kernels keep the addresses they were recorded with, for as long as the graph
 // or anything instantiated from it lives, and run in no order with the calls
@@ -1792,9 +1816,8 @@ th_status th_visual_hull_export(th_context* ctx, float* verts, int64_t* faces, v
         {
             if (!verts || !faces)
                 throw ArgError{ TH_ERR_INVALID_ARGUMENT, "verts or faces pointer is NULL" };
-            launch_export(s.plan, s.host->words, verts, faces, st);
+            export_on(s.done, st, [&] { launch_export(s.plan, s.host->words, verts, faces, st); });
         }
-        TH_CUDA(cudaEventRecord(s.done, st));
     });
 }
 
@@ -1811,13 +1834,15 @@ th_status th_visual_hull_export_candidates(th_context* ctx, int32_t level, int64
         {
             if (!dst)
                 throw ArgError{ TH_ERR_INVALID_ARGUMENT, "dst is NULL" };
-            // the leaves are written out on demand
-            if (level == s.plan.level)
-                launch_emit_leaves(s.plan, static_cast<cudaStream_t>(stream));
-            TH_CUDA(cudaMemcpyAsync(dst, s.plan.nodes + s.host->level_off[level], sizeof(int64_t) * n,
-                                    cudaMemcpyDeviceToDevice, static_cast<cudaStream_t>(stream)));
+            const cudaStream_t st = static_cast<cudaStream_t>(stream);
+            export_on(s.done, st, [&] {
+                // the leaves are written out on demand
+                if (level == s.plan.level)
+                    launch_emit_leaves(s.plan, st);
+                TH_CUDA(cudaMemcpyAsync(dst, s.plan.nodes + s.host->level_off[level], sizeof(int64_t) * n,
+                                        cudaMemcpyDeviceToDevice, st));
+            });
         }
-        TH_CUDA(cudaEventRecord(s.done, static_cast<cudaStream_t>(stream)));
     });
 }
 
@@ -1833,9 +1858,8 @@ th_status th_visual_hull_export_field(th_context* ctx, int64_t* indices, float* 
         {
             if (!indices || !values)
                 throw ArgError{ TH_ERR_INVALID_ARGUMENT, "indices or values pointer is NULL" };
-            launch_export_field(s.plan, n, indices, values, st);
+            export_on(s.done, st, [&] { launch_export_field(s.plan, n, indices, values, st); });
         }
-        TH_CUDA(cudaEventRecord(s.done, st));
     });
 }
 
@@ -1851,9 +1875,8 @@ th_status th_visual_hull_export_field_coo(th_context* ctx, int64_t* indices, flo
         {
             if (!indices || !values)
                 throw ArgError{ TH_ERR_INVALID_ARGUMENT, "indices or values pointer is NULL" };
-            launch_export_field_coo(s.plan, n, indices, values, st);
+            export_on(s.done, st, [&] { launch_export_field_coo(s.plan, n, indices, values, st); });
         }
-        TH_CUDA(cudaEventRecord(s.done, st));
     });
 }
 
@@ -1943,11 +1966,7 @@ th_status th_marching_cubes_export(th_context* ctx, float* verts, int64_t* faces
             if (!verts || !faces)
                 throw ArgError{ TH_ERR_INVALID_ARGUMENT, "verts or faces pointer is NULL" };
             const cudaStream_t st = static_cast<cudaStream_t>(stream);
-            launch_mc_emit(s.plan, verts, faces, st);
-            // an export recorded into a caller's graph is not ordered here: its
-            // event could not be waited on outside the graph
-            if (!in_capture(st))
-                TH_CUDA(cudaEventRecord(s.done, st));
+            export_on(s.done, st, [&] { launch_mc_emit(s.plan, verts, faces, st); });
         }
     });
 }
@@ -2019,9 +2038,8 @@ th_status th_visual_hull_batch_export(th_context* ctx, int32_t index, float* ver
         {
             if (!verts || !faces)
                 throw ArgError{ TH_ERR_INVALID_ARGUMENT, "verts or faces pointer is NULL" };
-            launch_export(s.plan, s.host->words, verts, faces, st);
+            export_on(s.done, st, [&] { launch_export(s.plan, s.host->words, verts, faces, st); });
         }
-        TH_CUDA(cudaEventRecord(s.done, st));
     });
 }
 
@@ -2043,6 +2061,10 @@ th_status th_visual_hull_batch_export_all(th_context* ctx, int32_t n, float* con
         auto st = static_cast<cudaStream_t>(stream);
         BatchState& bs = ctx->bstate;
         const int ns = std::min<int>(n, static_cast<int>(bs.streams.size()));
+        const bool recorded = in_capture(st); // export_on
+        if (!recorded)
+            for (int32_t i = 0; i < n; ++i)
+                TH_CUDA(cudaStreamWaitEvent(st, ctx->batch[i].done, 0));
         if (ns > 1)
         {
             // the exports side by side on the batch's streams, joined back into st
@@ -2064,8 +2086,9 @@ th_status th_visual_hull_batch_export_all(th_context* ctx, int32_t n, float* con
                 TH_CUDA(cudaStreamWaitEvent(st, bs.joins[i], 0));
             }
         }
-        for (int32_t i = 0; i < n; ++i)
-            TH_CUDA(cudaEventRecord(ctx->batch[i].done, st));
+        if (!recorded)
+            for (int32_t i = 0; i < n; ++i)
+                TH_CUDA(cudaEventRecord(ctx->batch[i].done, st));
     });
 }
 
