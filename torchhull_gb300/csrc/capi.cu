@@ -224,7 +224,8 @@ struct HullSlot
     ReqConsts* host_rq_d = nullptr; // its device address
     th_hull_info info{};
     bool has_result = false;
-    cudaEvent_t done = nullptr;
+    cudaEvent_t done = nullptr; // the last export that read the buffers
+    bool exported = false;      // one was queued since the last request waited for it
 
     // Captured pipelines, keyed by the plan with the per-request fields cleared.
     struct Graph
@@ -403,6 +404,7 @@ struct McSlot
     th_mc_info info{};
     bool has_result = false;
     cudaEvent_t done = nullptr; // the last export that read the buffers
+    bool exported = false;      // one was queued since the last call waited for it
 
     std::vector<const DevBuf*> buffers() const
     {
@@ -438,28 +440,30 @@ bool in_capture(cudaStream_t st)
     return status != cudaStreamCaptureStatusNone;
 }
 
-// Runs launch(), the kernels of an export on st, and records `done` behind them
-// for the next request.  Exports of one result may be on several streams: each
+// Runs launch(), the kernels of an export of slot s on st, and records s.done
+// behind them for the next request.  Exports of one result may be on several streams: each
 // waits for the one before, as some use scratch (the leaf list, the words of a
 // volume in slabs), and so the last event stands for them all.  An export
 // recorded into a caller's graph is not ordered here: its event could not be
 // waited on outside the graph.
-template <class F>
-void export_on(cudaEvent_t done, cudaStream_t st, F&& launch)
+template <class Slot, class F>
+void export_on(Slot& s, cudaStream_t st, F&& launch)
 {
     if (in_capture(st))
         return launch();
-    TH_CUDA(cudaStreamWaitEvent(st, done, 0));
+    if (s.exported)
+        TH_CUDA(cudaStreamWaitEvent(st, s.done, 0));
+    s.exported = true;
     try
     {
         launch();
     }
     catch (...)
     {
-        cudaEventRecord(done, st); // what is queued
+        cudaEventRecord(s.done, st); // what is queued
         throw;
     }
-    TH_CUDA(cudaEventRecord(done, st));
+    TH_CUDA(cudaEventRecord(s.done, st));
 }
 
 // Scratch of the calls that a caller records into a graph.  The graph's
@@ -977,6 +981,7 @@ void run_hull_once(th_context* ctx,
 {
     if (s.done)
         TH_CUDA(cudaStreamWaitEvent(st, s.done, 0)); // the last request's exports read the pools
+    s.exported = false;
     s.has_result = false;
     const int L = a->level;
     for (int attempt = 0; attempt < 8; ++attempt)
@@ -1119,6 +1124,7 @@ void run_batch(th_context* ctx, const th_hull_args* args, int32_t n, cudaStream_
         HullSlot& s = ctx->batch[r];
         if (s.done)
             TH_CUDA(cudaStreamWaitEvent(st, s.done, 0)); // the last batch's exports read the pools
+        s.exported = false;
         s.has_result = false;
     }
     std::vector<int32_t> order(n);
@@ -1463,6 +1469,7 @@ void run_mc(McSlot& s, const th_mc_args* a, cudaStream_t st)
         TH_CUDA(cudaStreamWaitEvent(st, s.done, 0));
     else
         TH_CUDA(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
+    s.exported = false;
     if (!s.host)
         alloc_mapped(&s.host, &s.host_d);
     s.ctr.ensure(sizeof(McCounters), st);
@@ -1816,7 +1823,7 @@ th_status th_visual_hull_export(th_context* ctx, float* verts, int64_t* faces, v
         {
             if (!verts || !faces)
                 throw ArgError{ TH_ERR_INVALID_ARGUMENT, "verts or faces pointer is NULL" };
-            export_on(s.done, st, [&] { launch_export(s.plan, s.host->words, verts, faces, st); });
+            export_on(s, st, [&] { launch_export(s.plan, s.host->words, verts, faces, st); });
         }
     });
 }
@@ -1835,7 +1842,7 @@ th_status th_visual_hull_export_candidates(th_context* ctx, int32_t level, int64
             if (!dst)
                 throw ArgError{ TH_ERR_INVALID_ARGUMENT, "dst is NULL" };
             const cudaStream_t st = static_cast<cudaStream_t>(stream);
-            export_on(s.done, st, [&] {
+            export_on(s, st, [&] {
                 // the leaves are written out on demand
                 if (level == s.plan.level)
                     launch_emit_leaves(s.plan, st);
@@ -1858,7 +1865,7 @@ th_status th_visual_hull_export_field(th_context* ctx, int64_t* indices, float* 
         {
             if (!indices || !values)
                 throw ArgError{ TH_ERR_INVALID_ARGUMENT, "indices or values pointer is NULL" };
-            export_on(s.done, st, [&] { launch_export_field(s.plan, n, indices, values, st); });
+            export_on(s, st, [&] { launch_export_field(s.plan, n, indices, values, st); });
         }
     });
 }
@@ -1875,7 +1882,7 @@ th_status th_visual_hull_export_field_coo(th_context* ctx, int64_t* indices, flo
         {
             if (!indices || !values)
                 throw ArgError{ TH_ERR_INVALID_ARGUMENT, "indices or values pointer is NULL" };
-            export_on(s.done, st, [&] { launch_export_field_coo(s.plan, n, indices, values, st); });
+            export_on(s, st, [&] { launch_export_field_coo(s.plan, n, indices, values, st); });
         }
     });
 }
@@ -1966,7 +1973,7 @@ th_status th_marching_cubes_export(th_context* ctx, float* verts, int64_t* faces
             if (!verts || !faces)
                 throw ArgError{ TH_ERR_INVALID_ARGUMENT, "verts or faces pointer is NULL" };
             const cudaStream_t st = static_cast<cudaStream_t>(stream);
-            export_on(s.done, st, [&] { launch_mc_emit(s.plan, verts, faces, st); });
+            export_on(s, st, [&] { launch_mc_emit(s.plan, verts, faces, st); });
         }
     });
 }
@@ -2038,7 +2045,7 @@ th_status th_visual_hull_batch_export(th_context* ctx, int32_t index, float* ver
         {
             if (!verts || !faces)
                 throw ArgError{ TH_ERR_INVALID_ARGUMENT, "verts or faces pointer is NULL" };
-            export_on(s.done, st, [&] { launch_export(s.plan, s.host->words, verts, faces, st); });
+            export_on(s, st, [&] { launch_export(s.plan, s.host->words, verts, faces, st); });
         }
     });
 }
@@ -2064,7 +2071,11 @@ th_status th_visual_hull_batch_export_all(th_context* ctx, int32_t n, float* con
         const bool recorded = in_capture(st); // export_on
         if (!recorded)
             for (int32_t i = 0; i < n; ++i)
-                TH_CUDA(cudaStreamWaitEvent(st, ctx->batch[i].done, 0));
+            {
+                if (ctx->batch[i].exported)
+                    TH_CUDA(cudaStreamWaitEvent(st, ctx->batch[i].done, 0));
+                ctx->batch[i].exported = true;
+            }
         if (ns > 1)
         {
             // the exports side by side on the batch's streams, joined back into st
