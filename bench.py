@@ -82,11 +82,11 @@ WORKLOAD = ("partial-view visual hull: 32 views of 1024x1024 float32 masks, leve
             "unique_verts=True, OpenGL, 8 ellipsoids + 20 capsules")
 MEASURED_PEAKS = ROOT / "MEASURED_PEAKS.json"
 # DRAM bytes (read + write) per launch of a stage's dominant kernel, from one ncu capture of a
-# request of the same workload (not measured by this run): dram__bytes.sum.per_second times
-# the duration of the level-8 classify_items_kernel launch.
-NCU_TRAFFIC = {"carve_level_8": 56.1e6}
+# request of the same workload (not measured by this run): dram__bytes_read.sum and
+# dram__bytes_write.sum of the level-8 classify_items_kernel launch.
+NCU_TRAFFIC = {"carve_level_8": 40.9e6}
 NCU_TRAFFIC_SOURCE = ("ncu capture of classify_items_kernel, level 8, a request of this workload "
-                      "(dram__bytes.sum.per_second times its duration); a separate capture, not this run")
+                      "(dram__bytes_read.sum + dram__bytes_write.sum); a separate capture, not this run")
 
 
 def peaks() -> tuple[float, str]:
@@ -267,11 +267,11 @@ def host_copy(th, method: str):
     """The copy the end-to-end legs move their bytes with, on the current stream: "sm" is
     torchhull_gb300's copy kernel (th_copy: a few blocks of SMs over the pinned buffers' device
     mappings), "dma" is cudaMemcpyAsync (a copy engine).  The copy
-    engines are the default of both legs: plain hulls 422 hulls/s against 281 with the copy kernel,
-    batched ones 480 against 250, because the hulls' kernels leave its few blocks little room.  One
-    copy-engine loop in eight (one in three while a hull took 3.1 ms) loses 70-80 ms: a few
+    engines are the default of both legs: plain hulls 448 hulls/s against 285 with the copy kernel,
+    because the hulls' kernels leave its few blocks little room.  Some
+    copy-engine loops lose 70-80 ms: a few
     consecutive copies run at a tenth of their rate (raw cudaMemcpyAsync as well as torch's copies,
-    either direction; 239 hulls/s then).  The copy kernel showed no such stall."""
+    either direction); a run that met one gave 321 against 288.  The copy kernel showed no such stall."""
     if method == "sm":
         return th._C.copy_on_sms
 
@@ -292,7 +292,7 @@ def e2e_plain_pipelined(th, reqs, steps: int, dev, world: int, copy: str = "sm")
 
     The two directions share one stream, so one copy at a time runs beside a
     hull (per hull 134 MB in at ~130 GB/s and ~211 MB out at ~190 GB/s with
-    the copy kernel: ~2.2 ms, inside the ~3.1 ms hull)."""
+    the copy kernel: ~2.2 ms, about a hull's time)."""
     import torch
     import torch.distributed as dist
 

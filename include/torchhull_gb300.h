@@ -145,6 +145,10 @@ th_status th_visual_hull_export_field_coo(th_context* ctx, int64_t* indices, flo
  * out_dtype (float16/32/64).
  * Replaces torchhull::gaussian_blur (src/torchhull/_C/include/torchhull/gaussian_blur.h:10-15,
  * src/torchhull/_C/src/gaussian_blur.cpp:15-28, gaussian_blur_cuda.cu:73-518).
+ * May be recorded into a CUDA graph (a capture of the calling thread's stream),
+ * as may th_integral_image and the exports: a recorded blur or integral image has scratch
+ * of its own, held until the graph and all instantiated from it are destroyed;
+ * such graphs are not launched after th_context_destroy.
  */
 th_status th_gaussian_blur(th_context* ctx,
                            const void* images,
@@ -348,11 +352,10 @@ int64_t th_launch_count(void);
  * TH_ERR_INVALID_ARGUMENT.
  * The transfer runs on a few blocks of SMs instead of a DMA copy engine
  * (8 blocks when reading host memory, 6 when writing it, all SMs for device
- * to device), sized to overlap the hull kernels.  On GB300, a loop overlapping
- * hulls with cudaMemcpyAsync copies of their inputs and meshes lost ~70-80 ms
- * in about one run of three (a few consecutive copies at a tenth of their
- * rate); the same loop with this kernel showed no such stall in 40 runs and
- * ran ~5% below the stall-free copy-engine runs. */
+ * to device), beside the hull kernels, which leave it little room: a loop
+ * overlapping hulls with the copies of their inputs and meshes is faster with
+ * cudaMemcpyAsync, except that some such loops lose 70-80 ms (a few
+ * consecutive copies at a tenth of their rate), which this kernel never did. */
 th_status th_copy(void* dst, const void* src, int64_t bytes, void* stream);
 
 #ifdef __cplusplus

@@ -1423,9 +1423,11 @@ void run_mc(McSlot& s, const th_mc_args* a, cudaStream_t st)
         p.volume = a->volume;
     }
     // Rows of 32-point words.  A sparse volume takes them when they are at
-    // most kWordsPerEntry per entry (and always below kFewWords): clearing and
-    // counting a word costs about an eighth of what an entry's hash lookups
-    // do, and a word takes 40 bytes of scratch where an entry's table takes 60.
+    // most kWordsPerEntry per entry (and always below kFewWords).  The line
+    // bounds the scratch, not the time: a word takes 40 bytes where an entry's
+    // table takes 60, and words are faster well past it (512^3, calls with words
+    // against the table: one word per entry 415 us against 1313, 8 190 against
+    // 265, 16 162 against 214, 64 132 against 187).
     constexpr int64_t kWordsPerEntry = 8, kFewWords = int64_t{ 1 } << 18;
     p.wr = 0;
     if (W > 0 && H > 0 && D > 0)

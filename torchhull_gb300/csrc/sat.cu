@@ -173,7 +173,12 @@ __global__ void __launch_bounds__(32 * kRowWarps) sat_rows_kernel(float* __restr
 
 constexpr int kBandRows = 32; // rows to a word
 // The bands above a block's are counted by the block itself up to this many
-// (a word per column each), from a table of prefix counts beyond.
+// (a word per column each), from a table of prefix counts beyond: the launch
+// for the table costs few views more than the counting up to about 48 bands,
+// whose work grows with the square.  Integral images, counted against the
+// table: 4x1024^2 (32 bands) 45.8 us against 48.2, 64x1024^2 133.3 against
+// 129.8; 1x1536^2 (48) 53.6 against 54.0, 28x1536^2 142 against 136; 1x2048^2
+// (64) 65 against 61, 16x2048^2 159 against 144; 4x4096^2 237 against 162.
 constexpr int kCountedBands = 32;
 constexpr int kCountedWidth = 8192; // columns whose counts fit the block's shared memory
 

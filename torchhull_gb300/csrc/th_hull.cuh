@@ -22,10 +22,13 @@ enum OverflowBits : int64_t
 };
 
 // From this level on the corners of the leaves are marked by a launch of their
-// own: at level 7 (13 x 437x611) marking them in the last classify kernel took
-// 85 us for both against 91, but that kernel keeps 16 warps on an SM, too few for the
-// waits on the bitmap when there are many leaves (level 9 headline scene: 906
-// us against 625 + 103).
+// own: the last classify kernel keeps 16 warps on an SM, few for the waits on
+// the bitmap when there are many leaves, while a small request feels the
+// launch.  Whole calls, apart against in that kernel: level 6 24x512^2 193 us
+// against 185; level 7 230 against 237, 32x1024^2 partial 473 against 480; level
+// 8 308 against 318, 815 against 814; level 9 508 against 521, 1961 against
+// 1975; level 7 could go either way.  (Before that kernel shared its items between a block's warps, level 9
+// took 906 us against 625 + 103 for the two.)
 constexpr int kMarkApartLevel = 8;
 
 constexpr int kRowBlock = 32;           // words of row flags a block of rows_kernel owns
