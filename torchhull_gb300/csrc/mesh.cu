@@ -1041,7 +1041,9 @@ __global__ void __launch_bounds__(256) export_field_kernel(HullPlan p, int64_t n
         }
         else
             indices[t] = x + y * R + z * R * R;
-        values[t] = p.values[t];
+        // coalescing sums a point's values from 0, so no value of the tensor is -0 (a
+        // product of negative mask samples can be)
+        values[t] = COO ? __fadd_rn(p.values[t], 0.f) : p.values[t];
     }
 }
 
