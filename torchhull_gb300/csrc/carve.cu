@@ -466,6 +466,7 @@ struct ChildCount
     }
 };
 
+// The leaves, without view masks: nothing reads those.
 struct ChildEmit
 {
     HullPlan p;
@@ -484,8 +485,6 @@ struct ChildEmit
         const int64_t gx = 2 * (idx & mask), gy = 2 * ((idx >> li) & mask), gz = 2 * (idx >> (2 * li));
         const int sh = li + 1; // children ravel at resolution 2^(li+1)
         const uint32_t m = __ldg(p.child_masks + i);
-        // the masks of the children of the last level (the leaves) are never read
-        const bool has_skip = i < p.parent_cap && li + 1 < p.level;
         int64_t out = c->level_off[li + 1] + static_cast<int64_t>(off);
 #pragma unroll
         for (int k = 0; k < 8; ++k)
@@ -493,15 +492,7 @@ struct ChildEmit
             if (m >> k & 1u)
             {
                 if (out < p.node_cap)
-                {
                     p.nodes[out] = (gx + (k & 1)) | ((gy + (k >> 1 & 1)) << sh) | ((gz + (k >> 2 & 1)) << (2 * sh));
-                    for (int w = 0; w < p.mask_words; ++w)
-                    {
-                        const int64_t at = w * p.parent_cap * 8 + i * 8 + k;
-                        p.node_skip[w * p.node_cap + out] = has_skip ? __ldg(p.child_skip + at) : 0u;
-                        p.node_out[w * p.node_cap + out] = has_skip ? __ldg(p.child_out + at) : 0u;
-                    }
-                }
                 ++out;
             }
         }
