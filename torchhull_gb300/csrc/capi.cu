@@ -1298,6 +1298,7 @@ th_status guarded(th_context* ctx, F&& f)
     }
     catch (const CudaError& e)
     {
+        cudaGetLastError(); // reported here: the next launch's check, ours or the caller's, must not find it again
         const th_status st = (e.code == cudaErrorMemoryAllocation) ? TH_ERR_OUT_OF_MEMORY : TH_ERR_CUDA;
         return fail(ctx, st, std::string(cudaGetErrorString(e.code)) + " (" + e.where + ")");
     }
