@@ -1,7 +1,7 @@
 // CPU oracle for the visual-hull and Gaussian-blur path.
 //
-// TEST INFRASTRUCTURE ONLY.  This library is the checker: the parity tests,
-// the smoke check and the CPU baseline leg of the benchmark call it.  The
+// TEST INFRASTRUCTURE ONLY.  The parity tests, the smoke check and the CPU
+// baseline leg of the benchmark call it.  The
 // product path (the CUDA library and its Python/torch front end) never links,
 // loads or falls back to it.
 //

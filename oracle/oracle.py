@@ -1,7 +1,7 @@
 """ctypes front end of the CPU oracle (oracle.cpp): TEST INFRASTRUCTURE ONLY.
 
 Used by the tests, ``__graft_entry__.smoke()`` and the CPU-baseline leg of
-``bench.py`` as the checker.  The product path never imports this module.
+``bench.py``.  The product path never imports this module.
 See oracle.h for the parity status of the oracle.
 """
 
